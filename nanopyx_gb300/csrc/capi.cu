@@ -133,7 +133,6 @@ struct nx_esrrf_plan {
   nx::RgcScalars sc;
   const nx::FusedEntry* fused;
   int tile_variant;  // which instantiation `fused` is (0: default tiling)
-  int cy_base, cx_base;
   float cy[4], cx[4];
   int device;
   float* d_tbl;     // device: [tbl | inv_wsum | wfull]
@@ -291,8 +290,6 @@ static void fill_params(const nx_esrrf_plan* p, FusedParams& fp, const float* in
   fp.sens_mode_k[0] = p->sc.sens_mode;
   fp.sens_int_k[0] = p->sc.sens_int;
   fp.sens_k[0] = p->sc.sens;
-  fp.cy_base = p->cy_base;
-  fp.cx_base = p->cx_base;
   for (int t = 0; t < 4; ++t) {
     fp.cy[t] = p->cy[t];
     fp.cx[t] = p->cx[t];
@@ -417,8 +414,12 @@ int nx_esrrf_plan_create(nx_esrrf_plan** out, int H, int W, int magnification, f
     for (int mode = 0; mode < 3; ++mode)
       if (p->fused->smem[mode](1) > lim) p->fused = nullptr;
   }
-  clamp_taps(H, magnification, &p->cy_base, p->cy);
-  clamp_taps(W, magnification, &p->cx_base, p->cx);
+  int cy_base, cx_base;
+  clamp_taps(H, magnification, &cy_base, p->cy);
+  clamp_taps(W, magnification, &cx_base, p->cx);
+  // the fused kernel takes the clamped position's taps from H-2 (W-2) on, where
+  // (2 m H - 1) / (2 m) - 0.5 always puts them
+  if (cy_base != H - 2 || cx_base != W - 2) p->fused = nullptr;
   cudaGetDevice(&p->device);
   p->d_tbl = nullptr;
   if (p->fused) {

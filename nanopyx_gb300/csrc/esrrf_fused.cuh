@@ -1,22 +1,21 @@
 // Fused eSRRF frame-loop kernel (sm_103a), warp-specialised.
 //
 // One CTA works through units -- (stack, 32 x TY tile of input pixels = a
-// 32M x TY*M tile of output pixels, timepoint, frame chunk) -- two frames per
-// pass.  Its producer warps, per pass,
-//   1. receive the input tiles + halo by TMA (two sets of buffers, mbarrier),
-//      or by plain loads when the row pitch is not 16-byte aligned;
+// 32M x TY*M tile of output pixels, timepoint, frame chunk) -- two or four
+// frames per pass.  Its producer warps, per pass,
+//   1. receive the input tiles + halo by TMA (mbarrier), or by plain loads when
+//      the row pitch is not 16-byte aligned;
 //   2. compute Roberts-Cross gradients          (_c_gradients.c:53-73) and the
 //      row pass of the intensity magnification  (_c_interpolation_catmull_rom.c:21-52);
 //   3. Catmull-Rom-interpolate the gradients on the half-pixel grid -- the only
 //      positions the reference RGC ever reads from its 2m-magnified gradient
 //      images (rows/cols k*m, clamped to 2*m*H-1;
-//      _c_sr_radial_gradient_convergence.c:45-61) -- on packed f32x2
-//      arithmetic over the frame pair, and normalise them into a
-//      double-buffered slot;
+//      _c_sr_radial_gradient_convergence.c:45-61) -- walking down columns, and
+//      normalise them into a double-buffered slot;
 // while its consumer warps, one thread per input pixel and output row phase,
 //   4. evaluate RGC for the thread's M output pixels with FP64-derived phase
 //      tables of the distance weights      (_c_sr_radial_gradient_convergence.c:17-90),
-//      on packed f32x2 arithmetic (both frames in one register pair);
+//      on packed f32x2 arithmetic (two frames in one register pair);
 //   5. apply ^sensitivity, the intensity (column pass) and the margin, and
 //      either write the per-frame value (eSRRF_ST stack) or fold it into
 //      per-pixel streaming temporal moments kept in shared memory (Welford
@@ -24,6 +23,17 @@
 //      Moments).
 // Nothing of size (T, 2Hm, 2Wm) or (T, Hm, Wm) is ever materialised for the
 // temporal modes.
+//
+// What bounds it: the register reads and FMA pipe of step 4 (see rgc_sample).
+// 100 x 512 x 512, m = 5, R = 1.5, VAR + TAC2, of 5.79 ms: the RGC core 4.9,
+// the epilogue 0.5, the producers 0.35 (each found by leaving the others out).
+// How that kernel got there from 7.66 ms:
+//   saturating half-plane test, mirrored table entries           7.14
+//   gradients walked down columns instead of a column pass, its
+//   buffer and a row pass; 4 frames a pass in the shared memory
+//   that frees; intensity rows 5 outputs at a time               6.31
+//   epilogue in whole blocks (power, intensity, then moments):
+//   no register spills                                           5.79
 #pragma once
 
 #include <cuda.h>
@@ -53,8 +63,7 @@ struct FusedParams {
   int chunks;          // chunks per timepoint (the last timepoint uses min(chunks, its frames))
   int margin;
   int iw;
-  int cy_base, cx_base;  // first tap row/col of the clamped half-grid index 2H / 2W
-  float cy[4], cx[4];
+  float cy[4], cx[4];  // taps (rows H-2 .. H+1, cols W-2 ..) of the clamped index 2H / 2W
   const float* tbl;      // [M][2J+1][3][NS4*4]  (a = dx*w/d, b = dy*w/d, w) per sample
   const float* inv_wsum; // [M][M]
   const float* wfull;    // [M][M][2J+1][2J+1]
@@ -99,51 +108,46 @@ struct TileRows {
   static constexpr int TY = (M <= 2) ? 8 : (M <= 5 ? 4 : 2);
 };
 
-// Warp roles of the eSRRF kernel.  Each CTA runs 32 * TY * M consumer threads
-// (one per input pixel and output row phase: RGC, normalisation, temporal
-// update) and one producer warpgroup that prepares the gradient and intensity
+// Warp roles of the eSRRF kernel.  Each CTA runs 32 * TY * M / PYT consumer
+// threads (one per input pixel and PYT output row phases: RGC, normalisation,
+// temporal update) and producer warps that prepare the gradient and intensity
 // tiles of the next frames (TMA, Roberts-Cross, Catmull-Rom passes,
 // normalisation) into a double-buffered slot while the consumers work on the
-// current one.  The consumers' RGC is FMA-pipe bound and the preparation is
-// load/ALU bound, so the two overlap on the SM.
+// current one, so the two overlap on the SM.
 template <int M, int V = 0>
 struct EsrrfTile {
   // rows per tile: as many consumer warps as the registers allow without
-  // spilling (m = 5: 20 consumer + 4 producer warps at 80 registers measured
-  // 12 % faster than 15 + 4 at 96, 40 % faster than 10 + 4)
+  // spilling
   static constexpr int TY = (M <= 2) ? 8 : (M <= 5 ? 4 : (M == 6 ? 2 : 1));
+  // output row phases per consumer thread
+  static constexpr int PYT = 1;
   // producer threads: the preparation per input pixel is the same for every m
   // while the RGC work grows with m^2, so small m needs more producers.
-  // Measured (200 x 512 x 512, VAR): m = 5 best with one warpgroup (96 or 64
-  // threads slower); m = 2: 6.31 / 4.74 / 4.15 / 4.23 ms with 128 / 256 / 384 /
-  // 512; m = 3: 9.23 / 7.60 / 7.75 ms with 128 / 256 / 384; m = 4 (4 rows):
-  // 12.12 / 11.82 ms with 128 / 256 (3 rows: 12.41 / 12.48); m = 5: 16.92 /
-  // 18.11 ms with 128 / 256.
   // Tile variant V = 1 (instantiated for m = 2, 4, 5) has one producer warp
   // group fewer (m = 5: 3 warps), for the tiling autotuner to weigh against
   // the default on a given batch.
   static constexpr int NP_DEFAULT = (M <= 2) ? 384 : (M <= 4 ? 256 : 128);
   static constexpr int NP_ALT = (M <= 2) ? 256 : (M <= 4 ? 128 : 96);
   static constexpr int NP = V == 0 ? NP_DEFAULT : NP_ALT;
-  static constexpr int NT = 32 * TY * M + NP;
+  // most frames a pass carries (4 where the layout fits shared memory, else 2)
+  static constexpr int FP_MAX = 4;
   // one CTA per SM: registers for the consumers (m = 8 with 2 CTAs per SM at
   // 80 registers measured 11 % slower than 1 CTA)
   static constexpr int MIN_BLOCKS = 1;
 };
 
-// Frames per pass (FP).  With FP = 2 a consumer carries two consecutive frames
-// through each pass: the RGC core runs on packed f32x2 arithmetic (frame pair
-// in one register pair, one phase-table load for both frames) and the
-// producers share their index and weight work between the two frames.
-// Results are bit-identical to FP = 1 (the same IEEE operations per frame).
-// Instantiations whose FP = 2 shared-memory layout does not fit a CTA use FP = 1.
-template <int M, int J, int TY, int FP, int NP_ = EsrrfTile<M>::NP>
+// Frames per pass (FP = 2 or 4): a consumer carries FP / 2 pairs of consecutive
+// frames through each pass.  The RGC core runs on packed f32x2 arithmetic (a
+// frame pair in one register pair) and every phase-table load serves all the
+// pairs; the temporal state is read and written once per pass.
+template <int M, int J, int TY, int FP, int NP_ = EsrrfTile<M>::NP, int PYT_ = EsrrfTile<M>::PYT>
 struct Geo {
   static constexpr int TX = 32;
   static constexpr int W2 = 2 * J + 1;
   static constexpr int NQ = 2 * J + 2;
+  static constexpr int NPR = FP / 2;  // frame pairs per pass
+  static constexpr int PYT = PYT_;
   static constexpr int HG_R = 2 * TY + 2 * J;
-  static constexpr int HG_C = 2 * TX + 2 * J;
   static constexpr int HGP = TX + J;
   static constexpr int RLO = (J + 1) / 2 + 2;
   static constexpr int RHI = TY + (J - 1) / 2 + 2;
@@ -160,50 +164,54 @@ struct Geo {
   static constexpr int OY = TY * M;
   static constexpr int OX = TX * M;
   static constexpr int RIW = TX + 4;
-  static constexpr int NTC = 32 * TY * M;        // consumer threads
-  static constexpr int NP = NP_;                 // producer threads
+  static constexpr int NTC = 32 * TY * (M / PYT);  // consumer threads
+  static constexpr int NP = NP_;                   // producer threads
   static constexpr int NT = NTC + NP;
   // prepared passes in flight between producers and consumers (3 or 4
   // measured no faster: the producers keep up)
   static constexpr int NSLOT = 2;
-  // phase-table block per (py, jj), in float4:
-  //   FP = 1: a[NS4] b[NS4] w[NS4]   (4 samples per float4)
-  //   FP = 2: (a, b, -b, w) per sample, each value broadcast into a frame pair
-  //           (measured 12 % faster than storing the pairs duplicated)
-  static constexpr int TBLK = FP >= 2 ? 4 * NS4 : 3 * NS4;
-  // unit gradients of one slot: FP = 1: float2 (nx, ny) per half-grid sample;
-  // FP >= 2: one plane per frame pair of float4 (nx0, nx1, ny0, ny1)
+  // phase-table block per (py, jj): NE float4 entries, one per mirrored couple
+  // of samples (see rgc_core), each value broadcast into a frame pair
+  static constexpr int NE = (J + 1) * M + (M + 1) / 2;
+  // unit gradients of one slot: one plane per frame pair of float4
+  // (nx, nx', ny, ny')
   static constexpr int HG_PLANE = HG_R * 2 * HGP;  // samples per plane
+  // the gradient walk (see Producer::gradients): steps along an axis that each
+  // yield up to two half-grid samples, and rows of steps per walk
+  static constexpr int NB = TX + J + (J & 1);
+  static constexpr int NA = TY + J + (J & 1);
+  static constexpr int SEG = 4;
+  static constexpr int NSEG = (NA + SEG - 1) / SEG;
+  static constexpr int LEFT = NB - 32;  // columns beyond one warp
 
   __host__ __device__ static constexpr int al(int n) { return (n + 31) / 32 * 32; }
   // shared-memory layout (in floats, 128-byte aligned blocks)
   static constexpr int O_INB = 0;
-  static constexpr int S_INB = al(BH * BW);  // 2 * FP input tiles (two sets of FP frames)
-  static constexpr int O_G = O_INB + 2 * FP * S_INB;
-  static constexpr int S_G = al(NRY * NCX);  // Roberts-Cross gc, gr per frame
-  static constexpr int O_T1 = O_G + 2 * FP * S_G;
-  static constexpr int S_T1 = al(NRY * HG_C);  // column-pass gx, gy per frame
-  static constexpr int O_HG = O_T1 + 2 * FP * S_T1;
-  static constexpr int S_HG = al(HG_R * 2 * HGP * 2 * FP);  // one slot: float2 / float4 gradients
-  static constexpr int O_RI = O_HG + NSLOT * S_HG;          // NSLOT slots
-  static constexpr int S_RI = al(OY * RIW);  // intensity row pass per frame
-  static constexpr int O_TB = O_RI + NSLOT * FP * S_RI;     // NSLOT slots of FP planes
-  static constexpr int S_TB = al(M * W2 * TBLK * 4);
+  static constexpr int S_INB = al(BH * BW);  // FP input tiles
+  static constexpr int O_G = O_INB + FP * S_INB;
+  static constexpr int S_G = al(NRY * NCX * 4);  // per frame pair: (gc, gc', gr, gr')
+  static constexpr int O_HG = O_G + NPR * S_G;
+  static constexpr int S_HG = al(HG_PLANE * 4) * NPR;   // one slot
+  static constexpr int O_RI = O_HG + NSLOT * S_HG;      // NSLOT slots
+  static constexpr int S_RI = al(OY * RIW * 2);  // intensity row pass per frame pair (v, v')
+  static constexpr int O_TB = O_RI + NSLOT * NPR * S_RI;  // NSLOT slots of NPR planes
+  static constexpr int S_TB = al(M * W2 * NE * 4);
   static constexpr int O_RW = O_TB + S_TB;
-  static constexpr int S_RW = al(OY * 5);
+  static constexpr int S_RW = al(OY * 8);      // 5 weights per output row, rows of 8
   static constexpr int O_CW = O_RW + S_RW;
   static constexpr int S_CW = al(OX * 5);
-  // per-output temporal state kept out of registers, [px][consumer] planes:
+  // per-output temporal state kept out of registers, [output][consumer] planes:
   //   FULL: float4 (mean, M2, C, A) then float B;  SUM: the mean per sensitivity
+  static constexpr int NO = PYT * M;           // outputs per consumer
   static constexpr int O_TW = O_CW + S_CW;     // 1 / sum w per output
-  static constexpr int O_TK = O_TW + M * NTC;
-  static constexpr int S_TK_FULL = 5 * M * NTC;
+  static constexpr int O_TK = O_TW + NO * NTC;
+  static constexpr int S_TK_FULL = 5 * NO * NTC;
   static constexpr int O_BAR_FULL = O_TK + S_TK_FULL;
   // AVG mode keeps the running mean of ns_cap sensitivities per output
   __host__ __device__ static constexpr int o_bar(int mode, int ns_cap) {
-    return mode == 1 ? O_TK + ns_cap * M * NTC : (mode == 2 ? O_BAR_FULL : O_TK);
+    return mode == 1 ? O_TK + ns_cap * NO * NTC : (mode == 2 ? O_BAR_FULL : O_TK);
   }
-  // 2 NSLOT + 1 + 2 FP (<= 11) mbarriers after o_bar
+  // 2 NSLOT + 2 mbarriers after o_bar
   __host__ __device__ static constexpr size_t smem_bytes(int mode, int ns_cap) {
     return size_t(o_bar(mode, ns_cap) + 32) * 4;
   }
@@ -217,17 +225,20 @@ template <int M, int J, int MODE, int V = 0>
 struct FusedCfg {
   static constexpr int TY = EsrrfTile<M, V>::TY;
   static constexpr int NP = EsrrfTile<M, V>::NP;
+  static constexpr int PYT = EsrrfTile<M, V>::PYT;
   static constexpr int NSC = MODE == kModeSum ? kMaxSens : 1;
-  // FP = 4 (two frame pairs per pass sharing the table loads) is supported by
-  // the code but not selected: it does not fit shared memory with the VAR/TAC2
-  // or AVG state at m = 5, and in stack mode it measured 9 % slower.
-  static constexpr int FP = Geo<M, J, TY, 2, NP>::smem_bytes(MODE, NSC) <= kSmemBudget ? 2 : 1;
-  using G = Geo<M, J, TY, FP, NP>;
+  static constexpr int FP =
+      EsrrfTile<M, V>::FP_MAX >= 4 &&
+              Geo<M, J, TY, 4, NP, PYT>::smem_bytes(MODE, NSC) <= kSmemBudget ? 4 : 2;
+  using G = Geo<M, J, TY, FP, NP, PYT>;
 };
 
-__device__ __forceinline__ float f4c(const float4& v, int e) {
-  return e == 0 ? v.x : (e == 1 ? v.y : (e == 2 ? v.z : v.w));
-}
+// Unit gradients of a frame pair are kept scaled by 2^32: the half-plane test
+// t < 0 of a sample is then a saturating FMA of the scaled gradients, which
+// gives exactly 0 or 1 unless |t| < 2^-32, where the sample's contribution
+// w (1 - |sin|) is itself below w 2^-64.  A power of two, so nothing else rounds
+// differently.
+constexpr float kGradScale = 4294967296.f;
 
 __device__ __forceinline__ float apply_sens(float r, int mode, int n, float s) {
   if (mode == 1) {
@@ -239,6 +250,34 @@ __device__ __forceinline__ float apply_sens(float r, int mode, int n, float s) {
   return r;
 }
 
+// max(v, 0) that keeps a NaN
+__device__ __forceinline__ float clamp0(float v) {
+  float r;
+  asm("max.NaN.f32 %0, %1, 0f00000000;" : "=f"(r) : "f"(v));
+  return r;
+}
+
+// r ^ sensitivity of a thread's values (mode and n are uniform over the launch)
+template <int A, int B>
+__device__ __forceinline__ void apply_sens_all(float2 (&r)[A][B], int mode, int n, float s) {
+  if (mode == 0) return;
+  if (mode == 1 && n <= 3) {
+#pragma unroll
+    for (int i = 0; i < A; ++i)
+#pragma unroll
+      for (int j = 0; j < B; ++j) {
+        const float2 q = __fmul2_rn(r[i][j], r[i][j]);
+        r[i][j] = n == 3 ? __fmul2_rn(q, r[i][j]) : q;
+      }
+    return;
+  }
+#pragma unroll
+  for (int i = 0; i < A; ++i)
+#pragma unroll
+    for (int j = 0; j < B; ++j)
+      r[i][j] = make_float2(apply_sens(r[i][j].x, mode, n, s), apply_sens(r[i][j].y, mode, n, s));
+}
+
 // geometry of one unit (tile, timepoint, frame chunk), shared by both roles
 struct UnitGeo {
   int nx0, ny0, H, W, f0, f1;
@@ -246,332 +285,264 @@ struct UnitGeo {
 };
 
 // ---------------------------------------------------------------------------
-// producer warpgroup: input tiles -> slot s (unit gradients hg, intensity rows ri)
+// producer warps: input tiles -> slot s (unit gradients hg, intensity rows ri)
 // ---------------------------------------------------------------------------
-template <int M, int J, int TY, int FP, int NP>
+template <typename G, int M, int J>
 struct Producer {
-  using G = Geo<M, J, TY, FP, NP>;
   float* inb;
-  // Roberts-Cross gradients and the column pass's half-grid columns:
-  //   FP = 1: plane 0 gc / gx, plane 1 gr / gy;
-  //   FP >= 2: per frame pair pp one plane of float4 (gc, gc', gr, gr') /
-  //            (gx, gx', gy, gy'), so the passes run on packed frame pairs
-  float* gsm;
-  float* t1;
+  float* gsm;  // Roberts-Cross gradients, one plane of float4 per frame pair
   float* hg0;  // slot 0; slot s at hg0 + s * S_HG
-  float* ri0;  // slot s, frame fr at ri0 + (s * FP + fr) * S_RI
+  float* ri0;  // slot s, frame pair pp at ri0 + (s * NPR + pp) * S_RI
   const float* rw;
   int ptid;
 
-  __device__ void roberts_and_rows(const FusedParams& p, const UnitGeo& u, const float* const* tin,
+  // Roberts-Cross gradients and the intensity row pass of np frame pairs; tin:
+  // the input tile of every frame
+  __device__ void roberts_and_rows(const FusedParams& p, const UnitGeo& u, int nf, int np,
                                    int s) const {
-    for (int i = ptid; i < G::NRY * G::NCX; i += G::NP) {
-      const int rl = i / G::NCX, cl = i % G::NCX;
-      const int r = u.RY0 + rl, c = u.CX0 + cl;
-      const bool in = r >= 0 && r < u.H && c >= 0 && c < u.W;
-      const int r0 = r > 0 ? r - 1 : 0;
-      const int c0 = c > 0 ? c - 1 : 0;
-      const int ia = (r0 - u.y_start) * G::BW + (c - u.x_start);   // image[r0][c1]
-      const int ib = (r - u.y_start) * G::BW + (c0 - u.x_start);   // image[r1][c0]
-      const int id = (r0 - u.y_start) * G::BW + (c0 - u.x_start);  // image[r0][c0]
-      const int ie = (r - u.y_start) * G::BW + (c - u.x_start);    // image[r1][c1]
-      float gc[FP], gr[FP];
-#pragma unroll
-      for (int fr = 0; fr < FP; ++fr) {
-        gc[fr] = gr[fr] = 0.f;
-        if (in) {
-          const float a = tin[fr][ia], bb = tin[fr][ib], d = tin[fr][id], e = tin[fr][ie];
-          gc[fr] = __fsub_rn(__fadd_rn(__fsub_rn(a, bb), e), d);
-          gr[fr] = __fsub_rn(__fadd_rn(__fadd_rn(-a, bb), e), d);
+    for (int pp = 0; pp < np; ++pp) {
+      const float* t0 = inb + 2 * pp * G::S_INB;
+      // an odd last frame stands in for its missing partner
+      const float* t1 = 2 * pp + 1 < nf ? t0 + G::S_INB : t0;
+      float4* g4 = reinterpret_cast<float4*>(gsm + pp * G::S_G);
+      for (int i = ptid; i < G::NRY * G::NCX; i += G::NP) {
+        const int rl = i / G::NCX, cl = i % G::NCX;
+        const int r = u.RY0 + rl, c = u.CX0 + cl;
+        float4 g = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (r >= 0 && r < u.H && c >= 0 && c < u.W) {
+          const int ie = (r - u.y_start) * G::BW + (c - u.x_start);  // image[r1][c1]
+          const int ia = r > 0 ? ie - G::BW : ie;                    // image[r0][c1]
+          const int ib = c > 0 ? ie - 1 : ie;                        // image[r1][c0]
+          const int id = c > 0 ? ia - 1 : ia;                        // image[r0][c0]
+          const float a0 = t0[ia], b0 = t0[ib], d0 = t0[id], e0 = t0[ie];
+          const float a1 = t1[ia], b1 = t1[ib], d1 = t1[id], e1 = t1[ie];
+          g.x = __fsub_rn(__fadd_rn(__fsub_rn(a0, b0), e0), d0);
+          g.y = __fsub_rn(__fadd_rn(__fsub_rn(a1, b1), e1), d1);
+          g.z = __fsub_rn(__fadd_rn(__fadd_rn(-a0, b0), e0), d0);
+          g.w = __fsub_rn(__fadd_rn(__fadd_rn(-a1, b1), e1), d1);
         }
+        g4[i] = g;
       }
-      if constexpr (FP >= 2) {
-        // frame pair pp: float4 (gc, gc', gr, gr') per position
+      // intensity row pass: one input row and column at a time, whose 5 taps
+      // serve the M output rows
+      if (!p.iw) continue;
+      float2* ri = reinterpret_cast<float2*>(ri0 + (s * G::NPR + pp) * G::S_RI);
+      for (int i = ptid; i < (G::OY / M) * G::RIW; i += G::NP) {
+        const int ty = i / G::RIW, cc = i % G::RIW;
+        const int off = (u.ny0 + ty - 2 - u.y_start) * G::BW + (u.nx0 - 2 + cc - u.x_start);
+        float2 v[5];
 #pragma unroll
-        for (int pp = 0; pp < FP / 2; ++pp)
-          reinterpret_cast<float4*>(gsm)[pp * G::S_G + i] =
-              make_float4(gc[2 * pp], gc[2 * pp + 1], gr[2 * pp], gr[2 * pp + 1]);
-      } else {
-        gsm[i] = gc[0];
-        gsm[G::S_G + i] = gr[0];
-      }
-    }
-    float* ri = ri0 + s * FP * G::S_RI;
-    for (int i = ptid; i < G::OY * G::RIW; i += G::NP) {
-      const int oy = i / G::RIW, cc = i % G::RIW;
-      const int nyo = u.ny0 + oy / M;
-      float w5[5];
+        for (int k = 0; k < 5; ++k)
+          v[k] = make_float2(t0[off + k * G::BW], t1[off + k * G::BW]);
 #pragma unroll
-      for (int k = 0; k < 5; ++k) w5[k] = rw[oy * 5 + k];
-      const int off = (nyo - 2 - u.y_start) * G::BW + (u.nx0 - 2 + cc - u.x_start);
+        for (int py = 0; py < M; ++py) {
+          const float* w = rw + (ty * M + py) * 8;
+          const float4 wa = *reinterpret_cast<const float4*>(w);
+          const float w5[5] = {wa.x, wa.y, wa.z, wa.w, w[4]};
+          float2 sum = make_float2(0.f, 0.f);
 #pragma unroll
-      for (int fr = 0; fr < FP; ++fr) {
-        const float* col = tin[fr] + off;
-        float sum = 0.f;
-#pragma unroll
-        for (int k = 0; k < 5; ++k) sum = fmaf(w5[k], col[k * G::BW], sum);
-        ri[fr * G::S_RI + i] = sum;
+          for (int k = 0; k < 5; ++k) sum = __ffma2_rn(make_float2(w5[k], w5[k]), v[k], sum);
+          ri[(ty * M + py) * G::RIW + cc] = sum;
+        }
       }
     }
   }
 
-  // gradient column pass onto the half-grid columns
-  // (each row's even half-grid columns first, then its odd ones, so that the
-  // lanes of a warp mostly take the same odd / even branch).  With frame
-  // pairs the planes hold float4 (x, x', y, y') per position and the taps run
-  // as packed f32x2 operations: the same IEEE operations per frame.
-  __device__ void column_pass(const FusedParams& p, const UnitGeo& u) const {
-    const int twoW = 2 * u.W;
-    constexpr int HALF = (G::HG_C + 1) / 2;
-    for (int i = ptid; i < G::NRY * G::HG_C; i += G::NP) {
-      const int rl = i / G::HG_C, j = i - rl * G::HG_C;
-      const int kxl = j < HALF ? 2 * j : 2 * (j - HALF) + 1;
-      const int o = rl * G::HG_C + kxl;
-      const int kx = u.kb_x + kxl;
-      const bool valid = kx >= 1 && kx <= u.kmax_x;
-      if constexpr (FP >= 2) {
-#pragma unroll
-        for (int pp = 0; pp < FP / 2; ++pp) {
-          const float4* g4 = reinterpret_cast<const float4*>(gsm) + pp * G::S_G + rl * G::NCX;
-          float2 vc = make_float2(0.f, 0.f), vr = make_float2(0.f, 0.f);
-          if (valid) {
-            if (kx >= twoW) {
-#pragma unroll
-              for (int t = 0; t < 4; ++t) {
-                const float4 q = g4[p.cx_base + t - u.CX0];
-                const float2 w = make_float2(p.cx[t], p.cx[t]);
-                vc = __ffma2_rn(w, make_float2(q.x, q.y), vc);
-                vr = __ffma2_rn(w, make_float2(q.z, q.w), vr);
-              }
-            } else if (kx & 1) {
-              const float4 q = g4[((kx - 1) >> 1) - u.CX0];
-              vc = make_float2(q.x, q.y);
-              vr = make_float2(q.z, q.w);
-            } else {
-              const float4* g = g4 + (kx >> 1) - 2 - u.CX0;
-              const float2 c0 = make_float2(-0.0625f, -0.0625f);
-              const float2 c1 = make_float2(0.5625f, 0.5625f);
-              const float4 q0 = g[0], q1 = g[1], q2 = g[2], q3 = g[3];
-              vc = __fmul2_rn(c0, make_float2(q0.x, q0.y));
-              vr = __fmul2_rn(c0, make_float2(q0.z, q0.w));
-              vc = __ffma2_rn(c1, make_float2(q1.x, q1.y), vc);
-              vr = __ffma2_rn(c1, make_float2(q1.z, q1.w), vr);
-              vc = __ffma2_rn(c1, make_float2(q2.x, q2.y), vc);
-              vr = __ffma2_rn(c1, make_float2(q2.z, q2.w), vr);
-              vc = __ffma2_rn(c0, make_float2(q3.x, q3.y), vc);
-              vr = __ffma2_rn(c0, make_float2(q3.z, q3.w), vr);
-            }
-          }
-          reinterpret_cast<float4*>(t1)[pp * G::S_T1 + o] = make_float4(vc.x, vc.y, vr.x, vr.y);
-        }
-      } else {
-        const float* g0 = gsm + rl * G::NCX;
-        const float* g1 = gsm + G::S_G + rl * G::NCX;
-        float vc = 0.f, vr = 0.f;
-        if (valid) {
-          if (kx >= twoW) {
-#pragma unroll
-            for (int t = 0; t < 4; ++t) {
-              const int cl = p.cx_base + t - u.CX0;
-              vc = fmaf(p.cx[t], g0[cl], vc);
-              vr = fmaf(p.cx[t], g1[cl], vr);
-            }
-          } else if (kx & 1) {
-            const int cl = ((kx - 1) >> 1) - u.CX0;
-            vc = g0[cl];
-            vr = g1[cl];
-          } else {
-            const int cl = (kx >> 1) - 2 - u.CX0;
-            float c = -0.0625f * g0[cl], r = -0.0625f * g1[cl];
-            c = fmaf(0.5625f, g0[cl + 1], c);
-            r = fmaf(0.5625f, g1[cl + 1], r);
-            c = fmaf(0.5625f, g0[cl + 2], c);
-            r = fmaf(0.5625f, g1[cl + 2], r);
-            vc = fmaf(-0.0625f, g0[cl + 3], c);
-            vr = fmaf(-0.0625f, g1[cl + 3], r);
-          }
-        }
-        t1[o] = vc;
-        t1[G::S_T1 + o] = vr;
-      }
-    }
+  // one half-grid sample of a frame pair: normalise and store
+  __device__ __forceinline__ static void emit(const float4& v, bool valid, float4* dst) {
+    const float2 x = make_float2(v.x, v.y), y = make_float2(v.z, v.w);
+    const float2 m2 = __ffma2_rn(x, x, __fmul2_rn(y, y));
+    const float i0 = rsqrtf(m2.x) * kGradScale, i1 = rsqrtf(m2.y) * kGradScale;
+    const float2 inv = make_float2(i0, i1);
+    const float2 nx = __fmul2_rn(x, inv), ny = __fmul2_rn(y, inv);
+    const bool k0 = valid && m2.x > 0.f, k1 = valid && m2.y > 0.f;
+    *dst = make_float4(k0 ? nx.x : 0.f, k1 ? nx.y : 0.f, k0 ? ny.x : 0.f, k1 ? ny.y : 0.f);
   }
 
-  // gradient row pass and normalisation -> unit gradients of slot s
-  __device__ void row_pass(const FusedParams& p, const UnitGeo& u, int s) const {
-    const int twoH = 2 * u.H;
-    float* hgf = hg0 + s * G::S_HG;
-    for (int i = ptid; i < G::HG_R * G::HG_C; i += G::NP) {
-      const int kyl = i / G::HG_C, kxl = i % G::HG_C;
-      const int ky = u.kb_y + kyl, kx = u.kb_x + kxl;
-      const bool valid = ky >= 1 && ky <= u.kmax_y && kx >= 1 && kx <= u.kmax_x;
-      float gx[FP], gy[FP];
-#pragma unroll
-      for (int fr = 0; fr < FP; ++fr) gx[fr] = gy[fr] = 0.f;
-      if (valid) {
-        if constexpr (FP >= 2) {
-#pragma unroll
-          for (int pp = 0; pp < FP / 2; ++pp) {
-            const float4* c4 = reinterpret_cast<const float4*>(t1) + pp * G::S_T1 + kxl;
-            float2 x = make_float2(0.f, 0.f), y = make_float2(0.f, 0.f);
-            if (ky >= twoH) {
-#pragma unroll
-              for (int t = 0; t < 4; ++t) {
-                const float4 q = c4[(p.cy_base + t - u.RY0) * G::HG_C];
-                const float2 w = make_float2(p.cy[t], p.cy[t]);
-                x = __ffma2_rn(w, make_float2(q.x, q.y), x);
-                y = __ffma2_rn(w, make_float2(q.z, q.w), y);
-              }
-            } else if (ky & 1) {
-              const float4 q = c4[(((ky - 1) >> 1) - u.RY0) * G::HG_C];
-              x = make_float2(q.x, q.y);
-              y = make_float2(q.z, q.w);
-            } else {
-              const float4* c = c4 + ((ky >> 1) - 2 - u.RY0) * G::HG_C;
-              const float2 c0 = make_float2(-0.0625f, -0.0625f);
-              const float2 c1 = make_float2(0.5625f, 0.5625f);
-              const float4 q0 = c[0], q1 = c[G::HG_C], q2 = c[2 * G::HG_C], q3 = c[3 * G::HG_C];
-              x = __fmul2_rn(c0, make_float2(q0.x, q0.y));
-              y = __fmul2_rn(c0, make_float2(q0.z, q0.w));
-              x = __ffma2_rn(c1, make_float2(q1.x, q1.y), x);
-              y = __ffma2_rn(c1, make_float2(q1.z, q1.w), y);
-              x = __ffma2_rn(c1, make_float2(q2.x, q2.y), x);
-              y = __ffma2_rn(c1, make_float2(q2.z, q2.w), y);
-              x = __ffma2_rn(c0, make_float2(q3.x, q3.y), x);
-              y = __ffma2_rn(c0, make_float2(q3.z, q3.w), y);
-            }
-            gx[2 * pp] = x.x;
-            gx[2 * pp + 1] = x.y;
-            gy[2 * pp] = y.x;
-            gy[2 * pp + 1] = y.y;
-          }
-        } else {
-          const float* c0 = t1 + kxl;
-          const float* c1 = t1 + G::S_T1 + kxl;
-          if (ky >= twoH) {
-#pragma unroll
-            for (int t = 0; t < 4; ++t) {
-              const int rl = p.cy_base + t - u.RY0;
-              gx[0] = fmaf(p.cy[t], c0[rl * G::HG_C], gx[0]);
-              gy[0] = fmaf(p.cy[t], c1[rl * G::HG_C], gy[0]);
-            }
-          } else if (ky & 1) {
-            const int rl = ((ky - 1) >> 1) - u.RY0;
-            gx[0] = c0[rl * G::HG_C];
-            gy[0] = c1[rl * G::HG_C];
-          } else {
-            const int rl = (ky >> 1) - 2 - u.RY0;
-            const float* a0 = c0 + rl * G::HG_C;
-            const float* a1 = c1 + rl * G::HG_C;
-            float x = -0.0625f * a0[0], y = -0.0625f * a1[0];
-            x = fmaf(0.5625f, a0[G::HG_C], x);
-            y = fmaf(0.5625f, a1[G::HG_C], y);
-            x = fmaf(0.5625f, a0[2 * G::HG_C], x);
-            y = fmaf(0.5625f, a1[2 * G::HG_C], y);
-            gx[0] = fmaf(-0.0625f, a0[3 * G::HG_C], x);
-            gy[0] = fmaf(-0.0625f, a1[3 * G::HG_C], y);
-          }
-        }
-      }
-      float nxv[FP], nyv[FP];
-#pragma unroll
-      for (int fr = 0; fr < FP; ++fr) {
-        nxv[fr] = nyv[fr] = 0.f;
-        const float m2 = fmaf(gx[fr], gx[fr], gy[fr] * gy[fr]);
-        if (valid && m2 > 0.f) {
-          const float inv = rsqrtf(m2);
-          nxv[fr] = gx[fr] * inv;
-          nyv[fr] = gy[fr] * inv;
-        }
-      }
-      const int o = (kyl * 2 + (kxl & 1)) * G::HGP + (kxl >> 1);
-      if constexpr (FP >= 2) {
-#pragma unroll
-        for (int pp = 0; pp < FP / 2; ++pp)
-          reinterpret_cast<float4*>(hgf)[pp * G::HG_PLANE + o] =
-              make_float4(nxv[2 * pp], nxv[2 * pp + 1], nyv[2 * pp], nyv[2 * pp + 1]);
+  // w0 q0 + w1 q1 + w2 q2 + w3 q3 of a frame pair's (gx, gx', gy, gy')
+  __device__ __forceinline__ static float4 taps(const float4& q0, const float4& q1,
+                                                const float4& q2, const float4& q3,
+                                                const float (&w)[4]) {
+    auto tap = [](float wk, const float4& q, float2& x, float2& y) {
+      const float2 w2 = make_float2(wk, wk);
+      x = __ffma2_rn(w2, make_float2(q.x, q.y), x);
+      y = __ffma2_rn(w2, make_float2(q.z, q.w), y);
+    };
+    float2 x = __fmul2_rn(make_float2(w[0], w[0]), make_float2(q0.x, q0.y));
+    float2 y = __fmul2_rn(make_float2(w[0], w[0]), make_float2(q0.z, q0.w));
+    tap(w[1], q1, x, y);
+    tap(w[2], q2, x, y);
+    tap(w[3], q3, x, y);
+    return make_float4(x.x, x.y, y.x, y.y);
+  }
+
+  // Gradient Catmull-Rom on the half-grid and its normalisation -> slot s.
+  // Half-grid index 2 a takes the taps a-2 .. a+1 of its axis with weights
+  // (-1, 9, 9, -1) / 16, index 2 a + 1 is sample a itself; indices from 2 H
+  // (2 W) on are all the clamped last position, whose taps H-2 .. H+1 are
+  // those of a = H.  A thread takes one half-grid column and walks down the row
+  // steps of a segment with the four newest rows of its column in registers:
+  // per row 4 shared loads (an even index) or 1 (an odd one), per step two
+  // samples, without the buffer between a column and a row pass.  Lanes run
+  // along the columns of one parity; the LEFT columns beyond a warp are done
+  // one step per thread.
+  __device__ void gradients(const FusedParams& p, const UnitGeo& u, int np, int s) const {
+    const int a0 = u.ny0 - (J + 1) / 2, b0 = u.nx0 - (J + 1) / 2;
+    const int tH = u.H - a0;  // step of a = H
+    const int main_jobs = np * G::NSEG * 64;
+    const int jobs = main_jobs + np * G::NA * G::LEFT * 2;
+    for (int i = ptid; i < jobs; i += G::NP) {
+      int pp, c, t0, t1, odd;
+      if (i < main_jobs) {
+        const int wj = i >> 5;
+        odd = wj >= np * G::NSEG;
+        const int k = odd ? wj - np * G::NSEG : wj;
+        pp = k / G::NSEG;
+        t0 = (k - pp * G::NSEG) * G::SEG;
+        t1 = min(t0 + G::SEG, G::NA);
+        c = i & 31;
       } else {
-        reinterpret_cast<float2*>(hgf)[o] = make_float2(nxv[0], nyv[0]);
+        const int k = i - main_jobs;
+        const int pl = k / (G::NA * G::LEFT);
+        const int r = k - pl * (G::NA * G::LEFT);
+        odd = pl >= np;
+        pp = odd ? pl - np : pl;
+        t0 = r / G::LEFT;
+        t1 = t0 + 1;
+        c = 32 + r - t0 * G::LEFT;
+      }
+      // an odd J starts its tile at an odd half-grid index: the first even and
+      // the last odd index of the steps are outside the slot
+      if ((J & 1) && c == (odd ? G::NB - 1 : 0)) continue;
+      const int b = b0 + c;
+      const int kx = 2 * b + odd;
+      const bool vx = kx >= 1 && kx <= u.kmax_x;
+      const bool cclamp = b >= u.W;
+      const bool four = cclamp || !odd;
+      const float4* g4 = reinterpret_cast<const float4*>(gsm + pp * G::S_G) +
+                         (cclamp ? u.W - 2 - u.CX0 : (odd ? c + 2 : c));
+      // slot column of kx: [parity][index]
+      float4* hg = reinterpret_cast<float4*>(hg0 + s * G::S_HG) + pp * G::HG_PLANE +
+                   ((J & 1) ? (odd ? c : G::HGP + c - 1) : odd * G::HGP + c);
+      float4 win[4];
+      auto row = [&](int r) {
+        const float4* q = g4 + r * G::NCX;
+        float4 v = q[0];
+        if (four) {
+          float w[4] = {-0.0625f, 0.5625f, 0.5625f, -0.0625f};
+          if (cclamp) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) w[k] = p.cx[k];
+          }
+          v = taps(v, q[1], q[2], q[3], w);
+        }
+        return v;
+      };
+      const int ts = min(t0, tH);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) win[k + 1] = row(ts + k);
+#pragma unroll
+      for (int d = 0; d < G::SEG; ++d) {
+        const int t = t0 + d;
+        if (t >= t1) break;
+        if (d == 0 || t <= tH) {  // past a = H the window stays
+#pragma unroll
+          for (int k = 0; k < 3; ++k) win[k] = win[k + 1];
+          win[3] = row(min(t, tH) + 3);
+        }
+        const int a = a0 + t;
+        const int kyl = 2 * t - (J & 1);  // slot row of 2 a
+        const bool rclamp = a >= u.H;
+        float w[4] = {-0.0625f, 0.5625f, 0.5625f, -0.0625f};
+        if (rclamp) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) w[k] = p.cy[k];
+        }
+        const float4 e = taps(win[0], win[1], win[2], win[3], w);
+        if (!(J & 1) || t >= 1)
+          emit(e, vx && 2 * a >= 1 && 2 * a <= u.kmax_y, hg + kyl * 2 * G::HGP);
+        if (!(J & 1) || t < G::NA - 1)
+          emit(rclamp ? e : win[2], vx && a >= 0 && 2 * a + 1 <= u.kmax_y,
+               hg + (kyl + 1) * 2 * G::HGP);
       }
     }
   }
 };
 
-// Numerator of the horizontal offset of RGC sample (px, ii) from its output's
-// centre, 2 M dx = M (cpx + ii - J) - (2 px + 1); its sign is the sign of the
-// table's a = dx w / d (zero exactly when dx is).
+// Numerator of the horizontal offset of half-grid sample q (of the NQ a window
+// row spans) from the centre of output phase px, 2 M dx = M (q - J) - (2 px + 1);
+// zero only for the middle phase of an odd M at q = J + 1.
 template <int M, int J>
-__host__ __device__ constexpr int dx_num(int px, int ii) {
-  return M * ((2 * px + 1) / M + ii - J) - (2 * px + 1);
+__host__ __device__ constexpr int dx_num(int px, int q) {
+  return M * (q - J) - (2 * px + 1);
 }
 
-// RGC of one consumer's M outputs for the FP frames of slot hgf.
+// whether sample q lies in the window of output phase px
+template <int M, int J>
+__host__ __device__ constexpr bool in_window(int px, int q) {
+  const int ii = q - (2 * px + 1) / M;
+  return px >= 0 && px < M && ii >= 0 && ii < 2 * J + 1;
+}
+
+// One sample of the RGC for a frame pair: acc += [n.(a, b) < 0] (w - |n x (a, b)|).
+// With rho = b / a, n.(a, b) = a (gx + gy rho) and |n x (a, b)| = |a| |gy - gx rho|;
+// SIGN is the sign of dx (of a), a constant of the unrolled loops.  For dx = 0
+// the two are gy b and |b| |gx|, and rho, nab stand for sign b and -|b|.
+//
+// The test is a saturating scalar FMA per frame (kGradScale): 0 or 1 straight
+// from the FMA pipe.  In a loop of samples with their constants in registers
+// this form took 10.8 cycles per sample pair and scheduler, the comparison it
+// replaces (a packed FMA and two ALU set instructions) 12.1; four packed FMAs
+// alone take 10.8, because each reads six register operands.
+template <int SIGN>
+__device__ __forceinline__ void rgc_sample(const float4& g, float rho, float nrho, float nab,
+                                           float w, float2& acc) {
+  const float2 gx = make_float2(g.x, g.y), gy = make_float2(g.z, g.w);
+  float2 m, t2;
+  if (SIGN > 0) {
+    m = make_float2(__saturatef(__fmaf_rn(-gy.x, rho, -gx.x)),
+                    __saturatef(__fmaf_rn(-gy.y, rho, -gx.y)));
+  } else if (SIGN < 0) {
+    m = make_float2(__saturatef(__fmaf_rn(gy.x, rho, gx.x)),
+                    __saturatef(__fmaf_rn(gy.y, rho, gx.y)));
+  } else {
+    m = make_float2(__saturatef(__fmul_rn(-gy.x, rho)), __saturatef(__fmul_rn(-gy.y, rho)));
+  }
+  t2 = SIGN == 0 ? gx : __ffma2_rn(gx, make_float2(nrho, nrho), gy);
+  const float2 v = __ffma2_rn(make_float2(nab, nab), make_float2(fabsf(t2.x), fabsf(t2.y)),
+                              make_float2(w, w));
+  acc = __ffma2_rn(m, v, acc);
+}
+
+// RGC of one consumer's PYT * M outputs for NPR frame pairs of the slot at hgf.
 // Contribution of sample (phase, offset): (dp < 0) ? w - |u| : 0 with
 // dp = n.(a, b) and u = n x (a, b) (n the unit gradient).
-template <int M, int J, int TY, int FP>
+//
+// Mirror images share a table entry: sample q seen from phase px and sample
+// NQ - q seen from phase M - 1 - px lie at opposite dx and the same dy, so they
+// have the same weight and |a| and opposite rho.  Walking q from both ends loads
+// (J + 1) M + M / 2 entries per window row instead of M (2J + 1) (m = 5,
+// R = 1.5: 20 used for 35 samples).
+template <typename G, int M, int J, int NPR>
 __device__ __forceinline__ void rgc_core(const float* hgf, const float4* tb4, int ty, int py,
-                                         int lane, float (&acc)[FP][M]) {
-  using G = Geo<M, J, TY, FP>;
+                                         int lane, float2 (&acc)[NPR][M]) {
   const int cpy = (2 * py + 1) / M;
+  const float4* hg = reinterpret_cast<const float4*>(hgf);
 #pragma unroll
-  for (int fr = 0; fr < FP; ++fr)
+  for (int pp = 0; pp < NPR; ++pp)
 #pragma unroll
-    for (int px = 0; px < M; ++px) acc[fr][px] = 0.f;
-  if constexpr (FP == 1) {
-    const float2* hg = reinterpret_cast<const float2*>(hgf);
-#pragma unroll
-    for (int jj = 0; jj < G::W2; ++jj) {
-      const int kyl = 2 * ty + cpy + jj;
-      const float2* r0 = hg + (kyl * 2 + 0) * G::HGP + lane;
-      const float2* r1 = hg + (kyl * 2 + 1) * G::HGP + lane;
-      float2 sv[G::NQ];
-#pragma unroll
-      for (int q = 0; q < G::NQ; ++q) sv[q] = (q & 1) ? r1[q >> 1] : r0[q >> 1];
-      const float4* tb = tb4 + (size_t)(py * G::W2 + jj) * G::TBLK;
-#pragma unroll
-      for (int s4 = 0; s4 < G::NS4; ++s4) {
-        const float4 A = tb[s4];
-        const float4 B = tb[G::NS4 + s4];
-        const float4 Wv = tb[2 * G::NS4 + s4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int sidx = s4 * 4 + e;
-          if (sidx < G::NS) {
-            const int px = sidx / G::W2;
-            const int ii = sidx % G::W2;
-            const int cpx = (2 * px + 1) / M;
-            const float2 gv = sv[cpx + ii];
-            const float a = f4c(A, e), bb = f4c(B, e), w = f4c(Wv, e);
-            const float dp = fmaf(gv.x, a, gv.y * bb);
-            const float u = fmaf(gv.y, a, -(gv.x * bb));
-            const float v = w - fabsf(u);
-            acc[0][px] = (dp < 0.f) ? acc[0][px] + v : acc[0][px];
-          }
-        }
-      }
-    }
-  } else {
-    // frame pair in one register pair: gx = (gx0, gx1), gy = (gy0, gy1); every
-    // FMA-pipe operation is packed: v = w + (-|u|), acc += [dp < 0] * v
-    // (measured 6 % faster than scalar v and predicated scalar adds)
-    const float4* hg = reinterpret_cast<const float4*>(hgf);
-    constexpr int NPR = FP / 2;  // frame pairs per pass (share every table load)
-    float2 acc2[NPR][M];
-#pragma unroll
-    for (int pp = 0; pp < NPR; ++pp)
-#pragma unroll
-      for (int px = 0; px < M; ++px) acc2[pp][px] = make_float2(0.f, 0.f);
-    // window rows stay a loop: unrolled, the core's code outgrows the
-    // instruction cache (measured 2 % slower and with register spills)
+    for (int px = 0; px < M; ++px) acc[pp][px] = make_float2(0.f, 0.f);
+  // window rows stay a loop: unrolled, the core's code outgrows the
+  // instruction cache (measured 2 % slower and with register spills)
 #pragma unroll 1
-    for (int jj = 0; jj < G::W2; ++jj) {
-      const int kyl = 2 * ty + cpy + jj;
-      const float4* r0 = hg + (kyl * 2 + 0) * G::HGP + lane;
-      const float4* r1 = hg + (kyl * 2 + 1) * G::HGP + lane;
-      const float4* tb = tb4 + (size_t)(py * G::W2 + jj) * G::TBLK;
+  for (int jj = 0; jj < G::W2; ++jj) {
+    const int kyl = 2 * ty + cpy + jj;
+    const float4* r0 = hg + (kyl * 2 + 0) * G::HGP + lane;
+    const float4* r1 = hg + (kyl * 2 + 1) * G::HGP + lane;
+    const float4* tb = tb4 + (size_t)(py * G::W2 + jj) * G::NE;
+    if constexpr (M <= 2) {
       // gradient-major order: one half-grid sample at a time, applied to every
-      // output phase px whose window holds it (fewer live registers than
-      // loading the row first; measured 1.3 % faster)
+      // output phase px whose window holds it
 #pragma unroll
       for (int q = 0; q < G::NQ; ++q) {
         float4 g[NPR];
@@ -580,65 +551,67 @@ __device__ __forceinline__ void rgc_core(const float* hgf, const float4* tb4, in
           g[pp] = (q & 1) ? r1[pp * G::HG_PLANE + (q >> 1)] : r0[pp * G::HG_PLANE + (q >> 1)];
 #pragma unroll
         for (int px = 0; px < M; ++px) {
-          const int ii = q - (2 * px + 1) / M;
-          if (ii < 0 || ii >= G::W2) continue;
-          const int sidx = px * G::W2 + ii;
-          const float4 T = tb[sidx];
-          const float w = T.w;
-          const int dxn = dx_num<M, J>(px, ii);  // compile-time after unrolling
-          if (dxn != 0) {
-            // dp = a (gx + gy rho) and u = a (gy - gx rho), rho = b / a: the
-            // sign of a is the sign of dx, a constant of (px, ii), so
-            // [dp < 0] is a comparison of t1 = gx + gy rho in a fixed
-            // direction, and w - |u| = w + (-|a|) |t2|, t2 = gy - gx rho:
-            // 4 packed FMA-pipe operations per sample pair instead of 6
-            const float2 rho = make_float2(T.x, T.x), nrho = make_float2(T.y, T.y);
-            const float2 nab = make_float2(T.z, T.z);
+          if (!in_window<M, J>(px, q)) continue;
+          // entry (rho, -rho, -|a|, w) of this sample, or of its mirror image
+          const bool own = q <= J || (q == J + 1 && 2 * px < M);
+          const float4 T = own ? tb[q * M + px] : tb[(G::NQ - q) * M + M - 1 - px];
+          const float rho = own ? T.x : T.y, nrho = own ? T.y : T.x;
+          const int dxn = dx_num<M, J>(px, q);
 #pragma unroll
-            for (int pp = 0; pp < NPR; ++pp) {
-              const float2 gx = make_float2(g[pp].x, g[pp].y), gy = make_float2(g[pp].z, g[pp].w);
-              const float2 t1 = __ffma2_rn(gy, rho, gx);
-              const float2 t2 = __ffma2_rn(gx, nrho, gy);
-              const float2 at2 = make_float2(fabsf(t2.x), fabsf(t2.y));
-              const float2 v = __ffma2_rn(nab, at2, make_float2(w, w));
-              const float2 msk =
-                  dxn > 0 ? make_float2(t1.x < 0.f ? 1.f : 0.f, t1.y < 0.f ? 1.f : 0.f)
-                          : make_float2(t1.x > 0.f ? 1.f : 0.f, t1.y > 0.f ? 1.f : 0.f);
-              acc2[pp][px] = __ffma2_rn(msk, v, acc2[pp][px]);
+          for (int pp = 0; pp < NPR; ++pp) {
+            if (dxn > 0) {
+              rgc_sample<1>(g[pp], rho, nrho, T.z, T.w, acc[pp][px]);
+            } else if (dxn < 0) {
+              rgc_sample<-1>(g[pp], rho, nrho, T.z, T.w, acc[pp][px]);
+            } else {
+              rgc_sample<0>(g[pp], T.x, 0.f, T.z, T.w, acc[pp][px]);
             }
-          } else {
-            // dx = 0: dp = gy b, u = -gx b
-            const float2 a = make_float2(T.x, T.x), b = make_float2(T.y, T.y);
-            const float2 nb = make_float2(T.z, T.z);
+          }
+        }
+      }
+    } else {
 #pragma unroll
-            for (int pp = 0; pp < NPR; ++pp) {
-              const float2 gx = make_float2(g[pp].x, g[pp].y), gy = make_float2(g[pp].z, g[pp].w);
-              const float2 dp = __ffma2_rn(gx, a, __fmul2_rn(gy, b));
-              const float2 u = __ffma2_rn(gy, a, __fmul2_rn(gx, nb));
-              const float2 nu = make_float2(__int_as_float(__float_as_int(u.x) | 0x80000000),
-                                            __int_as_float(__float_as_int(u.y) | 0x80000000));
-              const float2 v = __fadd2_rn(make_float2(w, w), nu);
-              const float2 msk = make_float2(dp.x < 0.f ? 1.f : 0.f, dp.y < 0.f ? 1.f : 0.f);
-              acc2[pp][px] = __ffma2_rn(msk, v, acc2[pp][px]);
+      for (int q = 0; q <= J + 1; ++q) {
+        const int qm = G::NQ - q;  // the mirrored sample (none for q = 0)
+        float4 ga[NPR], gb[NPR];
+#pragma unroll
+        for (int pp = 0; pp < NPR; ++pp) {
+          ga[pp] = (q & 1) ? r1[pp * G::HG_PLANE + (q >> 1)] : r0[pp * G::HG_PLANE + (q >> 1)];
+          gb[pp] = ga[pp];
+          if (q >= 1 && qm != q)
+            gb[pp] = (qm & 1) ? r1[pp * G::HG_PLANE + (qm >> 1)]
+                              : r0[pp * G::HG_PLANE + (qm >> 1)];
+        }
+#pragma unroll
+        for (int px = 0; px < (q == J + 1 ? (M + 1) / 2 : M); ++px) {
+          const int pm = M - 1 - px;
+          const bool use_a = in_window<M, J>(px, q);
+          const bool use_b = q >= 1 && (q != qm || px != pm) && in_window<M, J>(pm, qm);
+          if (!use_a && !use_b) continue;
+          const float4 T = tb[q * M + px];  // (rho, -rho, -|a|, w) of (px, q)
+          const int dxn = dx_num<M, J>(px, q);
+#pragma unroll
+          for (int pp = 0; pp < NPR; ++pp) {
+            if (dxn > 0) {
+              if (use_a) rgc_sample<1>(ga[pp], T.x, T.y, T.z, T.w, acc[pp][px]);
+              if (use_b) rgc_sample<-1>(gb[pp], T.y, T.x, T.z, T.w, acc[pp][pm]);
+            } else if (dxn < 0) {
+              if (use_a) rgc_sample<-1>(ga[pp], T.x, T.y, T.z, T.w, acc[pp][px]);
+              if (use_b) rgc_sample<1>(gb[pp], T.y, T.x, T.z, T.w, acc[pp][pm]);
+            } else {
+              rgc_sample<0>(ga[pp], T.x, 0.f, T.z, T.w, acc[pp][px]);
             }
           }
         }
       }
     }
-#pragma unroll
-    for (int pp = 0; pp < NPR; ++pp)
-#pragma unroll
-      for (int px = 0; px < M; ++px) {
-        acc[2 * pp][px] = acc2[pp][px].x;
-        acc[2 * pp + 1][px] = acc2[pp][px].y;
-      }
   }
 }
 
-template <int M, int J, int TY, int FP, int MODE, int NP>
-__global__ void __launch_bounds__(32 * TY * M + NP, EsrrfTile<M>::MIN_BLOCKS)
+template <int M, int J, int TY, int FP, int MODE, int NP, int PYT>
+__global__ void __launch_bounds__(32 * TY * (M / PYT) + NP, EsrrfTile<M>::MIN_BLOCKS)
     esrrf_fused_kernel(const __grid_constant__ TmapPack maps, const UnitTable ut) {
-  using G = Geo<M, J, TY, FP, NP>;
+  using G = Geo<M, J, TY, FP, NP, PYT>;
   extern __shared__ __align__(128) float sm[];
   __shared__ FusedParams sp;
   __shared__ int s_unit;
@@ -646,22 +619,22 @@ __global__ void __launch_bounds__(32 * TY * M + NP, EsrrfTile<M>::MIN_BLOCKS)
   float4* tb4 = reinterpret_cast<float4*>(sm + G::O_TB);
   float* rw = sm + G::O_RW;
   float* cw = sm + G::O_CW;
-  float* tw = sm + G::O_TW;  // tw[px * NTC + tid]
+  float* tw = sm + G::O_TW;  // tw[output * NTC + tid]
   float* tk = sm + G::O_TK;
   uint64_t* bars = reinterpret_cast<uint64_t*>(sm + G::o_bar(MODE, ut.ns_cap));
   uint64_t* full = bars;                    // [NSLOT] slot prepared (NP arrivals)
   uint64_t* empty = bars + G::NSLOT;        // [NSLOT] slot released (NTC arrivals)
   uint64_t* pbar = bars + 2 * G::NSLOT;     // producer-group barrier (NP arrivals)
-  uint64_t* tbar = bars + 2 * G::NSLOT + 1; // [2 FP] TMA input tiles
+  uint64_t* tbar = bars + 2 * G::NSLOT + 1; // TMA input tiles of a pass
 
   const int tid = threadIdx.x;
   const bool producer = tid >= G::NTC;
   const int lane = tid & 31;
   const int warp = tid >> 5;
   const int ty = warp % TY;  // consumers
-  const int py = warp / TY;
-  Producer<M, J, TY, FP, NP> prod{sm + G::O_INB, sm + G::O_G, sm + G::O_T1, sm + G::O_HG,
-                              sm + G::O_RI, rw, tid - G::NTC};
+  const int py0 = warp / TY * PYT;
+  const Producer<G, M, J> prod{sm + G::O_INB, sm + G::O_G, sm + G::O_HG,
+                               sm + G::O_RI, rw, tid - G::NTC};
 
   if (tid == 0) {
     for (int k = 0; k < G::NSLOT; ++k) {
@@ -669,14 +642,14 @@ __global__ void __launch_bounds__(32 * TY * M + NP, EsrrfTile<M>::MIN_BLOCKS)
       mbar_init(&empty[k], G::NTC);
     }
     mbar_init(pbar, G::NP);
-    for (int k = 0; k < 2 * FP; ++k) mbar_init(&tbar[k], 1);
+    mbar_init(tbar, 1);
     fence_mbar_init();
     s_abort = 0;
   }
   __syncthreads();
   unsigned gp = 0;      // frame passes since launch: slot gp % NSLOT, use gp / NSLOT (all threads)
-  unsigned tphase = 0;  // producers: bit k = parity of the next completion of tbar[k]
-  unsigned tpend = 0;   // producers: bit k = a TMA load into input buffer k is in flight
+  unsigned tphase = 0;  // producers: parity of the next completion of tbar
+  bool tpend = false;   // producers: TMA loads into the input tiles are in flight
   unsigned pphase = 0;  // producers: parity of the next completion of pbar
   int cur_item = -1;
 
@@ -703,31 +676,34 @@ __global__ void __launch_bounds__(32 * TY * M + NP, EsrrfTile<M>::MIN_BLOCKS)
   if (item != cur_item) {
     if (tid == 0) sp = ut.items ? ut.items[item] : ut.single;
     __syncthreads();
-    if constexpr (FP == 1) {
-      const float4* src = reinterpret_cast<const float4*>(sp.tbl);
-      for (int i = tid; i < M * G::W2 * 3 * G::NS4; i += G::NT) tb4[i] = src[i];
-    } else {
-      // plan layout [py][jj]{a, b, w}[NS4 * 4] -> one float4 per sample:
-      //   dx != 0: (rho, -rho, -|a|, w) with rho = b / a (see rgc_core);
-      //   dx == 0: (a, b, -b, w) (a = 0);  outside the window: zeros
+    {
+      // plan layout [py][jj]{a, b, w}[NS4 * 4] -> one float4 per mirrored couple
+      // (see rgc_core), in the orientation of its sample (px, q):
+      //   dx != 0: (rho, -rho, -|a| / scale, w) with rho = b / a;
+      //   dx == 0: (sign b, 0, -|b| / scale, w);  outside the radius: zeros
       constexpr int N4 = G::NS4 * 4;
       const float* src = sp.tbl;
-      for (int i = tid; i < M * G::W2 * N4; i += G::NT) {
-        const int blk = i / N4, s = i % N4;
-        const float a = src[(blk * 3 + 0) * N4 + s];
-        const float b = src[(blk * 3 + 1) * N4 + s];
-        const float w = src[(blk * 3 + 2) * N4 + s];
-        const int px = s / G::W2, ii = s % G::W2;
+      for (int i = tid; i < M * G::W2 * G::NE; i += G::NT) {
+        const int blk = i / G::NE, k = i % G::NE;
+        const int q = k / M, px = k % M;
+        const bool own = in_window<M, J>(px, q);
+        const int sp_px = own ? px : M - 1 - px, sq = own ? q : G::NQ - q;
         float4 e = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (s < G::NS && w != 0.f) {
-          if (dx_num<M, J>(px, ii) == 0) {
-            e = make_float4(a, b, -b, w);
-          } else if (a != 0.f) {
-            const float rho = __fdiv_rn(b, a);
-            e = make_float4(rho, -rho, -fabsf(a), w);
+        if (in_window<M, J>(sp_px, sq)) {
+          const int s = sp_px * G::W2 + sq - (2 * sp_px + 1) / M;
+          const float a = own ? src[(blk * 3 + 0) * N4 + s] : -src[(blk * 3 + 0) * N4 + s];
+          const float b = src[(blk * 3 + 1) * N4 + s];
+          const float w = src[(blk * 3 + 2) * N4 + s];
+          if (w != 0.f) {
+            if (dx_num<M, J>(px, q) == 0) {
+              e = make_float4(b > 0.f ? 1.f : -1.f, 0.f, -fabsf(b) / kGradScale, w);
+            } else if (a != 0.f) {
+              const float rho = __fdiv_rn(b, a);
+              e = make_float4(rho, -rho, -fabsf(a) / kGradScale, w);
+            }
           }
         }
-        tb4[blk * G::TBLK + s] = e;
+        tb4[blk * G::NE + k] = e;
       }
     }
     cur_item = item;
@@ -780,7 +756,7 @@ __global__ void __launch_bounds__(32 * TY * M + NP, EsrrfTile<M>::MIN_BLOCKS)
       for (int kk = 0; kk < 5; ++kk) w5[kk] = (k == kk) ? w : w5[kk];
     }
 #pragma unroll
-    for (int k = 0; k < 5; ++k) rw[i * 5 + k] = w5[k];
+    for (int k = 0; k < 5; ++k) rw[i * 8 + k] = w5[k];
   }
   for (int i = tid; i < G::OX; i += G::NT) {
     const int xM = u.nx0 * M + i;
@@ -803,89 +779,87 @@ __global__ void __launch_bounds__(32 * TY * M + NP, EsrrfTile<M>::MIN_BLOCKS)
   // ---- consumer constants --------------------------------------------------
   const int ny = u.ny0 + ty;
   const int nx = u.nx0 + lane;
-  const int yM = ny * M + py;
-  unsigned omask = 0;  // bit px: output forced to 0 / not written; bit 31: outside the image
+  unsigned omask = 0;  // bit per output: forced to 0 / not written; bit 31: outside the image
   if (!producer) {
-    const int cpy = (2 * py + 1) / M;
-    const int ky_lo = 2 * ny + cpy - J, ky_hi = 2 * ny + cpy + J;
-    const bool by = (ky_lo < 1) || (ky_hi > u.kmax_y);
 #pragma unroll
-    for (int px = 0; px < M; ++px) {
-      const int cpx = (2 * px + 1) / M;
-      const int xM = nx * M + px;
-      const int kx_lo = 2 * nx + cpx - J, kx_hi = 2 * nx + cpx + J;
-      float iw = p.inv_wsum[py * M + px];
-      if (by || kx_lo < 1 || kx_hi > u.kmax_x) {
-        // window reaches invalid half-grid samples: they count in neither sum
-        const float* wf = p.wfull + (size_t)(py * M + px) * G::W2 * G::W2;
-        float s = 0.f;
-        for (int jj = 0; jj < G::W2; ++jj) {
-          const int ky = ky_lo + jj;
-          if (ky < 1 || ky > u.kmax_y) continue;
-          for (int ii = 0; ii < G::W2; ++ii) {
-            const int kx = kx_lo + ii;
-            if (kx < 1 || kx > u.kmax_x) continue;
-            s += wf[jj * G::W2 + ii];
+    for (int d = 0; d < PYT; ++d) {
+      const int py = py0 + d, yM = ny * M + py;
+      const int cpy = (2 * py + 1) / M;
+      const int ky_lo = 2 * ny + cpy - J, ky_hi = 2 * ny + cpy + J;
+      const bool by = (ky_lo < 1) || (ky_hi > u.kmax_y);
+#pragma unroll
+      for (int px = 0; px < M; ++px) {
+        const int cpx = (2 * px + 1) / M;
+        const int xM = nx * M + px;
+        const int kx_lo = 2 * nx + cpx - J, kx_hi = 2 * nx + cpx + J;
+        float iw = p.inv_wsum[py * M + px];
+        if (by || kx_lo < 1 || kx_hi > u.kmax_x) {
+          // window reaches invalid half-grid samples: they count in neither sum
+          const float* wf = p.wfull + (size_t)(py * M + px) * G::W2 * G::W2;
+          float s = 0.f;
+          for (int jj = 0; jj < G::W2; ++jj) {
+            const int ky = ky_lo + jj;
+            if (ky < 1 || ky > u.kmax_y) continue;
+            for (int ii = 0; ii < G::W2; ++ii) {
+              const int kx = kx_lo + ii;
+              if (kx < 1 || kx > u.kmax_x) continue;
+              s += wf[jj * G::W2 + ii];
+            }
           }
+          iw = s > 0.f ? 1.f / s : 0.f;
         }
-        iw = s > 0.f ? 1.f / s : 0.f;
+        tw[(d * M + px) * G::NTC + tid] = iw;
+        const bool outside = (ny >= u.H) || (nx >= u.W);
+        const bool in_margin = (yM < p.margin) || (yM >= p.rowsM - p.margin) ||
+                               (xM < p.margin) || (xM >= p.colsM - p.margin);
+        if (outside) omask |= (1u << (d * M + px)) | (1u << 31);
+        else if (in_margin) omask |= (1u << (d * M + px));
       }
-      tw[px * G::NTC + tid] = iw;
-      const bool outside = (ny >= u.H) || (nx >= u.W);
-      const bool in_margin = (yM < p.margin) || (yM >= p.rowsM - p.margin) ||
-                             (xM < p.margin) || (xM >= p.colsM - p.margin);
-      if (outside) omask |= (1u << px) | (1u << 31);
-      else if (in_margin) omask |= (1u << px);
     }
   }
   __syncthreads();
 
   if (producer) {
-    // ======================= producer warpgroup =============================
+    // ======================= producer warps =================================
     constexpr unsigned kTileBytes = unsigned(G::BH * G::BW * 4);
     const bool use_tma = p.tmap >= 0;
     const CUtensorMap* tmap = use_tma ? &maps.m[p.tmap] : nullptr;
     const bool leader = prod.ptid == 0;
-    if (use_tma && leader) {
-      // input buffer k = set * FP + fr holds frame f0 + k for the first two sets
+    // the input tiles of the pass whose first frame is f (leader only)
+    auto fetch = [&](int f) {
+      const int n = min(FP, f1 - f);
       fence_proxy_async_smem();
-      for (int k = 0; k < 2 * FP; ++k) {
-        if (f0 + k < f1) {
-          mbar_arrive_expect_tx(&tbar[k], kTileBytes);
-          tma_load_3d(prod.inb + k * G::S_INB, tmap, &tbar[k], u.x_start, u.y_start, f0 + k);
-          tpend |= 1u << k;
-        }
-      }
-    }
+      mbar_arrive_expect_tx(tbar, n * kTileBytes);
+      for (int k = 0; k < n; ++k)
+        tma_load_3d(prod.inb + k * G::S_INB, tmap, tbar, u.x_start, u.y_start, f + k);
+      tpend = true;
+    };
+    auto group_sync = [&]() {  // all producer threads
+      mbar_arrive(pbar);
+      const bool ok = mbar_wait_or_abort(pbar, pphase & 1u, &s_abort, lim);
+      pphase ^= 1u;
+      return ok;
+    };
+    if (use_tma && leader) fetch(f0);
     for (int j = 0; j < npass; ++j) {
       const unsigned g = gp + j;
       const int s = (int)(g % G::NSLOT);
       const unsigned use = g / G::NSLOT;
       const int fa = f0 + j * FP;
-      const int set = j & 1;
       const int nf = min(FP, f1 - fa);
-      const float* tin[FP];
-#pragma unroll
-      for (int fr = 0; fr < FP; ++fr)
-        tin[fr] = prod.inb + (set * FP + (fr < nf ? fr : 0)) * G::S_INB;
+      const int np = (nf + 1) / 2;
       // slot s is free once the consumers released its previous use
       bool ok = use == 0 || mbar_wait_or_abort(&empty[s], (use - 1) & 1u, &s_abort, lim);
       if (ok && use_tma) {
-#pragma unroll
-        for (int fr = 0; fr < FP; ++fr) {
-          const int k = set * FP + fr;
-          if (fr < nf && ok) {
-            ok = mbar_wait_or_abort(&tbar[k], (tphase >> k) & 1u, &s_abort, lim);
-            if (ok) {
-              tphase ^= 1u << k;
-              tpend &= ~(1u << k);
-            }
-          }
+        ok = mbar_wait_or_abort(tbar, tphase, &s_abort, lim);
+        if (ok) {
+          tphase ^= 1u;
+          tpend = false;
         }
       } else if (ok) {
         for (int fr = 0; fr < nf; ++fr) {
           const float* src = p.in + (size_t)(fa + fr) * u.H * u.W;
-          float* dst = prod.inb + (set * FP + fr) * G::S_INB;
+          float* dst = prod.inb + fr * G::S_INB;
           for (int i = prod.ptid; i < G::BH * G::BW; i += G::NP) {
             const int r = u.y_start + i / G::BW;
             const int c = u.x_start + i % G::BW;
@@ -893,46 +867,24 @@ __global__ void __launch_bounds__(32 * TY * M + NP, EsrrfTile<M>::MIN_BLOCKS)
                                                                : 0.f;
           }
         }
-        mbar_arrive(pbar);
-        ok = mbar_wait_or_abort(pbar, pphase & 1u, &s_abort, lim);
-        pphase ^= 1u;
+        ok = group_sync();
+      }
+      // (the group_sync at the end of the previous pass freed the gradient planes)
+      if (ok) {
+        prod.roberts_and_rows(p, u, nf, np, s);
+        ok = group_sync();
+      }
+      if (ok) {
+        // the input tiles are free: fetch the next pass's frames
+        if (use_tma && leader && fa + FP < f1) fetch(fa + FP);
+        prod.gradients(p, u, np, s);
+        if (!(p.test_withhold_full && iter == 0 && j == 0)) mbar_arrive(&full[s]);
+        ok = group_sync();
       }
       if (!ok) {
         *(volatile int*)&s_abort = 1;
         break;
       }
-      prod.roberts_and_rows(p, u, tin, s);
-      mbar_arrive(pbar);
-      ok = mbar_wait_or_abort(pbar, pphase & 1u, &s_abort, lim);
-      pphase ^= 1u;
-      if (!ok) {
-        *(volatile int*)&s_abort = 1;
-        break;
-      }
-      if (use_tma && leader) {
-        // this set's input buffers are free: fetch the frames two passes ahead
-        fence_proxy_async_smem();
-#pragma unroll
-        for (int fr = 0; fr < FP; ++fr) {
-          const int fn = fa + 2 * FP + fr;
-          const int k = set * FP + fr;
-          if (fn < f1) {
-            mbar_arrive_expect_tx(&tbar[k], kTileBytes);
-            tma_load_3d(prod.inb + k * G::S_INB, tmap, &tbar[k], u.x_start, u.y_start, fn);
-            tpend |= 1u << k;
-          }
-        }
-      }
-      prod.column_pass(p, u);
-      mbar_arrive(pbar);
-      ok = mbar_wait_or_abort(pbar, pphase & 1u, &s_abort, lim);
-      pphase ^= 1u;
-      if (!ok) {
-        *(volatile int*)&s_abort = 1;
-        break;
-      }
-      prod.row_pass(p, u, s);
-      if (!(p.test_withhold_full && iter == 0 && j == 0)) mbar_arrive(&full[s]);
     }
   } else {
     // ======================= consumers ======================================
@@ -947,21 +899,7 @@ __global__ void __launch_bounds__(32 * TY * M + NP, EsrrfTile<M>::MIN_BLOCKS)
         *(volatile int*)&s_abort = 1;
         break;
       }
-      float acc[FP][M];
-      rgc_core<M, J, TY, FP>(sm + G::O_HG + s * G::S_HG, tb4, ty, py, lane, acc);
-
-      // ---- normalise, ^sensitivity, intensity, margin, temporal ------------
-      // magnified intensity of this thread's outputs: column pass of the
-      // Catmull-Rom interpolation from the row-pass values (5 taps per output)
-      const float* ri = sm + G::O_RI + s * FP * G::S_RI;
-      float rv[FP][5];
-      if (p.iw) {
-#pragma unroll
-        for (int fr = 0; fr < FP; ++fr)
-#pragma unroll
-          for (int k = 0; k < 5; ++k) rv[fr][k] = ri[fr * G::S_RI + (ty * M + py) * G::RIW + lane + k];
-      }
-      mbar_arrive(&empty[s]);  // slot s fully read
+      const float* hgf = sm + G::O_HG + s * G::S_HG;
       const bool first = (fa == f0);
       // frame fa + fr is frame k = fa - f0 + fr of this unit's series; 1 / (k + 1)
       // by the fast reciprocal (the increment it scales is a deviation-sized term,
@@ -970,108 +908,162 @@ __global__ void __launch_bounds__(32 * TY * M + NP, EsrrfTile<M>::MIN_BLOCKS)
 #pragma unroll
       for (int fr = 0; fr < FP; ++fr) inv_n[fr] = __fdividef(1.0f, (float)(fa - f0 + fr + 1));
 #pragma unroll
+      for (int d = 0; d < PYT; ++d) {
+      const int py = py0 + d, yM = ny * M + py;
+      float2 acc[G::NPR][M];
+      if (G::NPR == 1 || nf > 2) {
+        rgc_core<G, M, J, G::NPR>(hgf, tb4, ty, py, lane, acc);
+      } else {  // the last pass of a chunk may hold one frame pair only
+        float2 acc1[1][M];
+        rgc_core<G, M, J, 1>(hgf, tb4, ty, py, lane, acc1);
+#pragma unroll
+        for (int px = 0; px < M; ++px) {
+          acc[0][px] = acc1[0][px];
+#pragma unroll
+          for (int pp = 1; pp < G::NPR; ++pp) acc[pp][px] = make_float2(0.f, 0.f);
+        }
+      }
+
+      // ---- normalise, ^sensitivity, intensity, margin, temporal ------------
+#pragma unroll
       for (int px = 0; px < M; ++px) {
-        const float twv = tw[px * G::NTC + tid];
-        const bool zero = (omask & (1u << px)) != 0;
-        float base[FP], ival[FP];
+        const float twv = tw[(d * M + px) * G::NTC + tid];
 #pragma unroll
-        for (int fr = 0; fr < FP; ++fr) {
-          base[fr] = acc[fr][px] * twv;
-          base[fr] = (base[fr] < 0.f) ? 0.f : base[fr];
-          ival[fr] = 1.f;
+        for (int pp = 0; pp < G::NPR; ++pp)
+          acc[pp][px] = make_float2(clamp0(acc[pp][px].x * twv), clamp0(acc[pp][px].y * twv));
+      }
+      if (MODE != kModeSum)
+        apply_sens_all(acc, p.sens_mode_k[0], p.sens_int_k[0], p.sens_k[0]);
+      // magnified intensity of this thread's outputs: column pass of the
+      // Catmull-Rom interpolation from the row-pass values (5 taps per output)
+      float2 ival[G::NPR][M];
+      if (p.iw) {
+        float2 rv[G::NPR][5];
+#pragma unroll
+        for (int pp = 0; pp < G::NPR; ++pp) {
+          const float2* ri = reinterpret_cast<const float2*>(
+              sm + G::O_RI + (s * G::NPR + pp) * G::S_RI) + (ty * M + py) * G::RIW + lane;
+#pragma unroll
+          for (int k = 0; k < 5; ++k) rv[pp][k] = ri[k];
         }
-        if (p.iw) {
-          float w5[5];
 #pragma unroll
-          for (int k = 0; k < 5; ++k) w5[k] = cw[(lane * M + px) * 5 + k];
-          if constexpr (FP >= 2) {
+        for (int px = 0; px < M; ++px) {
 #pragma unroll
-            for (int pp = 0; pp < FP / 2; ++pp) {
-              float2 s2 = make_float2(0.f, 0.f);
+          for (int pp = 0; pp < G::NPR; ++pp) ival[pp][px] = make_float2(0.f, 0.f);
 #pragma unroll
-              for (int k = 0; k < 5; ++k)
-                s2 = __ffma2_rn(make_float2(w5[k], w5[k]),
-                                make_float2(rv[2 * pp][k], rv[2 * pp + 1][k]), s2);
-              ival[2 * pp] = s2.x;
-              ival[2 * pp + 1] = s2.y;
-            }
-          } else {
-            float s1 = 0.f;
+          for (int k = 0; k < 5; ++k) {
+            const float w = cw[(lane * M + px) * 5 + k];
 #pragma unroll
-            for (int k = 0; k < 5; ++k) s1 = fmaf(w5[k], rv[0][k], s1);
-            ival[0] = s1;
+            for (int pp = 0; pp < G::NPR; ++pp)
+              ival[pp][px] = __ffma2_rn(make_float2(w, w), rv[pp][k], ival[pp][px]);
+          }
+          if (MODE != kModeSum) {
+#pragma unroll
+            for (int pp = 0; pp < G::NPR; ++pp)
+              acc[pp][px] = __fmul2_rn(acc[pp][px], ival[pp][px]);
           }
         }
-        if (MODE == kModeSum) {
-          // unrolled over the sensitivity slots (a runtime-bounded loop here
-          // made the compiler re-materialise addresses in the RGC core: +14 %
-          // instructions); running mean per sensitivity (Welford)
+      } else if (MODE == kModeSum) {
 #pragma unroll
-          for (int k = 0; k < kMaxSens; ++k) {
-            if (k >= p.n_sens) break;
-            float* ks = tk + (k * M + px) * G::NTC + tid;
-            float mu = first ? 0.f : *ks;
+        for (int px = 0; px < M; ++px)
 #pragma unroll
-            for (int fr = 0; fr < FP; ++fr) {
-              if (fr < nf) {
-                float r = apply_sens(base[fr], p.sens_mode_k[k], p.sens_int_k[k], p.sens_k[k]);
-                r = zero ? 0.f : r * ival[fr];
-                mu = (first && fr == 0) ? r : fmaf(r - mu, inv_n[fr], mu);
-              }
-            }
-            *ks = mu;
-          }
-        } else if (MODE == kModeStack) {
+          for (int pp = 0; pp < G::NPR; ++pp) ival[pp][px] = make_float2(1.f, 1.f);
+      }
+      if (d == PYT - 1) mbar_arrive(&empty[s]);  // slot s fully read
+      // outputs in the margin are 0 whatever their intensity
+      const unsigned zmask = omask >> (d * M) & ((1u << M) - 1u);
+      if (MODE != kModeSum && zmask != 0) {
+#pragma unroll
+        for (int px = 0; px < M; ++px)
+          if (zmask >> px & 1u)
+#pragma unroll
+            for (int pp = 0; pp < G::NPR; ++pp) acc[pp][px] = make_float2(0.f, 0.f);
+      }
+      if (MODE == kModeStack) {
+        if (!(omask >> 31)) {
+          float* o = p.out + (size_t)fa * plane + (size_t)yM * p.colsM + (size_t)nx * M;
 #pragma unroll
           for (int fr = 0; fr < FP; ++fr) {
-            if (fr < nf) {
-              float r = apply_sens(base[fr], p.sens_mode_k[0], p.sens_int_k[0], p.sens_k[0]);
-              r = zero ? 0.f : r * ival[fr];
-              if (!(omask >> 31))
-                p.out[(size_t)(fa + fr) * plane + (size_t)yM * p.colsM + (size_t)nx * M + px] = r;
-            }
+            if (fr < nf)
+#pragma unroll
+              for (int px = 0; px < M; ++px)
+                o[fr * plane + px] = (fr & 1) ? acc[fr / 2][px].y : acc[fr / 2][px].x;
           }
-        } else {
-          float4* st = reinterpret_cast<float4*>(tk) + px * G::NTC + tid;
-          float* stl = tk + 4 * M * G::NTC + px * G::NTC + tid;
-          Moments mo{0.f, 0.f, 0.f, 0.f, 0.f};
+        }
+      } else if (MODE == kModeSum) {
+        // running mean per sensitivity; unrolled over the sensitivity slots (a
+        // runtime-bounded loop here made the compiler re-materialise addresses
+        // in the RGC core: +14 % instructions)
+#pragma unroll
+        for (int k = 0; k < kMaxSens; ++k) {
+          if (k >= p.n_sens) break;
+          const int smode = p.sens_mode_k[k], sint = p.sens_int_k[k];
+          const float sval = p.sens_k[k];
+#pragma unroll
+          for (int px = 0; px < M; ++px) {
+            float* ks = tk + (k * G::NO + d * M + px) * G::NTC + tid;
+            float2 r[G::NPR][1];
+#pragma unroll
+            for (int pp = 0; pp < G::NPR; ++pp) r[pp][0] = acc[pp][px];
+            apply_sens_all(r, smode, sint, sval);
+#pragma unroll
+            for (int pp = 0; pp < G::NPR; ++pp) {
+              r[pp][0] = __fmul2_rn(r[pp][0], ival[pp][px]);
+              if (zmask >> px & 1u) r[pp][0] = make_float2(0.f, 0.f);
+            }
+            float mu = first ? r[0][0].x : *ks;
+#pragma unroll
+            for (int fr = 0; fr < FP; ++fr)
+              if (fr < nf)
+                mu = fmaf(((fr & 1) ? r[fr / 2][0].y : r[fr / 2][0].x) - mu, inv_n[fr], mu);
+            *ks = mu;
+          }
+        }
+      } else {
+#pragma unroll
+        for (int px = 0; px < M; ++px) {
+          const int o = d * M + px;
+          float4* st = reinterpret_cast<float4*>(tk) + o * G::NTC + tid;
+          float* stl = tk + 4 * G::NO * G::NTC + o * G::NTC + tid;
+          Moments mo = moments_start(acc[0][px].x);
           if (!first) {
             const float4 t = *st;
             mo = Moments{t.x, t.y, t.z, t.w, *stl};
           }
 #pragma unroll
-          for (int fr = 0; fr < FP; ++fr) {
-            if (fr < nf) {
-              float r = apply_sens(base[fr], p.sens_mode_k[0], p.sens_int_k[0], p.sens_k[0]);
-              r = zero ? 0.f : r * ival[fr];
-              if (first && fr == 0) mo = moments_start(r);
-              else moments_push(mo, r, inv_n[fr]);
-            }
-          }
+          for (int fr = 0; fr < FP; ++fr)
+            if (fr < nf && !(first && fr == 0))
+              moments_push(mo, (fr & 1) ? acc[fr / 2][px].y : acc[fr / 2][px].x, inv_n[fr]);
           *st = make_float4(mo.mean, mo.m2, mo.c, mo.a);
           *stl = mo.b;
         }
       }
+      }  // output row phases
     }
   }
   if (!producer && s_abort == 0 && MODE != kModeStack && !(omask >> 31)) {
     const size_t plane = (size_t)p.rowsM * p.colsM;
-    float* rec = p.out + (size_t)(tp * p.chunks + chunk) * p.F * plane +
-                 (size_t)yM * p.colsM + (size_t)nx * M;
-    if (MODE == kModeSum) {
-      for (int k = 0; k < p.n_sens; ++k) {
 #pragma unroll
-        for (int px = 0; px < M; ++px) rec[k * plane + px] = tk[(k * M + px) * G::NTC + tid];
-      }
-    } else {
+    for (int d = 0; d < PYT; ++d) {
+      float* rec = p.out + (size_t)(tp * p.chunks + chunk) * p.F * plane +
+                   (size_t)(ny * M + py0 + d) * p.colsM + (size_t)nx * M;
+      if (MODE == kModeSum) {
+        for (int k = 0; k < p.n_sens; ++k) {
 #pragma unroll
-      for (int px = 0; px < M; ++px) {
-        const float4 t = reinterpret_cast<const float4*>(tk)[px * G::NTC + tid];
-        rec[px] = t.x;
-        rec[plane + px] = t.y;
-        rec[2 * plane + px] = t.z;
-        rec[3 * plane + px] = t.w;
-        rec[4 * plane + px] = tk[4 * M * G::NTC + px * G::NTC + tid];
+          for (int px = 0; px < M; ++px)
+            rec[k * plane + px] = tk[(k * G::NO + d * M + px) * G::NTC + tid];
+        }
+      } else {
+#pragma unroll
+        for (int px = 0; px < M; ++px) {
+          const int o = d * M + px;
+          const float4 t = reinterpret_cast<const float4*>(tk)[o * G::NTC + tid];
+          rec[px] = t.x;
+          rec[plane + px] = t.y;
+          rec[2 * plane + px] = t.z;
+          rec[3 * plane + px] = t.w;
+          rec[4 * plane + px] = tk[4 * G::NO * G::NTC + o * G::NTC + tid];
+        }
       }
     }
   }
@@ -1082,8 +1074,7 @@ __global__ void __launch_bounds__(32 * TY * M + NP, EsrrfTile<M>::MIN_BLOCKS)
     // still in flight, then every thread leaves without writing more
     if (producer && prod.ptid == 0 && p.status) atomicOr(p.status, kDevTmaTimeout);
     if (producer && prod.ptid == 0) {
-      for (int k = 0; k < 2 * FP; ++k)
-        if (tpend & (1u << k)) (void)mbar_wait_bounded(&tbar[k], (tphase >> k) & 1u);
+      if (tpend) (void)mbar_wait_bounded(tbar, tphase);
     }
     return;
   }
@@ -1101,7 +1092,7 @@ cudaError_t launch_fused(const UnitTable& ut, const TmapPack& maps, int grid,
                          cudaStream_t stream) {
   using C = FusedCfg<M, J, MODE, V>;
   using G = typename C::G;
-  auto kern = esrrf_fused_kernel<M, J, C::TY, C::FP, MODE, C::NP>;
+  auto kern = esrrf_fused_kernel<M, J, C::TY, C::FP, MODE, C::NP, C::PYT>;
   const size_t smem = G::smem_bytes(MODE, MODE == kModeSum ? ut.ns_cap : 1);
   if (smem > kSmemBudget) return cudaErrorInvalidValue;
   static int attr_done = -1;  // device the attributes were last set for
@@ -1127,7 +1118,7 @@ template <int M, int J, int MODE, int V = 0>
 int fused_occupancy(int ns_cap) {
   using C = FusedCfg<M, J, MODE, V>;
   using G = typename C::G;
-  auto kern = esrrf_fused_kernel<M, J, C::TY, C::FP, MODE, C::NP>;
+  auto kern = esrrf_fused_kernel<M, J, C::TY, C::FP, MODE, C::NP, C::PYT>;
   const size_t smem = G::smem_bytes(MODE, MODE == kModeSum ? ns_cap : 1);
   if (smem > kSmemBudget) return 0;
   // cached per device and sensitivity count (queried once; launches ask per call)
@@ -1156,7 +1147,7 @@ struct FusedGeometry {
 
 template <int M, int J, int V = 0>
 FusedGeometry fused_geometry() {
-  using G = Geo<M, J, EsrrfTile<M, V>::TY, 1>;
+  using G = Geo<M, J, EsrrfTile<M, V>::TY, 2>;
   return FusedGeometry{EsrrfTile<M, V>::TY, G::IX, G::IY, G::BW, G::BH};
 }
 
