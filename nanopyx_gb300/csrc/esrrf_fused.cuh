@@ -73,7 +73,7 @@ struct FusedParams {
   int tiles_y;
   int F;                 // record fields: 5 (VAR/TAC2) or n_sens (AVG: the mean per sensitivity)
   int n_sens;            // AVG mode: sensitivities evaluated on the same RGC (others: 1)
-  int sens_mode_k[kMaxSens];  // 0: none (s <= 1), 1: integer power sens_int_k, 2: powf(sens_k)
+  int sens_mode_k[kMaxSens];  // see apply_sensitivity (common.cuh)
   int sens_int_k[kMaxSens];
   float sens_k[kMaxSens];
   unsigned long long wait_ns;  // bound of every producer/consumer wait (0: kWaitLimitNs)
@@ -119,15 +119,22 @@ struct EsrrfTile {
   // rows per tile: as many consumer warps as the registers allow without
   // spilling
   static constexpr int TY = (M <= 2) ? 8 : (M <= 5 ? 4 : (M == 6 ? 2 : 1));
-  // output row phases per consumer thread
-  static constexpr int PYT = 1;
+  // output row phases per consumer thread: both at m = 2, where a gradient
+  // sample meets only 4 outputs and its loads (shared by the phases of a thread)
+  // fill the shared-memory pipe.  100 x 512 x 512, R = 1.5, VAR: 1.32 ms with
+  // one phase and 384 producer threads, 1.25 ms with two and 256 (384: 1.28,
+  // 512: 1.48).  At m = 3 .. 8 one phase and the threads it gives are better
+  // (m = 3: 0.64 against 0.70 ms, m = 6: 1.09 / 1.44, m = 8: 2.06 / 2.00).
+  static constexpr int PYT = M == 2 ? 2 : 1;
   // producer threads: the preparation per input pixel is the same for every m
-  // while the RGC work grows with m^2, so small m needs more producers.
+  // while the RGC work grows with m^2, so small m needs more producers
+  // (m = 3, 128 / 256 threads: 0.71 / 0.64 ms; m = 4: 0.70 / 0.65 at R = 1 and
+  // 2.20 / 2.23 at R = 2.5; m = 5, 96 / 128 / 160: 6.04 / 5.84 / 6.07).
   // Tile variant V = 1 (instantiated for m = 2, 4, 5) has one producer warp
   // group fewer (m = 5: 3 warps), for the tiling autotuner to weigh against
   // the default on a given batch.
-  static constexpr int NP_DEFAULT = (M <= 2) ? 384 : (M <= 4 ? 256 : 128);
-  static constexpr int NP_ALT = (M <= 2) ? 256 : (M <= 4 ? 128 : 96);
+  static constexpr int NP_DEFAULT = M == 1 ? 384 : (M <= 4 ? 256 : 128);
+  static constexpr int NP_ALT = M == 1 ? 256 : (M <= 4 ? 128 : 96);
   static constexpr int NP = V == 0 ? NP_DEFAULT : NP_ALT;
   // most frames a pass carries (4 where the layout fits shared memory, else 2)
   static constexpr int FP_MAX = 4;
@@ -240,16 +247,6 @@ struct FusedCfg {
 // differently.
 constexpr float kGradScale = 4294967296.f;
 
-__device__ __forceinline__ float apply_sens(float r, int mode, int n, float s) {
-  if (mode == 1) {
-    const float base = r;
-    for (int k = 1; k < n; ++k) r *= base;
-  } else if (mode == 2) {
-    r = powf(r, s);
-  }
-  return r;
-}
-
 // max(v, 0) that keeps a NaN
 __device__ __forceinline__ float clamp0(float v) {
   float r;
@@ -261,13 +258,16 @@ __device__ __forceinline__ float clamp0(float v) {
 template <int A, int B>
 __device__ __forceinline__ void apply_sens_all(float2 (&r)[A][B], int mode, int n, float s) {
   if (mode == 0) return;
-  if (mode == 1 && n <= 3) {
+  if (mode != 2 && n <= 3) {
+    // n = 1 .. 3, times the square root for a half-integer power
 #pragma unroll
     for (int i = 0; i < A; ++i)
 #pragma unroll
       for (int j = 0; j < B; ++j) {
-        const float2 q = __fmul2_rn(r[i][j], r[i][j]);
-        r[i][j] = n == 3 ? __fmul2_rn(q, r[i][j]) : q;
+        const float2 b = r[i][j], q = __fmul2_rn(b, b);
+        float2 v = n == 1 ? b : (n == 3 ? __fmul2_rn(q, b) : q);
+        if (mode == 3) v = __fmul2_rn(v, make_float2(__fsqrt_rn(b.x), __fsqrt_rn(b.y)));
+        r[i][j] = v;
       }
     return;
   }
@@ -275,7 +275,8 @@ __device__ __forceinline__ void apply_sens_all(float2 (&r)[A][B], int mode, int 
   for (int i = 0; i < A; ++i)
 #pragma unroll
     for (int j = 0; j < B; ++j)
-      r[i][j] = make_float2(apply_sens(r[i][j].x, mode, n, s), apply_sens(r[i][j].y, mode, n, s));
+      r[i][j] = make_float2(apply_sensitivity(r[i][j].x, mode, n, s),
+                            apply_sensitivity(r[i][j].y, mode, n, s));
 }
 
 // geometry of one unit (tile, timepoint, frame chunk), shared by both roles
@@ -523,23 +524,38 @@ __device__ __forceinline__ void rgc_sample(const float4& g, float rho, float nrh
 // have the same weight and |a| and opposite rho.  Walking q from both ends loads
 // (J + 1) M + M / 2 entries per window row instead of M (2J + 1) (m = 5,
 // R = 1.5: 20 used for 35 samples).
+//
+// The phases of a thread share every gradient load (LDS.128, four wavefronts a
+// warp) of a half-grid row.  Phases of the lower half of a pixel (cpy = 0) use
+// row k as window row k, those of the upper half (cpy = 1) as window row k - 1;
+// with both in one thread (PYT = M) the first and the last row serve one half.
 template <typename G, int M, int J, int NPR>
-__device__ __forceinline__ void rgc_core(const float* hgf, const float4* tb4, int ty, int py,
-                                         int lane, float2 (&acc)[NPR][M]) {
-  const int cpy = (2 * py + 1) / M;
-  const float4* hg = reinterpret_cast<const float4*>(hgf);
-#pragma unroll
-  for (int pp = 0; pp < NPR; ++pp)
-#pragma unroll
-    for (int px = 0; px < M; ++px) acc[pp][px] = make_float2(0.f, 0.f);
-  // window rows stay a loop: unrolled, the core's code outgrows the
-  // instruction cache (measured 2 % slower and with register spills)
-#pragma unroll 1
-  for (int jj = 0; jj < G::W2; ++jj) {
-    const int kyl = 2 * ty + cpy + jj;
-    const float4* r0 = hg + (kyl * 2 + 0) * G::HGP + lane;
-    const float4* r1 = hg + (kyl * 2 + 1) * G::HGP + lane;
-    const float4* tb = tb4 + (size_t)(py * G::W2 + jj) * G::NE;
+struct RgcCore {
+  static constexpr int PYT = G::PYT;
+  const float4* hg;   // this lane's first sample of row 2 ty
+  const float4* tb4;  // phase table of row phase py0
+  int cpy;            // of every phase of the thread unless PYT = M
+
+  // row k of the slot (rows from 2 ty on) for the phases d0 .. d1 - 1
+  template <int D0, int D1>
+  __device__ __forceinline__ void row(int k, float2 (&acc)[NPR][PYT * M]) const {
+    const float4* r0 = hg + (k * 2 + 0) * G::HGP;
+    const float4* r1 = hg + (k * 2 + 1) * G::HGP;
+    auto grad = [&](int pp, int q) {
+      return (q & 1) ? r1[pp * G::HG_PLANE + (q >> 1)] : r0[pp * G::HG_PLANE + (q >> 1)];
+    };
+    // window row of phase d: k - cpy(d)
+    auto table = [&](int d) {
+      const int c = PYT == M ? (2 * d + 1) / M : cpy;
+      return tb4 + (d * G::W2 + k - c) * G::NE;
+    };
+    auto sample = [&](int px, int q, const float4& g, float rho, float nrho, const float4& T,
+                      float2& a) {
+      const int dxn = dx_num<M, J>(px, q);
+      if (dxn > 0) rgc_sample<1>(g, rho, nrho, T.z, T.w, a);
+      else if (dxn < 0) rgc_sample<-1>(g, rho, nrho, T.z, T.w, a);
+      else rgc_sample<0>(g, rho, nrho, T.z, T.w, a);
+    };
     if constexpr (M <= 2) {
       // gradient-major order: one half-grid sample at a time, applied to every
       // output phase px whose window holds it
@@ -547,27 +563,19 @@ __device__ __forceinline__ void rgc_core(const float* hgf, const float4* tb4, in
       for (int q = 0; q < G::NQ; ++q) {
         float4 g[NPR];
 #pragma unroll
-        for (int pp = 0; pp < NPR; ++pp)
-          g[pp] = (q & 1) ? r1[pp * G::HG_PLANE + (q >> 1)] : r0[pp * G::HG_PLANE + (q >> 1)];
+        for (int pp = 0; pp < NPR; ++pp) g[pp] = grad(pp, q);
 #pragma unroll
-        for (int px = 0; px < M; ++px) {
-          if (!in_window<M, J>(px, q)) continue;
-          // entry (rho, -rho, -|a|, w) of this sample, or of its mirror image
-          const bool own = q <= J || (q == J + 1 && 2 * px < M);
-          const float4 T = own ? tb[q * M + px] : tb[(G::NQ - q) * M + M - 1 - px];
-          const float rho = own ? T.x : T.y, nrho = own ? T.y : T.x;
-          const int dxn = dx_num<M, J>(px, q);
+        for (int d = D0; d < D1; ++d)
 #pragma unroll
-          for (int pp = 0; pp < NPR; ++pp) {
-            if (dxn > 0) {
-              rgc_sample<1>(g[pp], rho, nrho, T.z, T.w, acc[pp][px]);
-            } else if (dxn < 0) {
-              rgc_sample<-1>(g[pp], rho, nrho, T.z, T.w, acc[pp][px]);
-            } else {
-              rgc_sample<0>(g[pp], T.x, 0.f, T.z, T.w, acc[pp][px]);
-            }
+          for (int px = 0; px < M; ++px) {
+            if (!in_window<M, J>(px, q)) continue;
+            // entry (rho, -rho, -|a|, w) of this sample, or of its mirror image
+            const bool own = q <= J || (q == J + 1 && 2 * px < M);
+            const float4 T = table(d)[own ? q * M + px : (G::NQ - q) * M + M - 1 - px];
+#pragma unroll
+            for (int pp = 0; pp < NPR; ++pp)
+              sample(px, q, g[pp], own ? T.x : T.y, own ? T.y : T.x, T, acc[pp][d * M + px]);
           }
-        }
       }
     } else {
 #pragma unroll
@@ -576,37 +584,47 @@ __device__ __forceinline__ void rgc_core(const float* hgf, const float4* tb4, in
         float4 ga[NPR], gb[NPR];
 #pragma unroll
         for (int pp = 0; pp < NPR; ++pp) {
-          ga[pp] = (q & 1) ? r1[pp * G::HG_PLANE + (q >> 1)] : r0[pp * G::HG_PLANE + (q >> 1)];
-          gb[pp] = ga[pp];
-          if (q >= 1 && qm != q)
-            gb[pp] = (qm & 1) ? r1[pp * G::HG_PLANE + (qm >> 1)]
-                              : r0[pp * G::HG_PLANE + (qm >> 1)];
+          ga[pp] = grad(pp, q);
+          gb[pp] = (q >= 1 && qm != q) ? grad(pp, qm) : ga[pp];
         }
 #pragma unroll
-        for (int px = 0; px < (q == J + 1 ? (M + 1) / 2 : M); ++px) {
-          const int pm = M - 1 - px;
-          const bool use_a = in_window<M, J>(px, q);
-          const bool use_b = q >= 1 && (q != qm || px != pm) && in_window<M, J>(pm, qm);
-          if (!use_a && !use_b) continue;
-          const float4 T = tb[q * M + px];  // (rho, -rho, -|a|, w) of (px, q)
-          const int dxn = dx_num<M, J>(px, q);
+        for (int d = D0; d < D1; ++d)
 #pragma unroll
-          for (int pp = 0; pp < NPR; ++pp) {
-            if (dxn > 0) {
-              if (use_a) rgc_sample<1>(ga[pp], T.x, T.y, T.z, T.w, acc[pp][px]);
-              if (use_b) rgc_sample<-1>(gb[pp], T.y, T.x, T.z, T.w, acc[pp][pm]);
-            } else if (dxn < 0) {
-              if (use_a) rgc_sample<-1>(ga[pp], T.x, T.y, T.z, T.w, acc[pp][px]);
-              if (use_b) rgc_sample<1>(gb[pp], T.y, T.x, T.z, T.w, acc[pp][pm]);
-            } else {
-              rgc_sample<0>(ga[pp], T.x, 0.f, T.z, T.w, acc[pp][px]);
+          for (int px = 0; px < (q == J + 1 ? (M + 1) / 2 : M); ++px) {
+            const int pm = M - 1 - px;
+            const bool use_a = in_window<M, J>(px, q);
+            const bool use_b = q >= 1 && (q != qm || px != pm) && in_window<M, J>(pm, qm);
+            if (!use_a && !use_b) continue;
+            const float4 T = table(d)[q * M + px];  // (rho, -rho, -|a|, w) of (px, q)
+#pragma unroll
+            for (int pp = 0; pp < NPR; ++pp) {
+              if (use_a) sample(px, q, ga[pp], T.x, T.y, T, acc[pp][d * M + px]);
+              if (use_b) sample(pm, qm, gb[pp], T.y, T.x, T, acc[pp][d * M + pm]);
             }
           }
-        }
       }
     }
   }
-}
+
+  __device__ __forceinline__ void run(float2 (&acc)[NPR][PYT * M]) const {
+#pragma unroll
+    for (int pp = 0; pp < NPR; ++pp)
+#pragma unroll
+      for (int o = 0; o < PYT * M; ++o) acc[pp][o] = make_float2(0.f, 0.f);
+    // window rows stay a loop: unrolled, the core's code outgrows the
+    // instruction cache (measured 2 % slower and with register spills)
+    if constexpr (PYT == M && M > 1) {
+      constexpr int DH = M / 2;  // phases d < DH have cpy = 0
+      row<0, DH>(0, acc);
+#pragma unroll 1
+      for (int k = 1; k < G::NQ - 1; ++k) row<0, M>(k, acc);
+      row<DH, M>(G::NQ - 1, acc);
+    } else {
+#pragma unroll 1
+      for (int k = cpy; k < cpy + G::W2; ++k) row<0, PYT>(k, acc);
+    }
+  }
+};
 
 template <int M, int J, int TY, int FP, int MODE, int NP, int PYT>
 __global__ void __launch_bounds__(32 * TY * (M / PYT) + NP, EsrrfTile<M>::MIN_BLOCKS)
@@ -632,7 +650,7 @@ __global__ void __launch_bounds__(32 * TY * (M / PYT) + NP, EsrrfTile<M>::MIN_BL
   const int lane = tid & 31;
   const int warp = tid >> 5;
   const int ty = warp % TY;  // consumers
-  const int py0 = warp / TY * PYT;
+  const int py0 = PYT == M ? 0 : warp / TY * PYT;
   const Producer<G, M, J> prod{sm + G::O_INB, sm + G::O_G, sm + G::O_HG,
                                sm + G::O_RI, rw, tid - G::NTC};
 
@@ -907,33 +925,38 @@ __global__ void __launch_bounds__(32 * TY * (M / PYT) + NP, EsrrfTile<M>::MIN_BL
       float inv_n[FP];
 #pragma unroll
       for (int fr = 0; fr < FP; ++fr) inv_n[fr] = __fdividef(1.0f, (float)(fa - f0 + fr + 1));
+      float2 acc[G::NPR][G::NO];
+      {
+        const int cpy = PYT == M ? (M > 1 ? 0 : 1) : (2 * py0 + 1) / M;
+        const float4* g0 = reinterpret_cast<const float4*>(hgf) + 4 * ty * G::HGP + lane;
+        const float4* t0 = tb4 + py0 * G::W2 * G::NE;
+        if (G::NPR == 1 || nf > 2) {
+          RgcCore<G, M, J, G::NPR>{g0, t0, cpy}.run(acc);
+        } else {  // the last pass of a chunk may hold one frame pair only
+          float2 acc1[1][G::NO];
+          RgcCore<G, M, J, 1>{g0, t0, cpy}.run(acc1);
 #pragma unroll
-      for (int d = 0; d < PYT; ++d) {
-      const int py = py0 + d, yM = ny * M + py;
-      float2 acc[G::NPR][M];
-      if (G::NPR == 1 || nf > 2) {
-        rgc_core<G, M, J, G::NPR>(hgf, tb4, ty, py, lane, acc);
-      } else {  // the last pass of a chunk may hold one frame pair only
-        float2 acc1[1][M];
-        rgc_core<G, M, J, 1>(hgf, tb4, ty, py, lane, acc1);
+          for (int o = 0; o < G::NO; ++o) {
+            acc[0][o] = acc1[0][o];
 #pragma unroll
-        for (int px = 0; px < M; ++px) {
-          acc[0][px] = acc1[0][px];
-#pragma unroll
-          for (int pp = 1; pp < G::NPR; ++pp) acc[pp][px] = make_float2(0.f, 0.f);
+            for (int pp = 1; pp < G::NPR; ++pp) acc[pp][o] = make_float2(0.f, 0.f);
+          }
         }
       }
 
       // ---- normalise, ^sensitivity, intensity, margin, temporal ------------
 #pragma unroll
-      for (int px = 0; px < M; ++px) {
-        const float twv = tw[(d * M + px) * G::NTC + tid];
+      for (int o = 0; o < G::NO; ++o) {
+        const float twv = tw[o * G::NTC + tid];
 #pragma unroll
         for (int pp = 0; pp < G::NPR; ++pp)
-          acc[pp][px] = make_float2(clamp0(acc[pp][px].x * twv), clamp0(acc[pp][px].y * twv));
+          acc[pp][o] = make_float2(clamp0(acc[pp][o].x * twv), clamp0(acc[pp][o].y * twv));
       }
       if (MODE != kModeSum)
         apply_sens_all(acc, p.sens_mode_k[0], p.sens_int_k[0], p.sens_k[0]);
+#pragma unroll
+      for (int d = 0; d < PYT; ++d) {
+      const int py = py0 + d, yM = ny * M + py;
       // magnified intensity of this thread's outputs: column pass of the
       // Catmull-Rom interpolation from the row-pass values (5 taps per output)
       float2 ival[G::NPR][M];
@@ -960,7 +983,7 @@ __global__ void __launch_bounds__(32 * TY * (M / PYT) + NP, EsrrfTile<M>::MIN_BL
           if (MODE != kModeSum) {
 #pragma unroll
             for (int pp = 0; pp < G::NPR; ++pp)
-              acc[pp][px] = __fmul2_rn(acc[pp][px], ival[pp][px]);
+              acc[pp][d * M + px] = __fmul2_rn(acc[pp][d * M + px], ival[pp][px]);
           }
         }
       } else if (MODE == kModeSum) {
@@ -977,7 +1000,7 @@ __global__ void __launch_bounds__(32 * TY * (M / PYT) + NP, EsrrfTile<M>::MIN_BL
         for (int px = 0; px < M; ++px)
           if (zmask >> px & 1u)
 #pragma unroll
-            for (int pp = 0; pp < G::NPR; ++pp) acc[pp][px] = make_float2(0.f, 0.f);
+            for (int pp = 0; pp < G::NPR; ++pp) acc[pp][d * M + px] = make_float2(0.f, 0.f);
       }
       if (MODE == kModeStack) {
         if (!(omask >> 31)) {
@@ -987,7 +1010,7 @@ __global__ void __launch_bounds__(32 * TY * (M / PYT) + NP, EsrrfTile<M>::MIN_BL
             if (fr < nf)
 #pragma unroll
               for (int px = 0; px < M; ++px)
-                o[fr * plane + px] = (fr & 1) ? acc[fr / 2][px].y : acc[fr / 2][px].x;
+                o[fr * plane + px] = (fr & 1) ? acc[fr / 2][d * M + px].y : acc[fr / 2][d * M + px].x;
           }
         }
       } else if (MODE == kModeSum) {
@@ -1004,7 +1027,7 @@ __global__ void __launch_bounds__(32 * TY * (M / PYT) + NP, EsrrfTile<M>::MIN_BL
             float* ks = tk + (k * G::NO + d * M + px) * G::NTC + tid;
             float2 r[G::NPR][1];
 #pragma unroll
-            for (int pp = 0; pp < G::NPR; ++pp) r[pp][0] = acc[pp][px];
+            for (int pp = 0; pp < G::NPR; ++pp) r[pp][0] = acc[pp][d * M + px];
             apply_sens_all(r, smode, sint, sval);
 #pragma unroll
             for (int pp = 0; pp < G::NPR; ++pp) {
@@ -1025,7 +1048,7 @@ __global__ void __launch_bounds__(32 * TY * (M / PYT) + NP, EsrrfTile<M>::MIN_BL
           const int o = d * M + px;
           float4* st = reinterpret_cast<float4*>(tk) + o * G::NTC + tid;
           float* stl = tk + 4 * G::NO * G::NTC + o * G::NTC + tid;
-          Moments mo = moments_start(acc[0][px].x);
+          Moments mo = moments_start(acc[0][o].x);
           if (!first) {
             const float4 t = *st;
             mo = Moments{t.x, t.y, t.z, t.w, *stl};
@@ -1033,7 +1056,7 @@ __global__ void __launch_bounds__(32 * TY * (M / PYT) + NP, EsrrfTile<M>::MIN_BL
 #pragma unroll
           for (int fr = 0; fr < FP; ++fr)
             if (fr < nf && !(first && fr == 0))
-              moments_push(mo, (fr & 1) ? acc[fr / 2][px].y : acc[fr / 2][px].x, inv_n[fr]);
+              moments_push(mo, (fr & 1) ? acc[fr / 2][o].y : acc[fr / 2][o].x, inv_n[fr]);
           *st = make_float4(mo.mean, mo.m2, mo.c, mo.a);
           *stl = mo.b;
         }

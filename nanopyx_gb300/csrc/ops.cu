@@ -219,16 +219,6 @@ __global__ void roberts_cross_kernel(const float* __restrict__ in, int T, int H,
   }
 }
 
-__device__ __forceinline__ float apply_sensitivity(float r, int mode, int n, float s) {
-  if (mode == 1) {
-    const float base = r;
-    for (int k = 1; k < n; ++k) r *= base;
-  } else if (mode == 2) {
-    r = powf(r, s);
-  }
-  return r;
-}
-
 // _c_calculate_rgc (src/include/_c_sr_radial_gradient_convergence.c:17-90) per
 // output pixel, float32 as the reference (the FP64 distance weight is
 // evaluated in float), reading the given 2m-magnified gradient images.
@@ -793,6 +783,9 @@ RgcScalars rgc_scalars(int M, float radius, float sensitivity, int pad_edges) {
     sc.sens_mode = 0;
   } else if (sensitivity == std::floor(sensitivity) && sensitivity <= 16.0f) {
     sc.sens_mode = 1;
+    sc.sens_int = (int)sensitivity;
+  } else if (sensitivity - 0.5f == std::floor(sensitivity) && sensitivity <= 16.0f) {
+    sc.sens_mode = 3;
     sc.sens_int = (int)sensitivity;
   } else {
     sc.sens_mode = 2;
