@@ -639,16 +639,11 @@ int nx_esrrf_run_stage2(const nx_esrrf_plan* p, int T, int fpt, int corr_mask, i
     cur += align256(generic_frame_floats(p) * sizeof(float));
   }
   float* map = (float*)cur;
-  for (int tp = 0; tp < n_tp; ++tp) {
-    const int nf = std::min(fpt, T - tp * fpt);
-    const int nch = std::min(chunks, nf);
-    cudaError_t e = launch_finalize(rec + (size_t)tp * chunks * Fr * planeM, Fr, nch, nf, planeM,
-                                    corr_mask, d_out + (size_t)tp * planeM,
-                                    (long long)n_tp * planeM, Fr == 5, s);
-    if (e != cudaSuccess) return cuda_status(e, "temporal finalize");
-  }
+  cudaError_t e = launch_finalize(rec, Fr, chunks, T, fpt, n_tp, planeM, corr_mask, d_out,
+                                  (long long)n_tp * planeM, Fr == 5, s);
+  if (e != cudaSuccess) return cuda_status(e, "temporal finalize");
   if (mpc) {
-    cudaError_t e = launch_mpc(d_out, ncorr * n_tp, p->rowsM, p->colsM, p->M, map, s);
+    e = launch_mpc(d_out, ncorr * n_tp, p->rowsM, p->colsM, p->M, map, s);
     if (e != cudaSuccess) return cuda_status(e, "macro-pixel correction");
   }
   return NX_OK;
@@ -736,8 +731,8 @@ int nx_esrrf_accum_finalize(const nx_esrrf_plan* p, const void* d_accum, int tot
   }
   cudaStream_t s = (cudaStream_t)stream;
   const long long planeM = (long long)p->rowsM * p->colsM;
-  cudaError_t e = launch_finalize((const float*)d_accum, 5, 1, total_frames, planeM, corr_mask,
-                                  d_out, planeM, true, s);
+  cudaError_t e = launch_finalize((const float*)d_accum, 5, 1, total_frames, total_frames, 1,
+                                  planeM, corr_mask, d_out, planeM, true, s);
   if (e != cudaSuccess) return cuda_status(e, "temporal finalize");
   if (mpc) {
     float* map = (float*)((char*)d_ws + kStatusBytes);

@@ -78,8 +78,6 @@ cudaError_t launch_record_push_frame(const float* frame, long long n, float* rec
                                      cudaStream_t s);
 cudaError_t launch_record_merge(float* acc, const float* blk, long long n, int n_acc, int n_blk,
                                 cudaStream_t s);
-// combine `nchunks` consecutive records (each F planes) of one timepoint with frame
-// counts derived from nf, and write the correlations of corr_mask to out[ci*out_stride]
 // one temporal finalisation of a batch: the chunk records of one timepoint
 // (rec, F fields, nchunks chunks over nf frames, n pixels) -> the output
 // planes at out (out_stride apart), VAR/TAC2/AVG per corr_mask, or the mean
@@ -94,9 +92,11 @@ struct FinalizeJob {
 // its blocks)
 cudaError_t launch_finalize_jobs(const FinalizeJob* jobs, int njobs, int total_blocks,
                                  cudaStream_t s);
-cudaError_t launch_finalize(const float* rec, int F, int nchunks, int nf, long long n,
-                            int corr_mask, float* out, long long out_stride, bool full,
-                            cudaStream_t s);
+// every timepoint (fpt frames, the last one what is left of T) in one launch:
+// `chunks` records of F planes per timepoint -> out[ci*out_stride + tp*n]
+cudaError_t launch_finalize(const float* rec, int F, int chunks, int T, int fpt, int n_tp,
+                            long long n, int corr_mask, float* out, long long out_stride,
+                            bool full, cudaStream_t s);
 cudaError_t launch_temporal_stack(const float* stack, int T, long long n, int corr, float* out,
                                   cudaStream_t s);
 cudaError_t launch_srrf_temporal(const float* stack, int T, long long n, int order, float* out,
