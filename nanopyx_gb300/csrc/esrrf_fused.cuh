@@ -101,13 +101,6 @@ struct UnitTable {
   FusedParams single;
 };
 
-template <int M>
-struct TileRows {
-  // input-pixel rows per CTA tile (32*TY*M threads <= 640); measured: TY = 4 beats
-  // TY = 2 at m = 5 by 4 % despite one CTA per SM (less halo work per pixel)
-  static constexpr int TY = (M <= 2) ? 8 : (M <= 5 ? 4 : 2);
-};
-
 // Warp roles of the eSRRF kernel.  Each CTA runs 32 * TY * M / PYT consumer
 // threads (one per input pixel and PYT output row phases: RGC, normalisation,
 // temporal update) and producer warps that prepare the gradient and intensity

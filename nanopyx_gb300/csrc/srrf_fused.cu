@@ -11,6 +11,13 @@
 // the tap rows / columns and Catmull-Rom weights of every (output row, ring
 // point) and (output column, ring point) are tabulated once per tile in shared
 // memory, in the reference's own float32 arithmetic (x0 rounded, x0 / m IEEE).
+//
+// What bounds it: shared-memory wavefronts (column weights and row sums, 64 % of
+// the pipe) and issue (60 %).  100 x 256 x 256, m = 5, ring 0.5 px: one frame a
+// pass, all 12 row passes at once 4.98 ms; frame pairs on packed arithmetic with
+// the row passes in groups 2.94; tile rows per magnification and chunks that fill
+// the last wave 2.86; the next pass's input loaded behind the ring points 2.71;
+// no comparisons in the ring sum 2.65.
 #include <algorithm>
 #include <cstring>
 
@@ -24,23 +31,34 @@ namespace {
 constexpr int kRing = 12;
 constexpr int kHalo = 5;  // input rows/cols around the tile: ring radius <= 2 px
 
+// Two consecutive frames per pass: the interpolation weights, ring tables and
+// offsets of a pass serve both, and the arithmetic runs on packed f32x2 (the
+// same IEEE operations per frame).
 template <int M>
 struct SrrfTile {
-  // tile rows: the eSRRF kernel's, except m = 5, where 6 rows (960 threads,
-  // 64 registers, no spills) measured 2.5 % faster than 4 (640 threads, 95
-  // registers) on the 500 x 512 x 512 stack: more warps hide the shared loads
-  static constexpr int TY = (M == 5) ? 6 : TileRows<M>::TY;
+  // tile rows, measured (100 x 256 x 256; m = 6, 8: 50 frames): m = 2: 4 / 8 / 12
+  // rows 0.68 / 0.83 / 0.77 ms; m = 3: 2 / 4 / 8 rows 1.34 / 1.54 / 1.25; m = 4:
+  // 2 / 4 / 6 rows 2.06 / 2.13 / 1.96; m = 5: 3 / 4 / 5 / 6 rows 3.13 / 2.86 /
+  // 3.15 / 2.94; m = 6: 1 / 2 / 4 rows 2.48 / 2.55 / 1.97; m = 8: 1 / 2 / 3 rows
+  // 3.68 / 3.49 / 3.69
+  static constexpr int TY =
+      M == 2 ? 4 : M == 3 ? 8 : M == 4 ? 6 : M == 5 ? 4 : M == 6 ? 4 : 2;
   static constexpr int TX = 32;
   static constexpr int NT = 32 * TY * M;
   static constexpr int IH = TY + 2 * kHalo;  // input tile rows
   static constexpr int IW = TX + 2 * kHalo;
   static constexpr int OY = TY * M, OX = TX * M;
   static constexpr int RIW = TX + 4;
+  // ring points whose row pass is formed at a time: the buffer of a warp is 1.3 KB
+  // instead of 8 for all 12 (100 x 256 x 256, m = 5: 2 / 3 / 4 points 2.71 / 2.78 /
+  // 2.89 ms)
+  static constexpr int RG = 2;
   static constexpr int al(int n) { return (n + 31) / 32 * 32; }
-  static constexpr int O_IN = 0;                        // input tile
-  static constexpr int O_G = O_IN + al(IH * IW);        // gradient float2 (gx, gy)
-  static constexpr int O_RI = O_G + al(IH * IW * 2);    // intensity row pass
-  static constexpr int O_RW = O_RI + al(OY * RIW);      // intensity row weights [OY][5]
+  static constexpr int O_IN = 0;                        // input tiles (2 frames)
+  static constexpr int S_IN = al(IH * IW);
+  static constexpr int O_G = O_IN + 2 * S_IN;           // gradients float4 (gx, gx', gy, gy')
+  static constexpr int O_RI = O_G + al(IH * IW * 4);    // intensity row pass float2 (v, v')
+  static constexpr int O_RW = O_RI + al(OY * RIW * 2);  // intensity row weights [OY][5]
   static constexpr int O_CW = O_RW + al(OY * 5);        // intensity col weights [OX][5]
   static constexpr int O_RT = O_CW + al(OX * 5);        // ring row taps [OY][12][8]
   // ring column taps of output column (lane, px) as 5 weights on the columns
@@ -50,9 +68,9 @@ struct SrrfTile {
   static constexpr int O_CW4 = O_RT + al(OY * kRing * 8);
   static constexpr int O_CW1 = O_CW4 + al(kRing * M * TX * 4);
   static constexpr int O_CB = O_CW1 + al(kRing * M * TX);  // [ring][lane] int: cb - x_start
-  // per-warp row pass of the gradient interpolation: [warp][ring][IW] float2,
-  // plus one zeroed float2 after the last ring (read with weight 0)
-  static constexpr int RBW = kRing * IW * 2 + 2;
+  // per-warp row pass of the gradient interpolation: [ring of the group][IW]
+  // float4, plus one zeroed float4 after the last (read with weight 0)
+  static constexpr int RBW = (RG * IW + 1) * 4;
   static constexpr int O_RB = O_CB + al(kRing * TX);
   static constexpr int FLOATS = O_RB + (NT / 32) * RBW;
   static constexpr size_t SMEM = size_t(FLOATS) * 4;
@@ -85,21 +103,28 @@ __device__ __forceinline__ void ring_entry(float* e, float c, float ring, int M,
   e[7] = 0.f;
 }
 
+constexpr float kTiny = 1.17549435e-38f;  // 2^-126
+
+// v >= 0 with the sign opposite to d's
+__device__ __forceinline__ float against(float v, float d) {
+  return __int_as_float(__float_as_int(v) ^ (~__float_as_int(d) & 0x80000000));
+}
+
 template <int M>
 __global__ void __launch_bounds__(SrrfTile<M>::NT, 1) srrf_fused_kernel(const SrrfParams p) {
   using G = SrrfTile<M>;
   constexpr int TY = G::TY;
   extern __shared__ __align__(128) float sm[];
   float* tin = sm + G::O_IN;
-  float2* grad = reinterpret_cast<float2*>(sm + G::O_G);
-  float* ri = sm + G::O_RI;
+  float4* grad = reinterpret_cast<float4*>(sm + G::O_G);
+  float2* ri = reinterpret_cast<float2*>(sm + G::O_RI);
   float* rw = sm + G::O_RW;
   float* cw = sm + G::O_CW;
   float* rt = sm + G::O_RT;
   float4* cw4 = reinterpret_cast<float4*>(sm + G::O_CW4);
   float* cw1 = sm + G::O_CW1;
   int* cbt = reinterpret_cast<int*>(sm + G::O_CB);
-  float2* rb = reinterpret_cast<float2*>(sm + G::O_RB + (threadIdx.x >> 5) * G::RBW);
+  float4* rb = reinterpret_cast<float4*>(sm + G::O_RB + (threadIdx.x >> 5) * G::RBW);
 
   const int tid = threadIdx.x;
   const int lane = tid & 31;
@@ -107,8 +132,10 @@ __global__ void __launch_bounds__(SrrfTile<M>::NT, 1) srrf_fused_kernel(const Sr
   const int ty = warp % TY;
   const int py = warp / TY;
   const int tile = blockIdx.x;
-  const int f_begin = (int)((long long)blockIdx.y * p.T / p.chunks);
-  const int f_end = (int)((long long)(blockIdx.y + 1) * p.T / p.chunks);
+  // chunks of whole frame pairs (the last pair may be one frame)
+  const int pairs = (p.T + 1) / 2;
+  const int f_begin = 2 * (int)((long long)blockIdx.y * pairs / p.chunks);
+  const int f_end = min(p.T, 2 * (int)((long long)(blockIdx.y + 1) * pairs / p.chunks));
   const int nx0 = (tile % p.tiles_x) * G::TX;
   const int ny0 = (tile / p.tiles_x) * TY;
   const int h = p.h, w = p.w;
@@ -172,7 +199,7 @@ __global__ void __launch_bounds__(SrrfTile<M>::NT, 1) srrf_fused_kernel(const Sr
     }
     cbt[s * G::TX + ln] = cb - x_start;
   }
-  if ((tid & 31) == 0) rb[kRing * G::IW] = make_float2(0.f, 0.f);
+  if ((tid & 31) == 0) rb[G::RG * G::IW] = make_float4(0.f, 0.f, 0.f, 0.f);
 
   const int ny = ny0 + ty, nx = nx0 + lane;
   const int j = ny * M + py;  // output row
@@ -183,23 +210,48 @@ __global__ void __launch_bounds__(SrrfTile<M>::NT, 1) srrf_fused_kernel(const Sr
   const size_t plane = (size_t)rowsM * colsM;
 
   const bool own_intensity = p.interp == nullptr;
-  for (int f = f_begin; f < f_end; ++f) {
-    __syncthreads();  // tables ready / previous frame's shared data consumed
+  // the next pass's input values, loaded while the current pass computes
+  constexpr int NPF = (G::IH * G::IW + G::NT - 1) / G::NT;
+  float2 pf[NPF];
+  auto fetch = [&](int f) {
     const float* src = p.in + (size_t)f * h * w;
-    for (int i = tid; i < G::IH * G::IW; i += G::NT) {
+    const float* src1 = f + 1 < f_end ? src + (size_t)h * w : src;
+#pragma unroll
+    for (int k = 0; k < NPF; ++k) {
+      const int i = tid + k * G::NT;
       const int r = y_start + i / G::IW, c = x_start + i % G::IW;
-      tin[i] = (r >= 0 && r < h && c >= 0 && c < w) ? __ldg(src + (size_t)r * w + c) : 0.f;
+      const bool in = i < G::IH * G::IW && r >= 0 && r < h && c >= 0 && c < w;
+      const size_t o = (size_t)r * w + c;
+      pf[k] = in ? make_float2(__ldg(src + o), __ldg(src1 + o)) : make_float2(0.f, 0.f);
     }
+  };
+  if (f_begin < f_end) fetch(f_begin);
+  for (int f = f_begin; f < f_end; f += 2) {
+    const bool two = f + 1 < f_end;  // an odd last frame stands in for its partner
+    __syncthreads();  // tables ready / previous pass's shared data consumed
+#pragma unroll
+    for (int k = 0; k < NPF; ++k) {
+      const int i = tid + k * G::NT;
+      if (i < G::IH * G::IW) {
+        tin[i] = pf[k].x;
+        tin[G::S_IN + i] = pf[k].y;
+      }
+    }
+    if (f + 2 < f_end) fetch(f + 2);
     __syncthreads();
     // gradients (zero outside rows/cols 1..n-2) and the intensity row pass
     for (int i = tid; i < G::IH * G::IW; i += G::NT) {
       const int rl = i / G::IW, cl = i % G::IW;
       const int r = y_start + rl, c = x_start + cl;
-      float2 g = make_float2(0.f, 0.f);
+      float4 g = make_float4(0.f, 0.f, 0.f, 0.f);
       if (r >= 1 && r < h - 1 && c >= 1 && c < w - 1 && rl >= 1 && rl < G::IH - 1 && cl >= 1 &&
           cl < G::IW - 1) {
-        g.x = __fadd_rn(-tin[i - 1], tin[i + 1]);
-        g.y = __fadd_rn(-tin[i - G::IW], tin[i + G::IW]);
+        const float* t0 = tin + i;
+        const float* t1 = t0 + G::S_IN;
+        g.x = __fadd_rn(-t0[-1], t0[1]);
+        g.y = __fadd_rn(-t1[-1], t1[1]);
+        g.z = __fadd_rn(-t0[-G::IW], t0[G::IW]);
+        g.w = __fadd_rn(-t1[-G::IW], t1[G::IW]);
       }
       grad[i] = g;
     }
@@ -208,96 +260,119 @@ __global__ void __launch_bounds__(SrrfTile<M>::NT, 1) srrf_fused_kernel(const Sr
       const int nyo = ny0 + oy / M;
       const float* w5 = rw + oy * 5;
       const float* col = tin + (nyo - 2 - y_start) * G::IW + (nx0 - 2 + cc - x_start);
-      float sum = 0.f;
+      float2 sum = make_float2(0.f, 0.f);
 #pragma unroll
-      for (int k = 0; k < 5; ++k) sum = fmaf(w5[k], col[k * G::IW], sum);
+      for (int k = 0; k < 5; ++k)
+        sum = __ffma2_rn(make_float2(w5[k], w5[k]),
+                         make_float2(col[k * G::IW], col[G::S_IN + k * G::IW]), sum);
       ri[i] = sum;
     }
     __syncthreads();
-    // row pass of the ring interpolation: the ring points of this warp's output
-    // row share their tap rows and weights, so each (ring point, tile column)
-    // sum over the 4 tap rows is formed once per warp (same fma order as the
-    // 16-tap form: rows first, then columns)
-    for (int idx = lane; idx < kRing * G::IW; idx += 32) {
-      const int s = idx / G::IW, c = idx - s * G::IW;
-      const float4 rA = *reinterpret_cast<const float4*>(rrow + s * 8);
-      const float4 rB = *reinterpret_cast<const float4*>(rrow + s * 8 + 4);
-      float2 v = make_float2(0.f, 0.f);
-      if (rB.z != 0.f) {
-        const int r0 = __float_as_int(rA.x) - y_start;
-        const float wr[4] = {rA.y, rA.z, rA.w, rB.x};
-        const float2* gp = grad + r0 * G::IW + c;
+    float2 div[M];
 #pragma unroll
-        for (int t = 0; t < 4; ++t) {
-          const float2 g = gp[t * G::IW];
-          v.x = fmaf(g.x, wr[t], v.x);
-          v.y = fmaf(g.y, wr[t], v.y);
-        }
-      }
-      rb[idx] = v;
-    }
-    __syncwarp();
-    // radiality of this thread's M outputs, ring point by ring point: the M
-    // columns share one window of 5 row-pass columns (cb .. cb + 4), each
-    // output weights it with its own 5-vector (its 4 taps and a zero), which
-    // is the 4-tap fma sequence of the reference with a + 0 at one end
-    float div[M];
-#pragma unroll
-    for (int px = 0; px < M; ++px) div[px] = 0.f;
+    for (int px = 0; px < M; ++px) div[px] = make_float2(0.f, 0.f);
     const float yc = (float)j + 0.5f;
-#pragma unroll 2
-    for (int s = 0; s < kRing; ++s) {
-      const float dy = __fsub_rn(yc, __fadd_rn(yc, p.yr[s]));  // yc - y0
-      const float2* rp = rb + s * G::IW + cbt[s * G::TX + lane];
-      float2 col[5];
+#pragma unroll 1
+    for (int sg = 0; sg < kRing; sg += G::RG) {
+      // row pass of the ring interpolation: the ring points of this warp's output
+      // row share their tap rows and weights, so each (ring point, tile column)
+      // sum over the 4 tap rows is formed once per warp (same fma order as the
+      // 16-tap form: rows first, then columns)
+      __syncwarp();
+      for (int idx = lane; idx < G::RG * G::IW; idx += 32) {
+        const int s = idx / G::IW, c = idx - s * G::IW;
+        const float4 rA = *reinterpret_cast<const float4*>(rrow + (sg + s) * 8);
+        const float4 rB = *reinterpret_cast<const float4*>(rrow + (sg + s) * 8 + 4);
+        float2 vx = make_float2(0.f, 0.f), vy = make_float2(0.f, 0.f);
+        if (rB.z != 0.f) {
+          const int r0 = __float_as_int(rA.x) - y_start;
+          const float wr[4] = {rA.y, rA.z, rA.w, rB.x};
+          const float4* gp = grad + r0 * G::IW + c;
 #pragma unroll
-      for (int k = 0; k < 5; ++k) col[k] = rp[k];
-#pragma unroll
-      for (int px = 0; px < M; ++px) {
-        const float4 wa = cw4[(s * M + px) * G::TX + lane];
-        const float we = cw1[(s * M + px) * G::TX + lane];
-        const float wv[5] = {wa.x, wa.y, wa.z, wa.w, we};
-        const float xc = (float)(nx * M + px) + 0.5f;
-        const float dx = __fsub_rn(xc, __fadd_rn(xc, p.xr[s]));  // xc - x0
-        float vgx = 0.f, vgy = 0.f;
-#pragma unroll
-        for (int k = 0; k < 5; ++k) {
-          vgx = fmaf(col[k].x, wv[k], vgx);
-          vgy = fmaf(col[k].y, wv[k], vgy);
+          for (int t = 0; t < 4; ++t) {
+            const float4 g = gp[t * G::IW];
+            const float2 wt = make_float2(wr[t], wr[t]);
+            vx = __ffma2_rn(make_float2(g.x, g.y), wt, vx);
+            vy = __ffma2_rn(make_float2(g.z, g.w), wt, vy);
+          }
         }
-        float dk = 0.f;
-        const float g2 = vgx * vgx + vgy * vgy;
-        if (g2 != 0.f) {
-          // |vGy (xc - x0) - vGx (yc - y0)| / GMag / ringRadius
-          dk = 1.f - fabsf(vgy * dx - vgx * dy) * rsqrtf(g2) * p.inv_rr;
-          dk = dk * dk;
+        rb[idx] = make_float4(vx.x, vx.y, vy.x, vy.y);
+      }
+      __syncwarp();
+      // radiality of this thread's M outputs, ring point by ring point: the M
+      // columns share one window of 5 row-pass columns (cb .. cb + 4), each
+      // output weights it with its own 5-vector (its 4 taps and a zero), which
+      // is the 4-tap fma sequence of the reference with a + 0 at one end
+#pragma unroll 1
+      for (int s = sg; s < sg + G::RG; ++s) {
+        const float dy = __fsub_rn(yc, __fadd_rn(yc, p.yr[s]));  // yc - y0
+        const float4* rp = rb + (s - sg) * G::IW + cbt[s * G::TX + lane];
+        float4 col[5];
+#pragma unroll
+        for (int k = 0; k < 5; ++k) col[k] = rp[k];
+#pragma unroll
+        for (int px = 0; px < M; ++px) {
+          const float4 wa = cw4[(s * M + px) * G::TX + lane];
+          const float we = cw1[(s * M + px) * G::TX + lane];
+          const float wv[5] = {wa.x, wa.y, wa.z, wa.w, we};
+          const float xc = (float)(nx * M + px) + 0.5f;
+          const float dx = __fsub_rn(xc, __fadd_rn(xc, p.xr[s]));  // xc - x0
+          float2 vgx = make_float2(0.f, 0.f), vgy = make_float2(0.f, 0.f);
+#pragma unroll
+          for (int k = 0; k < 5; ++k) {
+            const float2 wk = make_float2(wv[k], wv[k]);
+            vgx = __ffma2_rn(make_float2(col[k].x, col[k].y), wk, vgx);
+            vgy = __ffma2_rn(make_float2(col[k].z, col[k].w), wk, vgy);
+          }
+          // dk = (1 - |vGy (xc - x0) - vGx (yc - y0)| / GMag / ringRadius)^2, 0
+          // without a gradient; subtracted where the gradient points outwards.
+          // No comparisons (the ALU pipe was the busiest): kTiny, absorbed by any
+          // squared gradient above it, keeps rsqrt finite, a saturating FMA
+          // turns "any gradient" into 0 or 1, and the dot product's sign is
+          // moved onto dk by a logic operation (dk is 0 where it is 0).
+          const float2 g2 = __ffma2_rn(vgx, vgx, __ffma2_rn(vgy, vgy, make_float2(kTiny, kTiny)));
+          const float2 any = make_float2(__saturatef(__fmaf_rn(g2.x, 1.f / kTiny, -1.f)),
+                                         __saturatef(__fmaf_rn(g2.y, 1.f / kTiny, -1.f)));
+          const float2 cr = __ffma2_rn(vgy, make_float2(dx, dx),
+                                       __fmul2_rn(vgx, make_float2(-dy, -dy)));
+          const float2 rs = __fmul2_rn(make_float2(rsqrtf(g2.x), rsqrtf(g2.y)),
+                                       make_float2(-p.inv_rr, -p.inv_rr));
+          float2 dk = __ffma2_rn(make_float2(fabsf(cr.x), fabsf(cr.y)), rs, make_float2(1.f, 1.f));
+          dk = __fmul2_rn(dk, dk);
+          const float2 dot = __ffma2_rn(vgx, make_float2(p.xr[s], p.xr[s]),
+                                        __fmul2_rn(vgy, make_float2(p.yr[s], p.yr[s])));
+          dk = make_float2(against(dk.x, dot.x), against(dk.y, dot.y));
+          div[px] = __ffma2_rn(any, dk, div[px]);
         }
-        if (vgx * p.xr[s] + vgy * p.yr[s] > 0.f) div[px] -= dk;
-        else div[px] += dk;
       }
     }
 #pragma unroll
     for (int px = 0; px < M; ++px) {
       const int i = nx * M + px;  // output column
-      float val = 0.f;
+      float2 val = make_float2(0.f, 0.f);
+      const size_t o = (size_t)f * plane + (size_t)j * colsM + i;
       if (row_ok && nx < w && i >= lo_i && i < hi_i) {
-        const float dv = div[px] / 12.f;
-        val = p.positivity ? fmaxf(dv, 0.f) : dv;
+        val = make_float2(div[px].x / 12.f, div[px].y / 12.f);
+        if (p.positivity) val = make_float2(fmaxf(val.x, 0.f), fmaxf(val.y, 0.f));
         if (p.iw) {
           if (own_intensity) {
             // column pass of the intensity magnification (5 taps of the row pass)
             const float* w5 = cw + (lane * M + px) * 5;
-            const float* rr = ri + (ty * M + py) * G::RIW + lane;
-            float sum = 0.f;
+            const float2* rr = ri + (ty * M + py) * G::RIW + lane;
+            float2 sum = make_float2(0.f, 0.f);
 #pragma unroll
-            for (int k = 0; k < 5; ++k) sum = fmaf(w5[k], rr[k], sum);
-            val *= sum;
+            for (int k = 0; k < 5; ++k) sum = __ffma2_rn(make_float2(w5[k], w5[k]), rr[k], sum);
+            val = __fmul2_rn(val, sum);
           } else {
-            val *= __ldg(p.interp + (size_t)f * plane + (size_t)j * colsM + i);
+            val.x *= __ldg(p.interp + o);
+            if (two) val.y *= __ldg(p.interp + o + plane);
           }
         }
       }
-      if (ny < h && nx < w) p.out[(size_t)f * plane + (size_t)j * colsM + i] = val;
+      if (ny < h && nx < w) {
+        p.out[o] = val.x;
+        if (two) p.out[o + plane] = val.y;
+      }
     }
   }
 }
@@ -321,7 +396,21 @@ cudaError_t launch_srrf_m(const SrrfParams& prm, cudaStream_t s) {
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const long long tiles = (long long)q.tiles_x * q.tiles_y;
-  q.chunks = (int)std::max<long long>(1, std::min<long long>(prm.T, (2LL * sms + tiles - 1) / tiles));
+  int per_sm = 1;
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, srrf_fused_kernel<M>, G::NT, G::SMEM);
+  if (e != cudaSuccess) return e;
+  // frame chunks: the count with the fewest passes on the busiest SM, a block
+  // costing its frame pairs plus about one pair for its tables
+  const long long pairs = ((long long)prm.T + 1) / 2, slots = (long long)sms * std::max(1, per_sm);
+  long long best = -1;
+  q.chunks = 1;
+  for (long long c = 1; c <= std::min<long long>(pairs, 64); ++c) {
+    const long long cost = (tiles * c + slots - 1) / slots * ((pairs + c - 1) / c + 1);
+    if (best < 0 || cost < best) {
+      best = cost;
+      q.chunks = (int)c;
+    }
+  }
   srrf_fused_kernel<M><<<dim3((unsigned)tiles, (unsigned)q.chunks), G::NT, G::SMEM, s>>>(q);
   return cudaGetLastError();
 }
