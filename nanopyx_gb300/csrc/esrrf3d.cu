@@ -1,7 +1,7 @@
 // eSRRF-3D: radial gradient convergence of volumes
 // (src/nanopyx/core/transform/_le_esrrf3d.pyx:65-140).
 //
-// Per frame of a (T, S, H, W) stack, as the reference:
+// Per pair of consecutive frames of a (T, S, H, W) stack, as the reference:
 //   1. gradients at the input resolution: central differences along x and y,
 //      the backward difference along z, halved, indices clamped
 //      (src/include/_c_gradients.c:75-116);
@@ -9,18 +9,29 @@
 //      every slice; the reference's "linear" z step then repeats each slice
 //      mz times (its slice coordinate sM / mz is an integer division, so the
 //      second weight is 0, _interpolation.pyx:54-88) -- here the repeat is an
-//      index mapping, never materialised;
+//      index mapping, never materialised.  One kernel does both and stores the
+//      gradients normalised, the two frames side by side;
 //   3. at every output voxel inside the margins the RGC over the window of
 //      input-pixel offsets (src/include/_c_sr_radial_gradient_convergence.c:
-//      92-204) in the reference's float32 operation order (its few double
-//      steps -- exp, pow, the quotient of square roots -- in float32, within
-//      a few ulp: FP64 runs at a small fraction of FP32 here), to the power
-//      `sensitivity`, times the interpolated intensity;
+//      92-204) on packed f32x2 arithmetic (FP64 steps of the reference -- exp,
+//      pow, the quotient of square roots -- in float32 or in the host's table),
+//      to the power `sensitivity`, times the interpolated intensity;
 //   4. the running mean (mode "average") or Welford variance (mode "std",
 //      sqrt(M2 / T) at the end) over the frames, in the reference's order.
+//
+// The window samples of the mz voxels of one input slice are the same gradients
+// at the same offsets, so their RGC is evaluated once wherever the same samples
+// lie inside the volume for all of them.
+//
+// What bounds it: issue and register reads of step 3 (15 packed operations per
+// sample and frame pair) and the L1 wavefronts of its two gradient loads.
+// 20 x 16 x 128 x 128, mxy = mz = 2, R = 1.5: one frame at a time, three scalar
+// gradients normalised at every sample and every voxel by itself 5.9 ms; frame
+// pairs, gradients normalised once, shared z voxels 1.5 ms.
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <vector>
 
@@ -34,120 +45,253 @@ struct Rgc3d {
   int S, H, W, mxy, mz, Hm, Wm, Sm;
   int margin, margin_z;
   int s0, s1, z0, z1;  // window offsets, inclusive
-  float tSS, tSO, tSS_z, tSO_z, sensitivity;
+  int sens_mode, sens_int;
+  float sensitivity;
   int iw, mode;
-  // floor(x / mz) = (x * mz_magic) >> 32 in 64-bit arithmetic for 0 <= x,
-  // x * mz < 2^32
-  // (mz_magic = floor(2^32 / mz) + 1: the excess x (mz_magic - 2^32 / mz) / 2^32
-  // stays below 1 / mz, so it never crosses the next integer)
-  unsigned long long mz_magic;
 };
 
-__global__ void gradient3d_kernel(const float* __restrict__ v, int S, int H, int W,
-                                  float* __restrict__ gc, float* __restrict__ gr,
-                                  float* __restrict__ gs) {
-  const long long n = (long long)S * H * W;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n;
-       e += (long long)gridDim.x * blockDim.x) {
-    const int x = (int)(e % W), y = (int)((e / W) % H), z = (int)(e / ((long long)H * W));
-    const int xp = x >= W - 1 ? W - 1 : x + 1, xm = x <= 0 ? 0 : x - 1;
-    const int yp = y >= H - 1 ? H - 1 : y + 1, ym = y <= 0 ? 0 : y - 1;
-    const int zm = z <= 0 ? 0 : z - 1;
-    const float* sl = v + (size_t)z * H * W;
-    gc[e] = __fsub_rn(sl[(size_t)y * W + xp], sl[(size_t)y * W + xm]) / 2;
-    gr[e] = __fsub_rn(sl[(size_t)yp * W + x], sl[(size_t)ym * W + x]) / 2;
-    gs[e] = __fsub_rn(sl[(size_t)y * W + x], v[((size_t)zm * H + y) * W + x]) / 2;
+// Steps 1 and 2 for a frame pair: a block covers kPrepCols x kPrepRows output
+// pixels of one slice.  The gradients and the value of every input pixel the
+// taps reach go to shared memory as (gx, gx', gy, gy') (gz, gz', v, v') -- zero
+// outside the image, the reference's skipped taps -- then each thread keeps one
+// output column and a run of rows: 8 shared loads give a row's 4-tap column sums
+// of all quantities, and the four newest rows stay in registers.
+constexpr int kPrepCols = 64, kPrepRows = 16, kPrepThreads = 256;
+constexpr int kPrepRun = kPrepRows / (kPrepThreads / kPrepCols);  // rows per thread
+
+__host__ __device__ inline int prep_extent(int n_out, int mag) { return (n_out - 1) / mag + 6; }
+
+struct Quad {  // float4 (gx, gx', gy, gy') and (gz, gz', v, v')
+  float4 a, b;
+};
+
+__device__ __forceinline__ void quad_fma(Quad& q, float w, const Quad& v) {
+  const float2 w2 = make_float2(w, w);
+  float2 x = __ffma2_rn(make_float2(v.a.x, v.a.y), w2, make_float2(q.a.x, q.a.y));
+  float2 y = __ffma2_rn(make_float2(v.a.z, v.a.w), w2, make_float2(q.a.z, q.a.w));
+  q.a = make_float4(x.x, x.y, y.x, y.y);
+  x = __ffma2_rn(make_float2(v.b.x, v.b.y), w2, make_float2(q.b.x, q.b.y));
+  y = __ffma2_rn(make_float2(v.b.z, v.b.w), w2, make_float2(q.b.z, q.b.w));
+  q.b = make_float4(x.x, x.y, y.x, y.y);
+}
+
+// 1 / |g| for the normalisation; 0 without a gradient.  An infinite gradient is
+// not normalised (scale 1, see unit): its RGC then overflows to NaN where the
+// reference's quotient does.
+__device__ __forceinline__ float unit_scale(float x, float y, float z) {
+  const float d = fmaf(z, z, fmaf(y, y, x * x));
+  return d > 0.f ? (d < INFINITY ? rsqrtf(d) : 1.f) : d == 0.f ? 0.f : d;
+}
+
+__device__ __forceinline__ float unit(float g, float s) {
+  return fminf(fabsf(g), 3.4e38f) == fabsf(g) ? g * s : (g != g ? g : copysignf(3.4e38f, g));
+}
+
+__global__ void __launch_bounds__(kPrepThreads)
+    prep3d_kernel(const float* __restrict__ v0, const float* __restrict__ v1, int H, int W, int m,
+                  int z_first, float4* __restrict__ A, float2* __restrict__ B, float2* __restrict__ I) {
+  extern __shared__ __align__(16) float4 patch[];  // [PR][PC][2]
+  const int Hm = H * m, Wm = W * m;
+  const int nbx = (Wm + kPrepCols - 1) / kPrepCols;
+  const int z = z_first + blockIdx.y;
+  const int x0 = blockIdx.x % nbx * kPrepCols, y0 = blockIdx.x / nbx * kPrepRows;
+  const int PR = prep_extent(kPrepRows, m), PC = prep_extent(kPrepCols, m);
+  const int r0 = y0 / m - 2, c0 = x0 / m - 2;  // first input row / column of the patch
+  const size_t plane = (size_t)H * W;
+  const float* f0 = v0 + z * plane;
+  const float* f1 = v1 + z * plane;
+  const ptrdiff_t back = z > 0 ? -(ptrdiff_t)plane : 0;  // the slice below (clamped)
+  for (int i = threadIdx.x; i < PR * PC; i += kPrepThreads) {
+    const int y = r0 + i / PC, x = c0 + i % PC;
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+    if (y >= 0 && y < H && x >= 0 && x < W) {
+      const size_t o = (size_t)y * W + x;
+      const int xp = x < W - 1 ? 1 : 0, xm = x > 0 ? 1 : 0;
+      const int yp = y < H - 1 ? W : 0, ym = y > 0 ? W : 0;
+      auto grad = [&](const float* f, float& gx, float& gy, float& gz, float& val) {
+        val = __ldg(f + o);
+        gx = __fsub_rn(__ldg(f + o + xp), __ldg(f + o - xm)) / 2;
+        gy = __fsub_rn(__ldg(f + o + yp), __ldg(f + o - ym)) / 2;
+        gz = __fsub_rn(val, __ldg(f + o + back)) / 2;
+      };
+      grad(f0, a.x, a.z, b.x, b.z);
+      grad(f1, a.y, a.w, b.y, b.w);
+    }
+    patch[2 * i] = a;
+    patch[2 * i + 1] = b;
+  }
+  __syncthreads();
+  const int x = x0 + threadIdx.x % kPrepCols;
+  const int yb = y0 + threadIdx.x / kPrepCols * kPrepRun;
+  if (x >= Wm) return;
+  auto store = [&](int y, const Quad& q) {
+    const float s0 = unit_scale(q.a.x, q.a.z, q.b.x), s1 = unit_scale(q.a.y, q.a.w, q.b.y);
+    const size_t o = ((size_t)z * Hm + y) * Wm + x;
+    A[o] = make_float4(unit(q.a.x, s0), unit(q.a.y, s1), unit(q.a.z, s0), unit(q.a.w, s1));
+    B[o] = make_float2(unit(q.b.x, s0), unit(q.b.y, s1));
+    I[o] = make_float2(q.b.z, q.b.w);
+  };
+  if (m == 1) {  // not magnified: the values themselves
+    for (int y = yb; y < min(yb + kPrepRun, Hm); ++y) {
+      const int i = (y - r0) * PC + x - c0;
+      store(y, Quad{patch[2 * i], patch[2 * i + 1]});
+    }
+    return;
+  }
+  const float col = __fdiv_rn((float)x, (float)m);
+  const int cb = (int)floorf(col - 0.5f) - 1;
+  const bool cin = col < (float)W;
+  float wc[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) wc[k] = cin ? cr_cubic(col - ((float)(cb + k) + 0.5f)) : 0.f;
+  auto across = [&](int r) {  // 4-tap sums of input row r
+    Quad q{make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
+    const float4* p = patch + 2 * ((r - r0) * PC + cb - c0);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) quad_fma(q, wc[k], Quad{p[2 * k], p[2 * k + 1]});
+    return q;
+  };
+  Quad win[4];
+  int top = INT_MIN;  // input row of win[0]
+#pragma unroll 1
+  for (int y = yb; y < min(yb + kPrepRun, Hm); ++y) {
+    const float row = __fdiv_rn((float)y, (float)m);
+    const int rb = (int)floorf(row - 0.5f) - 1;
+    if (rb == top + 1) {
+#pragma unroll
+      for (int k = 0; k < 3; ++k) win[k] = win[k + 1];
+      win[3] = across(rb + 3);
+    } else if (rb != top) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) win[k] = across(rb + k);
+    }
+    top = rb;
+    Quad q{make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
+    if (row < (float)H) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        quad_fma(q, cr_cubic(row - ((float)(rb + k) + 0.5f)), win[k]);
+    }
+    store(y, q);
   }
 }
 
-// one thread per output voxel inside the margins; gx/gy/gz/img: (S, Hm, Wm),
-// the xy-magnified volumes (slice zM of the z-magnified volume is slice
-// zM / mz of these).  The window samples sit at whole input-pixel offsets
-// (i, j, k) from the voxel's centre, so their distance weights, validity
-// (distance != 0, xy distance <= tSO, signed z offset <= tSO_z) and inverse
-// distances depend on the offset alone: `tab` holds (weight, 1 / distance)
-// per offset, weight 0 where a sample does not count.  Per voxel only the
-// in-volume tests and the gradient indices use the voxel's float coordinates,
-// exactly as the reference forms them.
-__global__ void __launch_bounds__(256) rgc3d_kernel(const __grid_constant__ Rgc3d p,
-                                                    const float* __restrict__ gx,
-                                                    const float* __restrict__ gy,
-                                                    const float* __restrict__ gz,
-                                                    const float* __restrict__ img,
-                                                    const float2* __restrict__ tab, int frame,
-                                                    float* __restrict__ out,
-                                                    float* __restrict__ mean) {
-  const int nx = p.Wm - 2 * p.margin, ny = p.Hm - 2 * p.margin, nz = p.Sm - 2 * p.margin_z;
-  const long long n = (long long)nx * ny * nz;
+// Steps 3 and 4 for a frame pair: a block covers 32 x 8 output pixels inside the
+// margins and the mz voxels of one input slice.  tab holds, per window offset
+// [k][j][i], the unit offset and the weight (0: does not count); sample columns
+// and rows, from the voxel's float32 coordinates as the reference forms them,
+// are tabulated per block (-1: outside the image).
+constexpr int kMaxWin = 64;  // window offsets per axis are at most 2 int(radius) + 2
+
+__global__ void __launch_bounds__(256)
+    rgc3d_kernel(const __grid_constant__ Rgc3d p, const float4* __restrict__ A,
+                 const float2* __restrict__ B, const float2* __restrict__ I,
+                 const float4* __restrict__ tab, int s_first, int frame, int two,
+                 float* __restrict__ out, float* __restrict__ mean) {
+  __shared__ int cidx[kMaxWin][32], ridx[kMaxWin][8];
+  const int nI = p.s1 - p.s0 + 1;
+  const int lane = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int nbx = (p.Wm - 2 * p.margin + 31) / 32;
+  const int c0 = p.margin + blockIdx.x % nbx * 32, r0 = p.margin + blockIdx.x / nbx * 8;
+  for (int e = threadIdx.x; e < nI * 40; e += 256) {
+    const int i = e / 40, t = e % 40;
+    const bool isrow = t >= 32;
+    const int n = isrow ? p.H : p.W, nm = isrow ? p.Hm : p.Wm;
+    // threads past the last voxel of a row or column repeat it
+    const int M = min(isrow ? r0 + t - 32 : c0 + t, nm - p.margin - 1);
+    const float v = __fadd_rn(__fdiv_rn((float)M, (float)p.mxy), (float)(p.s0 + i));
+    const int idx =
+        0.f < v && v <= (float)(n - 1) ? min((int)__fmul_rn((float)p.mxy, v), nm - 1) : -1;
+    if (isrow) ridx[i][t - 32] = idx;
+    else cidx[i][t] = idx;
+  }
+  __syncthreads();
+  const int cM = c0 + lane, rM = r0 + ty;
+  const bool active = cM < p.Wm - p.margin && rM < p.Hm - p.margin;
+  bool all_in = true;
+  for (int i = 0; i < nI; ++i) all_in = all_in && cidx[i][lane] >= 0 && ridx[i][ty] >= 0;
+  const bool interior = __all_sync(0xffffffffu, all_in);
   const size_t plane = (size_t)p.Hm * p.Wm;
-  const int nI = p.s1 - p.s0 + 1, nK = p.z1 - p.z0 + 1;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n;
-       e += (long long)gridDim.x * blockDim.x) {
-    int cM, rM, sM;
-    if (n < (1LL << 31)) {  // 32-bit index arithmetic
-      const unsigned u = (unsigned)e;
-      cM = p.margin + (int)(u % (unsigned)nx);
-      rM = p.margin + (int)((u / (unsigned)nx) % (unsigned)ny);
-      sM = p.margin_z + (int)(u / ((unsigned)nx * (unsigned)ny));
-    } else {
-      cM = p.margin + (int)(e % nx);
-      rM = p.margin + (int)((e / nx) % ny);
-      sM = p.margin_z + (int)(e / ((long long)nx * ny));
-    }
-    const float xc = __fdiv_rn((float)cM, (float)p.mxy);
-    const float yc = __fdiv_rn((float)rM, (float)p.mxy);
-    const float zc = __fdiv_rn((float)sM, (float)p.mz);
-    float rgc = 0.f, wsum = 0.f;
-    for (int j = p.s0; j <= p.s1; ++j) {
-      const float vy = __fadd_rn(yc, (float)j);
-      if (!(0.f < vy && vy <= (float)(p.H - 1))) continue;
-      const size_t ry = (size_t)(int)__fmul_rn((float)p.mxy, vy) * p.Wm;
-      for (int i = p.s0; i <= p.s1; ++i) {
-        const float vx = __fadd_rn(xc, (float)i);
-        if (!(0.f < vx && vx <= (float)(p.W - 1))) continue;
-        const size_t rxy = ry + (int)__fmul_rn((float)p.mxy, vx);
-        const float2* trow = tab + ((size_t)(j - p.s0) * nI + (i - p.s0)) * nK;
-        for (int k = p.z0; k <= p.z1; ++k) {
-          const float2 t = __ldg(trow + (k - p.z0));
-          if (t.x == 0.f) continue;
-          const float vz = __fadd_rn(zc, (float)k);
-          if (!(0.f < vz && vz <= (float)(p.S - 1))) continue;
-          // slice of the xy-magnified volumes: (int)(vz mz) / mz, vz > 0
-          const unsigned zm = (unsigned)(int)__fmul_rn(vz, (float)p.mz);
-          const size_t li = (size_t)((zm * p.mz_magic) >> 32) * plane + rxy;
-          const float Gx = __ldg(gx + li), Gy = __ldg(gy + li), Gz = __ldg(gz + li);
-          wsum = __fadd_rn(wsum, t.x);
-          const float fi = (float)i, fj = (float)j, fk = (float)k;
-          const float gdr = fmaf(Gz, fk, fmaf(Gy, fj, Gx * fi));
-          if (gdr < 0.f) {
-            const float c1 = fmaf(Gy, fk, -Gz * fj);
-            const float c2 = fmaf(Gz, fi, -Gx * fk);
-            const float c3 = fmaf(Gx, fj, -Gy * fi);
-            const float num = fmaf(c3, c3, fmaf(c2, c2, c1 * c1));
-            const float den = fmaf(Gz, Gz, fmaf(Gy, Gy, Gx * Gx));
-            // |c| / |G| / distance; 0 / 0 (no gradient) counts as the distance
-            // itself in the reference, i.e. a zero contribution
-            const float dk = den > 0.f ? sqrtf(num) * rsqrtf(den) * t.y : 1.f;
-            rgc = fmaf(1.f - dk, t.x, rgc);
-          }
+  // voxels sM = s mz + r, r0 <= r < r1, inside the z margins
+  const int s = s_first + blockIdx.y;
+  const int ra = max(0, p.margin_z - s * p.mz);
+  const int rb = min(p.mz, p.Sm - p.margin_z - s * p.mz);
+  auto z_in = [&](int r, int k) {
+    const float vz = __fadd_rn(__fdiv_rn((float)(s * p.mz + r), (float)p.mz), (float)k);
+    return 0.f < vz && vz <= (float)(p.S - 1);
+  };
+  bool same = true;  // the same samples lie inside the volume for every r
+  for (int k = p.z0; k <= p.z1; ++k)
+    for (int r = ra + 1; r < rb; ++r) same = same && z_in(r, k) == z_in(ra, k);
+  for (int r = ra; r < rb; r = same ? rb : r + 1) {
+    float2 acc = make_float2(0.f, 0.f);
+    float wsum = 0.f;
+    for (int k = p.z0; k <= p.z1; ++k) {
+      if (!z_in(r, k)) continue;
+      // slice of the magnified volumes: (int)(vz mz) / mz = s + k (vz mz rounds
+      // to s mz + k mz + r or, for r > 0, at worst just below it)
+      const float4* Ak = A + (size_t)(s + k) * plane;
+      const float2* Bk = B + (size_t)(s + k) * plane;
+      const float4* tk = tab + (size_t)(k - p.z0) * nI * nI;
+      for (int j = 0; j < nI; ++j) {
+        const int ry = ridx[j][ty];
+        const float4* Aj = Ak + (size_t)max(ry, 0) * p.Wm;
+        const float2* Bj = Bk + (size_t)max(ry, 0) * p.Wm;
+#pragma unroll 4
+        for (int i = 0; i < nI; ++i) {
+          const float4 t = __ldg(tk + j * nI + i);
+          if (t.w == 0.f) continue;
+          const int cx = cidx[i][lane];
+          const bool ok = interior || (ry >= 0 && cx >= 0);
+          const float4 a = __ldg(Aj + max(cx, 0));
+          const float2 nz = __ldg(Bj + max(cx, 0));
+          const float2 nx = make_float2(a.x, a.y), ny = make_float2(a.z, a.w);
+          const float2 rx = make_float2(t.x, t.x), ryv = make_float2(t.y, t.y),
+                       rz = make_float2(t.z, t.z);
+          const float2 mx = make_float2(-t.x, -t.x), my = make_float2(-t.y, -t.y),
+                       mzv = make_float2(-t.z, -t.z);
+          const float2 dot = __ffma2_rn(nz, rz, __ffma2_rn(ny, ryv, __fmul2_rn(nx, rx)));
+          const float2 c1 = __ffma2_rn(ny, rz, __fmul2_rn(nz, my));
+          const float2 c2 = __ffma2_rn(nz, rx, __fmul2_rn(nx, mzv));
+          const float2 c3 = __ffma2_rn(nx, ryv, __fmul2_rn(ny, mx));
+          // the smallest normal number keeps rsqrt finite for a zero cross product
+          const float tiny = 1.17549435e-38f;
+          const float2 q = __ffma2_rn(
+              c3, c3, __ffma2_rn(c2, c2, __ffma2_rn(c1, c1, make_float2(tiny, tiny))));
+          const float2 dk = __fmul2_rn(q, make_float2(rsqrtf(q.x), rsqrtf(q.y)));
+          const float2 v = __ffma2_rn(dk, make_float2(-t.w, -t.w), make_float2(t.w, t.w));
+          acc = __fadd2_rn(acc, make_float2(ok && dot.x < 0.f ? v.x : 0.f,
+                                            ok && dot.y < 0.f ? v.y : 0.f));
+          wsum += ok ? t.w : 0.f;
         }
       }
     }
-    rgc = __fdiv_rn(rgc, wsum);
-    if (rgc >= 0.f && p.sensitivity > 1.f)
-      rgc = powf(rgc, p.sensitivity);
-    else if (rgc < 0.f)
-      rgc = 0.f;
-    if (p.iw) rgc = __fmul_rn(rgc, __ldg(img + (size_t)(sM / p.mz) * plane + (size_t)rM * p.Wm + cM));
-    const size_t o = ((size_t)sM * p.Hm + rM) * p.Wm + cM;
-    const float fr = (float)(frame + 1);
-    if (p.mode == 0) {
-      out[o] = __fadd_rn(out[o], __fdiv_rn(__fsub_rn(rgc, out[o]), fr));
-    } else {
-      const float delta = __fsub_rn(rgc, mean[o]);
-      mean[o] = __fadd_rn(mean[o], __fdiv_rn(delta, fr));
-      const float delta2 = __fsub_rn(rgc, mean[o]);
-      out[o] = __fadd_rn(out[o], __fmul_rn(delta, delta2));
+    if (!active) continue;
+    float2 val = make_float2(__fdiv_rn(acc.x, wsum), __fdiv_rn(acc.y, wsum));
+    auto power = [&](float g) {
+      if (g >= 0.f) return apply_sensitivity(g, p.sens_mode, p.sens_int, p.sensitivity);
+      return g < 0.f ? 0.f : g;
+    };
+    val.x = power(val.x);
+    val.y = power(val.y);
+    if (p.iw)
+      val = __fmul2_rn(val, __ldg(I + (size_t)s * plane + (size_t)rM * p.Wm + cM));
+    // voxels that share their samples share their whole history
+    size_t o = ((size_t)(s * p.mz + r) * p.Hm + rM) * p.Wm + cM;
+    float cur = out[o], mu = p.mode ? mean[o] : 0.f;
+    for (int f = 0; f <= two; ++f) {
+      const float g = f ? val.y : val.x, fr = (float)(frame + f + 1);
+      if (p.mode == 0) {
+        cur = __fadd_rn(cur, __fdiv_rn(__fsub_rn(g, cur), fr));
+      } else {
+        const float delta = __fsub_rn(g, mu);
+        mu = __fadd_rn(mu, __fdiv_rn(delta, fr));
+        cur = __fadd_rn(cur, __fmul_rn(delta, __fsub_rn(g, mu)));
+      }
+    }
+    for (int q = r; q < (same ? rb : r + 1); ++q, o += plane) {
+      out[o] = cur;
+      if (p.mode) mean[o] = mu;
     }
   }
 }
@@ -171,18 +315,14 @@ using namespace nx;
 
 extern "C" {
 
-// window offsets per axis are at most 2 int(radius) + 2 <= kMaxWin
-constexpr int kMaxWin = 64;
-
 size_t nx_esrrf3d_workspace_bytes(int S, int H, int W, int magnification_xy,
                                   int magnification_z, int mode) {
   if (S < 1 || H < 1 || W < 1 || magnification_xy < 1 || magnification_z < 1) return 256;
-  const size_t vol = (size_t)S * H * W;
   const size_t volm = (size_t)S * H * magnification_xy * W * magnification_xy;
   const size_t out = volm * magnification_z;
-  return 256 + rup(3 * (size_t)S * sizeof(float)) + rup(3 * vol * sizeof(float)) +
-         rup(4 * volm * sizeof(float)) + (mode ? rup(out * sizeof(float)) : 0) +
-         rup((size_t)kMaxWin * kMaxWin * kMaxWin * sizeof(float2));
+  return 256 + rup(volm * sizeof(float4)) + 2 * rup(volm * sizeof(float2)) +
+         (mode ? rup(out * sizeof(float)) : 0) +
+         rup((size_t)kMaxWin * kMaxWin * kMaxWin * sizeof(float4));
 }
 
 int nx_esrrf3d_st(const float* d_in, int T, int S, int H, int W, int magnification_xy,
@@ -214,93 +354,85 @@ int nx_esrrf3d_st(const float* d_in, int T, int S, int H, int W, int magnificati
   p.Sm = S * mz;
   if ((unsigned long long)p.Sm * (unsigned long long)mz >= (1ULL << 32))
     return nx::set_error("S * magnification_z^2 must be below 2^32"), NX_ERR_INVALID_ARG;
-  p.mz_magic = (1ULL << 32) / (unsigned long long)mz + 1;
   // the reference's scalars (_le_esrrf3d.pyx:73-86): radius and radius_z are
   // Python floats, sigma and the thresholds C floats
   const float sigma = (float)(radius / 2.355);
   const float sigma_z = (float)(radius_z / 2.355);
   p.margin = (int)(radius * mxy);
   p.margin_z = (int)(radius_z * mz);
-  p.tSS = 2 * sigma * sigma;
-  p.tSO = 2 * sigma + 1;
-  p.tSS_z = 2 * sigma_z * sigma_z;
-  p.tSO_z = 2 * sigma_z + 1;
+  const float tSS = 2 * sigma * sigma, tSO = 2 * sigma + 1;
+  const float tSS_z = 2 * sigma_z * sigma_z, tSO_z = 2 * sigma_z + 1;
   const float fwhm = (float)radius, fwhm_z = (float)radius_z;
   p.s0 = -(int)fwhm;
   p.s1 = (int)(fwhm + 1);
   p.z0 = -(int)fwhm_z;
   p.z1 = (int)(fwhm_z + 1);
+  const RgcScalars power = rgc_scalars(1, 1.f, sensitivity, 0);
+  p.sens_mode = power.sens_mode;
+  p.sens_int = power.sens_int;
   p.sensitivity = sensitivity;
   p.iw = do_intensity_weighting ? 1 : 0;
   p.mode = mode;
   const int nI = p.s1 - p.s0 + 1, nK = p.z1 - p.z0 + 1;
   if (nI > kMaxWin || nK > kMaxWin)
     return nx::set_error("radius too large for the 3-D window"), NX_ERR_INVALID_ARG;
-  // per-offset (weight, 1 / distance), the reference's _c_calculate_dw3D
-  // (src/include/_c_sr_radial_gradient_convergence.c:96-102) at whole-pixel
-  // offsets; weight 0 where the sample does not count
-  std::vector<float2> tab((size_t)nI * nI * nK);
-  for (int j = p.s0; j <= p.s1; ++j)
-    for (int i = p.s0; i <= p.s1; ++i)
-      for (int k = p.z0; k <= p.z1; ++k) {
+  // per offset its unit vector and the weight of the reference's
+  // _c_calculate_dw3D (src/include/_c_sr_radial_gradient_convergence.c:96-102);
+  // weight 0 where the sample does not count
+  std::vector<float4> tab((size_t)nI * nI * nK);
+  for (int k = p.z0; k <= p.z1; ++k)
+    for (int j = p.s0; j <= p.s1; ++j)
+      for (int i = p.s0; i <= p.s1; ++i) {
         const double dxy2 = (double)i * i + (double)j * j;
         const double d = std::sqrt(dxy2 + (double)k * k), dxy = std::sqrt(dxy2);
-        float w = 0.f, inv = 0.f;
-        if (d != 0 && dxy <= (double)p.tSO && (double)k <= (double)p.tSO_z) {
-          const float wxy = (float)std::exp(-dxy2 / (double)p.tSS);
-          const float wz = (float)std::exp(-(double)k * k / (double)p.tSS_z);
+        float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (d != 0 && dxy <= (double)tSO && (double)k <= (double)tSO_z) {
+          const float wxy = (float)std::exp(-dxy2 / (double)tSS);
+          const float wz = (float)std::exp(-(double)k * k / (double)tSS_z);
           const float D = (float)(d * (double)(wxy * wz));
-          w = (float)std::pow((double)D, 4.0);
-          inv = (float)(1.0 / d);
+          t = make_float4((float)(i / d), (float)(j / d), (float)(k / d),
+                          (float)std::pow((double)D, 4.0));
         }
-        tab[((size_t)(j - p.s0) * nI + (i - p.s0)) * nK + (k - p.z0)] = make_float2(w, inv);
+        tab[((size_t)(k - p.z0) * nI + (j - p.s0)) * nI + (i - p.s0)] = t;
       }
   const size_t vol = (size_t)S * H * W;
   const size_t volm = (size_t)S * p.Hm * p.Wm;
   const long long nout = (long long)p.Sm * p.Hm * p.Wm;
   char* b = (char*)d_ws + 256;
-  float* zeros = (float*)b;
-  b += rup(3 * (size_t)S * sizeof(float));
-  float* G = (float*)b;  // (3, S, H, W)
-  b += rup(3 * vol * sizeof(float));
-  float* M = (float*)b;  // (4, S, Hm, Wm): image, gx, gy, gz magnified in xy
-  b += rup(4 * volm * sizeof(float));
+  float4* A = (float4*)b;  // magnified unit gradients of a frame pair (x, x', y, y')
+  b += rup(volm * sizeof(float4));
+  float2* B = (float2*)b;  // (z, z')
+  b += rup(volm * sizeof(float2));
+  float2* I = (float2*)b;  // magnified frames (v, v')
+  b += rup(volm * sizeof(float2));
   float* mean = mode ? (float*)b : nullptr;
   if (mode) b += rup((size_t)nout * sizeof(float));
-  float2* dtab = (float2*)b;
-  NX_CUDA_TRY(cudaMemcpyAsync(dtab, tab.data(), tab.size() * sizeof(float2),
+  float4* dtab = (float4*)b;
+  NX_CUDA_TRY(cudaMemcpyAsync(dtab, tab.data(), tab.size() * sizeof(float4),
                               cudaMemcpyHostToDevice, s));
-  NX_CUDA_TRY(cudaMemsetAsync(zeros, 0, 3 * (size_t)S * sizeof(float), s));
   NX_CUDA_TRY(cudaMemsetAsync(d_out, 0, (size_t)nout * sizeof(float), s));
   if (mean) NX_CUDA_TRY(cudaMemsetAsync(mean, 0, (size_t)nout * sizeof(float), s));
-  const bool inside = p.Wm - 2 * p.margin > 0 && p.Hm - 2 * p.margin > 0 &&
-                      p.Sm - 2 * p.margin_z > 0;
-  const long long ninner = inside ? (long long)(p.Wm - 2 * p.margin) *
-                                        (p.Hm - 2 * p.margin) * (p.Sm - 2 * p.margin_z)
-                                  : 0;
-  for (int f = 0; f < T; ++f) {
-    const float* frame = d_in + (size_t)f * vol;
-    gradient3d_kernel<<<grid_of((long long)vol), 256, 0, s>>>(frame, S, H, W, G, G + vol,
-                                                               G + 2 * vol);
-    NX_CUDA_TRY(cudaGetLastError());
-    const float *img, *gx, *gy, *gz;
-    if (mxy > 1) {
-      NX_CUDA_TRY(launch_cr_shift_magnify(frame, S, H, W, zeros, zeros, (float)mxy, (float)mxy,
-                                          p.Hm, p.Wm, M, s));
-      NX_CUDA_TRY(launch_cr_shift_magnify(G, 3 * S, H, W, zeros, zeros, (float)mxy, (float)mxy,
-                                          p.Hm, p.Wm, M + volm, s));
-      img = M;
-      gx = M + volm;
-      gy = M + 2 * volm;
-      gz = M + 3 * volm;
-    } else {
-      img = frame;
-      gx = G;
-      gy = G + vol;
-      gz = G + 2 * vol;
+  const int ncol = p.Wm - 2 * p.margin, nrow = p.Hm - 2 * p.margin, nz = p.Sm - 2 * p.margin_z;
+  const bool inside = ncol > 0 && nrow > 0 && nz > 0;
+  // input slices that hold a voxel inside the z margins
+  const int sa = p.margin_z / mz, sb = inside ? (p.Sm - p.margin_z - 1) / mz : sa - 1;
+  const unsigned prep_blocks = (unsigned)((p.Wm + kPrepCols - 1) / kPrepCols) *
+                               (unsigned)((p.Hm + kPrepRows - 1) / kPrepRows);
+  const unsigned rgc_blocks =
+      inside ? (unsigned)((ncol + 31) / 32) * (unsigned)((nrow + 7) / 8) : 0;
+  const size_t smem =
+      (size_t)prep_extent(kPrepRows, mxy) * prep_extent(kPrepCols, mxy) * 2 * sizeof(float4);
+  for (int f = 0; f < T && inside; f += 2) {
+    const float* f0 = d_in + (size_t)f * vol;
+    const int two = f + 1 < T;  // an odd last frame stands in for its partner
+    for (int z = 0; z < S; z += 65535) {  // grid.y limit
+      prep3d_kernel<<<dim3(prep_blocks, (unsigned)std::min(S - z, 65535)), kPrepThreads, smem,
+                      s>>>(f0, two ? f0 + vol : f0, H, W, mxy, z, A, B, I);
+      NX_CUDA_TRY(cudaGetLastError());
     }
-    if (ninner > 0) {
-      rgc3d_kernel<<<grid_of(ninner), 256, 0, s>>>(p, gx, gy, gz, img, dtab, f, d_out, mean);
+    for (int z = sa; z <= sb; z += 65535) {
+      rgc3d_kernel<<<dim3(rgc_blocks, (unsigned)std::min(sb - z + 1, 65535)), 256, 0, s>>>(
+          p, A, B, I, dtab, z, f, two, d_out, mean);
       NX_CUDA_TRY(cudaGetLastError());
     }
   }
