@@ -16,8 +16,10 @@
 //   A[i][n] = (1/L) sum_{f=-(N-N2)}^{N2-1} e^{2 pi i f (i/L - n/N)}, N2 = ceil(N/2)
 //   C[j][m] = (1/L) sum_{k=0}^{N/2} c_k e^{2 pi i k (j/L - m/N)}, c_0 = 1, else 2
 // (the one unpaired y frequency makes A complex; the half spectrum along x
-// gives C), so the interpolation is two batched FP32 GEMMs with operators
-// formed once in float64 on the host.  FP32 on the CUDA cores, not TF32 on the
+// gives C).  That frequency alone makes A_im: A_im[i][n] = -(-1)^n sin(pi i / mag)
+// / L, so the second term is the outer product of s_i = sin(pi i / mag) / L and
+// r = (sum_n (-1)^n X[n]) C_im^T, and the interpolation is two batched FP32
+// GEMMs plus a rank-1 update, with operators formed once in float64 on the host.  FP32 on the CUDA cores, not TF32 on the
 // tensor cores: the reference transforms in float64, and a 10-bit mantissa
 // would not hold the 1e-4 parity bar.
 #include <cuda_runtime.h>
@@ -42,71 +44,6 @@ int pow2_ceil(int n) {
   int p = 1;
   while (p < n) p <<= 1;
   return p;
-}
-
-// ---------------------------------------------------------------------------
-// batched FP32 GEMM, row major: C = A B, 64 x 64 tiles, 4 x 4 per thread
-// ---------------------------------------------------------------------------
-struct GemmBatch {
-  int inner;                    // batch index z = outer * inner + inner_index
-  long long sa_o, sa_i, sb_o, sb_i, sc_o, sc_i;
-};
-
-constexpr int kGB = 64, kGK = 16;
-
-__global__ void __launch_bounds__(256) sgemm_kernel(const float* __restrict__ A,
-                                                    const float* __restrict__ B,
-                                                    float* __restrict__ C, int M, int N, int K,
-                                                    int lda, int ldb, int ldc, GemmBatch bt) {
-  __shared__ __align__(16) float As[kGK][kGB + 4];
-  __shared__ __align__(16) float Bs[kGK][kGB + 4];
-  const int zo = blockIdx.z / bt.inner, zi = blockIdx.z % bt.inner;
-  A += zo * bt.sa_o + zi * bt.sa_i;
-  B += zo * bt.sb_o + zi * bt.sb_i;
-  C += zo * bt.sc_o + zi * bt.sc_i;
-  const int m0 = blockIdx.y * kGB, n0 = blockIdx.x * kGB;
-  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-  float acc[4][4] = {};
-  for (int k0 = 0; k0 < K; k0 += kGK) {
-    for (int e = threadIdx.x; e < kGB * kGK; e += 256) {
-      const int r = e / kGK, c = e % kGK;  // A tile: row r, column c
-      const int gm = m0 + r, gk = k0 + c;
-      As[c][r] = (gm < M && gk < K) ? __ldg(A + (size_t)gm * lda + gk) : 0.f;
-      const int br = e / kGB, bc = e % kGB;  // B tile: row br, column bc
-      const int bk = k0 + br, bn = n0 + bc;
-      Bs[br][bc] = (bk < K && bn < N) ? __ldg(B + (size_t)bk * ldb + bn) : 0.f;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < kGK; ++k) {
-      const float4 a = *reinterpret_cast<const float4*>(&As[k][ty * 4]);
-      const float4 b = *reinterpret_cast<const float4*>(&Bs[k][tx * 4]);
-      const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int gm = m0 + ty * 4 + i;
-    if (gm >= M) continue;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int gn = n0 + tx * 4 + j;
-      if (gn < N) C[(size_t)gm * ldc + gn] = acc[i][j];
-    }
-  }
-}
-
-cudaError_t gemm(const float* A, const float* B, float* C, int M, int N, int K, int lda, int ldb,
-                 int ldc, int batches, const GemmBatch& bt, cudaStream_t s) {
-  const dim3 grid((unsigned)((N + kGB - 1) / kGB), (unsigned)((M + kGB - 1) / kGB),
-                  (unsigned)batches);
-  sgemm_kernel<<<grid, 256, 0, s>>>(A, B, C, M, N, K, lda, ldb, ldc, bt);
-  return cudaGetLastError();
 }
 
 // order-preserving int image of a float, for atomicMin / atomicMax
@@ -140,6 +77,252 @@ __device__ __forceinline__ void block_minmax(float lo, float hi, int* slot) {
   }
 }
 
+// ---------------------------------------------------------------------------
+// batched FP32 GEMM, row major: C = A B, 64 x 64 tiles, 4 x 4 per thread
+// ---------------------------------------------------------------------------
+struct GemmBatch {
+  int inner;                    // batch index z = outer * inner + inner_index
+  long long sa_o, sa_i, sb_o, sb_i, sc_o, sc_i;
+};
+
+// The second product's epilogue: z += s_i r_j (s given), and (min, max) of all z
+// into mm[4 batch + 2 ..] (mm given).
+struct Rank1 {
+  const float* s;     // s_i at s[i * lds]
+  long long lds;
+  const float* r;     // r_j of a batch at r[batch * N + j]
+  int* mm;
+};
+
+constexpr int kGB = 64, kGK = 16;
+
+__global__ void __launch_bounds__(256) sgemm_kernel(const float* __restrict__ A,
+                                                    const float* __restrict__ B,
+                                                    float* __restrict__ C, int M, int N, int K,
+                                                    int lda, int ldb, int ldc, GemmBatch bt,
+                                                    Rank1 u) {
+  __shared__ __align__(16) float As[kGK][kGB + 4];
+  __shared__ __align__(16) float Bs[kGK][kGB + 4];
+  const int zo = blockIdx.z / bt.inner, zi = blockIdx.z % bt.inner;
+  A += zo * bt.sa_o + zi * bt.sa_i;
+  B += zo * bt.sb_o + zi * bt.sb_i;
+  C += zo * bt.sc_o + zi * bt.sc_i;
+  const int m0 = blockIdx.y * kGB, n0 = blockIdx.x * kGB;
+  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
+  float acc[4][4] = {};
+  for (int k0 = 0; k0 < K; k0 += kGK) {
+    for (int e = threadIdx.x; e < kGB * kGK; e += 256) {
+      const int r = e / kGK, c = e % kGK;  // A tile: row r, column c
+      const int gm = m0 + r, gk = k0 + c;
+      As[c][r] = (gm < M && gk < K) ? __ldg(A + (size_t)gm * lda + gk) : 0.f;
+      const int br = e / kGB, bc = e % kGB;  // B tile: row br, column bc
+      const int bk = k0 + br, bn = n0 + bc;
+      Bs[br][bc] = (bk < K && bn < N) ? __ldg(B + (size_t)bk * ldb + bn) : 0.f;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kGK; ++k) {
+      const float4 a = *reinterpret_cast<const float4*>(&As[k][ty * 4]);
+      const float4 b = *reinterpret_cast<const float4*>(&Bs[k][tx * 4]);
+      const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+    }
+    __syncthreads();
+  }
+  float lo = INFINITY, hi = -INFINITY;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int gm = m0 + ty * 4 + i;
+    if (gm >= M) continue;
+    const float si = u.s ? __ldg(u.s + gm * u.lds) : 0.f;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int gn = n0 + tx * 4 + j;
+      if (gn >= N) continue;
+      float v = acc[i][j];
+      if (u.s) v = fmaf(si, __ldg(u.r + (size_t)blockIdx.z * N + gn), v);
+      lo = fminf(lo, v);
+      hi = fmaxf(hi, v);
+      C[(size_t)gm * ldc + gn] = v;
+    }
+  }
+  if (u.mm) block_minmax(lo, hi, u.mm + 4 * blockIdx.z + 2);
+}
+
+
+// The same product in 128 x 128 tiles, 8 x 8 per thread on packed f32x2 (two
+// columns per register pair), the next K slice loaded into registers behind the
+// current one and stored to the other half of a double buffer.  Needs K a
+// multiple of 16, N and the leading dimensions multiples of 4 and 16-byte
+// aligned operands; M is guarded per row.
+constexpr int kBT = 128, kBK = 16;
+__global__ void __launch_bounds__(256, 2)
+    sgemm_big_kernel(const float* __restrict__ A, const float* __restrict__ B,
+                     float* __restrict__ C, int M, int N, int K, int lda, int ldb, int ldc,
+                     GemmBatch bt, Rank1 u) {
+  __shared__ __align__(16) float As[2][kBK][kBT + 4];
+  __shared__ __align__(16) float Bs[2][kBK][kBT];
+  const int zo = blockIdx.z / bt.inner, zi = blockIdx.z % bt.inner;
+  A += zo * bt.sa_o + zi * bt.sa_i;
+  B += zo * bt.sb_o + zi * bt.sb_i;
+  C += zo * bt.sc_o + zi * bt.sc_i;
+  const int m0 = blockIdx.y * kBT, n0 = blockIdx.x * kBT;
+  const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
+  // staging: thread t loads A rows t / 4 and + 64, K quad t % 4, and B rows
+  // t / 32 and + 8, column quad t % 32
+  const int ar = tid / 4, ak = tid % 4 * 4, br = tid / 32, bc = tid % 32 * 4;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 pa[2], pb[2];
+  auto load = [&](int k0) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int gm = m0 + ar + 64 * h;
+      pa[h] = gm < M ? __ldg(reinterpret_cast<const float4*>(A + (size_t)gm * lda + k0 + ak)) : zero;
+      pb[h] = n0 + bc < N ? __ldg(reinterpret_cast<const float4*>(
+                                B + (size_t)(k0 + br + 8 * h) * ldb + n0 + bc))
+                          : zero;
+    }
+  };
+  auto store = [&](int b) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      As[b][ak][ar + 64 * h] = pa[h].x;
+      As[b][ak + 1][ar + 64 * h] = pa[h].y;
+      As[b][ak + 2][ar + 64 * h] = pa[h].z;
+      As[b][ak + 3][ar + 64 * h] = pa[h].w;
+      *reinterpret_cast<float4*>(&Bs[b][br + 8 * h][bc]) = pb[h];
+    }
+  };
+  // rows ty * 4 + {0..3} and 64 + ..., columns tx * 4 + {0..3} and 64 + ...
+  float2 acc[8][4];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = make_float2(0.f, 0.f);
+  load(0);
+  store(0);
+  __syncthreads();
+  int b = 0;
+  for (int k0 = 0; k0 < K; k0 += kBK, b ^= 1) {
+    const bool more = k0 + kBK < K;
+    if (more) load(k0 + kBK);
+#pragma unroll
+    for (int k = 0; k < kBK; ++k) {
+      const float4 a0 = *reinterpret_cast<const float4*>(&As[b][k][ty * 4]);
+      const float4 a1 = *reinterpret_cast<const float4*>(&As[b][k][64 + ty * 4]);
+      const float4 b0 = *reinterpret_cast<const float4*>(&Bs[b][k][tx * 4]);
+      const float4 b1 = *reinterpret_cast<const float4*>(&Bs[b][k][64 + tx * 4]);
+      const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+      const float2 bv[4] = {make_float2(b0.x, b0.y), make_float2(b0.z, b0.w),
+                            make_float2(b1.x, b1.y), make_float2(b1.z, b1.w)};
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          acc[i][j] = __ffma2_rn(make_float2(av[i], av[i]), bv[j], acc[i][j]);
+    }
+    if (more) store(b ^ 1);
+    __syncthreads();
+  }
+  float lo = INFINITY, hi = -INFINITY;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int gm = m0 + ty * 4 + (i & 3) + (i >> 2) * 64;
+    if (gm >= M) continue;
+    const float si = u.s ? __ldg(u.s + gm * u.lds) : 0.f;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int gn = n0 + tx * 4 + 64 * h;
+      if (gn >= N) continue;
+      float4 v = make_float4(acc[i][2 * h].x, acc[i][2 * h].y, acc[i][2 * h + 1].x,
+                             acc[i][2 * h + 1].y);
+      if (u.s) {
+        const float4 r = __ldg(reinterpret_cast<const float4*>(u.r + (size_t)blockIdx.z * N + gn));
+        v = make_float4(fmaf(si, r.x, v.x), fmaf(si, r.y, v.y), fmaf(si, r.z, v.z),
+                        fmaf(si, r.w, v.w));
+      }
+      lo = fminf(lo, fminf(fminf(v.x, v.y), fminf(v.z, v.w)));
+      hi = fmaxf(hi, fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)));
+      *reinterpret_cast<float4*>(C + (size_t)gm * ldc + gn) = v;
+    }
+  }
+  if (u.mm) block_minmax(lo, hi, u.mm + 4 * blockIdx.z + 2);
+}
+
+// operands the big tiles can take, and sizes they fill; else 64 x 64 tiles.
+// The 8 frames of 300 x 260 at m = 2 (24 products of 256- and 128-pixel squares):
+// 2.97 ms in 64 x 64 tiles with both parts of A, 1.08 ms now.
+bool big_tiles(const float* A, const float* B, const float* C, int M, int N, int K, int lda,
+               int ldb, int ldc, const GemmBatch& bt, const Rank1& u) {
+  const uintptr_t ptrs = reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) |
+                         reinterpret_cast<uintptr_t>(C) | reinterpret_cast<uintptr_t>(u.r);
+  const long long strides = lda | ldb | ldc | bt.sa_o | bt.sa_i | bt.sb_o | bt.sb_i | bt.sc_o |
+                            bt.sc_i;
+  return (ptrs & 15u) == 0 && strides % 4 == 0 && K % kBK == 0 && N % 4 == 0 && M >= 96 && N >= 96;
+}
+
+cudaError_t gemm(const float* A, const float* B, float* C, int M, int N, int K, int lda, int ldb,
+                 int ldc, int batches, const GemmBatch& bt, const Rank1& u, cudaStream_t s) {
+  if (big_tiles(A, B, C, M, N, K, lda, ldb, ldc, bt, u)) {
+    const dim3 grid((unsigned)((N + kBT - 1) / kBT), (unsigned)((M + kBT - 1) / kBT),
+                    (unsigned)batches);
+    sgemm_big_kernel<<<grid, 256, 0, s>>>(A, B, C, M, N, K, lda, ldb, ldc, bt, u);
+  } else {
+    const dim3 grid((unsigned)((N + kGB - 1) / kGB), (unsigned)((M + kGB - 1) / kGB),
+                    (unsigned)batches);
+    sgemm_kernel<<<grid, 256, 0, s>>>(A, B, C, M, N, K, lda, ldb, ldc, bt, u);
+  }
+  return cudaGetLastError();
+}
+
+// a[z][c] = sum_n (-1)^n X[z][n][c]
+__global__ void __launch_bounds__(256) fht_alternate_kernel(const float* __restrict__ X, int N,
+                                                            float* __restrict__ a) {
+  __shared__ float red[8][32];
+  const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
+  const int c = blockIdx.x * 32 + lane;
+  const float* x = X + (size_t)blockIdx.y * N * N;
+  float even = 0.f, odd = 0.f;  // rows g, g + 8, ... have one parity
+  if (c < N)
+    for (int n = g; n < N; n += 8) {
+      if (n & 1) odd += __ldg(x + (size_t)n * N + c);
+      else even += __ldg(x + (size_t)n * N + c);
+    }
+  red[g][lane] = even - odd;
+  __syncthreads();
+  if (g == 0 && c < N) {
+    float t = 0.f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) t += red[k][lane];
+    a[(size_t)blockIdx.y * N + c] = t;
+  }
+}
+
+// r[z][j] = sum_c a[z][c] Cim[c][j]
+__global__ void __launch_bounds__(256) fht_rank1_kernel(const float* __restrict__ a,
+                                                        const float* __restrict__ Cim, int N,
+                                                        int L, float* __restrict__ r) {
+  __shared__ float red[8][32];
+  const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
+  const int j = blockIdx.x * 32 + lane;
+  const float* az = a + (size_t)blockIdx.y * N;
+  float t = 0.f;
+  if (j < L) {
+#pragma unroll 4
+    for (int c = g; c < N; c += 8) t = fmaf(__ldg(az + c), __ldg(Cim + (size_t)c * L + j), t);
+  }
+  red[g][lane] = t;
+  __syncthreads();
+  if (g == 0 && j < L) {
+#pragma unroll
+    for (int k = 1; k < 8; ++k) t += red[k][lane];
+    r[(size_t)blockIdx.y * L + j] = t;
+  }
+}
+
 // mirror-padded N x N square of tile (r0, c0, th, tw) of every frame of the
 // chunk; slot[z] = (min, max) of the tile (every tile pixel is in the square:
 // the upright centre copy lies inside the central crop)
@@ -167,32 +350,19 @@ __global__ void fht_mm_init_kernel(int* __restrict__ mm, int n) {
   for (int k = threadIdx.x; k < 4 * n; k += blockDim.x) mm[k] = (k & 1) ? INT_MIN : INT_MAX;
 }
 
-__global__ void fht_zminmax_kernel(const float* __restrict__ Z, long long n,
-                                   int* __restrict__ mm) {
-  const int z = blockIdx.y;
-  const float* p = Z + (size_t)z * n;
-  float lo = INFINITY, hi = -INFINITY;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n;
-       e += (long long)gridDim.x * blockDim.x) {
-    const float v = p[e];
-    lo = fminf(lo, v);
-    hi = fmaxf(hi, v);
-  }
-  block_minmax(lo, hi, mm + 4 * z + 2);
-}
-
 // rescale onto the tile's [min, max] (the reference's float32 steps
 // -= out_min, *= scale, += orig_min), crop, and either store (one piece) or
 // add the Hann-weighted piece (tiled: output += piece * outer(wr, wc)).
 // The scale is a float64 quotient of the float32 extremes rounded once
 // (interpolation.py takes the extremes as Python floats), or float32
 // arithmetic throughout (f32_scale: _interpolation.pyx keeps them in C floats).
+constexpr int kFinishRows = 8;  // rows per thread: no index division, loads in flight
 __global__ void fht_finish_kernel(const float* __restrict__ Z, int L, const int* __restrict__ mm,
                                   int oh, int ow, int y_roi, int x_roi,
                                   const float* __restrict__ wr, const float* __restrict__ wc,
                                   float* __restrict__ out, int outH, int outW, int R0, int C0,
                                   int f32_scale) {
-  const int z = blockIdx.y;
+  const int z = blockIdx.z;
   const float lo = unordered(mm[4 * z]), hi = unordered(mm[4 * z + 1]);
   const float zlo = unordered(mm[4 * z + 2]), zhi = unordered(mm[4 * z + 3]);
   const bool resc = zhi != zlo;
@@ -201,20 +371,19 @@ __global__ void fht_finish_kernel(const float* __restrict__ Z, int L, const int*
     scale = f32_scale ? __fdiv_rn(__fsub_rn(hi, lo), __fsub_rn(zhi, zlo))
                       : __double2float_rn(__ddiv_rn((double)hi - (double)lo,
                                                     (double)zhi - (double)zlo));
-  const float* zp = Z + (size_t)z * L * L;
-  float* o = out + (size_t)z * outH * outW;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < (long long)oh * ow;
-       e += (long long)gridDim.x * blockDim.x) {
-    const int y = (int)(e / ow), x = (int)(e % ow);
-    float v = zp[(size_t)(y_roi + y) * L + (x_roi + x)];
+  const int x = blockIdx.x * blockDim.x + threadIdx.x;
+  if (x >= ow) return;
+  const float wx = wr ? wc[x] : 1.f;
+  const int y1 = min(oh, (int)(blockIdx.y + 1) * kFinishRows);
+  int y = blockIdx.y * kFinishRows;
+  const float* zp = Z + (size_t)z * L * L + (size_t)(y_roi + y) * L + x_roi + x;
+  float* o = out + (size_t)z * outH * outW + (size_t)(R0 + y) * outW + C0 + x;
+#pragma unroll 4
+  for (; y < y1; ++y, zp += L, o += outW) {
+    float v = *zp;
     if (resc) v = __fadd_rn(__fmul_rn(__fsub_rn(v, zlo), scale), lo);
-    const size_t oi = (size_t)(R0 + y) * outW + (C0 + x);
-    if (wr) {
-      const float win = __fmul_rn(wr[y], wc[x]);
-      o[oi] = __fadd_rn(o[oi], __fmul_rn(v, win));
-    } else {
-      o[oi] = v;
-    }
+    if (wr) *o = __fadd_rn(*o, __fmul_rn(v, __fmul_rn(wr[y], wx)));
+    else *o = v;
   }
 }
 
@@ -229,12 +398,16 @@ __global__ void fht_weight_kernel(const float* __restrict__ wr, const float* __r
   }
 }
 
+// a pixel's weight is read once for all frames
 __global__ void fht_normalize_kernel(float* __restrict__ out, const float* __restrict__ wgt,
                                      long long plane, int frames) {
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < plane * frames;
+  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < plane;
        e += (long long)gridDim.x * blockDim.x) {
-    const float w = wgt[e % plane];
-    if (w > 0.f) out[e] = __fdiv_rn(out[e], w);
+    const float w = wgt[e];
+    if (!(w > 0.f)) continue;
+    float* o = out + e;
+#pragma unroll 4
+    for (int f = 0; f < frames; ++f, o += plane) *o = __fdiv_rn(*o, w);
   }
 }
 
@@ -415,7 +588,9 @@ int nx_fht_plan_create_ex(nx_fht_plan** out, int H, int W, int magnification, in
     }
   for (const auto& o : p->ops)
     p->frame_floats = std::max(p->frame_floats,
-                               (size_t)o.N * o.N + (size_t)2 * o.N * o.L + (size_t)o.L * o.L);
+                               (size_t)o.N * o.N +
+                                   (size_t)(variant == NX_FHT_FULL_SPECTRUM ? 2 : 1) * o.N * o.L +
+                                   (size_t)o.L * o.L + o.L + o.N);
   if (p->tiled) {
     // blending weights: the windows summed in the reference's tile order
     const size_t plane = (size_t)H * magnification * W * magnification;
@@ -469,6 +644,7 @@ int nx_fht_interpolate(const nx_fht_plan* p, const float* d_in, int T, float* d_
   }
   cudaStream_t s = (cudaStream_t)stream;
   const int mag = p->mag;
+  const bool full = p->variant == NX_FHT_FULL_SPECTRUM;
   const int outH = p->H * mag, outW = p->W * mag;
   const long long plane = (long long)outH * outW;
   char* base = (char*)d_ws + 256;
@@ -485,7 +661,9 @@ int nx_fht_interpolate(const nx_fht_plan* p, const float* d_in, int T, float* d_
       const int N = o.N, L = o.L;
       float* X = work;
       float* U = X + (size_t)tc * N * N;
-      float* Z = U + (size_t)tc * 2 * N * L;
+      float* Z = U + (size_t)tc * (full ? 2 : 1) * N * L;
+      float* r = Z + (size_t)tc * L * L;
+      float* alt = r + (size_t)tc * L;
       // (min, max) slots of the tile input and of the interpolated square
       fht_mm_init_kernel<<<1, 32, 0, s>>>(mm, tc);
       NX_CUDA_TRY(cudaGetLastError());
@@ -493,25 +671,41 @@ int nx_fht_interpolate(const nx_fht_plan* p, const float* d_in, int T, float* d_
                           s>>>(in, p->H, p->W, t.r0, t.c0, t.th, t.tw, N, t.kh, t.kw, t.y_roi,
                                t.x_roi, X, mm);
       NX_CUDA_TRY(cudaGetLastError());
-      // U = X [C_re^T | C_im^T] stacked: batch (frame, part)
-      GemmBatch b1{2, (long long)N * N, 0, 0, (long long)N * L, (long long)2 * N * L,
-                   (long long)N * L};
-      NX_CUDA_TRY(gemm(X, o.ct, U, N, L, N, N, L, L, 2 * tc, b1, s));
-      // Z = [A_re | -A_im] [U_re ; U_im]
-      GemmBatch b2{1, 0, 0, (long long)2 * N * L, 0, (long long)L * L, 0};
-      NX_CUDA_TRY(gemm(o.acat, U, Z, L, L, 2 * N, 2 * N, L, L, tc, b2, s));
-      fht_zminmax_kernel<<<dim3(blocks_for((long long)L * L, 256, 512), (unsigned)tc), 256, 0,
-                           s>>>(Z, (long long)L * L, mm);
-      NX_CUDA_TRY(cudaGetLastError());
+      if (full) {
+        // U = X [C_re^T | C_im^T] stacked (batch (frame, part)), then
+        // Z = [A_re | -A_im] [U_re ; U_im]: one image per sweep, whose scores
+        // keep their bits
+        const GemmBatch b1{2, (long long)N * N, 0, 0, (long long)N * L, (long long)2 * N * L,
+                           (long long)N * L};
+        NX_CUDA_TRY(gemm(X, o.ct, U, N, L, N, N, L, L, 2 * tc, b1, Rank1{}, s));
+        const GemmBatch b2{1, 0, 0, (long long)2 * N * L, 0, (long long)L * L, 0};
+        NX_CUDA_TRY(gemm(o.acat, U, Z, L, L, 2 * N, 2 * N, L, L, tc, b2,
+                         Rank1{nullptr, 0, nullptr, mm}, s));
+      } else {
+        // r of the rank-1 term, then U = X C_re^T (the frames' squares stacked) and
+        // Z = A_re U + s r^T
+        fht_alternate_kernel<<<dim3((unsigned)((N + 31) / 32), (unsigned)tc), 256, 0, s>>>(X, N,
+                                                                                           alt);
+        NX_CUDA_TRY(cudaGetLastError());
+        fht_rank1_kernel<<<dim3((unsigned)((L + 31) / 32), (unsigned)tc), 256, 0, s>>>(
+            alt, o.ct + (size_t)N * L, N, L, r);
+        NX_CUDA_TRY(cudaGetLastError());
+        NX_CUDA_TRY(gemm(X, o.ct, U, tc * N, L, N, N, L, L, 1, GemmBatch{1, 0, 0, 0, 0, 0, 0},
+                         Rank1{}, s));
+        const GemmBatch b2{1, 0, 0, (long long)N * L, 0, (long long)L * L, 0};
+        NX_CUDA_TRY(gemm(o.acat, U, Z, L, L, N, 2 * N, L, L, tc, b2,
+                         Rank1{o.acat + N, 2LL * N, r, mm}, s));
+      }
       const int oh = t.th * mag, ow = t.tw * mag;
-      fht_finish_kernel<<<dim3(blocks_for((long long)oh * ow, 256, 1024), (unsigned)tc), 256, 0,
-                          s>>>(Z, L, mm, oh, ow, (L - oh) / 2, (L - ow) / 2,
+      fht_finish_kernel<<<dim3((unsigned)((ow + 127) / 128),
+                               (unsigned)((oh + kFinishRows - 1) / kFinishRows), (unsigned)tc),
+                          128, 0, s>>>(Z, L, mm, oh, ow, (L - oh) / 2, (L - ow) / 2,
                                p->tiled ? t.wr : nullptr, p->tiled ? t.wc : nullptr, out, outH,
-                               outW, t.r0 * mag, t.c0 * mag, p->variant == NX_FHT_FULL_SPECTRUM);
+                               outW, t.r0 * mag, t.c0 * mag, full);
       NX_CUDA_TRY(cudaGetLastError());
     }
     if (p->tiled) {
-      fht_normalize_kernel<<<blocks_for(plane * tc), 256, 0, s>>>(out, p->wgt, plane, tc);
+      fht_normalize_kernel<<<blocks_for(plane), 256, 0, s>>>(out, p->wgt, plane, tc);
       NX_CUDA_TRY(cudaGetLastError());
     }
   }
