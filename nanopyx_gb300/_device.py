@@ -89,12 +89,14 @@ def stream_ptr(device=None) -> int:
     return torch.cuda.current_stream(device).cuda_stream
 
 
-def workspace(nbytes: int, device=None) -> torch.Tensor:
+def workspace(nbytes: int, device=None, zero_status: bool = True) -> torch.Tensor:
     """Device scratch for one C-ABI call; its first 256 bytes (the device status
-    word the kernels report bounded-wait timeouts into) start at zero."""
+    word the kernels report bounded-wait timeouts into) start at zero, unless the
+    call clears its status itself (``zero_status=False``: one launch less)."""
     device = device if device is not None else torch.device("cuda", torch.cuda.current_device())
     ws = torch.empty(max(int(nbytes), 256), dtype=torch.uint8, device=device)
-    ws[:256].zero_()
+    if zero_status:
+        ws[:256].zero_()
     return ws
 
 

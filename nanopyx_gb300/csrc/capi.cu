@@ -222,23 +222,43 @@ static int check_plan(const nx_esrrf_plan* p) {
   return NX_OK;
 }
 
-// chunking of each timepoint's frames across CTAs (deterministic in its inputs)
-// Frame chunks per timepoint of a launch over `tiles` x `n_tp` units.  The
-// resident CTAs stride over (tile, timepoint, chunk) units, so a CTA runs
-// about ceil(units / resident) units, each costing its frame passes plus a
-// start-up of ~0.65 pass (the unit's first pass is not overlapped with the
-// producer warps' preparation).  The chunk count with the smallest estimate
-// wins: few chunks for large stacks, enough to fill every SM for small ones,
-// and >= 4 frames per chunk.
+// Frame chunks per timepoint of a launch over `tiles` x `n_tp` units
+// (deterministic in its inputs).  The resident CTAs stride over (tile, timepoint,
+// chunk) units, so a CTA runs about ceil(units / resident) units, each costing
+// its frame pairs plus a start-up of about 1.35 pairs (its constants and the
+// first pass, which nothing overlaps: 100 x 256 x 256, m = 5 in chunks of 1, 2,
+// 4, 6, 50, 100 frames takes 19.0, 19.1, 27.4, 36.2, 213, 411 us per unit at
+// 8.2 us a pair).  The chunk count with the smallest estimate wins: few chunks
+// for large stacks, enough to fill every SM for small ones; stacks below 8 frames
+// (two passes) stay whole, so that they give the bits of a streamed block.
 static int best_chunks(long long tiles, int n_tp, int fpt, int min_nf, long long resident) {
+  int best = 1;
+  double best_cost = 1e300;
+  const int cmax = min_nf < 8 ? 1 : std::min(min_nf / 2, 64);
+  for (int c = 1; c <= cmax; ++c) {
+    const long long units = tiles * n_tp * c;
+    const double per_cta = (double)((units + resident - 1) / resident);
+    const double pairs = ((fpt + c - 1) / c + 1) / 2;
+    const double cost = per_cta * (pairs + 1.35);
+    if (cost < best_cost * 0.999) {
+      best_cost = cost;
+      best = c;
+    }
+  }
+  return best;
+}
+
+// The chunks of an AVG sweep at m <= 2, the scored sweep's magnification: its
+// scores are published to full precision, so the split of its sums stays what
+// it was (passes of two frames, a start-up of 0.65 pass, >= 4 frames a chunk).
+static int sweep_chunks(long long tiles, int n_tp, int fpt, int min_nf, long long resident) {
   int best = 1;
   double best_cost = 1e300;
   const int cmax = std::max(1, std::min(min_nf / 4, 64));
   for (int c = 1; c <= cmax; ++c) {
     const long long units = tiles * n_tp * c;
     const double per_cta = (double)((units + resident - 1) / resident);
-    const double passes = std::ceil((double)fpt / c / 2.0);
-    const double cost = per_cta * (passes + 0.65);
+    const double cost = per_cta * (std::ceil((double)fpt / c / 2.0) + 0.65);
     if (cost < best_cost * 0.999) {
       best_cost = cost;
       best = c;
@@ -834,7 +854,8 @@ int nx_esrrf_batch_create(nx_esrrf_batch** out, const nx_esrrf_item* items, int 
       const long long tiles = (long long)((p->W + 31) / 32) * ((p->H + p->fused->geo.TY - 1) / p->fused->geo.TY);
       const long long resident =
           (long long)std::max(1, p->fused->occupancy[bi.mode](std::max(1, it.n_sens))) * sms;
-      const int c = best_chunks(tiles, bi.n_tp, bi.fpt, min_nf, resident);
+      const auto rule = it.n_sens > 0 && p->M <= 2 ? sweep_chunks : best_chunks;
+      const int c = rule(tiles, bi.n_tp, bi.fpt, min_nf, resident);
       fpu = std::max(1, (min_nf + c - 1) / c);
     }
     bi.chunks = std::max(1, std::min(min_nf, (min_nf + fpu - 1) / fpu));

@@ -247,20 +247,37 @@ __device__ __forceinline__ float clamp0(float v) {
   return r;
 }
 
-// r ^ sensitivity of a thread's values (mode and n are uniform over the launch)
-template <int A, int B>
+// The powers that are not worth their code in every unrolled use.
+static __device__ __noinline__ float apply_sensitivity_slow(float r, int mode, int n, float s) {
+  return apply_sensitivity(r, mode, n, s);
+}
+
+// r ^ sensitivity of a thread's values (mode and n are uniform over the launch):
+// squares and cubes, and (HALF) the half-integer powers below 4, in place; the
+// others by call -- with powf and the square root inlined per sensitivity and
+// column, the AVG kernels' code outgrew the instruction cache (4 x 4 sweep of
+// 200 x 256 x 256, m = 4: 13.46 against 12.39 ms).
+template <bool HALF, int A, int B>
 __device__ __forceinline__ void apply_sens_all(float2 (&r)[A][B], int mode, int n, float s) {
   if (mode == 0) return;
-  if (mode != 2 && n <= 3) {
-    // n = 1 .. 3, times the square root for a half-integer power
+  if (mode == 1 && n <= 3) {
+#pragma unroll
+    for (int i = 0; i < A; ++i)
+#pragma unroll
+      for (int j = 0; j < B; ++j) {
+        const float2 q = __fmul2_rn(r[i][j], r[i][j]);
+        r[i][j] = n == 3 ? __fmul2_rn(q, r[i][j]) : q;
+      }
+    return;
+  }
+  if (HALF && mode == 3 && n <= 3) {
 #pragma unroll
     for (int i = 0; i < A; ++i)
 #pragma unroll
       for (int j = 0; j < B; ++j) {
         const float2 b = r[i][j], q = __fmul2_rn(b, b);
-        float2 v = n == 1 ? b : (n == 3 ? __fmul2_rn(q, b) : q);
-        if (mode == 3) v = __fmul2_rn(v, make_float2(__fsqrt_rn(b.x), __fsqrt_rn(b.y)));
-        r[i][j] = v;
+        const float2 v = n == 1 ? b : (n == 3 ? __fmul2_rn(q, b) : q);
+        r[i][j] = __fmul2_rn(v, make_float2(__fsqrt_rn(b.x), __fsqrt_rn(b.y)));
       }
     return;
   }
@@ -268,8 +285,8 @@ __device__ __forceinline__ void apply_sens_all(float2 (&r)[A][B], int mode, int 
   for (int i = 0; i < A; ++i)
 #pragma unroll
     for (int j = 0; j < B; ++j)
-      r[i][j] = make_float2(apply_sensitivity(r[i][j].x, mode, n, s),
-                            apply_sensitivity(r[i][j].y, mode, n, s));
+      r[i][j] = make_float2(apply_sensitivity_slow(r[i][j].x, mode, n, s),
+                            apply_sensitivity_slow(r[i][j].y, mode, n, s));
 }
 
 // geometry of one unit (tile, timepoint, frame chunk), shared by both roles
@@ -529,18 +546,16 @@ struct RgcCore {
   const float4* tb4;  // phase table of row phase py0
   int cpy;            // of every phase of the thread unless PYT = M
 
-  // row k of the slot (rows from 2 ty on) for the phases d0 .. d1 - 1
+  // one row of the slot (at r) for the phases D0 .. D1 - 1; tb: the table of
+  // phase 0 at that row, were its cpy that of every phase
   template <int D0, int D1>
-  __device__ __forceinline__ void row(int k, float2 (&acc)[NPR][PYT * M]) const {
-    const float4* r0 = hg + (k * 2 + 0) * G::HGP;
-    const float4* r1 = hg + (k * 2 + 1) * G::HGP;
+  __device__ __forceinline__ static void row(const float4* r, const float4* tb,
+                                             float2 (&acc)[NPR][PYT * M]) {
     auto grad = [&](int pp, int q) {
-      return (q & 1) ? r1[pp * G::HG_PLANE + (q >> 1)] : r0[pp * G::HG_PLANE + (q >> 1)];
+      return r[(q & 1) * G::HGP + pp * G::HG_PLANE + (q >> 1)];
     };
-    // window row of phase d: k - cpy(d)
     auto table = [&](int d) {
-      const int c = PYT == M ? (2 * d + 1) / M : cpy;
-      return tb4 + (d * G::W2 + k - c) * G::NE;
+      return tb + (d * G::W2 - (PYT == M && M > 1 ? (2 * d + 1) / M : 0)) * G::NE;
     };
     auto sample = [&](int px, int q, const float4& g, float rho, float nrho, const float4& T,
                       float2& a) {
@@ -606,15 +621,21 @@ struct RgcCore {
       for (int o = 0; o < PYT * M; ++o) acc[pp][o] = make_float2(0.f, 0.f);
     // window rows stay a loop: unrolled, the core's code outgrows the
     // instruction cache (measured 2 % slower and with register spills)
+    const float4* r = hg + cpy * 2 * G::HGP;
+    const float4* t = tb4;
     if constexpr (PYT == M && M > 1) {
       constexpr int DH = M / 2;  // phases d < DH have cpy = 0
-      row<0, DH>(0, acc);
+      row<0, DH>(r, t, acc);
 #pragma unroll 1
-      for (int k = 1; k < G::NQ - 1; ++k) row<0, M>(k, acc);
-      row<DH, M>(G::NQ - 1, acc);
+      for (int k = 1; k < G::NQ - 1; ++k) {
+        r += 2 * G::HGP;
+        t += G::NE;
+        row<0, M>(r, t, acc);
+      }
+      row<DH, M>(r + 2 * G::HGP, t + G::NE, acc);
     } else {
 #pragma unroll 1
-      for (int k = cpy; k < cpy + G::W2; ++k) row<0, PYT>(k, acc);
+      for (int k = 0; k < G::W2; ++k, r += 2 * G::HGP, t += G::NE) row<0, PYT>(r, t, acc);
     }
   }
 };
@@ -946,7 +967,7 @@ __global__ void __launch_bounds__(32 * TY * (M / PYT) + NP, EsrrfTile<M>::MIN_BL
           acc[pp][o] = make_float2(clamp0(acc[pp][o].x * twv), clamp0(acc[pp][o].y * twv));
       }
       if (MODE != kModeSum)
-        apply_sens_all(acc, p.sens_mode_k[0], p.sens_int_k[0], p.sens_k[0]);
+        apply_sens_all<true>(acc, p.sens_mode_k[0], p.sens_int_k[0], p.sens_k[0]);
 #pragma unroll
       for (int d = 0; d < PYT; ++d) {
       const int py = py0 + d, yM = ny * M + py;
@@ -1021,7 +1042,7 @@ __global__ void __launch_bounds__(32 * TY * (M / PYT) + NP, EsrrfTile<M>::MIN_BL
             float2 r[G::NPR][1];
 #pragma unroll
             for (int pp = 0; pp < G::NPR; ++pp) r[pp][0] = acc[pp][d * M + px];
-            apply_sens_all(r, smode, sint, sval);
+            apply_sens_all<false>(r, smode, sint, sval);
 #pragma unroll
             for (int pp = 0; pp < G::NPR; ++pp) {
               r[pp][0] = __fmul2_rn(r[pp][0], ival[pp][px]);

@@ -59,7 +59,8 @@ def esrrf_device(stack: torch.Tensor, magnification: int = 5, radius: float = 1.
     m = int(magnification)
     plan = get_plan(H, W, m, radius, sensitivity, doIntensityWeighting)
     L = N.lib()
-    ws = workspace(L.nx_esrrf_workspace_bytes(plan.handle, T, fpt, mask), stack.device)
+    ws = workspace(L.nx_esrrf_workspace_bytes(plan.handle, T, fpt, mask), stack.device,
+                   zero_status=False)
     order = [b for b in ("AVG", "VAR", "TAC2") if mask & N.CORR_BITS[b]]
     out = torch.empty((len(order), n_tp, H * m, W * m), dtype=torch.float32, device=stack.device)
     N.check(L.nx_esrrf_run(plan.handle, stack.data_ptr(), T, fpt, mask,
@@ -270,7 +271,7 @@ def SRRF(image, magnification: int = 5, ringRadius: float = 0.5, border: int = 0
     m = int(magnification)
     L = N.lib()
     out = torch.empty((T, h * m, w * m), dtype=torch.float32, device=st.t.device)
-    ws = workspace(L.nx_srrf_workspace_bytes(T, h, w, m), st.t.device)
+    ws = workspace(L.nx_srrf_workspace_bytes(T, h, w, m), st.t.device, zero_status=False)
     N.check(L.nx_srrf(st.ptr(), T, h, w, m, float(ringRadius), int(border),
                       1 if radialityPositivityConstraint else 0, 1 if doIntensityWeighting else 0,
                       1 if macro_pixel_correction else 0, out.data_ptr(), ws.data_ptr(),

@@ -214,7 +214,8 @@ class eSRRF_ST(LiquidEngine):
         plan = get_plan(H, W, m, radius, sensitivity, doIntensityWeighting)
         out = _empty((T, H * m, W * m), img)
         L = N.lib()
-        ws = workspace(L.nx_esrrf_st_workspace_bytes(plan.handle, T), img.t.device)
+        ws = workspace(L.nx_esrrf_st_workspace_bytes(plan.handle, T), img.t.device,
+                       zero_status=T == 0)  # a call without frames clears nothing
         N.check(L.nx_esrrf_st(plan.handle, img.ptr(), T, _ptr(out), _ptr(ws), ws.numel(),
                               stream_ptr()), "eSRRF_ST")
         N.check(L.nx_workspace_status(_ptr(ws), stream_ptr()), "eSRRF_ST")
