@@ -329,6 +329,15 @@ size_t nx_moment_sums_workspace_bytes(int batch);
 int nx_moment_sums(const float* d_x, const float* d_y, long long n, int batch, double* d_sums,
                    void* d_ws, size_t ws_bytes, void* stream);
 
+/* One step of the error map's blur-width search: n images of the stack d_in
+ * (image src_index[i], or i) blurred as nx_gaussian_blur_batch and their
+ * moments against d_y (H, W) as nx_moment_sums, in one call.  h_sums (n, 6) is
+ * page-locked host memory (or device memory); the sums are there on return.  */
+size_t nx_blur_moments_workspace_bytes(int H, int W, int n);
+int nx_blur_moments(const float* d_in, int H, int W, int n, const int* src_index,
+                    const double* sigma, const float* d_y, double* h_sums, void* d_ws,
+                    size_t ws_bytes, void* stream);
+
 /* Fourier ring correlation sums of `pairs` image pairs
  * (src/nanopyx/core/analysis/frc.pyx:108-143,150-179,181-198): in pair q the
  * N x N windows at (r0, c0) of d_img1 + q stride and d_img2 + q stride (row

@@ -112,6 +112,8 @@ _SIGS = {
     "nx_decorr_coefs": (_I, [_P, _P, _P, _I, _I, C.c_float, C.c_float, _I, _P, _P, _P, _SZ, _P]),
     "nx_moment_sums_workspace_bytes": (_SZ, [_I]),
     "nx_moment_sums": (_I, [_P, _P, C.c_longlong, _I, _P, _P, _SZ, _P]),
+    "nx_blur_moments_workspace_bytes": (_SZ, [_I, _I, _I]),
+    "nx_blur_moments": (_I, [_P, _I, _I, _I, _P, _P, _P, _P, _P, _SZ, _P]),
     "nx_frc_plan_create": (_I, [C.POINTER(_P), _I]),
     "nx_frc_plan_destroy": (_I, [_P]),
     "nx_frc_rings": (_I, [_P]),

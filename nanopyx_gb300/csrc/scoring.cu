@@ -316,38 +316,31 @@ __global__ void __launch_bounds__(256) moment_mean_kernel(const float* __restric
   }
 }
 
-// per image: the two sums in fixed order, and the means rounded to float
-// (sums: batch x 2 doubles; fmeans: batch x 2 floats)
-__global__ void __launch_bounds__(256) moment_mean_final_kernel(const double* __restrict__ part,
-                                                                int nparts, long long n,
-                                                                double* __restrict__ sums,
-                                                                float* __restrict__ fmeans) {
-  __shared__ double red[2 * 256];
-  double v[2] = {0, 0};
-  for (int b = threadIdx.x; b < nparts; b += blockDim.x) {
-    v[0] += part[((size_t)blockIdx.x * nparts + b) * 2 + 0];
-    v[1] += part[((size_t)blockIdx.x * nparts + b) * 2 + 1];
-  }
-  block_sum(v, 2, red);
-  if (threadIdx.x == 0) {
-    sums[blockIdx.x * 2 + 0] = v[0];
-    sums[blockIdx.x * 2 + 1] = v[1];
-    fmeans[blockIdx.x * 2 + 0] = (float)(v[0] / (double)n);
-    fmeans[blockIdx.x * 2 + 1] = (float)(v[1] / (double)n);
-  }
-}
-
-// pass 2: products about the float32-rounded means, and (x - y)^2
+// pass 2: products about the float32-rounded means, and (x - y)^2.  Every block
+// adds up pass 1's partials (mpart) in fixed order itself, and block 0 of an
+// image keeps the two sums (batch x 2 doubles): a launch less in the chain that
+// a search step waits for.
 __global__ void __launch_bounds__(256) moment_centred_kernel(const float* __restrict__ x,
                                                              const float* __restrict__ y,
                                                              long long n,
-                                                             const float* __restrict__ fmeans,
+                                                             const double* __restrict__ mpart,
+                                                             double* __restrict__ sums,
                                                              double* __restrict__ part) {
   __shared__ double red[4 * 256];
-  const int z = blockIdx.y;
+  const int z = blockIdx.y, nparts = gridDim.x;
   const float* xs = x + (size_t)z * n;
-  const float mx = fmeans[2 * z], my = fmeans[2 * z + 1];
   double v[4] = {0, 0, 0, 0};
+  for (int b = threadIdx.x; b < nparts; b += blockDim.x) {
+    v[0] += mpart[((size_t)z * nparts + b) * 2 + 0];
+    v[1] += mpart[((size_t)z * nparts + b) * 2 + 1];
+  }
+  block_sum(v, 2, red);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    sums[z * 2 + 0] = v[0];
+    sums[z * 2 + 1] = v[1];
+  }
+  const float mx = (float)(v[0] / (double)n), my = (float)(v[1] / (double)n);
+  v[0] = v[1] = 0;
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i0 = blockIdx.x * (long long)blockDim.x + threadIdx.x; i0 < n;
        i0 += stride * kSumRun) {
@@ -946,8 +939,7 @@ int nx_gaussian_blur(const float* d_in, int H, int W, double sigma, int affine, 
 
 size_t nx_moment_sums_workspace_bytes(int batch) {
   const size_t b = (size_t)std::max(batch, 1);
-  return 256 + b * kSumMaxBlocks * 4 * sizeof(double) + b * 2 * sizeof(double) +
-         b * 2 * sizeof(float);
+  return 256 + b * kSumMaxBlocks * 6 * sizeof(double) + b * 2 * sizeof(double);
 }
 
 int nx_moment_sums(const float* d_x, const float* d_y, long long n, int batch, double* d_sums,
@@ -961,17 +953,45 @@ int nx_moment_sums(const float* d_x, const float* d_y, long long n, int batch, d
   }
   cudaStream_t s = (cudaStream_t)stream;
   double* part = (double*)((char*)d_ws + 256);                    // batch x blocks x 4
-  double* means = part + (size_t)batch * kSumMaxBlocks * 4;       // batch x 2 (the sums)
-  float* fmeans = (float*)(means + (size_t)batch * 2);            // batch x 2
+  double* mpart = part + (size_t)batch * kSumMaxBlocks * 4;       // batch x blocks x 2
+  double* sums = mpart + (size_t)batch * kSumMaxBlocks * 2;       // batch x 2
   const int nb = sum_blocks(n);
-  moment_mean_kernel<<<dim3(nb, batch), 256, 0, s>>>(d_x, d_y, n, part);
+  moment_mean_kernel<<<dim3(nb, batch), 256, 0, s>>>(d_x, d_y, n, mpart);
   NX_CUDA_TRY(cudaGetLastError());
-  moment_mean_final_kernel<<<batch, 256, 0, s>>>(part, nb, n, means, fmeans);
+  moment_centred_kernel<<<dim3(nb, batch), 256, 0, s>>>(d_x, d_y, n, mpart, sums, part);
   NX_CUDA_TRY(cudaGetLastError());
-  moment_centred_kernel<<<dim3(nb, batch), 256, 0, s>>>(d_x, d_y, n, fmeans, part);
+  moment_final_kernel<<<batch, 256, 0, s>>>(part, nb, n, sums, d_sums);
   NX_CUDA_TRY(cudaGetLastError());
-  moment_final_kernel<<<batch, 256, 0, s>>>(part, nb, n, means, d_sums);
-  NX_CUDA_TRY(cudaGetLastError());
+  return NX_OK;
+}
+
+static size_t up256(size_t b) { return (b + 255) / 256 * 256; }
+
+size_t nx_blur_moments_workspace_bytes(int H, int W, int n) {
+  if (H < 1 || W < 1 || n < 1) return 256;
+  return up256(nx_gaussian_blur_batch_workspace_bytes(H, W, n)) +
+         up256(nx_moment_sums_workspace_bytes(n)) + (size_t)n * H * W * sizeof(float);
+}
+
+int nx_blur_moments(const float* d_in, int H, int W, int n, const int* src_index,
+                    const double* sigma, const float* d_y, double* h_sums, void* d_ws,
+                    size_t ws_bytes, void* stream) {
+  if (H < 1 || W < 1 || n < 1) return nx::set_error("need H, W, n >= 1"), NX_ERR_INVALID_ARG;
+  if (!d_y || !h_sums) return nx::set_error("NULL pointer"), NX_ERR_INVALID_ARG;
+  if (!d_ws || ws_bytes < nx_blur_moments_workspace_bytes(H, W, n)) {
+    nx::set_error("workspace too small: need %zu bytes", nx_blur_moments_workspace_bytes(H, W, n));
+    return NX_ERR_WORKSPACE;
+  }
+  const size_t nblur = nx_gaussian_blur_batch_workspace_bytes(H, W, n);
+  const size_t nsums = nx_moment_sums_workspace_bytes(n);
+  char* wsum = (char*)d_ws + up256(nblur);
+  float* blurred = (float*)(wsum + up256(nsums));
+  int rc = nx_gaussian_blur_batch_ex(d_in, H, W, n, src_index, sigma, nullptr, nullptr, 0, blurred,
+                                     d_ws, nblur, stream);
+  if (rc) return rc;
+  rc = nx_moment_sums(blurred, d_y, (long long)H * W, n, h_sums, wsum, nsums, stream);
+  if (rc) return rc;
+  NX_CUDA_TRY(cudaStreamSynchronize((cudaStream_t)stream));
   return NX_OK;
 }
 

@@ -91,6 +91,33 @@ def moment_sums(x: torch.Tensor, y: torch.Tensor) -> np.ndarray:
     return out.cpu().numpy()
 
 
+class _BlurMoments:
+    """The blur-and-moments step of the blur-width search over a (B, H, W) stack
+    against one image, with its workspace and page-locked result kept for the
+    whole search: a step is one native call."""
+
+    def __init__(self, stack: torch.Tensor, y: torch.Tensor):
+        self.stack, self.y = stack, y
+        B, H, W = stack.shape
+        self.fn = N.lib().nx_blur_moments
+        self.ws = workspace(N.lib().nx_blur_moments_workspace_bytes(H, W, B), stack.device,
+                            zero_status=False)
+        self.sums = torch.empty((B, _SUMS), dtype=torch.float64, pin_memory=True)
+        self.view = self.sums.numpy()
+        self.sig, self.idx = (C.c_double * B)(), (C.c_int * B)()
+        self.stream = stream_ptr(stack.device)
+
+    def __call__(self, batch: dict) -> dict:
+        """{image: sigma} -> {image: its 6 moments}."""
+        for j, (k, v) in enumerate(batch.items()):
+            self.idx[j], self.sig[j] = k, v
+        _, H, W = self.stack.shape
+        N.check(self.fn(self.stack.data_ptr(), H, W, len(batch), self.idx, self.sig,
+                        self.y.data_ptr(), self.sums.data_ptr(), self.ws.data_ptr(),
+                        self.ws.numel(), self.stream), "Gaussian blur")
+        return {k: self.view[j].copy() for j, k in enumerate(batch)}
+
+
 def _pearson(s, n: int) -> float:
     """Pearson correlation from the moments; 0 where a variance vanishes
     (pearson_correlation.pyx:60-77)."""
@@ -280,13 +307,12 @@ def error_maps(ref: torch.Tensor, srs: torch.Tensor, fixed_sigmas=None, ref_int=
     fixed = [0] * B if fixed_sigmas is None else list(fixed_sigmas)
     evals = [0] * B
 
+    step = _BlurMoments(srs.contiguous(), y)
+
     def fits(batch):  # {image: sigma} -> {image: (slope, intercept, rmse)}
-        keys = list(batch)
-        for k in keys:
+        for k in batch:
             evals[k] += 1
-        g = gaussian_blur_batch(srs, [batch[k] for k in keys], keys)
-        sums = moment_sums(g, y)
-        return {k: _regression(sums[j], n) for j, k in enumerate(keys)}
+        return {k: _regression(v, n) for k, v in step(batch).items()}
 
     max_sigma_boundary = (4 / 2.35482) * m
     sig = [f * m for f in fixed]
