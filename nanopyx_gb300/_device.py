@@ -92,7 +92,8 @@ def stream_ptr(device=None) -> int:
 def workspace(nbytes: int, device=None, zero_status: bool = True) -> torch.Tensor:
     """Device scratch for one C-ABI call; its first 256 bytes (the device status
     word the kernels report bounded-wait timeouts into) start at zero, unless the
-    call clears its status itself (``zero_status=False``: one launch less)."""
+    call clears its status itself or has none (``zero_status=False``: one launch
+    less)."""
     device = device if device is not None else torch.device("cuda", torch.cuda.current_device())
     ws = torch.empty(max(int(nbytes), 256), dtype=torch.uint8, device=device)
     if zero_status:

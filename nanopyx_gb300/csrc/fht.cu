@@ -301,18 +301,40 @@ __global__ void __launch_bounds__(256) fht_alternate_kernel(const float* __restr
   }
 }
 
-// r[z][j] = sum_c a[z][c] Cim[c][j]
-__global__ void __launch_bounds__(256) fht_rank1_kernel(const float* __restrict__ a,
+// r[z][j] = sum_c a[z][c] Cim[c][j].  Up to kAltInline rows a block forms a
+// itself from the square (X given), a launch less; and block 0 clears the
+// extremes the next tile will use (next_mm, n of them).
+constexpr int kAltInline = 128;
+__global__ void __launch_bounds__(256) fht_rank1_kernel(const float* __restrict__ X,
+                                                        const float* __restrict__ a,
                                                         const float* __restrict__ Cim, int N,
-                                                        int L, float* __restrict__ r) {
+                                                        int L, float* __restrict__ r,
+                                                        int* __restrict__ next_mm, int n) {
   __shared__ float red[8][32];
+  __shared__ float as[kAltInline];
   const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
   const int j = blockIdx.x * 32 + lane;
+  if (blockIdx.x == 0 && blockIdx.y == 0)
+    for (int k = threadIdx.x; k < 4 * n; k += 256) next_mm[k] = (k & 1) ? INT_MIN : INT_MAX;
   const float* az = a + (size_t)blockIdx.y * N;
+  if (X) {
+    const float* x = X + (size_t)blockIdx.y * N * N;
+    for (int c = threadIdx.x; c < N; c += 256) {
+      float even = 0.f, odd = 0.f;
+#pragma unroll 4
+      for (int k = 0; k < N; k += 2) {
+        even += __ldg(x + (size_t)k * N + c);
+        if (k + 1 < N) odd += __ldg(x + (size_t)(k + 1) * N + c);
+      }
+      as[c] = even - odd;
+    }
+    __syncthreads();
+    az = as;
+  }
   float t = 0.f;
   if (j < L) {
 #pragma unroll 4
-    for (int c = g; c < N; c += 8) t = fmaf(__ldg(az + c), __ldg(Cim + (size_t)c * L + j), t);
+    for (int c = g; c < N; c += 8) t = fmaf(az[c], __ldg(Cim + (size_t)c * L + j), t);
   }
   red[g][lane] = t;
   __syncthreads();
@@ -626,7 +648,7 @@ size_t nx_fht_workspace_bytes(const nx_fht_plan* p, int T) {
   if (!p || T < 1) return 256;
   const size_t tc = (size_t)std::min(T, kFhtChunk);
   return 256 + ((tc * p->frame_floats * sizeof(float) + 255) / 256) * 256 +
-         tc * 4 * sizeof(int);
+         2 * tc * 4 * sizeof(int);
 }
 
 int nx_fht_interpolate(const nx_fht_plan* p, const float* d_in, int T, float* d_out, void* d_ws,
@@ -649,8 +671,11 @@ int nx_fht_interpolate(const nx_fht_plan* p, const float* d_in, int T, float* d_
   const long long plane = (long long)outH * outW;
   char* base = (char*)d_ws + 256;
   float* work = (float*)base;
-  int* mm = (int*)(base + ((std::min(T, kFhtChunk) * p->frame_floats * sizeof(float) + 255) /
-                           256) * 256);
+  int* const mm0 = (int*)(base + ((std::min(T, kFhtChunk) * p->frame_floats * sizeof(float) + 255) /
+                                  256) * 256);
+  int* const mms[2] = {mm0, mm0 + 4 * std::min(T, kFhtChunk)};
+  int set = 0;
+  bool clear = true;
   for (int t0 = 0; t0 < T; t0 += kFhtChunk) {
     const int tc = std::min(kFhtChunk, T - t0);
     const float* in = d_in + (size_t)t0 * p->H * p->W;
@@ -664,9 +689,14 @@ int nx_fht_interpolate(const nx_fht_plan* p, const float* d_in, int T, float* d_
       float* Z = U + (size_t)tc * (full ? 2 : 1) * N * L;
       float* r = Z + (size_t)tc * L * L;
       float* alt = r + (size_t)tc * L;
-      // (min, max) slots of the tile input and of the interpolated square
-      fht_mm_init_kernel<<<1, 32, 0, s>>>(mm, tc);
-      NX_CUDA_TRY(cudaGetLastError());
+      // (min, max) slots of the tile input and of the interpolated square: two sets
+      // in turn, each cleared while the other's tile runs (the first by itself)
+      int* mm = mms[set];
+      if (clear) {
+        fht_mm_init_kernel<<<1, 32, 0, s>>>(mm, tc);
+        NX_CUDA_TRY(cudaGetLastError());
+        clear = full;
+      }
       fht_gather_kernel<<<dim3(blocks_for((long long)N * N, 256, 256), (unsigned)tc), 256, 0,
                           s>>>(in, p->H, p->W, t.r0, t.c0, t.th, t.tw, N, t.kh, t.kw, t.y_roi,
                                t.x_roi, X, mm);
@@ -684,11 +714,14 @@ int nx_fht_interpolate(const nx_fht_plan* p, const float* d_in, int T, float* d_
       } else {
         // r of the rank-1 term, then U = X C_re^T (the frames' squares stacked) and
         // Z = A_re U + s r^T
-        fht_alternate_kernel<<<dim3((unsigned)((N + 31) / 32), (unsigned)tc), 256, 0, s>>>(X, N,
-                                                                                           alt);
-        NX_CUDA_TRY(cudaGetLastError());
+        const bool own = N <= kAltInline;
+        if (!own) {
+          fht_alternate_kernel<<<dim3((unsigned)((N + 31) / 32), (unsigned)tc), 256, 0, s>>>(X, N,
+                                                                                             alt);
+          NX_CUDA_TRY(cudaGetLastError());
+        }
         fht_rank1_kernel<<<dim3((unsigned)((L + 31) / 32), (unsigned)tc), 256, 0, s>>>(
-            alt, o.ct + (size_t)N * L, N, L, r);
+            own ? X : nullptr, alt, o.ct + (size_t)N * L, N, L, r, mms[set ^ 1], tc);
         NX_CUDA_TRY(cudaGetLastError());
         NX_CUDA_TRY(gemm(X, o.ct, U, tc * N, L, N, N, L, L, 1, GemmBatch{1, 0, 0, 0, 0, 0, 0},
                          Rank1{}, s));
@@ -703,6 +736,7 @@ int nx_fht_interpolate(const nx_fht_plan* p, const float* d_in, int T, float* d_
                                p->tiled ? t.wr : nullptr, p->tiled ? t.wc : nullptr, out, outH,
                                outW, t.r0 * mag, t.c0 * mag, full);
       NX_CUDA_TRY(cudaGetLastError());
+      set ^= 1;
     }
     if (p->tiled) {
       fht_normalize_kernel<<<blocks_for(plane), 256, 0, s>>>(out, p->wgt, plane, tc);

@@ -51,7 +51,8 @@ def gaussian_blur_batch(stack: torch.Tensor, sigmas, index=None, alpha=None,
     if n == 0:
         return out
     L = N.lib()
-    ws = workspace(L.nx_gaussian_blur_batch_workspace_bytes(H, W, n), stack.device)
+    ws = workspace(L.nx_gaussian_blur_batch_workspace_bytes(H, W, n), stack.device,
+                   zero_status=False)
     sig = (C.c_double * n)(*[float(v) for v in sigmas])
     ix = (C.c_int * n)(*idx)
     al = be = None
@@ -85,7 +86,7 @@ def moment_sums(x: torch.Tensor, y: torch.Tensor) -> np.ndarray:
     B = xs.shape[0]
     L = N.lib()
     out = torch.empty((B, _SUMS), dtype=torch.float64, device=x.device)
-    ws = workspace(L.nx_moment_sums_workspace_bytes(B), x.device)
+    ws = workspace(L.nx_moment_sums_workspace_bytes(B), x.device, zero_status=False)
     N.check(L.nx_moment_sums(xs.data_ptr(), y.data_ptr(), y.numel(), B, out.data_ptr(),
                              ws.data_ptr(), ws.numel(), stream_ptr()), "moment sums")
     return out.cpu().numpy()

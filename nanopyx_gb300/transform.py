@@ -232,7 +232,7 @@ def _fht_device(t: torch.Tensor, magnification: int, variant: int = 0) -> torch.
         return out
     plan = get_fht_plan(H, W, m, variant)
     L = N.lib()
-    ws = workspace(L.nx_fht_workspace_bytes(plan.handle, T), t.device)
+    ws = workspace(L.nx_fht_workspace_bytes(plan.handle, T), t.device, zero_status=False)
     N.check(L.nx_fht_interpolate(plan.handle, _ptr(t), T, _ptr(out), _ptr(ws), ws.numel(),
                                  stream_ptr()), "FHT interpolation")
     return out
@@ -355,7 +355,7 @@ def macro_pixel_corrector(img, magnification: int):
         raise ValueError("Buffer has wrong number of dimensions (expected 3)")
     S, rowsM, colsM = t.shape
     m = int(magnification)
-    ws = workspace(N.lib().nx_macro_pixel_workspace_bytes(S, m), t.device)
+    ws = workspace(N.lib().nx_macro_pixel_workspace_bytes(S, m), t.device, zero_status=False)
     N.check(N.lib().nx_macro_pixel_correct(_ptr(t), S, rowsM, colsM, m, _ptr(ws), ws.numel(),
                                            stream_ptr()),
             "macro_pixel_corrector")
@@ -414,7 +414,8 @@ class eSRRF3D_ST(LiquidEngine):
         out = torch.empty((S * mz, H * mxy, W * mxy), dtype=torch.float32, device=t.device)
         md = 1 if mode == "std" else 0
         L = N.lib()
-        ws = workspace(L.nx_esrrf3d_workspace_bytes(S, H, W, mxy, mz, md), t.device)
+        ws = workspace(L.nx_esrrf3d_workspace_bytes(S, H, W, mxy, mz, md), t.device,
+                       zero_status=False)
         N.check(L.nx_esrrf3d_st(_ptr(t), T, S, H, W, mxy, mz, float(radius), float(radius_z),
                                 float(sensitivity), md, 1 if doIntensityWeighting else 0,
                                 _ptr(out), _ptr(ws), ws.numel(), stream_ptr()), "eSRRF3D")
