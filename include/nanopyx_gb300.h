@@ -189,6 +189,14 @@ int nx_workspace_status(const void* d_ws, void* stream);
  * Standalone Liquid-Engine ops of the path
  * ------------------------------------------------------------------------ */
 
+/* n camera pixels (8- or 16-bit integers) to float32, exactly; the source
+ * aligned to its type.                                                       */
+#define NX_TYPE_U8 0
+#define NX_TYPE_I8 1
+#define NX_TYPE_U16 2
+#define NX_TYPE_I16 3
+int nx_to_float32(const void* d_src, int type, long long n, float* d_dst, void* stream);
+
 /* Catmull-Rom ShiftAndMagnify; per-frame shifts (length T, device arrays).
  *   src/nanopyx/core/transform/_le_interpolation_catmull_rom.pyx:17,143-160
  *   src/include/_c_interpolation_catmull_rom.c:6-52

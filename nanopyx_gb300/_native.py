@@ -29,6 +29,10 @@ NX_CORR_TAC2 = 4
 CORR_BITS = {"AVG": NX_CORR_AVG, "VAR": NX_CORR_VAR, "TAC2": NX_CORR_TAC2}
 
 
+# camera pixel types of nx_to_float32, by NumPy type character (native byte order)
+PIXEL_TYPES = {"B": 0, "b": 1, "H": 2, "h": 3}
+
+
 class EsrrfItem(C.Structure):
     """nx_esrrf_item of include/nanopyx_gb300.h."""
 
@@ -82,6 +86,7 @@ _SIGS = {
     "nx_esrrf_batch_bind": (_I, [_P, _P, _SZ, _P]),
     "nx_esrrf_batch_launch": (_I, [_P, _P]),
     "nx_esrrf_batch_destroy": (_I, [_P]),
+    "nx_to_float32": (_I, [_P, _I, _LL, _P, _P]),
     "nx_cr_shift_magnify": (_I, [_P, _I, _I, _I, _P, _P, _FL, _FL, _P, _P]),
     "nx_roberts_cross": (_I, [_P, _I, _I, _I, _P, _P, _P]),
     "nx_rgc": (_I, [_P, _P, _P, _I, _I, _I, _I, _FL, _FL, _I, _I, _P, _P]),

@@ -1100,6 +1100,15 @@ int nx_workspace_status(const void* d_ws, void* stream) {
   return NX_OK;
 }
 
+int nx_to_float32(const void* d_src, int type, long long n, float* d_dst, void* stream) {
+  if (n < 0) return invalid("n must be >= 0");
+  if (type < NX_TYPE_U8 || type > NX_TYPE_I16) return invalid("unknown pixel type");
+  if (n > 0 && (!d_src || !d_dst)) return invalid("NULL input/output");
+  cudaError_t e = launch_to_float32(d_src, type, n, d_dst, (cudaStream_t)stream);
+  if (e != cudaSuccess) return cuda_status(e, "pixel conversion");
+  return NX_OK;
+}
+
 int nx_cr_shift_magnify(const float* d_in, int T, int H, int W, const float* d_shift_row,
                         const float* d_shift_col, float mag_row, float mag_col, float* d_out,
                         void* stream) {

@@ -39,6 +39,8 @@ const FusedEntry* fused_entry_m5_alt(int J);
 // ---------------------------------------------------------------------------
 // standalone op launchers (ops.cu)
 // ---------------------------------------------------------------------------
+cudaError_t launch_to_float32(const void* src, int type, long long n, float* dst,
+                              cudaStream_t s);
 cudaError_t launch_cr_shift_magnify(const float* in, int T, int H, int W, const float* shift_r,
                                     const float* shift_c, float mag_r, float mag_c, int rowsM,
                                     int colsM, float* out, cudaStream_t s);

@@ -737,6 +737,41 @@ __global__ void srrf_acrf_integrated_kernel(float* __restrict__ im, int T, long 
   }
 }
 
+// Camera integers to float32, exact.  HBM-bound: 8 values per thread from one
+// vector load (16 bytes of 16-bit, 8 of 8-bit pixels) into two 16-byte stores;
+// scalar where the pointers do not allow it and for the rest.
+template <typename S>
+__global__ void __launch_bounds__(256)
+    to_float_kernel(const S* __restrict__ src, long long n, int vec, float* __restrict__ dst) {
+  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  const long long stride = (long long)gridDim.x * blockDim.x;
+  const long long n8 = vec ? n / 8 : 0;
+  for (long long i = t; i < n8; i += stride) {
+    union {
+      uint4 q;
+      uint2 d;
+      S v[8];
+    } u;
+    if constexpr (sizeof(S) == 2) u.q = __ldg(reinterpret_cast<const uint4*>(src) + i);
+    else u.d = __ldg(reinterpret_cast<const uint2*>(src) + i);
+    float4* o = reinterpret_cast<float4*>(dst) + 2 * i;
+    o[0] = make_float4((float)u.v[0], (float)u.v[1], (float)u.v[2], (float)u.v[3]);
+    o[1] = make_float4((float)u.v[4], (float)u.v[5], (float)u.v[6], (float)u.v[7]);
+  }
+  for (long long i = n8 * 8 + t; i < n; i += stride) dst[i] = (float)src[i];
+}
+
+template <typename S>
+cudaError_t launch_to_float(const void* src, long long n, float* dst, cudaStream_t s) {
+  const uintptr_t a = reinterpret_cast<uintptr_t>(src), b = reinterpret_cast<uintptr_t>(dst);
+  const int vec = a % (8 * sizeof(S)) == 0 && b % 16 == 0;
+  const long long items = vec ? (n + 7) / 8 : n;
+  const unsigned grid = (unsigned)std::max<long long>(1, std::min<long long>((items + 255) / 256,
+                                                                             152LL * 32));
+  to_float_kernel<S><<<grid, 256, 0, s>>>(static_cast<const S*>(src), n, vec, dst);
+  return cudaGetLastError();
+}
+
 // macro-pixel map, stage 1: block (s, py, chunk) sums the macro-pixel rows
 // [chunk*rpc, (chunk+1)*rpc) of phase row py; thread t owns phase px = t % M
 // (blockDim is a multiple of M); Kahan sums, fixed-order block reduction.
@@ -876,6 +911,17 @@ __global__ void __launch_bounds__(kMpcThreads)
 // ---------------------------------------------------------------------------
 // host launchers
 // ---------------------------------------------------------------------------
+cudaError_t launch_to_float32(const void* src, int type, long long n, float* dst,
+                              cudaStream_t s) {
+  if (n == 0) return cudaSuccess;
+  switch (type) {
+    case NX_TYPE_U8: return launch_to_float<uint8_t>(src, n, dst, s);
+    case NX_TYPE_I8: return launch_to_float<int8_t>(src, n, dst, s);
+    case NX_TYPE_U16: return launch_to_float<uint16_t>(src, n, dst, s);
+    default: return launch_to_float<int16_t>(src, n, dst, s);
+  }
+}
+
 cudaError_t launch_cr_shift_magnify(const float* in, int T, int H, int W, const float* shift_r,
                                     const float* shift_c, float mag_r, float mag_c, int rowsM,
                                     int colsM, float* out, cudaStream_t s) {

