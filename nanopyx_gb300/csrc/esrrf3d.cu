@@ -27,7 +27,8 @@
 // sample and frame pair) and the L1 wavefronts of its two gradient loads.
 // 20 x 16 x 128 x 128, mxy = mz = 2, R = 1.5: one frame at a time, three scalar
 // gradients normalised at every sample and every voxel by itself 5.9 ms; frame
-// pairs, gradients normalised once, shared z voxels 1.5 ms.
+// pairs, gradients normalised once, shared z voxels 1.5 ms; window columns in
+// registers 1.3 ms.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -181,15 +182,25 @@ __global__ void __launch_bounds__(kPrepThreads)
 // [k][j][i], the unit offset and the weight (0: does not count); sample columns
 // and rows, from the voxel's float32 coordinates as the reference forms them,
 // are tabulated per block (-1: outside the image).
+// NI: window columns known at compile time (4: radius 1 to below 2; 0: any) --
+// the columns' indices stay in registers and a window row's loads are in flight
+// together (whole call, 20 x 16 x 128 x 128, R = 1.5: 1.51 ms with the general
+// loop, 1.28 with NI = 4; NI = 6 at R = 2 lost, 3.2 against 2.3: a third of its loads
+// belong to samples outside the radius).
 constexpr int kMaxWin = 64;  // window offsets per axis are at most 2 int(radius) + 2
+constexpr int kMaxTab = 64;  // table entries kept in shared memory (NI > 0)
 
+template <int NI>
 __global__ void __launch_bounds__(256)
     rgc3d_kernel(const __grid_constant__ Rgc3d p, const float4* __restrict__ A,
                  const float2* __restrict__ B, const float2* __restrict__ I,
                  const float4* __restrict__ tab, int s_first, int frame, int two,
                  float* __restrict__ out, float* __restrict__ mean) {
-  __shared__ int cidx[kMaxWin][32], ridx[kMaxWin][8];
-  const int nI = p.s1 - p.s0 + 1;
+  __shared__ int cidx[NI > 0 ? NI : kMaxWin][32], ridx[NI > 0 ? NI : kMaxWin][8];
+  __shared__ float4 stab[NI > 0 ? kMaxTab : 1];
+  const int nI = NI > 0 ? NI : p.s1 - p.s0 + 1;
+  if (NI > 0)
+    for (int e = threadIdx.x; e < (p.z1 - p.z0 + 1) * nI * nI; e += 256) stab[e] = __ldg(tab + e);
   const int lane = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int nbx = (p.Wm - 2 * p.margin + 31) / 32;
   const int c0 = p.margin + blockIdx.x % nbx * 32, r0 = p.margin + blockIdx.x / nbx * 8;
@@ -211,6 +222,15 @@ __global__ void __launch_bounds__(256)
   bool all_in = true;
   for (int i = 0; i < nI; ++i) all_in = all_in && cidx[i][lane] >= 0 && ridx[i][ty] >= 0;
   const bool interior = __all_sync(0xffffffffu, all_in);
+  int cx[NI > 0 ? NI : 1];
+  unsigned cin = 0;  // bit i: column i lies inside the image
+  if constexpr (NI > 0) {
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+      cx[i] = max(cidx[i][lane], 0);
+      cin |= (cidx[i][lane] >= 0 ? 1u : 0u) << i;
+    }
+  }
   const size_t plane = (size_t)p.Hm * p.Wm;
   // voxels sM = s mz + r, r0 <= r < r1, inside the z margins
   const int s = s_first + blockIdx.y;
@@ -226,43 +246,61 @@ __global__ void __launch_bounds__(256)
   for (int r = ra; r < rb; r = same ? rb : r + 1) {
     float2 acc = make_float2(0.f, 0.f);
     float wsum = 0.f;
+    // one sample: unit gradients of the pair against the unit offset t (weight w)
+    auto sample = [&](const float4& t, const float4& a, const float2& nz, bool ok) {
+      const float2 nx = make_float2(a.x, a.y), ny = make_float2(a.z, a.w);
+      const float2 rx = make_float2(t.x, t.x), ry = make_float2(t.y, t.y),
+                   rz = make_float2(t.z, t.z);
+      const float2 mx = make_float2(-t.x, -t.x), my = make_float2(-t.y, -t.y),
+                   mz = make_float2(-t.z, -t.z);
+      const float2 dot = __ffma2_rn(nz, rz, __ffma2_rn(ny, ry, __fmul2_rn(nx, rx)));
+      const float2 c1 = __ffma2_rn(ny, rz, __fmul2_rn(nz, my));
+      const float2 c2 = __ffma2_rn(nz, rx, __fmul2_rn(nx, mz));
+      const float2 c3 = __ffma2_rn(nx, ry, __fmul2_rn(ny, mx));
+      // the smallest normal number keeps rsqrt finite for a zero cross product
+      const float tiny = 1.17549435e-38f;
+      const float2 q = __ffma2_rn(
+          c3, c3, __ffma2_rn(c2, c2, __ffma2_rn(c1, c1, make_float2(tiny, tiny))));
+      const float2 dk = __fmul2_rn(q, make_float2(rsqrtf(q.x), rsqrtf(q.y)));
+      const float2 v = __ffma2_rn(dk, make_float2(-t.w, -t.w), make_float2(t.w, t.w));
+      acc = __fadd2_rn(acc, make_float2(ok && dot.x < 0.f ? v.x : 0.f,
+                                        ok && dot.y < 0.f ? v.y : 0.f));
+      wsum += ok ? t.w : 0.f;
+    };
     for (int k = p.z0; k <= p.z1; ++k) {
       if (!z_in(r, k)) continue;
       // slice of the magnified volumes: (int)(vz mz) / mz = s + k (vz mz rounds
       // to s mz + k mz + r or, for r > 0, at worst just below it)
       const float4* Ak = A + (size_t)(s + k) * plane;
       const float2* Bk = B + (size_t)(s + k) * plane;
-      const float4* tk = tab + (size_t)(k - p.z0) * nI * nI;
+      const float4* tk = (NI > 0 ? stab : tab) + (size_t)(k - p.z0) * nI * nI;
       for (int j = 0; j < nI; ++j) {
         const int ry = ridx[j][ty];
         const float4* Aj = Ak + (size_t)max(ry, 0) * p.Wm;
         const float2* Bj = Bk + (size_t)max(ry, 0) * p.Wm;
+        if constexpr (NI > 0) {
+          float4 a[NI];
+          float2 nz[NI];
+#pragma unroll
+          for (int i = 0; i < NI; ++i) {
+            a[i] = __ldg(Aj + cx[i]);
+            nz[i] = __ldg(Bj + cx[i]);
+          }
+#pragma unroll
+          for (int i = 0; i < NI; ++i) {
+            const float4 t = tk[j * NI + i];
+            if (t.w == 0.f) continue;  // does not count
+            sample(t, a[i], nz[i], interior || (ry >= 0 && (cin >> i & 1u)));
+          }
+        } else {
 #pragma unroll 4
-        for (int i = 0; i < nI; ++i) {
-          const float4 t = __ldg(tk + j * nI + i);
-          if (t.w == 0.f) continue;
-          const int cx = cidx[i][lane];
-          const bool ok = interior || (ry >= 0 && cx >= 0);
-          const float4 a = __ldg(Aj + max(cx, 0));
-          const float2 nz = __ldg(Bj + max(cx, 0));
-          const float2 nx = make_float2(a.x, a.y), ny = make_float2(a.z, a.w);
-          const float2 rx = make_float2(t.x, t.x), ryv = make_float2(t.y, t.y),
-                       rz = make_float2(t.z, t.z);
-          const float2 mx = make_float2(-t.x, -t.x), my = make_float2(-t.y, -t.y),
-                       mzv = make_float2(-t.z, -t.z);
-          const float2 dot = __ffma2_rn(nz, rz, __ffma2_rn(ny, ryv, __fmul2_rn(nx, rx)));
-          const float2 c1 = __ffma2_rn(ny, rz, __fmul2_rn(nz, my));
-          const float2 c2 = __ffma2_rn(nz, rx, __fmul2_rn(nx, mzv));
-          const float2 c3 = __ffma2_rn(nx, ryv, __fmul2_rn(ny, mx));
-          // the smallest normal number keeps rsqrt finite for a zero cross product
-          const float tiny = 1.17549435e-38f;
-          const float2 q = __ffma2_rn(
-              c3, c3, __ffma2_rn(c2, c2, __ffma2_rn(c1, c1, make_float2(tiny, tiny))));
-          const float2 dk = __fmul2_rn(q, make_float2(rsqrtf(q.x), rsqrtf(q.y)));
-          const float2 v = __ffma2_rn(dk, make_float2(-t.w, -t.w), make_float2(t.w, t.w));
-          acc = __fadd2_rn(acc, make_float2(ok && dot.x < 0.f ? v.x : 0.f,
-                                            ok && dot.y < 0.f ? v.y : 0.f));
-          wsum += ok ? t.w : 0.f;
+          for (int i = 0; i < nI; ++i) {
+            const float4 t = __ldg(tk + j * nI + i);
+            if (t.w == 0.f) continue;
+            const int c = cidx[i][lane];
+            sample(t, __ldg(Aj + max(c, 0)), __ldg(Bj + max(c, 0)),
+                   interior || (ry >= 0 && c >= 0));
+          }
         }
       }
     }
@@ -395,6 +433,16 @@ int nx_esrrf3d_st(const float* d_in, int T, int S, int H, int W, int magnificati
         }
         tab[((size_t)(k - p.z0) * nI + (j - p.s0)) * nI + (i - p.s0)] = t;
       }
+  // slices at the end of the window in which nothing counts
+  while (p.z1 > p.z0) {
+    bool any = false;
+    for (size_t e = (size_t)(p.z1 - p.z0) * nI * nI; e < (size_t)(p.z1 - p.z0 + 1) * nI * nI; ++e)
+      any = any || tab[e].w != 0.f;
+    if (any) break;
+    --p.z1;
+  }
+  const bool small = (p.z1 - p.z0 + 1) * nI * nI <= kMaxTab;
+  const auto rgc = small && nI == 4 ? rgc3d_kernel<4> : rgc3d_kernel<0>;
   const size_t vol = (size_t)S * H * W;
   const size_t volm = (size_t)S * p.Hm * p.Wm;
   const long long nout = (long long)p.Sm * p.Hm * p.Wm;
@@ -431,7 +479,7 @@ int nx_esrrf3d_st(const float* d_in, int T, int S, int H, int W, int magnificati
       NX_CUDA_TRY(cudaGetLastError());
     }
     for (int z = sa; z <= sb; z += 65535) {
-      rgc3d_kernel<<<dim3(rgc_blocks, (unsigned)std::min(sb - z + 1, 65535)), 256, 0, s>>>(
+      rgc<<<dim3(rgc_blocks, (unsigned)std::min(sb - z + 1, 65535)), 256, 0, s>>>(
           p, A, B, I, dtab, z, f, two, d_out, mean);
       NX_CUDA_TRY(cudaGetLastError());
     }
