@@ -18,10 +18,12 @@
 // (the one unpaired y frequency makes A complex; the half spectrum along x
 // gives C).  That frequency alone makes A_im: A_im[i][n] = -(-1)^n sin(pi i / mag)
 // / L, so the second term is the outer product of s_i = sin(pi i / mag) / L and
-// r = (sum_n (-1)^n X[n]) C_im^T, and the interpolation is two batched FP32
-// GEMMs plus a rank-1 update, with operators formed once in float64 on the host.  FP32 on the CUDA cores, not TF32 on the
-// tensor cores: the reference transforms in float64, and a 10-bit mantissa
-// would not hold the 1e-4 parity bar.
+// r = (sum_n (-1)^n X[n]) C_im^T.  The mirror images are linear too: X = P_h T P_w^T
+// of the th x tw tile T, so P goes into the operators (A_re P_h, C P_w and the signs,
+// folded in float64 on the host) and the products run over the tile's own rows and
+// columns instead of N: two batched FP32 GEMMs plus a rank-1 update.  FP32 on the
+// CUDA cores, not TF32 on the tensor cores: the reference transforms in float64,
+// and a 10-bit mantissa would not hold the 1e-4 parity bar.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -254,7 +256,7 @@ __global__ void __launch_bounds__(256, 2)
 
 // operands the big tiles can take, and sizes they fill; else 64 x 64 tiles.
 // The 8 frames of 300 x 260 at m = 2 (24 products of 256- and 128-pixel squares):
-// 2.97 ms in 64 x 64 tiles with both parts of A, 1.08 ms now.
+// 2.97 ms in 64 x 64 tiles with both parts of A, 1.08 ms in these.
 bool big_tiles(const float* A, const float* B, const float* C, int M, int N, int K, int lda,
                int ldb, int ldc, const GemmBatch& bt, const Rank1& u) {
   const uintptr_t ptrs = reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) |
@@ -278,37 +280,39 @@ cudaError_t gemm(const float* A, const float* B, float* C, int M, int N, int K, 
   return cudaGetLastError();
 }
 
-// a[z][c] = sum_n (-1)^n X[z][n][c]
-__global__ void __launch_bounds__(256) fht_alternate_kernel(const float* __restrict__ X, int N,
-                                                            float* __restrict__ a) {
+// a[z][c] = sum_n e[n] X[z][n][c] over the nr rows of a tile (nc columns): e holds
+// the signs (-1)^n of the square's rows, summed over a tile row's images
+__global__ void __launch_bounds__(256) fht_alternate_kernel(const float* __restrict__ X,
+                                                            const float* __restrict__ e, int nr,
+                                                            int nc, float* __restrict__ a) {
   __shared__ float red[8][32];
   const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + lane;
-  const float* x = X + (size_t)blockIdx.y * N * N;
-  float even = 0.f, odd = 0.f;  // rows g, g + 8, ... have one parity
-  if (c < N)
-    for (int n = g; n < N; n += 8) {
-      if (n & 1) odd += __ldg(x + (size_t)n * N + c);
-      else even += __ldg(x + (size_t)n * N + c);
-    }
-  red[g][lane] = even - odd;
+  const float* x = X + (size_t)blockIdx.y * nr * nc;
+  float t = 0.f;
+  if (c < nc) {
+#pragma unroll 4
+    for (int n = g; n < nr; n += 8) t = fmaf(__ldg(e + n), __ldg(x + (size_t)n * nc + c), t);
+  }
+  red[g][lane] = t;
   __syncthreads();
-  if (g == 0 && c < N) {
-    float t = 0.f;
+  if (g == 0 && c < nc) {
+    t = 0.f;
 #pragma unroll
     for (int k = 0; k < 8; ++k) t += red[k][lane];
-    a[(size_t)blockIdx.y * N + c] = t;
+    a[(size_t)blockIdx.y * nc + c] = t;
   }
 }
 
-// r[z][j] = sum_c a[z][c] Cim[c][j].  Up to kAltInline rows a block forms a
-// itself from the square (X given), a launch less; and block 0 clears the
+// r[z][j] = sum_c a[z][c] Cim[c][j].  Up to kAltInline rows and columns a block forms
+// a itself from the tile (X given), a launch less; and block 0 clears the
 // extremes the next tile will use (next_mm, n of them).
 constexpr int kAltInline = 128;
 __global__ void __launch_bounds__(256) fht_rank1_kernel(const float* __restrict__ X,
+                                                        const float* __restrict__ e,
                                                         const float* __restrict__ a,
-                                                        const float* __restrict__ Cim, int N,
-                                                        int L, float* __restrict__ r,
+                                                        const float* __restrict__ Cim, int nr,
+                                                        int nc, int L, float* __restrict__ r,
                                                         int* __restrict__ next_mm, int n) {
   __shared__ float red[8][32];
   __shared__ float as[kAltInline];
@@ -316,17 +320,17 @@ __global__ void __launch_bounds__(256) fht_rank1_kernel(const float* __restrict_
   const int j = blockIdx.x * 32 + lane;
   if (blockIdx.x == 0 && blockIdx.y == 0)
     for (int k = threadIdx.x; k < 4 * n; k += 256) next_mm[k] = (k & 1) ? INT_MIN : INT_MAX;
-  const float* az = a + (size_t)blockIdx.y * N;
+  const float* az = a + (size_t)blockIdx.y * nc;
   if (X) {
-    const float* x = X + (size_t)blockIdx.y * N * N;
-    for (int c = threadIdx.x; c < N; c += 256) {
-      float even = 0.f, odd = 0.f;
+    const float* x = X + (size_t)blockIdx.y * nr * nc;
+    for (int c = threadIdx.x; c < nc; c += 256) {
+      float even = 0.f, odd = 0.f;  // nr is a multiple of 16
 #pragma unroll 4
-      for (int k = 0; k < N; k += 2) {
-        even += __ldg(x + (size_t)k * N + c);
-        if (k + 1 < N) odd += __ldg(x + (size_t)(k + 1) * N + c);
+      for (int k = 0; k < nr; k += 2) {
+        even = fmaf(__ldg(e + k), __ldg(x + (size_t)k * nc + c), even);
+        odd = fmaf(__ldg(e + k + 1), __ldg(x + (size_t)(k + 1) * nc + c), odd);
       }
-      as[c] = even - odd;
+      as[c] = even + odd;
     }
     __syncthreads();
     az = as;
@@ -334,7 +338,7 @@ __global__ void __launch_bounds__(256) fht_rank1_kernel(const float* __restrict_
   float t = 0.f;
   if (j < L) {
 #pragma unroll 4
-    for (int c = g; c < N; c += 8) t = fmaf(az[c], __ldg(Cim + (size_t)c * L + j), t);
+    for (int c = g; c < nc; c += 8) t = fmaf(az[c], __ldg(Cim + (size_t)c * L + j), t);
   }
   red[g][lane] = t;
   __syncthreads();
@@ -364,6 +368,28 @@ __global__ void fht_gather_kernel(const float* __restrict__ in, int H, int W, in
     X[(size_t)z * N * N + e] = v;
     lo = fminf(lo, v);
     hi = fmaxf(hi, v);
+  }
+  block_minmax(lo, hi, mm + 4 * z);
+}
+
+// tile (r0, c0, th, tw) of every frame of the chunk as nr x nc, zeros past its edges;
+// slot[z] = (min, max) of the tile
+__global__ void fht_tile_kernel(const float* __restrict__ in, int H, int W, int r0, int c0, int th,
+                                int tw, int nr, int nc, float* __restrict__ X,
+                                int* __restrict__ mm) {
+  const int z = blockIdx.y;
+  const float* f = in + (size_t)z * H * W + (size_t)r0 * W + c0;
+  float* o = X + (size_t)z * nr * nc;
+  float lo = INFINITY, hi = -INFINITY;
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < nr * nc; e += gridDim.x * blockDim.x) {
+    const int y = e / nc, x = e % nc;
+    float v = 0.f;
+    if (y < th && x < tw) {
+      v = __ldg(f + (size_t)y * W + x);
+      lo = fminf(lo, v);
+      hi = fmaxf(hi, v);
+    }
+    o[e] = v;
   }
   block_minmax(lo, hi, mm + 4 * z);
 }
@@ -444,18 +470,30 @@ unsigned blocks_for(long long n, int per = 256, long long cap = 4096) {
 // plan: tile layout, operators per padded size, windows, blending weights
 // ---------------------------------------------------------------------------
 struct nx_fht_plan {
-  struct Ops {
+  struct Ops {    // full-spectrum variant, per padded size
     int N, L;
     float* ct;    // [2][N][L]: C_re^T then C_im^T
     float* acat;  // [L][2N]: A_re | -A_im
   };
+  struct RowOps {  // per (padded size, tile height); n = th rounded up to 16
+    int N, th, n;
+    float* a;  // [L][n]: A_re with the mirror images folded in
+    float* s;  // [L]: the rank-1 term's column
+    float* e;  // [n]: its row signs
+  };
+  struct ColOps {  // per (padded size, tile width); n = tw rounded up to 16
+    int N, tw, n;
+    float* ct;  // [2][n][L]: C_re^T then C_im^T, folded
+  };
   struct Tile {
-    int r0, c0, th, tw, ops, kh, kw, y_roi, x_roi;
+    int r0, c0, th, tw, N, ops, rows, cols, kh, kw, y_roi, x_roi;
     float *wr, *wc;  // Hann windows (tiled path), device
   };
   int H, W, mag, device, variant;
   bool tiled;
   std::vector<Ops> ops;
+  std::vector<RowOps> row_ops;
+  std::vector<ColOps> col_ops;
   std::vector<Tile> tiles;
   std::vector<float*> bufs;  // every device allocation of the plan
   float* wgt = nullptr;      // (H mag, W mag) blending weights (tiled path)
@@ -473,42 +511,99 @@ std::vector<int> tile_starts(int dim) {
   return s;
 }
 
-// The float64 operators of one padded size, rounded once to float.  Both sums
-// are geometric series: sum_{f=a}^{b} e^{2 pi i f t} = e^{i pi (a+b) t}
-// sin(pi (b-a+1) t) / sin(pi t), and (b - a + 1) at t = 0 -- the only integer
-// phase, since t = (i - n mag) / L lies in (-1, 1).  With |t| >= 1 / L the
-// quotient is well conditioned.
-// full: both axes keep the whole complex spectrum f = -N/2 .. N/2-1 (the
-// fft2 / centred-block / ifft2 form of _interpolation.pyx:153-200), i.e. C = A.
-void build_ops(int N, int mag, bool full, std::vector<float>& ct, std::vector<float>& acat) {
-  const int L = N * mag;
-  const int N2 = (N + 1) / 2;
-  const int fa = -(N - N2), fb = N2 - 1;  // y frequencies kept
-  const int K = N / 2;                    // x frequencies kept: 0 .. K
-  const double pi = 3.14159265358979323846;
+// The float64 operators of one padded size.  Both sums are geometric series:
+// sum_{f=a}^{b} e^{2 pi i f t} = e^{i pi (a+b) t} sin(pi (b-a+1) t) / sin(pi t),
+// and (b - a + 1) at t = 0 -- the only integer phase, since t = (i - n mag) / L
+// lies in (-1, 1).  With |t| >= 1 / L the quotient is well conditioned.  An entry
+// depends on d = i - n mag only: every operator is read from tables over d.
+struct OpTables {
+  int N, mag, L;
+  std::vector<double> are, aim, cre, cim;  // [d + L]; aim holds -A_im
+  OpTables(int N_, int mag_) : N(N_), mag(mag_), L(N_ * mag_) {
+    const int N2 = (N + 1) / 2;
+    const int fa = -(N - N2), fb = N2 - 1;  // y frequencies kept
+    const int K = N / 2;                    // x frequencies kept: 0 .. K
+    const double pi = 3.14159265358979323846;
+    for (auto* v : {&are, &aim, &cre, &cim}) v->resize((size_t)2 * L);
+    for (int d = 1 - L; d < L; ++d) {
+      const double t = (double)d / L;  // i / L - n / N
+      // A: sum over f = fa .. fb
+      const double da = d == 0 ? (double)(fb - fa + 1)
+                               : std::sin(pi * (fb - fa + 1) * t) / std::sin(pi * t);
+      const double pa = pi * (fa + fb) * t;
+      are[d + L] = std::cos(pa) * da / L;
+      aim[d + L] = -std::sin(pa) * da / L;
+      // C: 2 sum_{k=0}^{K} e^{2 pi i k t} - 1
+      const double dc = d == 0 ? (double)(K + 1) : std::sin(pi * (K + 1) * t) / std::sin(pi * t);
+      const double pc = pi * K * t;
+      cre[d + L] = (2.0 * std::cos(pc) * dc - 1.0) / L;
+      cim[d + L] = 2.0 * std::sin(pc) * dc / L;
+    }
+  }
+  size_t at(int i, int n) const { return (size_t)(i - n * mag + L); }
+};
+
+// Both axes with the whole complex spectrum f = -N/2 .. N/2-1 (the fft2 /
+// centred-block / ifft2 form of _interpolation.pyx:153-200), i.e. C = A, rounded
+// once to float.
+void build_full_ops(const OpTables& o, std::vector<float>& ct, std::vector<float>& acat) {
+  const int N = o.N, L = o.L;
   ct.assign((size_t)2 * N * L, 0.f);
   acat.assign((size_t)L * 2 * N, 0.f);
   for (int i = 0; i < L; ++i)
     for (int n = 0; n < N; ++n) {
-      const double t = (double)(i - n * mag) / L;  // i / L - n / N
-      const bool zero = i == n * mag;
-      // A: sum over f = fa .. fb
-      const double da = zero ? (double)(fb - fa + 1)
-                             : std::sin(pi * (fb - fa + 1) * t) / std::sin(pi * t);
-      const double pa = pi * (fa + fb) * t;
-      acat[(size_t)i * 2 * N + n] = (float)(std::cos(pa) * da / L);
-      acat[(size_t)i * 2 * N + N + n] = (float)(-std::sin(pa) * da / L);
-      if (full) {
-        ct[(size_t)n * L + i] = acat[(size_t)i * 2 * N + n];
-        ct[(size_t)N * L + (size_t)n * L + i] = (float)(std::sin(pa) * da / L);
-        continue;
-      }
-      // C: 2 sum_{k=0}^{K} e^{2 pi i k t} - 1
-      const double dc = zero ? (double)(K + 1) : std::sin(pi * (K + 1) * t) / std::sin(pi * t);
-      const double pc = pi * K * t;
-      ct[(size_t)n * L + i] = (float)((2.0 * std::cos(pc) * dc - 1.0) / L);
-      ct[(size_t)N * L + (size_t)n * L + i] = (float)(2.0 * std::sin(pc) * dc / L);
+      acat[(size_t)i * 2 * N + n] = (float)o.are[o.at(i, n)];
+      acat[(size_t)i * 2 * N + N + n] = (float)o.aim[o.at(i, n)];
+      ct[(size_t)n * L + i] = (float)o.are[o.at(i, n)];
+      ct[(size_t)N * L + (size_t)n * L + i] = (float)-o.aim[o.at(i, n)];
     }
+}
+
+// the tile row (or column) that row n of the square shows: k copies of `size`,
+// the centre one upright, the square's first row roi rows into them
+int mirror_index(int n, int size, int k, int roi) {
+  const int copy = (n + roi) / size, in = (n + roi) % size;
+  return ((copy - (k - 1) / 2) & 1) ? size - 1 - in : in;
+}
+
+int round16(int n) { return (n + 15) / 16 * 16; }
+
+// A_re, s and the signs for tiles of th rows: the columns of a tile row's images
+// are added in float64 and rounded once
+void build_row_ops(const OpTables& o, int th, int k, int roi, std::vector<float>& a,
+                   std::vector<float>& s, std::vector<float>& e) {
+  const int N = o.N, L = o.L, nr = round16(th);
+  std::vector<double> row(nr), sign(nr, 0.0);
+  std::vector<int> of(N);
+  for (int n = 0; n < N; ++n) {
+    of[n] = mirror_index(n, th, k, roi);
+    sign[of[n]] += (n & 1) ? -1.0 : 1.0;
+  }
+  a.resize((size_t)L * nr);
+  s.resize(L);
+  for (int i = 0; i < L; ++i) {
+    std::fill(row.begin(), row.end(), 0.0);
+    for (int n = 0; n < N; ++n) row[of[n]] += o.are[o.at(i, n)];
+    for (int n = 0; n < nr; ++n) a[(size_t)i * nr + n] = (float)row[n];
+    s[i] = (float)o.aim[o.at(i, 0)];
+  }
+  e.assign(sign.begin(), sign.end());
+}
+
+// C_re^T and C_im^T for tiles of tw columns
+void build_col_ops(const OpTables& o, int tw, int k, int roi, std::vector<float>& ct) {
+  const int N = o.N, L = o.L, nc = round16(tw);
+  std::vector<double> acc((size_t)2 * nc * L, 0.0);
+  for (int n = 0; n < N; ++n) {
+    const int c = mirror_index(n, tw, k, roi);
+    double* re = acc.data() + (size_t)c * L;
+    double* im = re + (size_t)nc * L;
+    for (int i = 0; i < L; ++i) {
+      re[i] += o.cre[o.at(i, n)];
+      im[i] += o.cim[o.at(i, n)];
+    }
+  }
+  ct.assign(acc.begin(), acc.end());
 }
 
 std::vector<float> hann_inner(int n) {
@@ -528,6 +623,48 @@ int fht_upload(nx_fht_plan* p, const std::vector<float>& h, float** out) {
   if (e != cudaSuccess) return cuda_status(e, "FHT plan upload");
   *out = d;
   return NX_OK;
+}
+
+// the operators of a tile, shared by the tiles of the same sizes
+int build_tile_ops(nx_fht_plan* p, nx_fht_plan::Tile& t) {
+  t.ops = t.rows = t.cols = -1;
+  for (size_t k = 0; k < p->ops.size(); ++k)
+    if (p->ops[k].N == t.N) t.ops = (int)k;
+  for (size_t k = 0; k < p->row_ops.size(); ++k)
+    if (p->row_ops[k].N == t.N && p->row_ops[k].th == t.th) t.rows = (int)k;
+  for (size_t k = 0; k < p->col_ops.size(); ++k)
+    if (p->col_ops[k].N == t.N && p->col_ops[k].tw == t.tw) t.cols = (int)k;
+  const bool full = p->variant == NX_FHT_FULL_SPECTRUM;
+  if (full ? t.ops >= 0 : (t.rows >= 0 && t.cols >= 0)) return NX_OK;
+  const OpTables tab(t.N, p->mag);
+  std::vector<float> v, w, e;
+  int rc = NX_OK;
+  if (full) {
+    nx_fht_plan::Ops o{t.N, tab.L, nullptr, nullptr};
+    build_full_ops(tab, v, w);
+    rc = fht_upload(p, v, &o.ct);
+    if (!rc) rc = fht_upload(p, w, &o.acat);
+    p->ops.push_back(o);
+    t.ops = (int)p->ops.size() - 1;
+    return rc;
+  }
+  if (t.rows < 0) {
+    nx_fht_plan::RowOps o{t.N, t.th, round16(t.th), nullptr, nullptr, nullptr};
+    build_row_ops(tab, t.th, t.kh, t.y_roi, v, w, e);
+    rc = fht_upload(p, v, &o.a);
+    if (!rc) rc = fht_upload(p, w, &o.s);
+    if (!rc) rc = fht_upload(p, e, &o.e);
+    p->row_ops.push_back(o);
+    t.rows = (int)p->row_ops.size() - 1;
+  }
+  if (!rc && t.cols < 0) {
+    nx_fht_plan::ColOps o{t.N, t.tw, round16(t.tw), nullptr};
+    build_col_ops(tab, t.tw, t.kw, t.x_roi, v);
+    rc = fht_upload(p, v, &o.ct);
+    p->col_ops.push_back(o);
+    t.cols = (int)p->col_ops.size() - 1;
+  }
+  return rc;
 }
 
 void fht_plan_free(nx_fht_plan* p) {
@@ -582,24 +719,14 @@ int nx_fht_plan_create_ex(nx_fht_plan** out, int H, int W, int magnification, in
       t.kw += 1 - t.kw % 2;
       t.y_roi = (t.kh * t.th - N) / 2;
       t.x_roi = (t.kw * t.tw - N) / 2;
-      t.ops = -1;
-      for (size_t k = 0; k < p->ops.size(); ++k)
-        if (p->ops[k].N == N) t.ops = (int)k;
-      if (t.ops < 0) {
-        nx_fht_plan::Ops o{N, N * magnification, nullptr, nullptr};
-        std::vector<float> ct, acat;
-        build_ops(N, magnification, variant == NX_FHT_FULL_SPECTRUM, ct, acat);
-        int rc = fht_upload(p, ct, &o.ct);
-        if (!rc) rc = fht_upload(p, acat, &o.acat);
-        if (rc) {
-          fht_plan_free(p);
-          return rc;
-        }
-        p->ops.push_back(o);
-        t.ops = (int)p->ops.size() - 1;
+      t.N = N;
+      int rc = build_tile_ops(p, t);
+      if (rc) {
+        fht_plan_free(p);
+        return rc;
       }
       if (p->tiled) {
-        int rc = fht_upload(p, hann_inner(t.th * magnification), &t.wr);
+        rc = fht_upload(p, hann_inner(t.th * magnification), &t.wr);
         if (!rc) rc = fht_upload(p, hann_inner(t.tw * magnification), &t.wc);
         if (rc) {
           fht_plan_free(p);
@@ -608,11 +735,16 @@ int nx_fht_plan_create_ex(nx_fht_plan** out, int H, int W, int magnification, in
       }
       p->tiles.push_back(t);
     }
-  for (const auto& o : p->ops)
-    p->frame_floats = std::max(p->frame_floats,
-                               (size_t)o.N * o.N +
-                                   (size_t)(variant == NX_FHT_FULL_SPECTRUM ? 2 : 1) * o.N * o.L +
-                                   (size_t)o.L * o.L + o.L + o.N);
+  for (const auto& t : p->tiles) {
+    const size_t N = t.N, L = N * magnification;
+    if (variant == NX_FHT_FULL_SPECTRUM) {
+      p->frame_floats = std::max(p->frame_floats, N * N + 2 * N * L + L * L);
+    } else {  // tile, U, Z, r, alternating sums
+      const size_t nr = p->row_ops[t.rows].n, nc = p->col_ops[t.cols].n;
+      p->frame_floats = std::max(p->frame_floats,
+                                 nr * nc + std::min(nr, nc) * L + L * L + L + nc);
+    }
+  }
   if (p->tiled) {
     // blending weights: the windows summed in the reference's tile order
     const size_t plane = (size_t)H * magnification * W * magnification;
@@ -682,13 +814,7 @@ int nx_fht_interpolate(const nx_fht_plan* p, const float* d_in, int T, float* d_
     float* out = d_out + (size_t)t0 * plane;
     if (p->tiled) NX_CUDA_TRY(cudaMemsetAsync(out, 0, (size_t)tc * plane * sizeof(float), s));
     for (const auto& t : p->tiles) {
-      const auto& o = p->ops[t.ops];
-      const int N = o.N, L = o.L;
-      float* X = work;
-      float* U = X + (size_t)tc * N * N;
-      float* Z = U + (size_t)tc * (full ? 2 : 1) * N * L;
-      float* r = Z + (size_t)tc * L * L;
-      float* alt = r + (size_t)tc * L;
+      const int N = t.N, L = N * mag;
       // (min, max) slots of the tile input and of the interpolated square: two sets
       // in turn, each cleared while the other's tile runs (the first by itself)
       int* mm = mms[set];
@@ -697,11 +823,16 @@ int nx_fht_interpolate(const nx_fht_plan* p, const float* d_in, int T, float* d_
         NX_CUDA_TRY(cudaGetLastError());
         clear = full;
       }
-      fht_gather_kernel<<<dim3(blocks_for((long long)N * N, 256, 256), (unsigned)tc), 256, 0,
-                          s>>>(in, p->H, p->W, t.r0, t.c0, t.th, t.tw, N, t.kh, t.kw, t.y_roi,
-                               t.x_roi, X, mm);
-      NX_CUDA_TRY(cudaGetLastError());
+      float* const X = work;
+      float* Z;
       if (full) {
+        const auto& o = p->ops[t.ops];
+        float* U = X + (size_t)tc * N * N;
+        Z = U + (size_t)tc * 2 * N * L;
+        fht_gather_kernel<<<dim3(blocks_for((long long)N * N, 256, 256), (unsigned)tc), 256, 0,
+                            s>>>(in, p->H, p->W, t.r0, t.c0, t.th, t.tw, N, t.kh, t.kw, t.y_roi,
+                                 t.x_roi, X, mm);
+        NX_CUDA_TRY(cudaGetLastError());
         // U = X [C_re^T | C_im^T] stacked (batch (frame, part)), then
         // Z = [A_re | -A_im] [U_re ; U_im]: one image per sweep, whose scores
         // keep their bits
@@ -712,22 +843,43 @@ int nx_fht_interpolate(const nx_fht_plan* p, const float* d_in, int T, float* d_
         NX_CUDA_TRY(gemm(o.acat, U, Z, L, L, 2 * N, 2 * N, L, L, tc, b2,
                          Rank1{nullptr, 0, nullptr, mm}, s));
       } else {
-        // r of the rank-1 term, then U = X C_re^T (the frames' squares stacked) and
-        // Z = A_re U + s r^T
-        const bool own = N <= kAltInline;
+        const auto& ro = p->row_ops[t.rows];
+        const auto& co = p->col_ops[t.cols];
+        const int nr = ro.n, nc = co.n;
+        float* U = X + (size_t)tc * nr * nc;
+        Z = U + (size_t)tc * std::min(nr, nc) * L;
+        float* r = Z + (size_t)tc * L * L;
+        float* alt = r + (size_t)tc * L;
+        fht_tile_kernel<<<dim3(blocks_for((long long)nr * nc, 256, 256), (unsigned)tc), 256, 0,
+                          s>>>(in, p->H, p->W, t.r0, t.c0, t.th, t.tw, nr, nc, X, mm);
+        NX_CUDA_TRY(cudaGetLastError());
+        // r of the rank-1 term
+        const bool own = nr <= kAltInline && nc <= kAltInline;
         if (!own) {
-          fht_alternate_kernel<<<dim3((unsigned)((N + 31) / 32), (unsigned)tc), 256, 0, s>>>(X, N,
-                                                                                             alt);
+          fht_alternate_kernel<<<dim3((unsigned)((nc + 31) / 32), (unsigned)tc), 256, 0, s>>>(
+              X, ro.e, nr, nc, alt);
           NX_CUDA_TRY(cudaGetLastError());
         }
         fht_rank1_kernel<<<dim3((unsigned)((L + 31) / 32), (unsigned)tc), 256, 0, s>>>(
-            own ? X : nullptr, alt, o.ct + (size_t)N * L, N, L, r, mms[set ^ 1], tc);
+            own ? X : nullptr, ro.e, alt, co.ct + (size_t)nc * L, nr, nc, L, r, mms[set ^ 1], tc);
         NX_CUDA_TRY(cudaGetLastError());
-        NX_CUDA_TRY(gemm(X, o.ct, U, tc * N, L, N, N, L, L, 1, GemmBatch{1, 0, 0, 0, 0, 0, 0},
-                         Rank1{}, s));
-        const GemmBatch b2{1, 0, 0, (long long)N * L, 0, (long long)L * L, 0};
-        NX_CUDA_TRY(gemm(o.acat, U, Z, L, L, N, 2 * N, L, L, tc, b2,
-                         Rank1{o.acat + N, 2LL * N, r, mm}, s));
+        // the product onto the L x L square, the larger, runs over the tile's
+        // shorter side: U = X C_re^T (the frames' tiles stacked), Z = A_re U + s r^T,
+        // or U = A_re X, Z = U C_re^T + s r^T.  8 frames of 300 x 260 at m = 2 (three
+        // interpolations of tiles of 256 x 256, 256 x 36, 76 x 256 and 76 x 36): the
+        // products 1.08 ms over mirrored squares of N x N, 0.72 ms so.
+        const Rank1 u{ro.s, 1, r, mm};
+        if (nr <= nc) {
+          NX_CUDA_TRY(gemm(X, co.ct, U, tc * nr, L, nc, nc, L, L, 1,
+                           GemmBatch{1, 0, 0, 0, 0, 0, 0}, Rank1{}, s));
+          const GemmBatch b2{1, 0, 0, (long long)nr * L, 0, (long long)L * L, 0};
+          NX_CUDA_TRY(gemm(ro.a, U, Z, L, L, nr, nr, L, L, tc, b2, u, s));
+        } else {
+          const GemmBatch b1{1, 0, 0, (long long)nr * nc, 0, (long long)L * nc, 0};
+          NX_CUDA_TRY(gemm(ro.a, X, U, L, nc, nr, nr, nc, nc, tc, b1, Rank1{}, s));
+          const GemmBatch b2{1, (long long)L * nc, 0, 0, 0, (long long)L * L, 0};
+          NX_CUDA_TRY(gemm(U, co.ct, Z, L, L, nc, nc, L, L, tc, b2, u, s));
+        }
       }
       const int oh = t.th * mag, ow = t.tw * mag;
       fht_finish_kernel<<<dim3((unsigned)((ow + 127) / 128),
