@@ -155,55 +155,67 @@ __global__ void __launch_bounds__(256) sgemm_kernel(const float* __restrict__ A,
 }
 
 
-// The same product in 128 x 128 tiles, 8 x 8 per thread on packed f32x2 (two
-// columns per register pair), the next K slice loaded into registers behind the
-// current one and stored to the other half of a double buffer.  Needs K a
+// The same product in 64 HA x 64 HB tiles, 4 HA x 4 HB per thread on packed f32x2
+// (two columns per register pair), the next K slice loaded into registers behind
+// the current one and stored to the other half of a double buffer.  Needs K a
 // multiple of 16, N and the leading dimensions multiples of 4 and 16-byte
-// aligned operands; M is guarded per row.
-constexpr int kBT = 128, kBK = 16;
+// aligned operands; M is guarded per row.  Every output is one chain of fused
+// multiply-adds in ascending k, so the tile changes no bit.
+constexpr int kBK = 16;
+// more blocks than this for a tile to be taken: one for every SM.  The products of
+// 8 frames of 300 x 260 at m = 2 (20 to 512 blocks of 128 x 128): 696 us in 128 x 128
+// tiles alone, 602 / 579 / 606 us with the line at 76 / 152 / 304 blocks; one
+// 512 x 512 frame at m = 2 whole: 623, 427 / 428 / 424 us.
+constexpr int kGemmFill = 152;
+template <int HA, int HB>
 __global__ void __launch_bounds__(256, 2)
     sgemm_big_kernel(const float* __restrict__ A, const float* __restrict__ B,
                      float* __restrict__ C, int M, int N, int K, int lda, int ldb, int ldc,
                      GemmBatch bt, Rank1 u) {
-  __shared__ __align__(16) float As[2][kBK][kBT + 4];
-  __shared__ __align__(16) float Bs[2][kBK][kBT];
+  constexpr int BM = 64 * HA, BN = 64 * HB;
+  __shared__ __align__(16) float As[2][kBK][BM + 4];
+  __shared__ __align__(16) float Bs[2][kBK][BN];
   const int zo = blockIdx.z / bt.inner, zi = blockIdx.z % bt.inner;
   A += zo * bt.sa_o + zi * bt.sa_i;
   B += zo * bt.sb_o + zi * bt.sb_i;
   C += zo * bt.sc_o + zi * bt.sc_i;
-  const int m0 = blockIdx.y * kBT, n0 = blockIdx.x * kBT;
+  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
   const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
-  // staging: thread t loads A rows t / 4 and + 64, K quad t % 4, and B rows
-  // t / 32 and + 8, column quad t % 32
-  const int ar = tid / 4, ak = tid % 4 * 4, br = tid / 32, bc = tid % 32 * 4;
+  // staging: thread t loads A rows t / 4 + 64 h, K quad t % 4, and HB quads of the
+  // B slice, row by row
+  constexpr int QB = BN / 4, RB = 256 / QB;
+  const int ar = tid / 4, ak = tid % 4 * 4, br = tid / QB, bc = tid % QB * 4;
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-  float4 pa[2], pb[2];
+  float4 pa[HA], pb[HB];
   auto load = [&](int k0) {
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
+    for (int h = 0; h < HA; ++h) {
       const int gm = m0 + ar + 64 * h;
       pa[h] = gm < M ? __ldg(reinterpret_cast<const float4*>(A + (size_t)gm * lda + k0 + ak)) : zero;
-      pb[h] = n0 + bc < N ? __ldg(reinterpret_cast<const float4*>(
-                                B + (size_t)(k0 + br + 8 * h) * ldb + n0 + bc))
-                          : zero;
     }
+#pragma unroll
+    for (int h = 0; h < HB; ++h)
+      pb[h] = n0 + bc < N ? __ldg(reinterpret_cast<const float4*>(
+                                B + (size_t)(k0 + br + RB * h) * ldb + n0 + bc))
+                          : zero;
   };
   auto store = [&](int b) {
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
+    for (int h = 0; h < HA; ++h) {
       As[b][ak][ar + 64 * h] = pa[h].x;
       As[b][ak + 1][ar + 64 * h] = pa[h].y;
       As[b][ak + 2][ar + 64 * h] = pa[h].z;
       As[b][ak + 3][ar + 64 * h] = pa[h].w;
-      *reinterpret_cast<float4*>(&Bs[b][br + 8 * h][bc]) = pb[h];
     }
+#pragma unroll
+    for (int h = 0; h < HB; ++h) *reinterpret_cast<float4*>(&Bs[b][br + RB * h][bc]) = pb[h];
   };
-  // rows ty * 4 + {0..3} and 64 + ..., columns tx * 4 + {0..3} and 64 + ...
-  float2 acc[8][4];
+  // rows ty * 4 + {0..3} + 64 h, columns tx * 4 + {0..3} + 64 h
+  float2 acc[4 * HA][2 * HB];
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+  for (int i = 0; i < 4 * HA; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = make_float2(0.f, 0.f);
+    for (int j = 0; j < 2 * HB; ++j) acc[i][j] = make_float2(0.f, 0.f);
   load(0);
   store(0);
   __syncthreads();
@@ -213,30 +225,36 @@ __global__ void __launch_bounds__(256, 2)
     if (more) load(k0 + kBK);
 #pragma unroll
     for (int k = 0; k < kBK; ++k) {
-      const float4 a0 = *reinterpret_cast<const float4*>(&As[b][k][ty * 4]);
-      const float4 a1 = *reinterpret_cast<const float4*>(&As[b][k][64 + ty * 4]);
-      const float4 b0 = *reinterpret_cast<const float4*>(&Bs[b][k][tx * 4]);
-      const float4 b1 = *reinterpret_cast<const float4*>(&Bs[b][k][64 + tx * 4]);
-      const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-      const float2 bv[4] = {make_float2(b0.x, b0.y), make_float2(b0.z, b0.w),
-                            make_float2(b1.x, b1.y), make_float2(b1.z, b1.w)};
+      float4 av[HA];
+      float2 bv[2 * HB];
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
+      for (int h = 0; h < HA; ++h) av[h] = *reinterpret_cast<const float4*>(&As[b][k][64 * h + ty * 4]);
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-          acc[i][j] = __ffma2_rn(make_float2(av[i], av[i]), bv[j], acc[i][j]);
+      for (int h = 0; h < HB; ++h) {
+        const float4 v = *reinterpret_cast<const float4*>(&Bs[b][k][64 * h + tx * 4]);
+        bv[2 * h] = make_float2(v.x, v.y);
+        bv[2 * h + 1] = make_float2(v.z, v.w);
+      }
+#pragma unroll
+      for (int i = 0; i < 4 * HA; ++i) {
+        const float4 q = av[i >> 2];
+        const float a = (i & 3) == 0 ? q.x : (i & 3) == 1 ? q.y : (i & 3) == 2 ? q.z : q.w;
+#pragma unroll
+        for (int j = 0; j < 2 * HB; ++j)
+          acc[i][j] = __ffma2_rn(make_float2(a, a), bv[j], acc[i][j]);
+      }
     }
     if (more) store(b ^ 1);
     __syncthreads();
   }
   float lo = INFINITY, hi = -INFINITY;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
+  for (int i = 0; i < 4 * HA; ++i) {
     const int gm = m0 + ty * 4 + (i & 3) + (i >> 2) * 64;
     if (gm >= M) continue;
     const float si = u.s ? __ldg(u.s + gm * u.lds) : 0.f;
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
+    for (int h = 0; h < HB; ++h) {
       const int gn = n0 + tx * 4 + 64 * h;
       if (gn >= N) continue;
       float4 v = make_float4(acc[i][2 * h].x, acc[i][2 * h].y, acc[i][2 * h + 1].x,
@@ -254,29 +272,42 @@ __global__ void __launch_bounds__(256, 2)
   if (u.mm) block_minmax(lo, hi, u.mm + 4 * blockIdx.z + 2);
 }
 
-// operands the big tiles can take, and sizes they fill; else 64 x 64 tiles.
-// The 8 frames of 300 x 260 at m = 2 (24 products of 256- and 128-pixel squares):
-// 2.97 ms in 64 x 64 tiles with both parts of A, 1.08 ms in these.
-bool big_tiles(const float* A, const float* B, const float* C, int M, int N, int K, int lda,
-               int ldb, int ldc, const GemmBatch& bt, const Rank1& u) {
+// operands the vector form can take
+bool vector_operands(const float* A, const float* B, const float* C, int N, int K, int lda,
+                     int ldb, int ldc, const GemmBatch& bt, const Rank1& u) {
   const uintptr_t ptrs = reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) |
                          reinterpret_cast<uintptr_t>(C) | reinterpret_cast<uintptr_t>(u.r);
   const long long strides = lda | ldb | ldc | bt.sa_o | bt.sa_i | bt.sb_o | bt.sb_i | bt.sc_o |
                             bt.sc_i;
-  return (ptrs & 15u) == 0 && strides % 4 == 0 && K % kBK == 0 && N % 4 == 0 && M >= 96 && N >= 96;
+  return (ptrs & 15u) == 0 && strides % 4 == 0 && K % kBK == 0 && N % 4 == 0;
+}
+
+template <int HA, int HB>
+cudaError_t gemm_big(const float* A, const float* B, float* C, int M, int N, int K, int lda,
+                     int ldb, int ldc, int batches, const GemmBatch& bt, const Rank1& u,
+                     cudaStream_t s) {
+  const dim3 grid((unsigned)((N + 64 * HB - 1) / (64 * HB)), (unsigned)((M + 64 * HA - 1) / (64 * HA)),
+                  (unsigned)batches);
+  sgemm_big_kernel<HA, HB><<<grid, 256, 0, s>>>(A, B, C, M, N, K, lda, ldb, ldc, bt, u);
+  return cudaGetLastError();
 }
 
 cudaError_t gemm(const float* A, const float* B, float* C, int M, int N, int K, int lda, int ldb,
                  int ldc, int batches, const GemmBatch& bt, const Rank1& u, cudaStream_t s) {
-  if (big_tiles(A, B, C, M, N, K, lda, ldb, ldc, bt, u)) {
-    const dim3 grid((unsigned)((N + kBT - 1) / kBT), (unsigned)((M + kBT - 1) / kBT),
-                    (unsigned)batches);
-    sgemm_big_kernel<<<grid, 256, 0, s>>>(A, B, C, M, N, K, lda, ldb, ldc, bt, u);
-  } else {
-    const dim3 grid((unsigned)((N + kGB - 1) / kGB), (unsigned)((M + kGB - 1) / kGB),
-                    (unsigned)batches);
-    sgemm_kernel<<<grid, 256, 0, s>>>(A, B, C, M, N, K, lda, ldb, ldc, bt, u);
+  if (vector_operands(A, B, C, N, K, lda, ldb, ldc, bt, u)) {
+    // the largest tile that still gives every SM a block, else the smallest
+    const auto blocks = [&](int ha, int hb) {
+      return (long long)((N + 64 * hb - 1) / (64 * hb)) * ((M + 64 * ha - 1) / (64 * ha)) * batches;
+    };
+    if (blocks(2, 2) > kGemmFill)
+      return gemm_big<2, 2>(A, B, C, M, N, K, lda, ldb, ldc, batches, bt, u, s);
+    if (blocks(1, 2) > kGemmFill)
+      return gemm_big<1, 2>(A, B, C, M, N, K, lda, ldb, ldc, batches, bt, u, s);
+    return gemm_big<1, 1>(A, B, C, M, N, K, lda, ldb, ldc, batches, bt, u, s);
   }
+  const dim3 grid((unsigned)((N + kGB - 1) / kGB), (unsigned)((M + kGB - 1) / kGB),
+                  (unsigned)batches);
+  sgemm_kernel<<<grid, 256, 0, s>>>(A, B, C, M, N, K, lda, ldb, ldc, bt, u);
   return cudaGetLastError();
 }
 
@@ -867,7 +898,7 @@ int nx_fht_interpolate(const nx_fht_plan* p, const float* d_in, int T, float* d_
         // shorter side: U = X C_re^T (the frames' tiles stacked), Z = A_re U + s r^T,
         // or U = A_re X, Z = U C_re^T + s r^T.  8 frames of 300 x 260 at m = 2 (three
         // interpolations of tiles of 256 x 256, 256 x 36, 76 x 256 and 76 x 36): the
-        // products 1.08 ms over mirrored squares of N x N, 0.72 ms so.
+        // products 1.08 ms over mirrored squares of N x N, 0.72 ms so (0.58 ms now).
         const Rank1 u{ro.s, 1, r, mm};
         if (nr <= nc) {
           NX_CUDA_TRY(gemm(X, co.ct, U, tc * nr, L, nc, nc, L, L, 1,

@@ -25,3 +25,17 @@ TOL = 1e-5
 def test_folded_mirrors(shape, m):
     x = np.random.default_rng(m).poisson(50, shape).astype(np.float32)
     assert rel_err(nx.fht_space_interpolation(x, m), O.fht_space_interpolation(x, m)) <= TOL
+
+
+@pytest.mark.parametrize("shape,m", [((8, 256, 250), 4), ((8, 128, 120), 2), ((3, 200, 256), 3)])
+def test_product_tiles_by_size(shape, m):
+    """Products of enough blocks for each of the tile sizes, and partly filled ones."""
+    x = np.random.default_rng(m).poisson(50, shape).astype(np.float32)
+    assert rel_err(nx.fht_space_interpolation(x, m), O.fht_space_interpolation(x, m)) <= TOL
+
+
+@pytest.mark.parametrize("shape", [(2, 224, 257), (1, 225, 481), (2, 449, 30), (1, 500, 260)])
+def test_tiles_overlap(shape):
+    """Frames whose last tiles lie inside, at the edge of and beyond the one before."""
+    x = np.random.default_rng(shape[1]).poisson(50, shape).astype(np.float32)
+    assert rel_err(nx.fht_space_interpolation(x, 2), O.fht_space_interpolation(x, 2)) <= TOL
