@@ -248,9 +248,11 @@ static int best_chunks(long long tiles, int n_tp, int fpt, int min_nf, long long
   return best;
 }
 
-// The chunks of an AVG sweep at m <= 2, the scored sweep's magnification: its
-// scores are published to full precision, so the split of its sums stays what
-// it was (passes of two frames, a start-up of 0.65 pass, >= 4 frames a chunk).
+// The chunks of an AVG sweep at m <= 2.  Sweeps feed scores that are computed and
+// reported in float64; at m <= 2 the RGC adds its samples in ascending order, so
+// with this split (passes of two frames, a start-up of 0.65 pass, >= 4 frames a
+// chunk) the maps, and the scores with them, keep their bits from version to
+// version.
 static int sweep_chunks(long long tiles, int n_tp, int fpt, int min_nf, long long resident) {
   int best = 1;
   double best_cost = 1e300;

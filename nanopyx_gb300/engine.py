@@ -273,7 +273,7 @@ def sweep_batch(stack, magnification: int, sensitivities, radii, frames_per_time
 # ---------------------------------------------------------------------------
 # bumped whenever the kernels' tiling or unit structure changes, so that tunings
 # made with an older build are not reused
-TUNE_LAYOUT = "ws3"
+TUNE_LAYOUT = "ws4"
 
 
 def _gpu_key():
