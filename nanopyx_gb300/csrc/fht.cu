@@ -40,7 +40,12 @@ namespace {
 
 constexpr int kFhtTile = 256;     // tile side of the reference's tiled path
 constexpr int kFhtOverlap = 16;
-constexpr int kFhtChunk = 8;      // frames per GEMM batch
+// Frames per GEMM batch: as many as keep their interpolated squares within half of
+// the L2 (the finish kernel reads them back), at least 8 and at most 64, so that
+// small squares fill the SMs: 100 x 64 x 64 at m = 2 in 69 us, 16 x 256 x 256 at m = 4 in
+// 277, 16 x 200 x 200 at m = 4 in 225 (282 in chunks of 8)
+constexpr int kFhtChunkMin = 8, kFhtChunkMax = 64;
+constexpr size_t kFhtChunkBytes = 64u << 20;
 
 int pow2_ceil(int n) {
   int p = 1;
@@ -544,6 +549,7 @@ struct nx_fht_plan {
   std::vector<float*> bufs;  // every device allocation of the plan
   float* wgt = nullptr;      // (H mag, W mag) blending weights (tiled path)
   size_t frame_floats = 0;   // workspace floats per frame of a chunk
+  int chunk = 1;             // frames per chunk
 };
 
 namespace nx {
@@ -787,8 +793,10 @@ int nx_fht_plan_create_ex(nx_fht_plan** out, int H, int W, int magnification, in
       }
       p->tiles.push_back(t);
     }
+  size_t square = 1;
   for (const auto& t : p->tiles) {
     const size_t N = t.N, L = N * magnification;
+    square = std::max(square, L * L * sizeof(float));
     if (variant == NX_FHT_FULL_SPECTRUM) {
       p->frame_floats = std::max(p->frame_floats, N * N + 2 * N * L + L * L);
     } else {  // tile, U, Z, r, alternating sums
@@ -797,6 +805,7 @@ int nx_fht_plan_create_ex(nx_fht_plan** out, int H, int W, int magnification, in
                                  nr * nc + std::min(nr, nc) * L + L * L + L + nc);
     }
   }
+  p->chunk = (int)std::min<size_t>(kFhtChunkMax, std::max<size_t>(kFhtChunkMin, kFhtChunkBytes / square));
   if (p->tiled) {
     // blending weights: the windows summed in the reference's tile order
     const size_t plane = (size_t)H * magnification * W * magnification;
@@ -830,7 +839,7 @@ int nx_fht_plan_destroy(nx_fht_plan* p) {
 
 size_t nx_fht_workspace_bytes(const nx_fht_plan* p, int T) {
   if (!p || T < 1) return 256;
-  const size_t tc = (size_t)std::min(T, kFhtChunk);
+  const size_t tc = (size_t)std::min(T, p->chunk);
   return 256 + ((tc * p->frame_floats * sizeof(float) + 255) / 256) * 256 +
          2 * tc * 4 * sizeof(int);
 }
@@ -855,13 +864,13 @@ int nx_fht_interpolate(const nx_fht_plan* p, const float* d_in, int T, float* d_
   const long long plane = (long long)outH * outW;
   char* base = (char*)d_ws + 256;
   float* work = (float*)base;
-  int* const mm0 = (int*)(base + ((std::min(T, kFhtChunk) * p->frame_floats * sizeof(float) + 255) /
+  int* const mm0 = (int*)(base + ((std::min(T, p->chunk) * p->frame_floats * sizeof(float) + 255) /
                                   256) * 256);
-  int* const mms[2] = {mm0, mm0 + 4 * std::min(T, kFhtChunk)};
+  int* const mms[2] = {mm0, mm0 + 4 * std::min(T, p->chunk)};
   int set = 0;
   bool clear = true;
-  for (int t0 = 0; t0 < T; t0 += kFhtChunk) {
-    const int tc = std::min(kFhtChunk, T - t0);
+  for (int t0 = 0; t0 < T; t0 += p->chunk) {
+    const int tc = std::min(p->chunk, T - t0);
     const float* in = d_in + (size_t)t0 * p->H * p->W;
     float* out = d_out + (size_t)t0 * plane;
     for (const auto& t : p->tiles) {

@@ -277,12 +277,11 @@ def _esrrf_st_fht(x: torch.Tensor, m: int, radius, sensitivity, iw, pad_edges) -
         xb = x[a:a + chunk].contiguous()
         n = xb.shape[0]
         mag = _fht_device(xb, m)
-        gc = torch.empty_like(xb)
-        gr = torch.empty_like(xb)
-        N.check(L.nx_roberts_cross(_ptr(xb), n, H, W, _ptr(gc), _ptr(gr), s), "Roberts-Cross")
-        gci = _fht_device(gc, 2 * m)
-        gri = _fht_device(gr, 2 * m)
-        N.check(L.nx_rgc(_ptr(gci), _ptr(gri), _ptr(mag), n, H * m, W * m, m, float(radius),
+        # both gradients as one stack: one chain of launches for their interpolation
+        g = torch.empty((2 * n, H, W), dtype=torch.float32, device=xb.device)
+        N.check(L.nx_roberts_cross(_ptr(xb), n, H, W, _ptr(g), _ptr(g[n:]), s), "Roberts-Cross")
+        gi = _fht_device(g, 2 * m)
+        N.check(L.nx_rgc(_ptr(gi), _ptr(gi[n:]), _ptr(mag), n, H * m, W * m, m, float(radius),
                          float(sensitivity), 1 if iw else 0, 1 if pad_edges else 0,
                          _ptr(out[a:a + n]), s), "RadialGradientConvergence")
     return out
