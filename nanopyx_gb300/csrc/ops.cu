@@ -293,9 +293,9 @@ __global__ void rgc_kernel(const float* __restrict__ gc, const float* __restrict
 // shared load and seven arithmetic instructions.  A warp serves one output phase of
 // one input row, lanes along x; even and odd grid columns lie apart, so that its
 // lanes' gradients are neighbours.
-// 8 x 600 x 520, M = 2, R = 1.5: 128 us; 283 us with the gradients read and
-// normalised per sample, 409 us in the per-pixel kernel.  20 x 640 x 640, M = 5,
-// R = 2: 0.45 ms, 2.06 ms per pixel.
+// 8 x 600 x 520, M = 2, R = 1.5: 97 us (128 with the rows of the window not
+// unrolled); 283 us with the gradients read and normalised per sample, 409 us in
+// the per-pixel kernel.  20 x 640 x 640, M = 5, R = 2: 0.37 ms, 2.06 ms per pixel.
 constexpr int kRgcTableBytes = 48 * 1024;
 constexpr int kRgcTileRows = 8;
 constexpr int kRgcSharedMax = 128 * 1024;  // table and tile: at most 114,484 bytes (M = 1)
@@ -327,6 +327,8 @@ inline RgcTile rgc_tile(int M, int W2) {
   return t;
 }
 
+// W: the window's side (radii 0.5 to 3 in steps of 0.5, whose rows unroll), or 0
+template <int W>
 __global__ void __launch_bounds__(kBlock)
     rgc_table_kernel(const float* __restrict__ gc, const float* __restrict__ gr,
                      const float* __restrict__ img, int T, int rowsM, int colsM, int M,
@@ -335,7 +337,7 @@ __global__ void __launch_bounds__(kBlock)
   // table [py][px][j][i] of (unit offset, weight; 0: does not count, -); the
   // tile [row][column parity][column / 2]; sum of weights per phase
   extern __shared__ __align__(16) float4 rgct[];
-  const int W2 = sc.end - sc.start, MM = M * M;
+  const int W2 = W ? W : sc.end - sc.start, MM = M * M;
   float2* const cell = reinterpret_cast<float2*>(rgct + MM * W2 * W2);
   float* const wtot = reinterpret_cast<float*>(cell + tile.rows * 2 * tile.cols);
   for (int e = threadIdx.x; e < MM * W2 * W2; e += kBlock) {
@@ -403,11 +405,13 @@ __global__ void __launch_bounds__(kBlock)
       const float4* e = rgct + p * W2 * W2;
       float rgc = 0.f;
       for (int j = 0; j < W2; ++j, e += W2) {
+        // grid column cx + i: parity and index of even and odd i
         const float2* c = cell + (2 * yl + cy + j) * 2 * tile.cols + lane;
-#pragma unroll 4
+        const float2* c0 = cx ? c + tile.cols : c;
+        const float2* c1 = cx ? c + 1 : c + tile.cols;
+#pragma unroll(W ? W : 4)
         for (int i = 0; i < W2; ++i) {
-          const int q = cx + i;
-          const float2 g = c[(q & 1) * tile.cols + (q >> 1)];
+          const float2 g = (i & 1) ? c1[i >> 1] : c0[i >> 1];
           const float4 w = e[i];
           const float v = fmaf(-fabsf(fmaf(g.y, w.x, -(g.x * w.y))), w.z, w.z);
           if (fmaf(g.y, w.y, g.x * w.x) < 0.f) rgc += v;
@@ -1064,24 +1068,36 @@ cudaError_t launch_rgc(const float* gc, const float* gr, const float* img, int T
   const long long n = (long long)T * rowsM * colsM;
   if (n == 0) return cudaSuccess;
   // the table form where the table fits (e.g. M = 5 up to R = 2, M = 2 up to 6;
-  // 8 x 600 x 520, M = 2, R = 1.5: 128 against 409 us) and 32-bit positions hold
+  // 8 x 600 x 520, M = 2, R = 1.5: 97 against 409 us) and 32-bit positions hold
   const int W2 = sc.end - sc.start;
   const size_t table = (size_t)M * M * W2 * W2 * sizeof(float4);
   if (M <= 64 && table <= kRgcTableBytes && rowsM < (1 << 24) && colsM < (1 << 24)) {
     const RgcTile tile = rgc_tile(M, W2);
-    if (tile.bytes > 48 * 1024) {
-      const cudaError_t e = cudaFuncSetAttribute(
-          rgc_table_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRgcSharedMax);
-      if (e != cudaSuccess) return e;
+    const auto launch = [&](auto kernel) {
+      if (tile.bytes > 48 * 1024) {
+        const cudaError_t e = cudaFuncSetAttribute(
+            kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRgcSharedMax);
+        if (e != cudaSuccess) return e;
+      }
+      const long long units =
+          (long long)T * (((rowsM + M - 1) / M + kRgcTileRows - 1) / kRgcTileRows) *
+          (((colsM + M - 1) / M + 31) / 32);
+      // small images: several blocks per tile, so that every SM has two
+      const int parts = (int)std::min<long long>(M * M, std::max(1LL, 2 * 152 / units));
+      const dim3 grid((unsigned)std::min<long long>(units, 152LL * 8), (unsigned)parts);
+      kernel<<<grid, kBlock, tile.bytes, s>>>(gc, gr, img, T, rowsM, colsM, M, sc, iw, tile,
+                                              parts, out);
+      return cudaGetLastError();
+    };
+    switch (W2) {
+      case 3: return launch(rgc_table_kernel<3>);
+      case 5: return launch(rgc_table_kernel<5>);
+      case 7: return launch(rgc_table_kernel<7>);
+      case 9: return launch(rgc_table_kernel<9>);
+      case 11: return launch(rgc_table_kernel<11>);
+      case 13: return launch(rgc_table_kernel<13>);
+      default: return launch(rgc_table_kernel<0>);
     }
-    const long long units = (long long)T * (((rowsM + M - 1) / M + kRgcTileRows - 1) / kRgcTileRows) *
-                            (((colsM + M - 1) / M + 31) / 32);
-    // small images: several blocks per tile, so that every SM has two
-    const int parts = (int)std::min<long long>(M * M, std::max(1LL, 2 * 152 / units));
-    const dim3 grid((unsigned)std::min<long long>(units, 152LL * 8), (unsigned)parts);
-    rgc_table_kernel<<<grid, kBlock, tile.bytes, s>>>(gc, gr, img, T, rowsM, colsM, M, sc, iw,
-                                                      tile, parts, out);
-    return cudaGetLastError();
   }
   rgc_kernel<<<grid_for(n), kBlock, 0, s>>>(gc, gr, img, T, rowsM, colsM, M, sc, iw, out);
   return cudaGetLastError();

@@ -24,7 +24,8 @@ def inputs(m, T, h, w):
 
 
 @pytest.mark.parametrize("m,radius,h,w", [(1, 2.0, 17, 70), (2, 1.5, 8, 32), (2, 1.5, 9, 33),
-                                          (2, 6.0, 20, 40), (3, 2.0, 16, 31), (4, 1.0, 10, 65),
+                                          (2, 6.0, 20, 40), (3, 2.0, 16, 31), (3, 2.5, 9, 33),
+                                          (4, 1.0, 10, 65),
                                           (5, 2.0, 9, 35), (8, 1.0, 9, 33)])
 @pytest.mark.parametrize("pad", [False, True])
 def test_rgc_tiles(m, radius, h, w, pad):
