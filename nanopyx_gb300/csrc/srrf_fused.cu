@@ -103,7 +103,10 @@ __device__ __forceinline__ void ring_entry(float* e, float c, float ring, int M,
   e[7] = 0.f;
 }
 
-constexpr float kTiny = 1.17549435e-38f;  // 2^-126
+// Added to every squared gradient: keeps rsqrt finite without one, and no more
+// than a squared gradient's own rounding (an ulp up to 2^-125, half an ulp and
+// less above), so that radiality does not depend on a stack's units.
+constexpr float kTiny = 1.40129846e-45f;  // 2^-149, the smallest float
 
 // v >= 0 with the sign opposite to d's
 __device__ __forceinline__ float against(float v, float d) {
@@ -326,18 +329,19 @@ __global__ void __launch_bounds__(SrrfTile<M>::NT, 1) srrf_fused_kernel(const Sr
           }
           // dk = (1 - |vGy (xc - x0) - vGx (yc - y0)| / GMag / ringRadius)^2, 0
           // without a gradient; subtracted where the gradient points outwards.
-          // No comparisons (the ALU pipe was the busiest): kTiny, absorbed by any
-          // squared gradient above it, keeps rsqrt finite, a saturating FMA
-          // turns "any gradient" into 0 or 1, and the dot product's sign is
-          // moved onto dk by a logic operation (dk is 0 where it is 0).
+          // No comparisons (the ALU pipe was the busiest): rsqrt is 2^74.5 of
+          // kTiny alone and at most 2^74 with a gradient, so a saturating FMA
+          // of it turns "any gradient" into 0 or 1, and the dot product's sign
+          // is moved onto dk by a logic operation (dk is 0 where it is 0).
           const float2 g2 = __ffma2_rn(vgx, vgx, __ffma2_rn(vgy, vgy, make_float2(kTiny, kTiny)));
-          const float2 any = make_float2(__saturatef(__fmaf_rn(g2.x, 1.f / kTiny, -1.f)),
-                                         __saturatef(__fmaf_rn(g2.y, 1.f / kTiny, -1.f)));
+          const float2 rs = make_float2(rsqrtf(g2.x), rsqrtf(g2.y));
+          constexpr float kAnySlope = -2.11758237e-22f;  // -2^-72: 2^74.5 -> -5.66, 2^74 -> -4
+          const float2 any = make_float2(__saturatef(__fmaf_rn(rs.x, kAnySlope, 5.3f)),
+                                         __saturatef(__fmaf_rn(rs.y, kAnySlope, 5.3f)));
           const float2 cr = __ffma2_rn(vgy, make_float2(dx, dx),
                                        __fmul2_rn(vgx, make_float2(-dy, -dy)));
-          const float2 rs = __fmul2_rn(make_float2(rsqrtf(g2.x), rsqrtf(g2.y)),
-                                       make_float2(-p.inv_rr, -p.inv_rr));
-          float2 dk = __ffma2_rn(make_float2(fabsf(cr.x), fabsf(cr.y)), rs, make_float2(1.f, 1.f));
+          float2 dk = __ffma2_rn(__fmul2_rn(make_float2(fabsf(cr.x), fabsf(cr.y)), rs),
+                                 make_float2(-p.inv_rr, -p.inv_rr), make_float2(1.f, 1.f));
           dk = __fmul2_rn(dk, dk);
           const float2 dot = __ffma2_rn(vgx, make_float2(p.xr[s], p.xr[s]),
                                         __fmul2_rn(vgy, make_float2(p.yr[s], p.yr[s])));
