@@ -108,9 +108,9 @@ __device__ __forceinline__ void ring_entry(float* e, float c, float ring, int M,
 // less above), so that radiality does not depend on a stack's units.
 constexpr float kTiny = 1.40129846e-45f;  // 2^-149, the smallest float
 
-// v >= 0 with the sign opposite to d's
-__device__ __forceinline__ float against(float v, float d) {
-  return __int_as_float(__float_as_int(v) ^ (~__float_as_int(d) & 0x80000000));
+// v >= 0 with the sign of s
+__device__ __forceinline__ float with_sign(float v, float s) {
+  return __int_as_float(__float_as_int(v) | (__float_as_int(s) & 0x80000000));
 }
 
 template <int M>
@@ -331,8 +331,9 @@ __global__ void __launch_bounds__(SrrfTile<M>::NT, 1) srrf_fused_kernel(const Sr
           // without a gradient; subtracted where the gradient points outwards.
           // No comparisons (the ALU pipe was the busiest): rsqrt is 2^74.5 of
           // kTiny alone and at most 2^74 with a gradient, so a saturating FMA
-          // of it turns "any gradient" into 0 or 1, and the dot product's sign
-          // is moved onto dk by a logic operation (dk is 0 where it is 0).
+          // of it turns "any gradient" into 0 or 1, and the sign of the
+          // inward component (+0, never -0, where there is none: ring radius 0)
+          // is moved onto dk by a logic operation.
           const float2 g2 = __ffma2_rn(vgx, vgx, __ffma2_rn(vgy, vgy, make_float2(kTiny, kTiny)));
           const float2 rs = make_float2(rsqrtf(g2.x), rsqrtf(g2.y));
           constexpr float kAnySlope = -2.11758237e-22f;  // -2^-72: 2^74.5 -> -5.66, 2^74 -> -4
@@ -343,9 +344,10 @@ __global__ void __launch_bounds__(SrrfTile<M>::NT, 1) srrf_fused_kernel(const Sr
           float2 dk = __ffma2_rn(__fmul2_rn(make_float2(fabsf(cr.x), fabsf(cr.y)), rs),
                                  make_float2(-p.inv_rr, -p.inv_rr), make_float2(1.f, 1.f));
           dk = __fmul2_rn(dk, dk);
-          const float2 dot = __ffma2_rn(vgx, make_float2(p.xr[s], p.xr[s]),
-                                        __fmul2_rn(vgy, make_float2(p.yr[s], p.yr[s])));
-          dk = make_float2(against(dk.x, dot.x), against(dk.y, dot.y));
+          const float2 in = __ffma2_rn(vgx, make_float2(-p.xr[s], -p.xr[s]),
+                                       __ffma2_rn(vgy, make_float2(-p.yr[s], -p.yr[s]),
+                                                  make_float2(0.f, 0.f)));
+          dk = make_float2(with_sign(dk.x, in.x), with_sign(dk.y, in.y));
           div[px] = __ffma2_rn(any, dk, div[px]);
         }
       }
