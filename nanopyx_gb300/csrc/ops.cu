@@ -1239,7 +1239,9 @@ cudaError_t launch_mpc(float* img, int S, int rowsM, int colsM, int M, float* ma
   const bool vec = colsM % 4 == 0 && (reinterpret_cast<uintptr_t>(img) & 15u) == 0;
   const int gx = (colsM + kMpcThreads * (vec ? 4 : 1) - 1) / (kMpcThreads * (vec ? 4 : 1));
   const int npart = M * M * nch;
-  const int staged = npart <= kMpcStage;
+  // staged only where map and partials fit 48 KB together: from m = 79 on they do not,
+  // and the map alone (40 KB at m = 100) still does
+  const int staged = npart <= kMpcStage && (M * M + npart) * sizeof(float) <= 48 * 1024;
   const size_t smem = (size_t)(M * M + (staged ? npart : 0)) * sizeof(float);
   // rows per block: enough blocks for the chip (2048), but no more than 64 rows
   // (a longer walk gains nothing once the map is a small part of it); and within
