@@ -247,16 +247,50 @@ __device__ __forceinline__ float clamp0(float v) {
   return r;
 }
 
-// The powers that are not worth their code in every unrolled use.
-static __device__ __noinline__ float apply_sensitivity_slow(float r, int mode, int n, float s) {
-  return apply_sensitivity(r, mode, n, s);
+// r^1.5 of a frame pair, as power_compensated (common.cuh) forms it
+__device__ __forceinline__ float2 power_1p5(const float2& r) {
+  const float2 s = make_float2(__fsqrt_rn(r.x), __fsqrt_rn(r.y));
+  const float2 q = __fmul2_rn(r, s);
+  const float2 d = __ffma2_rn(make_float2(-s.x, -s.y), s, r);
+  const float2 e = __ffma2_rn(__fmul2_rn(make_float2(0.5f, 0.5f), d), s,
+                              __ffma2_rn(r, s, make_float2(-q.x, -q.y)));
+  const float2 v = __fadd2_rn(q, e);
+  return make_float2(v.x == v.x ? v.x : q.x, v.y == v.y ? v.y : q.y);
+}
+
+// The powers that are not worth their code in every unrolled use, a frame pair a
+// call (150 frames of 227 x 333, m = 5, s = 2.5: 3.27 ms, 3.54 with a call per value).
+static __device__ __noinline__ float2 apply_sensitivity_pair(float2 r, int mode, int n, float s) {
+  if (mode == 2) return make_float2(powf(r.x, s), powf(r.y, s));
+  float2 p = r, e = make_float2(0.f, 0.f), below = make_float2(1.f, 1.f);
+  if (mode == 1) {
+#pragma unroll 1
+    for (int k = 1; k < n; ++k) p = __fmul2_rn(p, r);
+    return p;
+  }
+  // power_compensated (common.cuh)
+#pragma unroll 1
+  for (int k = 1; k < n; ++k) {
+    const float2 q = __fmul2_rn(p, r);
+    e = __ffma2_rn(e, r, __ffma2_rn(p, r, make_float2(-q.x, -q.y)));
+    below = p;
+    p = q;
+  }
+  const float2 t = make_float2(__fsqrt_rn(r.x), __fsqrt_rn(r.y));
+  const float2 q = __fmul2_rn(p, t);
+  const float2 d = __ffma2_rn(make_float2(-t.x, -t.y), t, r);
+  e = __ffma2_rn(e, t, __ffma2_rn(p, t, make_float2(-q.x, -q.y)));
+  e = __ffma2_rn(__fmul2_rn(__fmul2_rn(make_float2(0.5f, 0.5f), below), d), t, e);
+  const float2 v = __fadd2_rn(q, e);
+  return make_float2(v.x == v.x ? v.x : q.x, v.y == v.y ? v.y : q.y);
 }
 
 // r ^ sensitivity of a thread's values (mode and n are uniform over the launch):
-// squares and cubes, and (HALF) the half-integer powers below 4, in place; the
-// others by call -- with powf and the square root inlined per sensitivity and
-// column, the AVG kernels' code outgrew the instruction cache (4 x 4 sweep of
-// 200 x 256 x 256, m = 4: 13.46 against 12.39 ms).
+// squares and cubes, and (HALF) the power 1.5, in place; the others by call --
+// with powf and the square root inlined per sensitivity and column, the AVG
+// kernels' code outgrew the instruction cache (4 x 4 sweep of 200 x 256 x 256,
+// m = 4: 13.46 against 12.39 ms), and the powers 2.5 and 3.5 in place cost every
+// kernel registers (m = 5: 30 to 70 bytes more spilled per thread).
 template <bool HALF, int A, int B>
 __device__ __forceinline__ void apply_sens_all(float2 (&r)[A][B], int mode, int n, float s) {
   if (mode == 0) return;
@@ -270,23 +304,17 @@ __device__ __forceinline__ void apply_sens_all(float2 (&r)[A][B], int mode, int 
       }
     return;
   }
-  if (HALF && mode == 3 && n <= 3) {
+  if (HALF && mode == 3 && n == 1) {
 #pragma unroll
     for (int i = 0; i < A; ++i)
 #pragma unroll
-      for (int j = 0; j < B; ++j) {
-        const float2 b = r[i][j], q = __fmul2_rn(b, b);
-        const float2 v = n == 1 ? b : (n == 3 ? __fmul2_rn(q, b) : q);
-        r[i][j] = __fmul2_rn(v, make_float2(__fsqrt_rn(b.x), __fsqrt_rn(b.y)));
-      }
+      for (int j = 0; j < B; ++j) r[i][j] = power_1p5(r[i][j]);
     return;
   }
 #pragma unroll
   for (int i = 0; i < A; ++i)
 #pragma unroll
-    for (int j = 0; j < B; ++j)
-      r[i][j] = make_float2(apply_sensitivity_slow(r[i][j].x, mode, n, s),
-                            apply_sensitivity_slow(r[i][j].y, mode, n, s));
+    for (int j = 0; j < B; ++j) r[i][j] = apply_sensitivity_pair(r[i][j], mode, n, s);
 }
 
 // geometry of one unit (tile, timepoint, frame chunk), shared by both roles
