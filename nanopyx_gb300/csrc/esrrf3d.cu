@@ -177,6 +177,12 @@ __global__ void __launch_bounds__(kPrepThreads)
   }
 }
 
+// g ^ sensitivity (modes 1 to 3 of apply_sensitivity), once a voxel and frame: called, so
+// that the kernel keeps to 64 registers (inlined 70, and 1.40 ms a call instead of 1.33)
+__device__ __noinline__ float power3d(float g, int mode, int n, float s) {
+  return mode == 2 ? powf(g, s) : power_compensated(g, n, mode == 3);
+}
+
 // Steps 3 and 4 for a frame pair: a block covers 32 x 8 output pixels inside the
 // margins and the mz voxels of one input slice.  tab holds, per window offset
 // [k][j][i], the unit offset and the weight (0: does not count); sample columns
@@ -307,8 +313,8 @@ __global__ void __launch_bounds__(256)
     if (!active) continue;
     float2 val = make_float2(__fdiv_rn(acc.x, wsum), __fdiv_rn(acc.y, wsum));
     auto power = [&](float g) {
-      if (g >= 0.f) return apply_sensitivity(g, p.sens_mode, p.sens_int, p.sensitivity);
-      return g < 0.f ? 0.f : g;
+      if (!(g >= 0.f)) return g < 0.f ? 0.f : g;
+      return p.sens_mode ? power3d(g, p.sens_mode, p.sens_int, p.sensitivity) : g;
     };
     val.x = power(val.x);
     val.y = power(val.y);
