@@ -76,16 +76,25 @@ __device__ __forceinline__ void quad_fma(Quad& q, float w, const Quad& v) {
   q.b = make_float4(x.x, x.y, y.x, y.y);
 }
 
-// 1 / |g| for the normalisation; 0 without a gradient.  An infinite gradient is
-// not normalised (scale 1, see unit): its RGC then overflows to NaN where the
-// reference's quotient does.
-__device__ __forceinline__ float unit_scale(float x, float y, float z) {
-  const float d = fmaf(z, z, fmaf(y, y, x * x));
-  return d > 0.f ? (d < INFINITY ? rsqrtf(d) : 1.f) : d == 0.f ? 0.f : d;
-}
-
-__device__ __forceinline__ float unit(float g, float s) {
-  return fminf(fabsf(g), 3.4e38f) == fabsf(g) ? g * s : (g != g ? g : copysignf(3.4e38f, g));
+// (x, y, z) to a unit vector; 0 without a gradient, and for an infinite one, whose
+// samples count nothing in the reference either (its quotient is NaN there)
+__device__ __forceinline__ void normalise(float& x, float& y, float& z) {
+  float d = fmaf(z, z, fmaf(y, y, x * x));
+  if (!(d > 1e-30f && d < 1e30f)) {  // the squares may not hold: scale first
+    const float m = fmaxf(fmaxf(fabsf(x), fabsf(y)), fabsf(z));
+    if (m == 0.f || isinf(m)) {
+      x = y = z = 0.f;
+      return;
+    }
+    x = __fdiv_rn(x, m);
+    y = __fdiv_rn(y, m);
+    z = __fdiv_rn(z, m);
+    d = fmaf(z, z, fmaf(y, y, x * x));
+  }
+  const float r = rsqrtf(d);
+  x *= r;
+  y *= r;
+  z *= r;
 }
 
 __global__ void __launch_bounds__(kPrepThreads)
@@ -125,11 +134,12 @@ __global__ void __launch_bounds__(kPrepThreads)
   const int x = x0 + threadIdx.x % kPrepCols;
   const int yb = y0 + threadIdx.x / kPrepCols * kPrepRun;
   if (x >= Wm) return;
-  auto store = [&](int y, const Quad& q) {
-    const float s0 = unit_scale(q.a.x, q.a.z, q.b.x), s1 = unit_scale(q.a.y, q.a.w, q.b.y);
+  auto store = [&](int y, Quad q) {
+    normalise(q.a.x, q.a.z, q.b.x);
+    normalise(q.a.y, q.a.w, q.b.y);
     const size_t o = ((size_t)z * Hm + y) * Wm + x;
-    A[o] = make_float4(unit(q.a.x, s0), unit(q.a.y, s1), unit(q.a.z, s0), unit(q.a.w, s1));
-    B[o] = make_float2(unit(q.b.x, s0), unit(q.b.y, s1));
+    A[o] = q.a;
+    B[o] = make_float2(q.b.x, q.b.y);
     I[o] = make_float2(q.b.z, q.b.w);
   };
   if (m == 1) {  // not magnified: the values themselves
