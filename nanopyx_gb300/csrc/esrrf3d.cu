@@ -23,12 +23,18 @@
 // at the same offsets, so their RGC is evaluated once wherever the same samples
 // lie inside the volume for all of them.
 //
-// What bounds it: issue and register reads of step 3 (15 packed operations per
-// sample and frame pair) and the L1 wavefronts of its two gradient loads.
-// 20 x 16 x 128 x 128, mxy = mz = 2, R = 1.5: one frame at a time, three scalar
-// gradients normalised at every sample and every voxel by itself 5.9 ms; frame
-// pairs, gradients normalised once, shared z voxels 1.5 ms; window columns in
-// registers 1.3 ms.
+// Rounding: weights formed in float64 and rounded once, gradients normalised to half
+// an ulp, |n x offset| from exact whole-pixel offsets by one square root good to
+// 2^-23, sums row by row.  Error against float64 at 20 x 16 x 128 x 128, mxy = mz = 2,
+// R = 1.5: 8.8e-8; with float32 unit offsets, q rsqrt(q) and one chain of sums 9.3e-8
+// (no magnification, R = 3, without intensity: 1.2e-7 against 5.6e-7).
+//
+// What bounds it: issue and register reads of step 3 (14 packed operations and two
+// square roots per sample and frame pair) and the L1 wavefronts of its two gradient
+// loads.  Same call: one frame at a time, three scalar gradients normalised at every
+// sample and every voxel by itself 5.9 ms; frame pairs, gradients normalised once,
+// shared z voxels 1.5 ms; window columns in registers 1.33 ms; one instruction for
+// the square root 1.24 ms.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -91,7 +97,8 @@ __device__ __forceinline__ void normalise(float& x, float& y, float& z) {
     z = __fdiv_rn(z, m);
     d = fmaf(z, z, fmaf(y, y, x * x));
   }
-  const float r = rsqrtf(d);
+  float r = rsqrtf(d);
+  r = fmaf(0.5f * r, fmaf(-d * r, r, 1.f), r);  // to half an ulp
   x *= r;
   y *= r;
   z *= r;
@@ -187,6 +194,14 @@ __global__ void __launch_bounds__(kPrepThreads)
   }
 }
 
+// square root to 2^-23 of |n x offset|^2, one instruction (a square below 2^-126
+// counts as 0: 1e-19 of a pixel)
+__device__ __forceinline__ float root(float q) {
+  float r;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(q));
+  return r;
+}
+
 // g ^ sensitivity (modes 1 to 3 of apply_sensitivity), once a voxel and frame: called, so
 // that the kernel keeps to 64 registers (inlined 70, and 1.40 ms a call instead of 1.33)
 __device__ __noinline__ float power3d(float g, int mode, int n, float s) {
@@ -195,9 +210,9 @@ __device__ __noinline__ float power3d(float g, int mode, int n, float s) {
 
 // Steps 3 and 4 for a frame pair: a block covers 32 x 8 output pixels inside the
 // margins and the mz voxels of one input slice.  tab holds, per window offset
-// [k][j][i], the unit offset and the weight (0: does not count); sample columns
-// and rows, from the voxel's float32 coordinates as the reference forms them,
-// are tabulated per block (-1: outside the image).
+// [k][j][i], the weight w (0: does not count) and w over the offset's length;
+// sample columns and rows, from the voxel's float32 coordinates as the reference
+// forms them, are tabulated per block (-1: outside the image).
 // NI: window columns known at compile time (4: radius 1 to below 2; 0: any) --
 // the columns' indices stay in registers and a window row's loads are in flight
 // together (whole call, 20 x 16 x 128 x 128, R = 1.5: 1.51 ms with the general
@@ -210,10 +225,10 @@ template <int NI>
 __global__ void __launch_bounds__(256)
     rgc3d_kernel(const __grid_constant__ Rgc3d p, const float4* __restrict__ A,
                  const float2* __restrict__ B, const float2* __restrict__ I,
-                 const float4* __restrict__ tab, int s_first, int frame, int two,
+                 const float2* __restrict__ tab, int s_first, int frame, int two,
                  float* __restrict__ out, float* __restrict__ mean) {
   __shared__ int cidx[NI > 0 ? NI : kMaxWin][32], ridx[NI > 0 ? NI : kMaxWin][8];
-  __shared__ float4 stab[NI > 0 ? kMaxTab : 1];
+  __shared__ float2 stab[NI > 0 ? kMaxTab : 1];
   const int nI = NI > 0 ? NI : p.s1 - p.s0 + 1;
   if (NI > 0)
     for (int e = threadIdx.x; e < (p.z1 - p.z0 + 1) * nI * nI; e += 256) stab[e] = __ldg(tab + e);
@@ -260,28 +275,26 @@ __global__ void __launch_bounds__(256)
   for (int k = p.z0; k <= p.z1; ++k)
     for (int r = ra + 1; r < rb; ++r) same = same && z_in(r, k) == z_in(ra, k);
   for (int r = ra; r < rb; r = same ? rb : r + 1) {
-    float2 acc = make_float2(0.f, 0.f);
-    float wsum = 0.f;
-    // one sample: unit gradients of the pair against the unit offset t (weight w)
-    auto sample = [&](const float4& t, const float4& a, const float2& nz, bool ok) {
+    // sums over window rows, then over the rows: short chains of roundings where one
+    // over all 44 samples (R = 1.5) cost most of the map's error
+    float2 acc = make_float2(0.f, 0.f), row = acc;
+    float wsum = 0.f, wrow = 0.f;
+    // one sample: unit gradients of the pair against the whole-pixel offset (x, y, z)
+    auto sample = [&](float x, float y, float z, const float2& t, const float4& a,
+                      const float2& nz, bool ok) {
       const float2 nx = make_float2(a.x, a.y), ny = make_float2(a.z, a.w);
-      const float2 rx = make_float2(t.x, t.x), ry = make_float2(t.y, t.y),
-                   rz = make_float2(t.z, t.z);
-      const float2 mx = make_float2(-t.x, -t.x), my = make_float2(-t.y, -t.y),
-                   mz = make_float2(-t.z, -t.z);
+      const float2 rx = make_float2(x, x), ry = make_float2(y, y), rz = make_float2(z, z);
+      const float2 mx = make_float2(-x, -x), my = make_float2(-y, -y), mz = make_float2(-z, -z);
       const float2 dot = __ffma2_rn(nz, rz, __ffma2_rn(ny, ry, __fmul2_rn(nx, rx)));
       const float2 c1 = __ffma2_rn(ny, rz, __fmul2_rn(nz, my));
       const float2 c2 = __ffma2_rn(nz, rx, __fmul2_rn(nx, mz));
       const float2 c3 = __ffma2_rn(nx, ry, __fmul2_rn(ny, mx));
-      // the smallest normal number keeps rsqrt finite for a zero cross product
-      const float tiny = 1.17549435e-38f;
-      const float2 q = __ffma2_rn(
-          c3, c3, __ffma2_rn(c2, c2, __ffma2_rn(c1, c1, make_float2(tiny, tiny))));
-      const float2 dk = __fmul2_rn(q, make_float2(rsqrtf(q.x), rsqrtf(q.y)));
-      const float2 v = __ffma2_rn(dk, make_float2(-t.w, -t.w), make_float2(t.w, t.w));
-      acc = __fadd2_rn(acc, make_float2(ok && dot.x < 0.f ? v.x : 0.f,
+      const float2 q = __ffma2_rn(c3, c3, __ffma2_rn(c2, c2, __fmul2_rn(c1, c1)));
+      const float2 dk = make_float2(root(q.x), root(q.y));
+      const float2 v = __ffma2_rn(dk, make_float2(-t.y, -t.y), make_float2(t.x, t.x));
+      row = __fadd2_rn(row, make_float2(ok && dot.x < 0.f ? v.x : 0.f,
                                         ok && dot.y < 0.f ? v.y : 0.f));
-      wsum += ok ? t.w : 0.f;
+      wrow += ok ? t.x : 0.f;
     };
     for (int k = p.z0; k <= p.z1; ++k) {
       if (!z_in(r, k)) continue;
@@ -289,9 +302,11 @@ __global__ void __launch_bounds__(256)
       // to s mz + k mz + r or, for r > 0, at worst just below it)
       const float4* Ak = A + (size_t)(s + k) * plane;
       const float2* Bk = B + (size_t)(s + k) * plane;
-      const float4* tk = (NI > 0 ? stab : tab) + (size_t)(k - p.z0) * nI * nI;
+      const float z = (float)k;
+      const float2* tk = (NI > 0 ? stab : tab) + (size_t)(k - p.z0) * nI * nI;
       for (int j = 0; j < nI; ++j) {
         const int ry = ridx[j][ty];
+        const float y = (float)(p.s0 + j);
         const float4* Aj = Ak + (size_t)max(ry, 0) * p.Wm;
         const float2* Bj = Bk + (size_t)max(ry, 0) * p.Wm;
         if constexpr (NI > 0) {
@@ -304,20 +319,25 @@ __global__ void __launch_bounds__(256)
           }
 #pragma unroll
           for (int i = 0; i < NI; ++i) {
-            const float4 t = tk[j * NI + i];
-            if (t.w == 0.f) continue;  // does not count
-            sample(t, a[i], nz[i], interior || (ry >= 0 && (cin >> i & 1u)));
+            const float2 t = tk[j * NI + i];
+            if (t.x == 0.f) continue;  // does not count
+            sample((float)(p.s0 + i), y, z, t, a[i], nz[i],
+                   interior || (ry >= 0 && (cin >> i & 1u)));
           }
         } else {
 #pragma unroll 4
           for (int i = 0; i < nI; ++i) {
-            const float4 t = __ldg(tk + j * nI + i);
-            if (t.w == 0.f) continue;
+            const float2 t = __ldg(tk + j * nI + i);
+            if (t.x == 0.f) continue;
             const int c = cidx[i][lane];
-            sample(t, __ldg(Aj + max(c, 0)), __ldg(Bj + max(c, 0)),
+            sample((float)(p.s0 + i), y, z, t, __ldg(Aj + max(c, 0)), __ldg(Bj + max(c, 0)),
                    interior || (ry >= 0 && c >= 0));
           }
         }
+        acc = __fadd2_rn(acc, row);
+        wsum += wrow;
+        row = make_float2(0.f, 0.f);
+        wrow = 0.f;
       }
     }
     if (!active) continue;
@@ -376,7 +396,7 @@ size_t nx_esrrf3d_workspace_bytes(int S, int H, int W, int magnification_xy,
   const size_t out = volm * magnification_z;
   return 256 + rup(volm * sizeof(float4)) + 2 * rup(volm * sizeof(float2)) +
          (mode ? rup(out * sizeof(float)) : 0) +
-         rup((size_t)kMaxWin * kMaxWin * kMaxWin * sizeof(float4));
+         rup((size_t)kMaxWin * kMaxWin * kMaxWin * sizeof(float2));
 }
 
 int nx_esrrf3d_st(const float* d_in, int T, int S, int H, int W, int magnification_xy,
@@ -430,22 +450,22 @@ int nx_esrrf3d_st(const float* d_in, int T, int S, int H, int W, int magnificati
   const int nI = p.s1 - p.s0 + 1, nK = p.z1 - p.z0 + 1;
   if (nI > kMaxWin || nK > kMaxWin)
     return nx::set_error("radius too large for the 3-D window"), NX_ERR_INVALID_ARG;
-  // per offset its unit vector and the weight of the reference's
-  // _c_calculate_dw3D (src/include/_c_sr_radial_gradient_convergence.c:96-102);
-  // weight 0 where the sample does not count
-  std::vector<float4> tab((size_t)nI * nI * nK);
+  // per offset the weight of the reference's _c_calculate_dw3D
+  // (src/include/_c_sr_radial_gradient_convergence.c:96-102), 0 where the sample
+  // does not count, and the weight over the offset's length; formed in float64 and
+  // rounded once (float32 factors to the fourth power are up to 2.4e-7 off)
+  std::vector<float2> tab((size_t)nI * nI * nK);
   for (int k = p.z0; k <= p.z1; ++k)
     for (int j = p.s0; j <= p.s1; ++j)
       for (int i = p.s0; i <= p.s1; ++i) {
         const double dxy2 = (double)i * i + (double)j * j;
         const double d = std::sqrt(dxy2 + (double)k * k), dxy = std::sqrt(dxy2);
-        float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+        float2 t = make_float2(0.f, 0.f);
         if (d != 0 && dxy <= (double)tSO && (double)k <= (double)tSO_z) {
-          const float wxy = (float)std::exp(-dxy2 / (double)tSS);
-          const float wz = (float)std::exp(-(double)k * k / (double)tSS_z);
-          const float D = (float)(d * (double)(wxy * wz));
-          t = make_float4((float)(i / d), (float)(j / d), (float)(k / d),
-                          (float)std::pow((double)D, 4.0));
+          const double D = d * std::exp(-dxy2 / (double)tSS - (double)k * k / (double)tSS_z);
+          const double w = D * D * D * D;
+          t.x = (float)w;
+          t.y = (float)(w / d);
         }
         tab[((size_t)(k - p.z0) * nI + (j - p.s0)) * nI + (i - p.s0)] = t;
       }
@@ -453,7 +473,7 @@ int nx_esrrf3d_st(const float* d_in, int T, int S, int H, int W, int magnificati
   while (p.z1 > p.z0) {
     bool any = false;
     for (size_t e = (size_t)(p.z1 - p.z0) * nI * nI; e < (size_t)(p.z1 - p.z0 + 1) * nI * nI; ++e)
-      any = any || tab[e].w != 0.f;
+      any = any || tab[e].x != 0.f;
     if (any) break;
     --p.z1;
   }
@@ -471,8 +491,8 @@ int nx_esrrf3d_st(const float* d_in, int T, int S, int H, int W, int magnificati
   b += rup(volm * sizeof(float2));
   float* mean = mode ? (float*)b : nullptr;
   if (mode) b += rup((size_t)nout * sizeof(float));
-  float4* dtab = (float4*)b;
-  NX_CUDA_TRY(cudaMemcpyAsync(dtab, tab.data(), tab.size() * sizeof(float4),
+  float2* dtab = (float2*)b;
+  NX_CUDA_TRY(cudaMemcpyAsync(dtab, tab.data(), tab.size() * sizeof(float2),
                               cudaMemcpyHostToDevice, s));
   NX_CUDA_TRY(cudaMemsetAsync(d_out, 0, (size_t)nout * sizeof(float), s));
   if (mean) NX_CUDA_TRY(cudaMemsetAsync(mean, 0, (size_t)nout * sizeof(float), s));
