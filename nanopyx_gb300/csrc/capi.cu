@@ -222,24 +222,19 @@ static int check_plan(const nx_esrrf_plan* p) {
   return NX_OK;
 }
 
-// Frame chunks per timepoint of a launch over `tiles` x `n_tp` units
-// (deterministic in its inputs).  The resident CTAs stride over (tile, timepoint,
-// chunk) units, so a CTA runs about ceil(units / resident) units, each costing
-// its frame pairs plus a start-up of about 1.35 pairs (its constants and the
-// first pass, which nothing overlaps: 100 x 256 x 256, m = 5 in chunks of 1, 2,
-// 4, 6, 50, 100 frames takes 19.0, 19.1, 27.4, 36.2, 213, 411 us per unit at
-// 8.2 us a pair).  The chunk count with the smallest estimate wins: few chunks
-// for large stacks, enough to fill every SM for small ones; stacks below 8 frames
-// (two passes) stay whole, so that they give the bits of a streamed block.
-static int best_chunks(long long tiles, int n_tp, int fpt, int min_nf, long long resident) {
-  int best = 1;
+// Of lo .. hi frame chunks per timepoint, the fewest with the smallest estimate
+// for a launch over `tiles` x `n_tp` units (deterministic in its inputs): the
+// resident CTAs stride over (tile, timepoint, chunk) units, so a CTA runs about
+// ceil(units / resident) units, each costing its frame pairs plus a start-up.
+static int cheapest_chunks(long long tiles, int n_tp, int fpt, long long resident, int lo, int hi,
+                           double start_up) {
+  int best = lo;
   double best_cost = 1e300;
-  const int cmax = min_nf < 8 ? 1 : std::min(min_nf / 2, 64);
-  for (int c = 1; c <= cmax; ++c) {
+  for (int c = lo; c <= hi; ++c) {
     const long long units = tiles * n_tp * c;
     const double per_cta = (double)((units + resident - 1) / resident);
     const double pairs = ((fpt + c - 1) / c + 1) / 2;
-    const double cost = per_cta * (pairs + 1.35);
+    const double cost = per_cta * (pairs + start_up);
     if (cost < best_cost * 0.999) {
       best_cost = cost;
       best = c;
@@ -248,25 +243,27 @@ static int best_chunks(long long tiles, int n_tp, int fpt, int min_nf, long long
   return best;
 }
 
-// The chunks of an AVG sweep at m <= 2.  Sweeps feed scores that are computed and
-// reported in float64; at m <= 2 the RGC adds its samples in ascending order, so
-// with this split (passes of two frames, a start-up of 0.65 pass, >= 4 frames a
-// chunk) the maps, and the scores with them, keep their bits from version to
-// version.
-static int sweep_chunks(long long tiles, int n_tp, int fpt, int min_nf, long long resident) {
-  int best = 1;
-  double best_cost = 1e300;
-  const int cmax = std::max(1, std::min(min_nf / 4, 64));
-  for (int c = 1; c <= cmax; ++c) {
-    const long long units = tiles * n_tp * c;
-    const double per_cta = (double)((units + resident - 1) / resident);
-    const double cost = per_cta * (std::ceil((double)fpt / c / 2.0) + 0.65);
-    if (cost < best_cost * 0.999) {
-      best_cost = cost;
-      best = c;
-    }
-  }
-  return best;
+// The fewest chunks a launch may have.  A chunk's running mean and moments are one
+// chain over its frames, whose rounding grows with the square root of their number,
+// and chunks are merged by few operations: with a start-up charged at 0.65 pairs, half
+// of what it costs, a near tie goes to the shorter chain (mean of 200 frames, 256 x 256,
+// m = 4: 5 chunks of 40, error 7.3e-8; 2 of 100 by the full charge, 1 % faster by the
+// estimate, 1.27e-7).  At least 4 frames, a full pass, each.
+static int least_chunks(long long tiles, int n_tp, int fpt, int min_nf, long long resident) {
+  return cheapest_chunks(tiles, n_tp, fpt, resident, 1, std::max(1, std::min(min_nf / 4, 64)),
+                         0.65);
+}
+
+// Frame chunks per timepoint: from least_chunks on, those with the smallest estimate
+// at the full start-up of about 1.35 pairs (a unit's constants and the first pass,
+// which nothing overlaps: 100 x 256 x 256, m = 5 in chunks of 1, 2, 4, 6, 50, 100
+// frames takes 19.0, 19.1, 27.4, 36.2, 213, 411 us per unit at 8.2 us a pair): few
+// chunks for large stacks, enough to fill every SM for small ones.  Stacks below 8
+// frames (two passes) stay whole, so that they give the bits of a streamed block.
+static int best_chunks(long long tiles, int n_tp, int fpt, int min_nf, long long resident) {
+  const int lo = least_chunks(tiles, n_tp, fpt, min_nf, resident);
+  const int hi = min_nf < 8 ? 1 : std::min(min_nf / 2, 64);
+  return cheapest_chunks(tiles, n_tp, fpt, resident, lo, std::max(lo, hi), 1.35);
 }
 
 static int plan_chunks(const nx_esrrf_plan* p, int T, int fpt, int n_tp) {
@@ -860,7 +857,10 @@ int nx_esrrf_batch_create(nx_esrrf_batch** out, const nx_esrrf_item* items, int 
       const long long tiles = (long long)((p->W + 31) / 32) * ((p->H + p->fused->geo.TY - 1) / p->fused->geo.TY);
       const long long resident =
           (long long)std::max(1, p->fused->occupancy[bi.mode](std::max(1, it.n_sens))) * sms;
-      const auto rule = it.n_sens > 0 && p->M <= 2 ? sweep_chunks : best_chunks;
+      // sweeps at m <= 2 feed scores reported in float64; the RGC adds its samples in
+      // ascending order there, and with the least chunks the maps, and the scores with
+      // them, are the same bits from version to version
+      const auto rule = it.n_sens > 0 && p->M <= 2 ? least_chunks : best_chunks;
       const int c = rule(tiles, bi.n_tp, bi.fpt, min_nf, resident);
       fpu = std::max(1, (min_nf + c - 1) / c);
     }
