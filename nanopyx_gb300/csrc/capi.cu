@@ -243,37 +243,39 @@ static int cheapest_chunks(long long tiles, int n_tp, int fpt, long long residen
   return best;
 }
 
-// The fewest chunks a launch may have.  A chunk's running mean and moments are one
-// chain over its frames, whose rounding grows with the square root of their number,
-// and chunks are merged by few operations: with a start-up charged at 0.65 pairs, half
-// of what it costs, a near tie goes to the shorter chain (mean of 200 frames, 256 x 256,
-// m = 4: 5 chunks of 40, error 7.3e-8; 2 of 100 by the full charge, 1 % faster by the
-// estimate, 1.27e-7).  At least 4 frames, a full pass, each.
+// The fewest chunks of a mean.  A chunk's running mean is one chain over its frames,
+// whose rounding grows with the square root of their number, and chunks are merged by
+// few operations: with a start-up charged at 0.65 pairs, half of what it costs, a near
+// tie goes to the shorter chain (mean of 200 frames, 256 x 256, m = 4: 5 chunks of 40,
+// error 7.3e-8; 2 of 100 by the full charge, 1 % faster by the estimate, 1.27e-7).  At
+// least 4 frames, a full pass, each.  The moments of VAR and TAC2 gain nothing: merging
+// theirs costs as much (322 frames of 26 x 64, TAC2: 17 chunks 3.4e-6, 21 4.8e-6).
 static int least_chunks(long long tiles, int n_tp, int fpt, int min_nf, long long resident) {
   return cheapest_chunks(tiles, n_tp, fpt, resident, 1, std::max(1, std::min(min_nf / 4, 64)),
                          0.65);
 }
 
-// Frame chunks per timepoint: from least_chunks on, those with the smallest estimate
-// at the full start-up of about 1.35 pairs (a unit's constants and the first pass,
-// which nothing overlaps: 100 x 256 x 256, m = 5 in chunks of 1, 2, 4, 6, 50, 100
-// frames takes 19.0, 19.1, 27.4, 36.2, 213, 411 us per unit at 8.2 us a pair): few
-// chunks for large stacks, enough to fill every SM for small ones.  Stacks below 8
+// Frame chunks per timepoint: those with the smallest estimate at the full start-up of
+// about 1.35 pairs (a unit's constants and the first pass, which nothing overlaps:
+// 100 x 256 x 256, m = 5 in chunks of 1, 2, 4, 6, 50, 100 frames takes 19.0, 19.1,
+// 27.4, 36.2, 213, 411 us per unit at 8.2 us a pair), for means from least_chunks on:
+// few chunks for large stacks, enough to fill every SM for small ones.  Stacks below 8
 // frames (two passes) stay whole, so that they give the bits of a streamed block.
-static int best_chunks(long long tiles, int n_tp, int fpt, int min_nf, long long resident) {
-  const int lo = least_chunks(tiles, n_tp, fpt, min_nf, resident);
+static int best_chunks(long long tiles, int n_tp, int fpt, int min_nf, long long resident,
+                       int mode) {
+  const int lo = mode == kModeSum ? least_chunks(tiles, n_tp, fpt, min_nf, resident) : 1;
   const int hi = min_nf < 8 ? 1 : std::min(min_nf / 2, 64);
   return cheapest_chunks(tiles, n_tp, fpt, resident, lo, std::max(lo, hi), 1.35);
 }
 
-static int plan_chunks(const nx_esrrf_plan* p, int T, int fpt, int n_tp) {
+static int plan_chunks(const nx_esrrf_plan* p, int mode, int T, int fpt, int n_tp) {
   if (!p->fused) return 1;
   const int TY = p->fused->geo.TY;
   const long long tiles = (long long)((p->W + 31) / 32) * ((p->H + TY - 1) / TY);
   const int min_nf = std::min(fpt, T - (n_tp - 1) * fpt);
   const long long resident =
       (long long)std::max(1, p->fused->occupancy[kModeFull](1)) * device_sms();
-  return best_chunks(tiles, n_tp, fpt, min_nf, resident);
+  return best_chunks(tiles, n_tp, fpt, min_nf, resident, mode);
 }
 
 static size_t align256(size_t b) { return (b + 255) / 256 * 256; }
@@ -288,6 +290,8 @@ static int corr_count(int mask) {
 static int fields_for(int corr_mask) {
   return (corr_mask & (NX_CORR_VAR | NX_CORR_TAC2)) ? 5 : 1;
 }
+
+static int record_mode(int fields) { return fields == 5 ? kModeFull : kModeSum; }
 
 static void fill_params(const nx_esrrf_plan* p, FusedParams& fp, const float* in, int T, int fpt,
                         int n_tp, int chunks, float* out, unsigned* status) {
@@ -545,8 +549,8 @@ int nx_esrrf_st(const nx_esrrf_plan* p, const float* d_in, int T, float* d_out, 
   // frames are independent, so chunks only balance the units (40 x 400 x 300,
   // m = 2, R = 1: 212 us in one chunk, 207 in two; 20 x 64 x 64, m = 5: 97 and 44)
   if (p->fused)
-    return launch_fused_mode(p, kModeStack, d_in, T, T, 1, plan_chunks(p, T, T, 1), d_out, status,
-                             s);
+    return launch_fused_mode(p, kModeStack, d_in, T, T, 1, plan_chunks(p, kModeStack, T, T, 1),
+                             d_out, status, s);
   float* scratch = (float*)((char*)d_ws + kStatusBytes);
   const size_t planeM = (size_t)p->rowsM * p->colsM;
   for (int t = 0; t < T; ++t) {
@@ -583,7 +587,7 @@ size_t nx_esrrf_workspace_bytes(const nx_esrrf_plan* p, int T, int fpt, int corr
   const int F = fields_for(corr_mask);
   size_t b = kStatusBytes;
   if (p->fused) {
-    const int chunks = plan_chunks(p, T, fpt, n_tp);
+    const int chunks = plan_chunks(p, record_mode(F), T, fpt, n_tp);
     b += align256((size_t)n_tp * chunks * F * planeM * sizeof(float));
   } else {
     b += align256((size_t)n_tp * 5 * planeM * sizeof(float));
@@ -622,8 +626,8 @@ int nx_esrrf_run_stage1(const nx_esrrf_plan* p, const float* d_in, int T, int fp
   NX_CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(unsigned), s));
   float* rec = (float*)cur;
   if (p->fused) {
-    const int chunks = plan_chunks(p, T, fpt, n_tp);
-    return launch_fused_mode(p, F == 5 ? kModeFull : kModeSum, d_in, T, fpt, n_tp, chunks, rec,
+    const int chunks = plan_chunks(p, record_mode(F), T, fpt, n_tp);
+    return launch_fused_mode(p, record_mode(F), d_in, T, fpt, n_tp, chunks, rec,
                              status, s);
   }
   cur += align256((size_t)n_tp * 5 * planeM * sizeof(float));
@@ -654,7 +658,7 @@ int nx_esrrf_run_stage2(const nx_esrrf_plan* p, int T, int fpt, int corr_mask, i
   float* rec = (float*)cur;
   int chunks = 1, Fr = 5;
   if (p->fused) {
-    chunks = plan_chunks(p, T, fpt, n_tp);
+    chunks = plan_chunks(p, record_mode(F), T, fpt, n_tp);
     Fr = F;
     cur += align256((size_t)n_tp * chunks * F * planeM * sizeof(float));
   } else {
@@ -710,7 +714,7 @@ int nx_esrrf_accum_push(const nx_esrrf_plan* p, const float* d_block, int T_bloc
   // block records: chunks merged in order into rec chunk 0 ... then into acc
   int chunks = 1;
   if (p->fused) {
-    chunks = plan_chunks(p, T_block, T_block, 1);
+    chunks = plan_chunks(p, kModeFull, T_block, T_block, 1);
     rc = launch_fused_mode(p, kModeFull, d_block, T_block, T_block, 1, chunks, rec, status, s);
     if (rc) return rc;
   } else {
@@ -860,8 +864,9 @@ int nx_esrrf_batch_create(nx_esrrf_batch** out, const nx_esrrf_item* items, int 
       // sweeps at m <= 2 feed scores reported in float64; the RGC adds its samples in
       // ascending order there, and with the least chunks the maps, and the scores with
       // them, are the same bits from version to version
-      const auto rule = it.n_sens > 0 && p->M <= 2 ? least_chunks : best_chunks;
-      const int c = rule(tiles, bi.n_tp, bi.fpt, min_nf, resident);
+      const int c = it.n_sens > 0 && p->M <= 2
+                        ? least_chunks(tiles, bi.n_tp, bi.fpt, min_nf, resident)
+                        : best_chunks(tiles, bi.n_tp, bi.fpt, min_nf, resident, bi.mode);
       fpu = std::max(1, (min_nf + c - 1) / c);
     }
     bi.chunks = std::max(1, std::min(min_nf, (min_nf + fpu - 1) / fpu));
