@@ -293,9 +293,14 @@ int nx_fht_interpolate(const nx_fht_plan* plan, const float* d_in, int T, float*
  * radius * PSF_ratio / voxel_ratio.  Voxels outside the margins are 0.
  *   src/nanopyx/core/transform/_le_esrrf3d.pyx:35-140
  *   src/include/_c_sr_radial_gradient_convergence.c:92-204
- *   src/include/_c_gradients.c:75-116                                        */
+ *   src/include/_c_gradients.c:75-116
+ * Two frames are taken at a time where ws_bytes allows: _range gives the least a
+ * call accepts and what frame pairs need (about twice that), _bytes the latter
+ * up to 4 GiB and the least for larger volumes.  The results are the same bits. */
 size_t nx_esrrf3d_workspace_bytes(int S, int H, int W, int magnification_xy,
                                   int magnification_z, int mode);
+void nx_esrrf3d_workspace_range(int S, int H, int W, int magnification_xy, int magnification_z,
+                                int mode, size_t* least, size_t* pairs);
 int nx_esrrf3d_st(const float* d_in, int T, int S, int H, int W, int magnification_xy,
                   int magnification_z, double radius, double radius_z, float sensitivity,
                   int mode, int do_intensity_weighting, float* d_out, void* d_ws,

@@ -104,6 +104,7 @@ _SIGS = {
     "nx_fht_workspace_bytes": (_SZ, [_P, _I]),
     "nx_fht_interpolate": (_I, [_P, _P, _I, _P, _P, _SZ, _P]),
     "nx_esrrf3d_workspace_bytes": (_SZ, [_I, _I, _I, _I, _I, _I]),
+    "nx_esrrf3d_workspace_range": (None, [_I, _I, _I, _I, _I, _I, C.POINTER(_SZ), C.POINTER(_SZ)]),
     "nx_esrrf3d_st": (_I, [_P, _I, _I, _I, _I, _I, _I, C.c_double, C.c_double, C.c_float, _I, _I,
                            _P, _P, _SZ, _P]),
     "nx_gaussian_blur_workspace_bytes": (_SZ, [_I, _I]),

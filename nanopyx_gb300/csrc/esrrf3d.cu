@@ -40,6 +40,7 @@
 #include <algorithm>
 #include <climits>
 #include <cmath>
+#include <type_traits>
 #include <vector>
 
 #include "common.cuh"
@@ -104,9 +105,34 @@ __device__ __forceinline__ void normalise(float& x, float& y, float& z) {
   z *= r;
 }
 
+size_t rup(size_t b) { return (b + 255) / 256 * 256; }
+
+// The magnified volumes between the two kernels: unit gradients (x, y) and z, and the
+// frame, of a frame pair side by side -- A (x, x', y, y'), B (z, z'), I (v, v') -- or
+// of one frame (A (x, y), B (z), I (v)) at half the memory.
+template <bool PAIR>
+struct Volumes {
+  using TA = typename std::conditional<PAIR, float4, float2>::type;
+  using TB = typename std::conditional<PAIR, float2, float>::type;
+  TA* __restrict__ A;
+  TB* __restrict__ B;
+  TB* __restrict__ I;
+  static size_t bytes(size_t voxels) {
+    return rup(voxels * sizeof(TA)) + 2 * rup(voxels * sizeof(TB));
+  }
+  explicit Volumes(char* base, size_t voxels)
+      : A((TA*)base), B((TB*)(base + rup(voxels * sizeof(TA)))),
+        I((TB*)(base + rup(voxels * sizeof(TA)) + rup(voxels * sizeof(TB)))) {}
+};
+__device__ __forceinline__ float4 both(const float4& a) { return a; }
+__device__ __forceinline__ float4 both(const float2& a) { return make_float4(a.x, a.x, a.y, a.y); }
+__device__ __forceinline__ float2 two_of(const float2& a) { return a; }
+__device__ __forceinline__ float2 two_of(float a) { return make_float2(a, a); }
+
+template <bool PAIR>
 __global__ void __launch_bounds__(kPrepThreads)
     prep3d_kernel(const float* __restrict__ v0, const float* __restrict__ v1, int H, int W, int m,
-                  int z_first, float4* __restrict__ A, float2* __restrict__ B, float2* __restrict__ I) {
+                  int z_first, const Volumes<PAIR> vol) {
   extern __shared__ __align__(16) float4 patch[];  // [PR][PC][2]
   const int Hm = H * m, Wm = W * m;
   const int nbx = (Wm + kPrepCols - 1) / kPrepCols;
@@ -145,9 +171,15 @@ __global__ void __launch_bounds__(kPrepThreads)
     normalise(q.a.x, q.a.z, q.b.x);
     normalise(q.a.y, q.a.w, q.b.y);
     const size_t o = ((size_t)z * Hm + y) * Wm + x;
-    A[o] = q.a;
-    B[o] = make_float2(q.b.x, q.b.y);
-    I[o] = make_float2(q.b.z, q.b.w);
+    if constexpr (PAIR) {
+      vol.A[o] = q.a;
+      vol.B[o] = make_float2(q.b.x, q.b.y);
+      vol.I[o] = make_float2(q.b.z, q.b.w);
+    } else {
+      vol.A[o] = make_float2(q.a.x, q.a.z);
+      vol.B[o] = q.b.x;
+      vol.I[o] = q.b.z;
+    }
   };
   if (m == 1) {  // not magnified: the values themselves
     for (int y = yb; y < min(yb + kPrepRun, Hm); ++y) {
@@ -219,14 +251,19 @@ __device__ __noinline__ float power3d(float g, int mode, int n, float s) {
 // loop, 1.28 with NI = 4; NI = 6 at R = 2 lost, 3.2 against 2.3: a third of its loads
 // belong to samples outside the radius).
 constexpr int kMaxWin = 64;  // window offsets per axis are at most 2 int(radius) + 2
+// up to this workspace nx_esrrf3d_workspace_bytes asks for frame pairs; above it for the
+// least, 16 bytes per magnified voxel instead of 32, so that a volume near the limit of
+// the memory still fits (one frame at a time: 2.17 ms a call instead of 1.24)
+constexpr size_t kPairBytes = 4ull << 30;
 constexpr int kMaxTab = 64;  // table entries kept in shared memory (NI > 0)
 
-template <int NI>
+template <int NI, bool PAIR>
 __global__ void __launch_bounds__(256)
-    rgc3d_kernel(const __grid_constant__ Rgc3d p, const float4* __restrict__ A,
-                 const float2* __restrict__ B, const float2* __restrict__ I,
+    rgc3d_kernel(const __grid_constant__ Rgc3d p, const Volumes<PAIR> vol,
                  const float2* __restrict__ tab, int s_first, int frame, int two,
                  float* __restrict__ out, float* __restrict__ mean) {
+  using TA = typename Volumes<PAIR>::TA;
+  using TB = typename Volumes<PAIR>::TB;
   __shared__ int cidx[NI > 0 ? NI : kMaxWin][32], ridx[NI > 0 ? NI : kMaxWin][8];
   __shared__ float2 stab[NI > 0 ? kMaxTab : 1];
   const int nI = NI > 0 ? NI : p.s1 - p.s0 + 1;
@@ -300,22 +337,22 @@ __global__ void __launch_bounds__(256)
       if (!z_in(r, k)) continue;
       // slice of the magnified volumes: (int)(vz mz) / mz = s + k (vz mz rounds
       // to s mz + k mz + r or, for r > 0, at worst just below it)
-      const float4* Ak = A + (size_t)(s + k) * plane;
-      const float2* Bk = B + (size_t)(s + k) * plane;
+      const TA* Ak = vol.A + (size_t)(s + k) * plane;
+      const TB* Bk = vol.B + (size_t)(s + k) * plane;
       const float z = (float)k;
       const float2* tk = (NI > 0 ? stab : tab) + (size_t)(k - p.z0) * nI * nI;
       for (int j = 0; j < nI; ++j) {
         const int ry = ridx[j][ty];
         const float y = (float)(p.s0 + j);
-        const float4* Aj = Ak + (size_t)max(ry, 0) * p.Wm;
-        const float2* Bj = Bk + (size_t)max(ry, 0) * p.Wm;
+        const TA* Aj = Ak + (size_t)max(ry, 0) * p.Wm;
+        const TB* Bj = Bk + (size_t)max(ry, 0) * p.Wm;
         if constexpr (NI > 0) {
           float4 a[NI];
           float2 nz[NI];
 #pragma unroll
           for (int i = 0; i < NI; ++i) {
-            a[i] = __ldg(Aj + cx[i]);
-            nz[i] = __ldg(Bj + cx[i]);
+            a[i] = both(__ldg(Aj + cx[i]));
+            nz[i] = two_of(__ldg(Bj + cx[i]));
           }
 #pragma unroll
           for (int i = 0; i < NI; ++i) {
@@ -330,8 +367,8 @@ __global__ void __launch_bounds__(256)
             const float2 t = __ldg(tk + j * nI + i);
             if (t.x == 0.f) continue;
             const int c = cidx[i][lane];
-            sample((float)(p.s0 + i), y, z, t, __ldg(Aj + max(c, 0)), __ldg(Bj + max(c, 0)),
-                   interior || (ry >= 0 && c >= 0));
+            sample((float)(p.s0 + i), y, z, t, both(__ldg(Aj + max(c, 0))),
+                   two_of(__ldg(Bj + max(c, 0))), interior || (ry >= 0 && c >= 0));
           }
         }
         acc = __fadd2_rn(acc, row);
@@ -349,7 +386,7 @@ __global__ void __launch_bounds__(256)
     val.x = power(val.x);
     val.y = power(val.y);
     if (p.iw)
-      val = __fmul2_rn(val, __ldg(I + (size_t)s * plane + (size_t)rM * p.Wm + cM));
+      val = __fmul2_rn(val, two_of(__ldg(vol.I + (size_t)s * plane + (size_t)rM * p.Wm + cM)));
     // voxels that share their samples share their whole history
     size_t o = ((size_t)(s * p.mz + r) * p.Hm + rM) * p.Wm + cM;
     float cur = out[o], mu = p.mode ? mean[o] : 0.f;
@@ -380,7 +417,6 @@ unsigned grid_of(long long n) {
   return (unsigned)std::max<long long>(1, std::min<long long>((n + 255) / 256, 152LL * 32));
 }
 
-size_t rup(size_t b) { return (b + 255) / 256 * 256; }
 
 }  // namespace
 }  // namespace nx
@@ -389,14 +425,25 @@ using namespace nx;
 
 extern "C" {
 
+void nx_esrrf3d_workspace_range(int S, int H, int W, int magnification_xy, int magnification_z,
+                                int mode, size_t* least, size_t* pairs) {
+  size_t rest = 0, one = 256, two = 256;
+  if (S >= 1 && H >= 1 && W >= 1 && magnification_xy >= 1 && magnification_z >= 1) {
+    const size_t volm = (size_t)S * H * magnification_xy * W * magnification_xy;
+    rest = 256 + (mode ? rup(volm * magnification_z * sizeof(float)) : 0) +
+           rup((size_t)kMaxWin * kMaxWin * kMaxWin * sizeof(float2));
+    one = rest + Volumes<false>::bytes(volm);
+    two = rest + Volumes<true>::bytes(volm);
+  }
+  if (least) *least = one;
+  if (pairs) *pairs = two;
+}
+
 size_t nx_esrrf3d_workspace_bytes(int S, int H, int W, int magnification_xy,
                                   int magnification_z, int mode) {
-  if (S < 1 || H < 1 || W < 1 || magnification_xy < 1 || magnification_z < 1) return 256;
-  const size_t volm = (size_t)S * H * magnification_xy * W * magnification_xy;
-  const size_t out = volm * magnification_z;
-  return 256 + rup(volm * sizeof(float4)) + 2 * rup(volm * sizeof(float2)) +
-         (mode ? rup(out * sizeof(float)) : 0) +
-         rup((size_t)kMaxWin * kMaxWin * kMaxWin * sizeof(float2));
+  size_t least, pairs;
+  nx_esrrf3d_workspace_range(S, H, W, magnification_xy, magnification_z, mode, &least, &pairs);
+  return pairs <= kPairBytes ? pairs : least;
 }
 
 int nx_esrrf3d_st(const float* d_in, int T, int S, int H, int W, int magnification_xy,
@@ -410,7 +457,8 @@ int nx_esrrf3d_st(const float* d_in, int T, int S, int H, int W, int magnificati
     return nx::set_error("radius and radius_z must be > 0"), NX_ERR_INVALID_ARG;
   if (mode != 0 && mode != 1) return nx::set_error("mode must be 0 (average) or 1 (std)"), NX_ERR_INVALID_ARG;
   if (!d_in || !d_out) return nx::set_error("NULL input/output"), NX_ERR_INVALID_ARG;
-  const size_t need = nx_esrrf3d_workspace_bytes(S, H, W, magnification_xy, magnification_z, mode);
+  size_t need, pair_need;
+  nx_esrrf3d_workspace_range(S, H, W, magnification_xy, magnification_z, mode, &need, &pair_need);
   if (!d_ws || ws_bytes < need) {
     nx::set_error("workspace too small: need %zu bytes", need);
     return NX_ERR_WORKSPACE;
@@ -478,17 +526,13 @@ int nx_esrrf3d_st(const float* d_in, int T, int S, int H, int W, int magnificati
     --p.z1;
   }
   const bool small = (p.z1 - p.z0 + 1) * nI * nI <= kMaxTab;
-  const auto rgc = small && nI == 4 ? rgc3d_kernel<4> : rgc3d_kernel<0>;
   const size_t vol = (size_t)S * H * W;
   const size_t volm = (size_t)S * p.Hm * p.Wm;
   const long long nout = (long long)p.Sm * p.Hm * p.Wm;
   char* b = (char*)d_ws + 256;
-  float4* A = (float4*)b;  // magnified unit gradients of a frame pair (x, x', y, y')
-  b += rup(volm * sizeof(float4));
-  float2* B = (float2*)b;  // (z, z')
-  b += rup(volm * sizeof(float2));
-  float2* I = (float2*)b;  // magnified frames (v, v')
-  b += rup(volm * sizeof(float2));
+  const bool pair = ws_bytes >= pair_need;
+  char* const volumes = b;
+  b += pair ? Volumes<true>::bytes(volm) : Volumes<false>::bytes(volm);
   float* mean = mode ? (float*)b : nullptr;
   if (mode) b += rup((size_t)nout * sizeof(float));
   float2* dtab = (float2*)b;
@@ -506,20 +550,27 @@ int nx_esrrf3d_st(const float* d_in, int T, int S, int H, int W, int magnificati
       inside ? (unsigned)((ncol + 31) / 32) * (unsigned)((nrow + 7) / 8) : 0;
   const size_t smem =
       (size_t)prep_extent(kPrepRows, mxy) * prep_extent(kPrepCols, mxy) * 2 * sizeof(float4);
-  for (int f = 0; f < T && inside; f += 2) {
-    const float* f0 = d_in + (size_t)f * vol;
-    const int two = f + 1 < T;  // an odd last frame stands in for its partner
-    for (int z = 0; z < S; z += 65535) {  // grid.y limit
-      prep3d_kernel<<<dim3(prep_blocks, (unsigned)std::min(S - z, 65535)), kPrepThreads, smem,
-                      s>>>(f0, two ? f0 + vol : f0, H, W, mxy, z, A, B, I);
-      NX_CUDA_TRY(cudaGetLastError());
+  const auto frames = [&](auto is_pair) {
+    constexpr bool PAIR = decltype(is_pair)::value;
+    const Volumes<PAIR> v(volumes, volm);
+    const auto rgc = small && nI == 4 ? rgc3d_kernel<4, PAIR> : rgc3d_kernel<0, PAIR>;
+    for (int f = 0; f < T && inside; f += PAIR ? 2 : 1) {
+      const float* f0 = d_in + (size_t)f * vol;
+      const int two = PAIR && f + 1 < T;  // an odd last frame stands in for its partner
+      for (int z = 0; z < S; z += 65535) {  // grid.y limit
+        prep3d_kernel<PAIR><<<dim3(prep_blocks, (unsigned)std::min(S - z, 65535)), kPrepThreads,
+                              smem, s>>>(f0, two ? f0 + vol : f0, H, W, mxy, z, v);
+        if (cudaError_t e = cudaGetLastError()) return e;
+      }
+      for (int z = sa; z <= sb; z += 65535) {
+        rgc<<<dim3(rgc_blocks, (unsigned)std::min(sb - z + 1, 65535)), 256, 0, s>>>(
+            p, v, dtab, z, f, two, d_out, mean);
+        if (cudaError_t e = cudaGetLastError()) return e;
+      }
     }
-    for (int z = sa; z <= sb; z += 65535) {
-      rgc<<<dim3(rgc_blocks, (unsigned)std::min(sb - z + 1, 65535)), 256, 0, s>>>(
-          p, A, B, I, dtab, z, f, two, d_out, mean);
-      NX_CUDA_TRY(cudaGetLastError());
-    }
-  }
+    return cudaSuccess;
+  };
+  NX_CUDA_TRY(pair ? frames(std::true_type{}) : frames(std::false_type{}));
   if (mode == 1) {
     std_finish_kernel<<<grid_of(nout), 256, 0, s>>>(d_out, nout, (float)T);
     NX_CUDA_TRY(cudaGetLastError());

@@ -19,6 +19,8 @@ stream).
 """
 from __future__ import annotations
 
+import ctypes as C
+
 import numpy as np
 import torch
 
@@ -413,8 +415,12 @@ class eSRRF3D_ST(LiquidEngine):
         out = torch.empty((S * mz, H * mxy, W * mxy), dtype=torch.float32, device=t.device)
         md = 1 if mode == "std" else 0
         L = N.lib()
-        ws = workspace(L.nx_esrrf3d_workspace_bytes(S, H, W, mxy, mz, md), t.device,
-                       zero_status=False)
+        least, pairs = C.c_size_t(), C.c_size_t()
+        L.nx_esrrf3d_workspace_range(S, H, W, mxy, mz, md, C.byref(least), C.byref(pairs))
+        try:
+            ws = workspace(pairs.value, t.device, zero_status=False)
+        except torch.cuda.OutOfMemoryError:  # one frame at a time, in half the memory
+            ws = workspace(least.value, t.device, zero_status=False)
         N.check(L.nx_esrrf3d_st(_ptr(t), T, S, H, W, mxy, mz, float(radius), float(radius_z),
                                 float(sensitivity), md, 1 if doIntensityWeighting else 0,
                                 _ptr(out), _ptr(ws), ws.numel(), stream_ptr()), "eSRRF3D")
