@@ -330,6 +330,7 @@ def error_maps(ref: torch.Tensor, srs: torch.Tensor, fixed_sigmas=None, ref_int=
         if abs(v - max_sigma_boundary) < 0.0001:
             print("RSF constrained, as no good minimum found")
     fit = fits({i: sig[i] for i in range(B)})
+    step = None  # its buffers go before the final blur's are made
     # the reference keeps these as C floats
     alpha = [float(np.float32(fit[i][0])) for i in range(B)]
     beta = [float(np.float32(fit[i][1])) for i in range(B)]
