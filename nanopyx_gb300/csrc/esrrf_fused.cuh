@@ -320,7 +320,7 @@ __device__ __forceinline__ void apply_sens_all(float2 (&r)[A][B], int mode, int 
 // geometry of one unit (tile, timepoint, frame chunk), shared by both roles
 struct UnitGeo {
   int nx0, ny0, H, W, f0, f1;
-  int kb_y, kb_x, RY0, CX0, y_start, x_start, kmax_y, kmax_x;
+  int RY0, CX0, y_start, x_start, kmax_y, kmax_x;
 };
 
 // ---------------------------------------------------------------------------
@@ -789,8 +789,6 @@ __global__ void __launch_bounds__(32 * TY * (M / PYT) + NP, EsrrfTile<M>::MIN_BL
   u.W = p.W;
   u.f0 = tp_f0 + (int)((long long)chunk * tp_nf / nch);
   u.f1 = tp_f0 + (int)((long long)(chunk + 1) * tp_nf / nch);
-  u.kb_y = 2 * u.ny0 - J;
-  u.kb_x = 2 * u.nx0 - J;
   u.RY0 = u.ny0 - G::RLO;
   u.CX0 = u.nx0 - G::CLO;
   u.y_start = u.ny0 - G::IY;

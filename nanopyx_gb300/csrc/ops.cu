@@ -327,7 +327,7 @@ inline RgcTile rgc_tile(int M, int W2) {
   return t;
 }
 
-// W: the window's side (radii 0.5 to 3 in steps of 0.5, whose rows unroll), or 0
+// W: the window's side where its rows unroll (3 to 13, radii from 0.5 to below 3.5), or 0
 template <int W>
 __global__ void __launch_bounds__(kBlock)
     rgc_table_kernel(const float* __restrict__ gc, const float* __restrict__ gr,
