@@ -341,8 +341,9 @@ __global__ void __launch_bounds__(SrrfTile<M>::NT, 1) srrf_fused_kernel(const Sr
                                          __saturatef(__fmaf_rn(rs.y, kAnySlope, 5.3f)));
           const float2 cr = __ffma2_rn(vgy, make_float2(dx, dx),
                                        __fmul2_rn(vgx, make_float2(-dy, -dy)));
-          float2 dk = __ffma2_rn(__fmul2_rn(make_float2(fabsf(cr.x), fabsf(cr.y)), rs),
-                                 make_float2(-p.inv_rr, -p.inv_rr), make_float2(1.f, 1.f));
+          float2 dk = __ffma2_rn(make_float2(fabsf(cr.x), fabsf(cr.y)),
+                                 __fmul2_rn(rs, make_float2(-p.inv_rr, -p.inv_rr)),
+                                 make_float2(1.f, 1.f));
           dk = __fmul2_rn(dk, dk);
           const float2 in = __ffma2_rn(vgx, make_float2(-p.xr[s], -p.xr[s]),
                                        __ffma2_rn(vgy, make_float2(-p.yr[s], -p.yr[s]),
@@ -441,7 +442,9 @@ cudaError_t launch_srrf_fused(const float* in, const float* img_interp, int T, i
   p.positivity = positivity;
   p.iw = iw;
   p.rr = rc.radius;
-  p.inv_rr = rc.radius != 0.f ? 1.f / rc.radius : 0.f;
+  // a ring below 2^-26 leaves every centre where it is, (xc + xr) - xc = 0, so its term
+  // is 1 for any factor; 0 keeps 2^74.5 / rr finite
+  p.inv_rr = rc.radius >= 1.49e-8f ? 1.f / rc.radius : 0.f;
   for (int k = 0; k < kRing; ++k) {
     p.xr[k] = rc.x[k];
     p.yr[k] = rc.y[k];

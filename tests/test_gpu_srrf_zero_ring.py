@@ -28,3 +28,16 @@ def test_every_term_counts(m, positivity):
             gx, gy = O.gradient_radiality(x[t])
             ref[t, m // 2::m, m // 2::m][(gx == 0) & (gy == 0)] = 0.0
     assert np.array_equal(got, ref)
+
+
+@pytest.mark.parametrize("m", [2, 3, 4, 5, 6, 8])
+def test_rings_below_the_coordinates_resolution(m):
+    """A ring too small to move a centre: every term is 1 with the sign of its outward
+    component, whatever the radius."""
+    x = torch.from_numpy(np.random.default_rng(m).poisson(100, (2, 17, 37)).astype(np.float32))
+    kw = dict(magnification=m, radialityPositivityConstraint=False, doIntensityWeighting=False,
+              macro_pixel_correction=False)
+    ref = nx.SRRF(x.cuda(), ringRadius=1e-12, **kw)
+    assert torch.isfinite(ref).all() and ref.abs().max() <= 1.0
+    for ring in (1e-20, 1e-30):
+        assert torch.equal(nx.SRRF(x.cuda(), ringRadius=ring, **kw), ref)
