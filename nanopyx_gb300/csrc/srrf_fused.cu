@@ -12,12 +12,12 @@
 // point) and (output column, ring point) are tabulated once per tile in shared
 // memory, in the reference's own float32 arithmetic (x0 rounded, x0 / m IEEE).
 //
-// What bounds it: shared-memory wavefronts (column weights and row sums, 64 % of
-// the pipe) and issue (60 %).  100 x 256 x 256, m = 5, ring 0.5 px: one frame a
+// What bounds it: shared-memory wavefronts (column weights and row sums, 67 % of
+// the pipe) and issue (59 %).  100 x 256 x 256, m = 5, ring 0.5 px: one frame a
 // pass, all 12 row passes at once 4.98 ms; frame pairs on packed arithmetic with
 // the row passes in groups 2.94; tile rows per magnification and chunks that fill
 // the last wave 2.86; the next pass's input loaded behind the ring points 2.71;
-// no comparisons in the ring sum 2.65.
+// no comparisons in the ring sum 2.65 (2.68 with weak gradients kept exact).
 #include <algorithm>
 #include <cstring>
 
