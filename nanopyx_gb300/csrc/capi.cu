@@ -711,7 +711,7 @@ int nx_esrrf_accum_push(const nx_esrrf_plan* p, const float* d_block, int T_bloc
   unsigned* status = (unsigned*)d_ws;
   float* rec = (float*)((char*)d_ws + kStatusBytes);
   float* acc = (float*)d_accum;
-  // block records: chunks merged in order into rec chunk 0 ... then into acc
+  // the block's records, one per chunk, then acc followed by them in order
   int chunks = 1;
   if (p->fused) {
     chunks = plan_chunks(p, kModeFull, T_block, T_block, 1);
@@ -727,19 +727,9 @@ int nx_esrrf_accum_push(const nx_esrrf_plan* p, const float* d_block, int T_bloc
       if (e != cudaSuccess) return cuda_status(e, "record push");
     }
   }
-  int n_acc = frames_before;
-  for (int c = 0; c < chunks; ++c) {
-    const int nc = (int)((long long)(c + 1) * T_block / chunks - (long long)c * T_block / chunks);
-    cudaError_t e;
-    if (n_acc == 0) {
-      e = cudaMemcpyAsync(acc, rec + (size_t)c * 5 * planeM, (size_t)5 * planeM * sizeof(float),
-                          cudaMemcpyDeviceToDevice, s);
-    } else {
-      e = launch_record_merge(acc, rec + (size_t)c * 5 * planeM, planeM, n_acc, nc, s);
-    }
-    if (e != cudaSuccess) return cuda_status(e, "accumulator merge");
-    n_acc += nc;
-  }
+  const cudaError_t e =
+      launch_record_merge(acc, rec, planeM, frames_before, T_block, chunks, s);
+  if (e != cudaSuccess) return cuda_status(e, "accumulator merge");
   return NX_OK;
 }
 

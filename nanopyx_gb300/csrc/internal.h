@@ -78,8 +78,9 @@ cudaError_t launch_srrf_fused(const float* in, const float* img_interp, int T, i
 // temporal records: fields mean, M2, C, A, B of Moments (planes of n_pixels)
 cudaError_t launch_record_push_frame(const float* frame, long long n, float* rec, int it,
                                      cudaStream_t s);
-cudaError_t launch_record_merge(float* acc, const float* blk, long long n, int n_acc, int n_blk,
-                                cudaStream_t s);
+// acc (n_acc frames, or none) followed by the n_blk frames of a block in `chunks` records
+cudaError_t launch_record_merge(float* acc, const float* rec, long long n, int n_acc, int n_blk,
+                                int chunks, cudaStream_t s);
 // one temporal finalisation of a batch: the chunk records of one timepoint
 // (rec, F fields, nchunks chunks over nf frames, n pixels) -> the output
 // planes at out (out_stride apart), VAR/TAC2/AVG per corr_mask, or the mean
