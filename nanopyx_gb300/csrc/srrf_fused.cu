@@ -19,6 +19,7 @@
 // the last wave 2.86; the next pass's input loaded behind the ring points 2.71;
 // no comparisons in the ring sum 2.65 (2.68 with weak gradients kept exact).
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 
 #include "common.cuh"
@@ -31,34 +32,82 @@ namespace {
 constexpr int kRing = 12;
 constexpr int kHalo = 5;  // input rows/cols around the tile: ring radius <= 2 px
 
-// Two consecutive frames per pass: the interpolation weights, ring tables and
+// FP = 2: two consecutive frames per pass: the interpolation weights, ring tables and
 // offsets of a pass serve both, and the arithmetic runs on packed f32x2 (the
-// same IEEE operations per frame).
-template <int M>
+// same IEEE operations per frame).  FP = 1: one, for one frame and for launches that leave
+// SMs idle (see launch_srrf_m), where a pair is only a longer pass.
+// V: a value of the pass's frames; Q: two of them (a gradient's x and y) as they lie
+// in shared memory.
+template <int FP>
+struct Frames;
+template <>
+struct Frames<1> {
+  using V = float;
+  using Q = float2;
+  __device__ static V all(float a) { return a; }
+  __device__ static V fma(V a, V b, V c) { return __fmaf_rn(a, b, c); }
+  __device__ static V mul(V a, V b) { return __fmul_rn(a, b); }
+  template <class F>
+  __device__ static V each(F f, V a) { return f(a); }
+  template <class F>
+  __device__ static V each(F f, V a, V b) { return f(a, b); }
+  template <class F>
+  __device__ static V of(F f) { return f(0); }
+  __device__ static V x(const Q& q) { return q.x; }
+  __device__ static V y(const Q& q) { return q.y; }
+  __device__ static Q both(V x, V y) { return make_float2(x, y); }
+  __device__ static float frame(V a, int) { return a; }
+};
+template <>
+struct Frames<2> {
+  using V = float2;
+  using Q = float4;
+  __device__ static V all(float a) { return make_float2(a, a); }
+  __device__ static V fma(V a, V b, V c) { return __ffma2_rn(a, b, c); }
+  __device__ static V mul(V a, V b) { return __fmul2_rn(a, b); }
+  template <class F>
+  __device__ static V each(F f, V a) { return make_float2(f(a.x), f(a.y)); }
+  template <class F>
+  __device__ static V each(F f, V a, V b) { return make_float2(f(a.x, b.x), f(a.y, b.y)); }
+  template <class F>
+  __device__ static V of(F f) { return make_float2(f(0), f(1)); }
+  __device__ static V x(const Q& q) { return make_float2(q.x, q.y); }
+  __device__ static V y(const Q& q) { return make_float2(q.z, q.w); }
+  __device__ static Q both(V x, V y) { return make_float4(x.x, x.y, y.x, y.y); }
+  __device__ static float frame(V a, int k) { return k ? a.y : a.x; }
+};
+
+template <int M, int FP>
 struct SrrfTile {
-  // tile rows, measured (100 x 256 x 256; m = 6, 8: 50 frames): m = 2: 4 / 8 / 12
+  // tile rows, measured.  Pairs (100 x 256 x 256; m = 6, 8: 50 frames): m = 2: 4 / 8 / 12
   // rows 0.68 / 0.83 / 0.77 ms; m = 3: 2 / 4 / 8 rows 1.34 / 1.54 / 1.25; m = 4:
   // 2 / 4 / 6 rows 2.06 / 2.13 / 1.96; m = 5: 3 / 4 / 5 / 6 rows 3.13 / 2.86 /
   // 3.15 / 2.94; m = 6: 1 / 2 / 4 rows 2.48 / 2.55 / 1.97; m = 8: 1 / 2 / 3 rows
-  // 3.68 / 3.49 / 3.69
+  // 3.68 / 3.49 / 3.69.  One frame of 30 x 30 and of 400 x 400, us: m = 3: 4 rows 12.5
+  // and 66, 8 rows 16 and 71; m = 4: 4 / 5 / 6 rows 15 / 16 / 18 and 114 / 100 / 94;
+  // m = 5: 4 / 5 / 6 rows 18 / 21 / 23 and 139 / 133 / 125; m = 6: 2 / 3 / 4 rows 16 /
+  // 19 / 21 and 255 / 201 / 175; m = 8: 1 / 2 rows 19 / 20 and 353 / 324
   static constexpr int TY =
-      M == 2 ? 4 : M == 3 ? 8 : M == 4 ? 6 : M == 5 ? 4 : M == 6 ? 4 : 2;
+      FP == 2 ? (M == 2 ? 4 : M == 3 ? 8 : M == 4 ? 6 : M == 5 ? 4 : M == 6 ? 4 : 2)
+              : (M == 4 || M == 5 ? 5 : M == 8 ? 2 : 4);
   static constexpr int TX = 32;
   static constexpr int NT = 32 * TY * M;
   static constexpr int IH = TY + 2 * kHalo;  // input tile rows
   static constexpr int IW = TX + 2 * kHalo;
   static constexpr int OY = TY * M, OX = TX * M;
   static constexpr int RIW = TX + 4;
-  // ring points whose row pass is formed at a time: the buffer of a warp is 1.3 KB
-  // instead of 8 for all 12 (100 x 256 x 256, m = 5: 2 / 3 / 4 points 2.71 / 2.78 /
-  // 2.89 ms)
-  static constexpr int RG = 2;
+  // ring points whose row pass is formed at a time: for pairs the buffer of a warp is
+  // 1.3 KB instead of 8 for all 12 (100 x 256 x 256, m = 5: 2 / 3 / 4 points 2.71 / 2.78 /
+  // 2.89 ms); a single frame's pass is too short to hide the waits between groups (one
+  // 400 x 400 frame, 2 / 4 / 12 points 145 / 145 / 140 us)
+  static constexpr int RG = FP == 2 ? 2 : 12;
+  static constexpr int UR = FP == 2 ? 1 : 2;  // ring points unrolled
   static constexpr int al(int n) { return (n + 31) / 32 * 32; }
-  static constexpr int O_IN = 0;                        // input tiles (2 frames)
+  static constexpr int O_IN = 0;                        // input tiles (FP frames)
   static constexpr int S_IN = al(IH * IW);
-  static constexpr int O_G = O_IN + 2 * S_IN;           // gradients float4 (gx, gx', gy, gy')
-  static constexpr int O_RI = O_G + al(IH * IW * 4);    // intensity row pass float2 (v, v')
-  static constexpr int O_RW = O_RI + al(OY * RIW * 2);  // intensity row weights [OY][5]
+  static constexpr int O_G = O_IN + FP * S_IN;          // gradients Q (gx, gx', gy, gy')
+  static constexpr int O_RI = O_G + al(IH * IW * 2 * FP);   // intensity row pass V (v, v')
+  static constexpr int O_RW = O_RI + al(OY * RIW * FP);     // intensity row weights [OY][5]
   static constexpr int O_CW = O_RW + al(OY * 5);        // intensity col weights [OX][5]
   static constexpr int O_RT = O_CW + al(OX * 5);        // ring row taps [OY][12][8]
   // ring column taps of output column (lane, px) as 5 weights on the columns
@@ -69,8 +118,8 @@ struct SrrfTile {
   static constexpr int O_CW1 = O_CW4 + al(kRing * M * TX * 4);
   static constexpr int O_CB = O_CW1 + al(kRing * M * TX);  // [ring][lane] int: cb - x_start
   // per-warp row pass of the gradient interpolation: [ring of the group][IW]
-  // float4, plus one zeroed float4 after the last (read with weight 0)
-  static constexpr int RBW = (RG * IW + 1) * 4;
+  // Q, plus one zeroed Q after the last (read with weight 0)
+  static constexpr int RBW = (RG * IW + 1) * 2 * FP;
   static constexpr int O_RB = O_CB + al(kRing * TX);
   static constexpr int FLOATS = O_RB + (NT / 32) * RBW;
   static constexpr size_t SMEM = size_t(FLOATS) * 4;
@@ -113,21 +162,24 @@ __device__ __forceinline__ float with_sign(float v, float s) {
   return __int_as_float(__float_as_int(v) | (__float_as_int(s) & 0x80000000));
 }
 
-template <int M>
-__global__ void __launch_bounds__(SrrfTile<M>::NT, 1) srrf_fused_kernel(const SrrfParams p) {
-  using G = SrrfTile<M>;
+template <int M, int FP>
+__global__ void __launch_bounds__(SrrfTile<M, FP>::NT, 1) srrf_fused_kernel(const SrrfParams p) {
+  using G = SrrfTile<M, FP>;
+  using F = Frames<FP>;
+  using V = typename F::V;
+  using Q = typename F::Q;
   constexpr int TY = G::TY;
   extern __shared__ __align__(128) float sm[];
   float* tin = sm + G::O_IN;
-  float4* grad = reinterpret_cast<float4*>(sm + G::O_G);
-  float2* ri = reinterpret_cast<float2*>(sm + G::O_RI);
+  Q* grad = reinterpret_cast<Q*>(sm + G::O_G);
+  V* ri = reinterpret_cast<V*>(sm + G::O_RI);
   float* rw = sm + G::O_RW;
   float* cw = sm + G::O_CW;
   float* rt = sm + G::O_RT;
   float4* cw4 = reinterpret_cast<float4*>(sm + G::O_CW4);
   float* cw1 = sm + G::O_CW1;
   int* cbt = reinterpret_cast<int*>(sm + G::O_CB);
-  float4* rb = reinterpret_cast<float4*>(sm + G::O_RB + (threadIdx.x >> 5) * G::RBW);
+  Q* rb = reinterpret_cast<Q*>(sm + G::O_RB + (threadIdx.x >> 5) * G::RBW);
 
   const int tid = threadIdx.x;
   const int lane = tid & 31;
@@ -135,10 +187,10 @@ __global__ void __launch_bounds__(SrrfTile<M>::NT, 1) srrf_fused_kernel(const Sr
   const int ty = warp % TY;
   const int py = warp / TY;
   const int tile = blockIdx.x;
-  // chunks of whole frame pairs (the last pair may be one frame)
-  const int pairs = (p.T + 1) / 2;
-  const int f_begin = 2 * (int)((long long)blockIdx.y * pairs / p.chunks);
-  const int f_end = min(p.T, 2 * (int)((long long)(blockIdx.y + 1) * pairs / p.chunks));
+  // chunks of whole passes (the last one may hold one frame of two)
+  const int passes = (p.T + FP - 1) / FP;
+  const int f_begin = FP * (int)((long long)blockIdx.y * passes / p.chunks);
+  const int f_end = min(p.T, FP * (int)((long long)(blockIdx.y + 1) * passes / p.chunks));
   const int nx0 = (tile % p.tiles_x) * G::TX;
   const int ny0 = (tile / p.tiles_x) * TY;
   const int h = p.h, w = p.w;
@@ -202,7 +254,7 @@ __global__ void __launch_bounds__(SrrfTile<M>::NT, 1) srrf_fused_kernel(const Sr
     }
     cbt[s * G::TX + ln] = cb - x_start;
   }
-  if ((tid & 31) == 0) rb[G::RG * G::IW] = make_float4(0.f, 0.f, 0.f, 0.f);
+  if ((tid & 31) == 0) rb[G::RG * G::IW] = F::both(F::all(0.f), F::all(0.f));
 
   const int ny = ny0 + ty, nx = nx0 + lane;
   const int j = ny * M + py;  // output row
@@ -215,46 +267,47 @@ __global__ void __launch_bounds__(SrrfTile<M>::NT, 1) srrf_fused_kernel(const Sr
   const bool own_intensity = p.interp == nullptr;
   // the next pass's input values, loaded while the current pass computes
   constexpr int NPF = (G::IH * G::IW + G::NT - 1) / G::NT;
-  float2 pf[NPF];
+  V pf[NPF];
   auto fetch = [&](int f) {
     const float* src = p.in + (size_t)f * h * w;
-    const float* src1 = f + 1 < f_end ? src + (size_t)h * w : src;
+    const float* src1 = f + 1 < f_end ? src + (size_t)h * w : src;  // FP = 2
 #pragma unroll
     for (int k = 0; k < NPF; ++k) {
       const int i = tid + k * G::NT;
       const int r = y_start + i / G::IW, c = x_start + i % G::IW;
       const bool in = i < G::IH * G::IW && r >= 0 && r < h && c >= 0 && c < w;
       const size_t o = (size_t)r * w + c;
-      pf[k] = in ? make_float2(__ldg(src + o), __ldg(src1 + o)) : make_float2(0.f, 0.f);
+      pf[k] = in ? F::of([&](int fr) { return __ldg((fr ? src1 : src) + o); }) : F::all(0.f);
     }
   };
   if (f_begin < f_end) fetch(f_begin);
-  for (int f = f_begin; f < f_end; f += 2) {
-    const bool two = f + 1 < f_end;  // an odd last frame stands in for its partner
+  for (int f = f_begin; f < f_end; f += FP) {
+    const bool two = FP == 2 && f + 1 < f_end;  // an odd last frame stands in for its partner
     __syncthreads();  // tables ready / previous pass's shared data consumed
 #pragma unroll
     for (int k = 0; k < NPF; ++k) {
       const int i = tid + k * G::NT;
       if (i < G::IH * G::IW) {
-        tin[i] = pf[k].x;
-        tin[G::S_IN + i] = pf[k].y;
+#pragma unroll
+        for (int fr = 0; fr < FP; ++fr) tin[fr * G::S_IN + i] = F::frame(pf[k], fr);
       }
     }
-    if (f + 2 < f_end) fetch(f + 2);
+    if (f + FP < f_end) fetch(f + FP);
     __syncthreads();
     // gradients (zero outside rows/cols 1..n-2) and the intensity row pass
     for (int i = tid; i < G::IH * G::IW; i += G::NT) {
       const int rl = i / G::IW, cl = i % G::IW;
       const int r = y_start + rl, c = x_start + cl;
-      float4 g = make_float4(0.f, 0.f, 0.f, 0.f);
+      Q g = F::both(F::all(0.f), F::all(0.f));
       if (r >= 1 && r < h - 1 && c >= 1 && c < w - 1 && rl >= 1 && rl < G::IH - 1 && cl >= 1 &&
           cl < G::IW - 1) {
-        const float* t0 = tin + i;
-        const float* t1 = t0 + G::S_IN;
-        g.x = __fadd_rn(-t0[-1], t0[1]);
-        g.y = __fadd_rn(-t1[-1], t1[1]);
-        g.z = __fadd_rn(-t0[-G::IW], t0[G::IW]);
-        g.w = __fadd_rn(-t1[-G::IW], t1[G::IW]);
+        const float* t = tin + i;
+        g = F::both(F::of([&](int fr) {
+                      return __fadd_rn(-t[fr * G::S_IN - 1], t[fr * G::S_IN + 1]);
+                    }),
+                    F::of([&](int fr) {
+                      return __fadd_rn(-t[fr * G::S_IN - G::IW], t[fr * G::S_IN + G::IW]);
+                    }));
       }
       grad[i] = g;
     }
@@ -263,17 +316,17 @@ __global__ void __launch_bounds__(SrrfTile<M>::NT, 1) srrf_fused_kernel(const Sr
       const int nyo = ny0 + oy / M;
       const float* w5 = rw + oy * 5;
       const float* col = tin + (nyo - 2 - y_start) * G::IW + (nx0 - 2 + cc - x_start);
-      float2 sum = make_float2(0.f, 0.f);
+      V sum = F::all(0.f);
 #pragma unroll
       for (int k = 0; k < 5; ++k)
-        sum = __ffma2_rn(make_float2(w5[k], w5[k]),
-                         make_float2(col[k * G::IW], col[G::S_IN + k * G::IW]), sum);
+        sum = F::fma(F::all(w5[k]), F::of([&](int fr) { return col[fr * G::S_IN + k * G::IW]; }),
+                     sum);
       ri[i] = sum;
     }
     __syncthreads();
-    float2 div[M];
+    V div[M];
 #pragma unroll
-    for (int px = 0; px < M; ++px) div[px] = make_float2(0.f, 0.f);
+    for (int px = 0; px < M; ++px) div[px] = F::all(0.f);
     const float yc = (float)j + 0.5f;
 #pragma unroll 1
     for (int sg = 0; sg < kRing; sg += G::RG) {
@@ -286,31 +339,31 @@ __global__ void __launch_bounds__(SrrfTile<M>::NT, 1) srrf_fused_kernel(const Sr
         const int s = idx / G::IW, c = idx - s * G::IW;
         const float4 rA = *reinterpret_cast<const float4*>(rrow + (sg + s) * 8);
         const float4 rB = *reinterpret_cast<const float4*>(rrow + (sg + s) * 8 + 4);
-        float2 vx = make_float2(0.f, 0.f), vy = make_float2(0.f, 0.f);
+        V vx = F::all(0.f), vy = vx;
         if (rB.z != 0.f) {
           const int r0 = __float_as_int(rA.x) - y_start;
           const float wr[4] = {rA.y, rA.z, rA.w, rB.x};
-          const float4* gp = grad + r0 * G::IW + c;
+          const Q* gp = grad + r0 * G::IW + c;
 #pragma unroll
           for (int t = 0; t < 4; ++t) {
-            const float4 g = gp[t * G::IW];
-            const float2 wt = make_float2(wr[t], wr[t]);
-            vx = __ffma2_rn(make_float2(g.x, g.y), wt, vx);
-            vy = __ffma2_rn(make_float2(g.z, g.w), wt, vy);
+            const Q g = gp[t * G::IW];
+            const V wt = F::all(wr[t]);
+            vx = F::fma(F::x(g), wt, vx);
+            vy = F::fma(F::y(g), wt, vy);
           }
         }
-        rb[idx] = make_float4(vx.x, vx.y, vy.x, vy.y);
+        rb[idx] = F::both(vx, vy);
       }
       __syncwarp();
       // radiality of this thread's M outputs, ring point by ring point: the M
       // columns share one window of 5 row-pass columns (cb .. cb + 4), each
       // output weights it with its own 5-vector (its 4 taps and a zero), which
       // is the 4-tap fma sequence of the reference with a + 0 at one end
-#pragma unroll 1
+#pragma unroll G::UR
       for (int s = sg; s < sg + G::RG; ++s) {
         const float dy = __fsub_rn(yc, __fadd_rn(yc, p.yr[s]));  // yc - y0
-        const float4* rp = rb + (s - sg) * G::IW + cbt[s * G::TX + lane];
-        float4 col[5];
+        const Q* rp = rb + (s - sg) * G::IW + cbt[s * G::TX + lane];
+        Q col[5];
 #pragma unroll
         for (int k = 0; k < 5; ++k) col[k] = rp[k];
 #pragma unroll
@@ -320,12 +373,12 @@ __global__ void __launch_bounds__(SrrfTile<M>::NT, 1) srrf_fused_kernel(const Sr
           const float wv[5] = {wa.x, wa.y, wa.z, wa.w, we};
           const float xc = (float)(nx * M + px) + 0.5f;
           const float dx = __fsub_rn(xc, __fadd_rn(xc, p.xr[s]));  // xc - x0
-          float2 vgx = make_float2(0.f, 0.f), vgy = make_float2(0.f, 0.f);
+          V vgx = F::all(0.f), vgy = vgx;
 #pragma unroll
           for (int k = 0; k < 5; ++k) {
-            const float2 wk = make_float2(wv[k], wv[k]);
-            vgx = __ffma2_rn(make_float2(col[k].x, col[k].y), wk, vgx);
-            vgy = __ffma2_rn(make_float2(col[k].z, col[k].w), wk, vgy);
+            const V wk = F::all(wv[k]);
+            vgx = F::fma(F::x(col[k]), wk, vgx);
+            vgy = F::fma(F::y(col[k]), wk, vgy);
           }
           // dk = (1 - |vGy (xc - x0) - vGx (yc - y0)| / GMag / ringRadius)^2, 0
           // without a gradient; subtracted where the gradient points outwards.
@@ -334,92 +387,121 @@ __global__ void __launch_bounds__(SrrfTile<M>::NT, 1) srrf_fused_kernel(const Sr
           // of it turns "any gradient" into 0 or 1, and the sign of the
           // inward component (+0, never -0, where there is none: ring radius 0)
           // is moved onto dk by a logic operation.
-          const float2 g2 = __ffma2_rn(vgx, vgx, __ffma2_rn(vgy, vgy, make_float2(kTiny, kTiny)));
-          const float2 rs = make_float2(rsqrtf(g2.x), rsqrtf(g2.y));
+          const V g2 = F::fma(vgx, vgx, F::fma(vgy, vgy, F::all(kTiny)));
+          const V rs = F::each([](float v) { return rsqrtf(v); }, g2);
           constexpr float kAnySlope = -2.11758237e-22f;  // -2^-72: 2^74.5 -> -5.66, 2^74 -> -4
-          const float2 any = make_float2(__saturatef(__fmaf_rn(rs.x, kAnySlope, 5.3f)),
-                                         __saturatef(__fmaf_rn(rs.y, kAnySlope, 5.3f)));
-          const float2 cr = __ffma2_rn(vgy, make_float2(dx, dx),
-                                       __fmul2_rn(vgx, make_float2(-dy, -dy)));
-          float2 dk = __ffma2_rn(make_float2(fabsf(cr.x), fabsf(cr.y)),
-                                 __fmul2_rn(rs, make_float2(-p.inv_rr, -p.inv_rr)),
-                                 make_float2(1.f, 1.f));
-          dk = __fmul2_rn(dk, dk);
-          const float2 in = __ffma2_rn(vgx, make_float2(-p.xr[s], -p.xr[s]),
-                                       __ffma2_rn(vgy, make_float2(-p.yr[s], -p.yr[s]),
-                                                  make_float2(0.f, 0.f)));
-          dk = make_float2(with_sign(dk.x, in.x), with_sign(dk.y, in.y));
-          div[px] = __ffma2_rn(any, dk, div[px]);
+          const V any =
+              F::each([](float v) { return __saturatef(__fmaf_rn(v, kAnySlope, 5.3f)); }, rs);
+          const V cr = F::fma(vgy, F::all(dx), F::mul(vgx, F::all(-dy)));
+          V dk = F::fma(F::each([](float v) { return fabsf(v); }, cr),
+                        F::mul(rs, F::all(-p.inv_rr)), F::all(1.f));
+          dk = F::mul(dk, dk);
+          const V in = F::fma(vgx, F::all(-p.xr[s]),
+                              F::fma(vgy, F::all(-p.yr[s]), F::all(0.f)));
+          dk = F::each(with_sign, dk, in);
+          div[px] = F::fma(any, dk, div[px]);
         }
       }
     }
 #pragma unroll
     for (int px = 0; px < M; ++px) {
       const int i = nx * M + px;  // output column
-      float2 val = make_float2(0.f, 0.f);
+      V val = F::all(0.f);
       const size_t o = (size_t)f * plane + (size_t)j * colsM + i;
       if (row_ok && nx < w && i >= lo_i && i < hi_i) {
-        val = make_float2(div[px].x / 12.f, div[px].y / 12.f);
-        if (p.positivity) val = make_float2(fmaxf(val.x, 0.f), fmaxf(val.y, 0.f));
+        val = F::each([](float v) { return v / 12.f; }, div[px]);
+        if (p.positivity) val = F::each([](float v) { return fmaxf(v, 0.f); }, val);
         if (p.iw) {
           if (own_intensity) {
             // column pass of the intensity magnification (5 taps of the row pass)
             const float* w5 = cw + (lane * M + px) * 5;
-            const float2* rr = ri + (ty * M + py) * G::RIW + lane;
-            float2 sum = make_float2(0.f, 0.f);
+            const V* rr = ri + (ty * M + py) * G::RIW + lane;
+            V sum = F::all(0.f);
 #pragma unroll
-            for (int k = 0; k < 5; ++k) sum = __ffma2_rn(make_float2(w5[k], w5[k]), rr[k], sum);
-            val = __fmul2_rn(val, sum);
+            for (int k = 0; k < 5; ++k) sum = F::fma(F::all(w5[k]), rr[k], sum);
+            val = F::mul(val, sum);
           } else {
-            val.x *= __ldg(p.interp + o);
-            if (two) val.y *= __ldg(p.interp + o + plane);
+            val = F::of([&](int fr) {
+              return fr && !two ? 0.f
+                                : F::frame(val, fr) * __ldg(p.interp + o + (fr ? plane : 0));
+            });
           }
         }
       }
       if (ny < h && nx < w) {
-        p.out[o] = val.x;
-        if (two) p.out[o + plane] = val.y;
+        p.out[o] = F::frame(val, 0);
+        if (two) p.out[o + plane] = F::frame(val, 1);
       }
     }
   }
 }
 
-template <int M>
-cudaError_t launch_srrf_m(const SrrfParams& prm, cudaStream_t s) {
-  using G = SrrfTile<M>;
-  static int attr_done = -1;
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  if (attr_done != dev) {
-    e = cudaFuncSetAttribute(srrf_fused_kernel<M>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)G::SMEM);
-    if (e != cudaSuccess) return e;
-    attr_done = dev;
+// blocks of a kernel resident on an SM, its shared memory allowed; asked once per device
+template <int M, int FP>
+cudaError_t srrf_resident(int dev, int* per_sm) {
+  using G = SrrfTile<M, FP>;
+  static std::atomic<int> known{-1};  // dev << 8 | blocks
+  const int k = known.load(std::memory_order_relaxed);
+  if (k >= 0 && k >> 8 == dev) {
+    *per_sm = k & 255;
+    return cudaSuccess;
   }
+  cudaError_t e = cudaFuncSetAttribute(srrf_fused_kernel<M, FP>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::SMEM);
+  if (e != cudaSuccess) return e;
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, srrf_fused_kernel<M, FP>, G::NT,
+                                                    G::SMEM);
+  if (e != cudaSuccess) return e;
+  *per_sm = std::min(std::max(*per_sm, 1), 255);
+  known.store(dev << 8 | *per_sm, std::memory_order_relaxed);
+  return cudaSuccess;
+}
+
+// frame chunks: the count with the fewest passes on the busiest SM, a block
+// costing its passes plus about one pass for its tables
+int srrf_chunks(long long tiles, long long passes, long long slots) {
+  long long best = -1;
+  int chunks = 1;
+  for (long long c = 1; c <= std::min<long long>(passes, 64); ++c) {
+    const long long cost = (tiles * c + slots - 1) / slots * ((passes + c - 1) / c + 1);
+    if (best < 0 || cost < best) {
+      best = cost;
+      chunks = (int)c;
+    }
+  }
+  return chunks;
+}
+
+template <int M, int FP>
+cudaError_t launch_srrf_f(const SrrfParams& prm, int dev, int sms, cudaStream_t s) {
+  using G = SrrfTile<M, FP>;
   SrrfParams q = prm;
   q.tiles_x = (prm.w + G::TX - 1) / G::TX;
   q.tiles_y = (prm.h + G::TY - 1) / G::TY;
+  int per_sm = 1;
+  cudaError_t e = srrf_resident<M, FP>(dev, &per_sm);
+  if (e != cudaSuccess) return e;
+  const long long tiles = (long long)q.tiles_x * q.tiles_y;
+  q.chunks = srrf_chunks(tiles, ((long long)prm.T + FP - 1) / FP, (long long)sms * per_sm);
+  srrf_fused_kernel<M, FP><<<dim3((unsigned)tiles, (unsigned)q.chunks), G::NT, G::SMEM, s>>>(q);
+  return cudaGetLastError();
+}
+
+template <int M>
+cudaError_t launch_srrf_m(const SrrfParams& prm, cudaStream_t s) {
+  using G = SrrfTile<M, 1>;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const long long tiles = (long long)q.tiles_x * q.tiles_y;
-  int per_sm = 1;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, srrf_fused_kernel<M>, G::NT, G::SMEM);
-  if (e != cudaSuccess) return e;
-  // frame chunks: the count with the fewest passes on the busiest SM, a block
-  // costing its frame pairs plus about one pair for its tables
-  const long long pairs = ((long long)prm.T + 1) / 2, slots = (long long)sms * std::max(1, per_sm);
-  long long best = -1;
-  q.chunks = 1;
-  for (long long c = 1; c <= std::min<long long>(pairs, 64); ++c) {
-    const long long cost = (tiles * c + slots - 1) / slots * ((pairs + c - 1) / c + 1);
-    if (best < 0 || cost < best) {
-      best = cost;
-      q.chunks = (int)c;
-    }
-  }
-  srrf_fused_kernel<M><<<dim3((unsigned)tiles, (unsigned)q.chunks), G::NT, G::SMEM, s>>>(q);
-  return cudaGetLastError();
+  // one frame a pass where there is one only (400 x 400, m = 5: 133 us, 182 as a pair of
+  // its own), or where every frame's tile finds an SM of its own (two frames of 64 x 64:
+  // 21 us, 23 as a pair); beyond that pairs (two frames of 200 x 200: 64 us, two single
+  // ones 80)
+  const long long tiles = (long long)((prm.w + G::TX - 1) / G::TX) * ((prm.h + G::TY - 1) / G::TY);
+  if (prm.T == 1 || tiles * prm.T <= sms) return launch_srrf_f<M, 1>(prm, dev, sms, s);
+  return launch_srrf_f<M, 2>(prm, dev, sms, s);
 }
 
 }  // namespace
