@@ -834,6 +834,32 @@ __global__ void __launch_bounds__(32 * TY * (M / PYT) + NP, EsrrfTile<M>::MIN_BL
     for (int k = 0; k < 5; ++k) cw[i * 5 + k] = w5[k];
   }
 
+  // ---- 1 / sum w of the outputs: several row phases per consumer --------------
+  // by all warps, so that the windows of an edge tile are no longer a chain than with one
+  // phase (a push of one frame of 64 x 64, m = 2: 24.9 us by the consumers alone, 20.3 so);
+  // with one phase the consumers' own loop below is the shorter (256 x 256, m = 5: 130 us
+  // a push, 147 by all warps)
+  if constexpr (PYT > 1) {
+    for (int e = tid; e < G::NO * G::NTC; e += G::NT) {
+      const int o = e / G::NTC, c = e % G::NTC;  // output o of consumer c
+      const int py = (PYT == M ? 0 : (c >> 5) / TY * PYT) + o / M, px = o % M;
+      const int ky_lo = 2 * (u.ny0 + (c >> 5) % TY) + (2 * py + 1) / M - J;
+      const int kx_lo = 2 * (u.nx0 + (c & 31)) + (2 * px + 1) / M - J;
+      float iw = p.inv_wsum[py * M + px];
+      if (ky_lo < 1 || ky_lo + 2 * J > u.kmax_y || kx_lo < 1 || kx_lo + 2 * J > u.kmax_x) {
+        const float* wf = p.wfull + (size_t)(py * M + px) * G::W2 * G::W2;
+        float s = 0.f;
+        for (int jj = 0; jj < G::W2; ++jj) {
+          if (ky_lo + jj < 1 || ky_lo + jj > u.kmax_y) continue;
+          for (int ii = 0; ii < G::W2; ++ii)
+            if (kx_lo + ii >= 1 && kx_lo + ii <= u.kmax_x) s += wf[jj * G::W2 + ii];
+        }
+        iw = s > 0.f ? 1.f / s : 0.f;
+      }
+      tw[e] = iw;
+    }
+  }
+
   // ---- consumer constants --------------------------------------------------
   const int ny = u.ny0 + ty;
   const int nx = u.nx0 + lane;
@@ -850,23 +876,25 @@ __global__ void __launch_bounds__(32 * TY * (M / PYT) + NP, EsrrfTile<M>::MIN_BL
         const int cpx = (2 * px + 1) / M;
         const int xM = nx * M + px;
         const int kx_lo = 2 * nx + cpx - J, kx_hi = 2 * nx + cpx + J;
-        float iw = p.inv_wsum[py * M + px];
-        if (by || kx_lo < 1 || kx_hi > u.kmax_x) {
-          // window reaches invalid half-grid samples: they count in neither sum
-          const float* wf = p.wfull + (size_t)(py * M + px) * G::W2 * G::W2;
-          float s = 0.f;
-          for (int jj = 0; jj < G::W2; ++jj) {
-            const int ky = ky_lo + jj;
-            if (ky < 1 || ky > u.kmax_y) continue;
-            for (int ii = 0; ii < G::W2; ++ii) {
-              const int kx = kx_lo + ii;
-              if (kx < 1 || kx > u.kmax_x) continue;
-              s += wf[jj * G::W2 + ii];
+        if constexpr (PYT == 1) {
+          float iw = p.inv_wsum[py * M + px];
+          if (by || kx_lo < 1 || kx_hi > u.kmax_x) {
+            // window reaches invalid half-grid samples: they count in neither sum
+            const float* wf = p.wfull + (size_t)(py * M + px) * G::W2 * G::W2;
+            float s = 0.f;
+            for (int jj = 0; jj < G::W2; ++jj) {
+              const int ky = ky_lo + jj;
+              if (ky < 1 || ky > u.kmax_y) continue;
+              for (int ii = 0; ii < G::W2; ++ii) {
+                const int kx = kx_lo + ii;
+                if (kx < 1 || kx > u.kmax_x) continue;
+                s += wf[jj * G::W2 + ii];
+              }
             }
+            iw = s > 0.f ? 1.f / s : 0.f;
           }
-          iw = s > 0.f ? 1.f / s : 0.f;
+          tw[(d * M + px) * G::NTC + tid] = iw;
         }
-        tw[(d * M + px) * G::NTC + tid] = iw;
         const bool outside = (ny >= u.H) || (nx >= u.W);
         const bool in_margin = (yM < p.margin) || (yM >= p.rowsM - p.margin) ||
                                (xM < p.margin) || (xM >= p.colsM - p.margin);
