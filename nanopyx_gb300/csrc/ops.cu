@@ -527,23 +527,63 @@ __global__ void record_push_frame_kernel(const float* __restrict__ frame, long l
   }
 }
 
-// acc (its moments over na frames; nothing there if 0) followed by the block's records in
-// frame order: nb frames in `chunks` records, as finalize_pixel takes them.  One launch
-// whatever the chunks: with one each, the 8 chunks of a 16-frame block of 48 x 60, m = 2,
-// took 53 us a push instead of 28.
+// a followed by b, the rounding of a's mean carried along: the mean is a.mean + lo
+__device__ __forceinline__ void moments_merge_lo(Moments& a, float& lo, const Moments& b, int na,
+                                                 int nb, bool full) {
+  const float q = __fdiv_rn((float)nb, (float)na + (float)nb);
+  const float before = a.mean, dl = b.mean - before;
+  moments_merge(a, b, na, nb, full);
+  if (na > 0 && nb > 0) lo = fmaf(lo, 1.f - q, fmaf(dl, q, before - a.mean));
+}
+__device__ __forceinline__ void mean_round(Moments& a, float lo) {
+  const float mean = a.mean + lo;
+  if (mean == mean) a.mean = mean;  // an infinite mean has no rounding to add
+}
+
+// The moments of pixel i over nf frames in `chunks` consecutive records (F fields of n
+// pixels; 5, or the mean only).  A merge rounds like a push, and small images split into
+// more chunks than one chain is short for: up to kMergeGroup records are one chain, more
+// are merged in groups of as many and the groups in order, the rounding of the means
+// carried along (mean of 32 frames of 26 x 64 in 16 chunks: 6.2e-8 in one chain, 3.9e-8 so).
+constexpr int kMergeGroup = 8;
+__device__ __forceinline__ Moments merge_records(const float* __restrict__ rec, int F, int chunks,
+                                                 int nf, long long n, bool full, long long i) {
+  Moments a{0.f, 0.f, 0.f, 0.f, 0.f};
+  int na = 0;
+  float lo = 0.f;
+  for (int g = 0; g < chunks; g += kMergeGroup) {
+    Moments s{0.f, 0.f, 0.f, 0.f, 0.f};
+    int ns = 0;
+    float ls = 0.f;
+    for (int c = g; c < min(g + kMergeGroup, chunks); ++c) {
+      const int nc = (int)((long long)(c + 1) * nf / chunks - (long long)c * nf / chunks);
+      const float* r = rec + (size_t)c * F * n;
+      Moments b{r[i], 0.f, 0.f, 0.f, 0.f};
+      if (full) b = Moments{r[i], r[n + i], r[2 * n + i], r[3 * n + i], r[4 * n + i]};
+      moments_merge_lo(s, ls, b, ns, nc, full);
+      ns += nc;
+    }
+    if (chunks <= kMergeGroup) return s;
+    mean_round(s, ls);
+    moments_merge_lo(a, lo, s, na, ns, full);
+    na += ns;
+  }
+  mean_round(a, lo);
+  return a;
+}
+
+// acc (its moments over na frames; nothing there if 0) followed by a block of nb frames in
+// `chunks` records, merged among themselves first, so that acc's chain is one of pushes
+// (100 frames of 26 x 64 in pushes of 16, m = 2: mean 4.8e-8, 1.1e-7 in one chain of
+// chunks).  One launch whatever the chunks: with one each, the 8 chunks of a 16-frame
+// block of 48 x 60, m = 2, took 53 us a push instead of 28.
 __global__ void record_merge_kernel(float* __restrict__ acc, const float* __restrict__ rec,
                                     long long n, int na, int nb, int chunks) {
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x) {
     Moments a{0.f, 0.f, 0.f, 0.f, 0.f};
     if (na > 0) a = Moments{acc[i], acc[n + i], acc[2 * n + i], acc[3 * n + i], acc[4 * n + i]};
-    int have = na;
-    for (int c = 0; c < chunks; ++c) {
-      const int nc = (int)((long long)(c + 1) * nb / chunks - (long long)c * nb / chunks);
-      const float* r = rec + (size_t)c * 5 * n + i;
-      moments_merge(a, Moments{r[0], r[n], r[2 * n], r[3 * n], r[4 * n]}, have, nc, true);
-      have += nc;
-    }
+    moments_merge(a, merge_records(rec, 5, chunks, nb, n, true, i), na, nb, true);
     acc[i] = a.mean;
     acc[n + i] = a.m2;
     acc[2 * n + i] = a.c;
@@ -560,17 +600,8 @@ __device__ __forceinline__ void finalize_pixel(const float* __restrict__ rec, in
                                                float* __restrict__ out, long long out_stride,
                                                bool full, long long i) {
   {
-    Moments a{0.f, 0.f, 0.f, 0.f, 0.f};
-    int na = 0;
-    for (int c = 0; c < nchunks; ++c) {
-      const int nc = (int)((long long)(c + 1) * nf / nchunks - (long long)c * nf / nchunks);
-      const float* r = rec + (size_t)c * F * n;
-      Moments b{r[i], 0.f, 0.f, 0.f, 0.f};
-      if (full) b = Moments{r[i], r[n + i], r[2 * n + i], r[3 * n + i], r[4 * n + i]};
-      moments_merge(a, b, na, nc, full);
-      na += nc;
-    }
-    const float fn = (float)na;
+    const Moments a = merge_records(rec, F, nchunks, nf, n, full, i);
+    const float fn = (float)nf;
     int ci = 0;
     if (corr_mask & NX_CORR_AVG) out[(ci++) * out_stride + i] = a.mean;
     if (corr_mask & NX_CORR_VAR) {
