@@ -784,6 +784,7 @@ struct nx_esrrf_batch {
     size_t params_off, starts_off;
     size_t jobs_off;      // the class's temporal finalisations (FinalizeJob list)
     int n_jobs, job_blocks;
+    bool job_groups;      // whether any of them merges its records in groups
     int grid;
     nx::TmapPack maps;
   };
@@ -992,6 +993,7 @@ int nx_esrrf_batch_bind(nx_esrrf_batch* b, void* d_ws, size_t ws_bytes, void* st
                                 cl.unit_start.size() * sizeof(int), cudaMemcpyHostToDevice, s));
     std::vector<FinalizeJob> jobs;
     jobs.reserve(cl.n_jobs);
+    cl.job_groups = false;
     int block0 = 0;
     for (int idx : cl.items) {
       const auto& bi = b->items[idx];
@@ -1018,8 +1020,10 @@ int nx_esrrf_batch_bind(nx_esrrf_batch* b, void* d_ws, size_t ws_bytes, void* st
           j.nf = nf;
           j.corr_mask = full ? bi.desc.corr_mask : NX_CORR_AVG;
           j.full = full ? 1 : 0;
+          j.chain = bi.desc.n_sens > 0 && p->M <= 2;  // maps whose scores keep their bits
           j.block0 = block0;
           block0 += nblk;
+          cl.job_groups = cl.job_groups || merges_in_groups(j);
           jobs.push_back(j);
         }
       }
@@ -1062,7 +1066,7 @@ int nx_esrrf_batch_launch(const nx_esrrf_batch* b, void* stream) {
     if (e != cudaSuccess) return cuda_status(e, "batched eSRRF launch");
     // every item's temporal finalisation of this class in one launch
     e = launch_finalize_jobs((const FinalizeJob*)(base + cl.jobs_off), cl.n_jobs, cl.job_blocks,
-                             cs);
+                             cl.job_groups, cs);
     if (e != cudaSuccess) return cuda_status(e, "batched temporal finalize");
     for (int idx : cl.items) {
       const auto& bi = b->items[idx];

@@ -84,16 +84,18 @@ cudaError_t launch_record_merge(float* acc, const float* rec, long long n, int n
 // one temporal finalisation of a batch: the chunk records of one timepoint
 // (rec, F fields, nchunks chunks over nf frames, n pixels) -> the output
 // planes at out (out_stride apart), VAR/TAC2/AVG per corr_mask, or the mean
-// only (!full); block0 = the job's first block in the launch
+// only (!full); chain: its records are merged in one chain however many; block0 = the
+// job's first block in the launch
 struct FinalizeJob {
   const float* rec;
   float* out;
   long long n, out_stride;
-  int F, nchunks, nf, corr_mask, full, block0;
+  int F, nchunks, nf, corr_mask, full, chain, block0;
 };
-// every job of a list in one launch (total_blocks = the last job's block0 +
-// its blocks)
-cudaError_t launch_finalize_jobs(const FinalizeJob* jobs, int njobs, int total_blocks,
+bool merges_in_groups(const FinalizeJob& j);
+// every job of a list in one launch (total_blocks = the last job's block0 + its blocks;
+// groups: whether any of them merges in groups)
+cudaError_t launch_finalize_jobs(const FinalizeJob* jobs, int njobs, int total_blocks, bool groups,
                                  cudaStream_t s);
 // every timepoint (fpt frames, the last one what is left of T) in one launch:
 // `chunks` records of F planes per timepoint -> out[ci*out_stride + tp*n]

@@ -540,30 +540,47 @@ __device__ __forceinline__ void mean_round(Moments& a, float lo) {
   if (mean == mean) a.mean = mean;  // an infinite mean has no rounding to add
 }
 
+__device__ __forceinline__ Moments record(const float* __restrict__ r, long long n, bool full) {
+  if (full) return Moments{r[0], r[n], r[2 * n], r[3 * n], r[4 * n]};
+  return Moments{r[0], 0.f, 0.f, 0.f, 0.f};
+}
+
 // The moments of pixel i over nf frames in `chunks` consecutive records (F fields of n
 // pixels; 5, or the mean only).  A merge rounds like a push, and small images split into
 // more chunks than one chain is short for: up to kMergeGroup records are one chain, more
 // are merged in groups of as many and the groups in order, the rounding of the means
-// carried along (mean of 32 frames of 26 x 64 in 16 chunks: 6.2e-8 in one chain, 3.9e-8 so).
+// carried along (mean of 32 frames of 26 x 64 in 16 chunks: 6.2e-8 in one chain, 3.9e-8).
+// chain: one chain whatever their number.  GROUPS: built for groups at all -- the kernels
+// of the usual few records are built without, whose registers keep them at memory speed
+// (20 x 512 x 512, m = 5, VAR: 44 us, 61 to 65 with the groups' code in).
 constexpr int kMergeGroup = 8;
+template <bool GROUPS>
 __device__ __forceinline__ Moments merge_records(const float* __restrict__ rec, int F, int chunks,
-                                                 int nf, long long n, bool full, long long i) {
+                                                 int nf, long long n, bool full, bool chain,
+                                                 long long i) {
+  auto frames = [&](int c) {
+    return (int)((long long)(c + 1) * nf / chunks - (long long)c * nf / chunks);
+  };
   Moments a{0.f, 0.f, 0.f, 0.f, 0.f};
   int na = 0;
+  if (!GROUPS || chain || chunks <= kMergeGroup) {
+    for (int c = 0; c < chunks; ++c) {
+      const int nc = frames(c);
+      moments_merge(a, record(rec + (size_t)c * F * n + i, n, full), na, nc, full);
+      na += nc;
+    }
+    return a;
+  }
   float lo = 0.f;
   for (int g = 0; g < chunks; g += kMergeGroup) {
     Moments s{0.f, 0.f, 0.f, 0.f, 0.f};
     int ns = 0;
     float ls = 0.f;
     for (int c = g; c < min(g + kMergeGroup, chunks); ++c) {
-      const int nc = (int)((long long)(c + 1) * nf / chunks - (long long)c * nf / chunks);
-      const float* r = rec + (size_t)c * F * n;
-      Moments b{r[i], 0.f, 0.f, 0.f, 0.f};
-      if (full) b = Moments{r[i], r[n + i], r[2 * n + i], r[3 * n + i], r[4 * n + i]};
-      moments_merge_lo(s, ls, b, ns, nc, full);
+      const int nc = frames(c);
+      moments_merge_lo(s, ls, record(rec + (size_t)c * F * n + i, n, full), ns, nc, full);
       ns += nc;
     }
-    if (chunks <= kMergeGroup) return s;
     mean_round(s, ls);
     moments_merge_lo(a, lo, s, na, ns, full);
     na += ns;
@@ -577,13 +594,19 @@ __device__ __forceinline__ Moments merge_records(const float* __restrict__ rec, 
 // (100 frames of 26 x 64 in pushes of 16, m = 2: mean 4.8e-8, 1.1e-7 in one chain of
 // chunks).  One launch whatever the chunks: with one each, the 8 chunks of a 16-frame
 // block of 48 x 60, m = 2, took 53 us a push instead of 28.
+// KIND 0: one record, 1: one chain of them, 2: groups.
+template <int KIND>
 __global__ void record_merge_kernel(float* __restrict__ acc, const float* __restrict__ rec,
                                     long long n, int na, int nb, int chunks) {
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x) {
-    Moments a{0.f, 0.f, 0.f, 0.f, 0.f};
-    if (na > 0) a = Moments{acc[i], acc[n + i], acc[2 * n + i], acc[3 * n + i], acc[4 * n + i]};
-    moments_merge(a, merge_records(rec, 5, chunks, nb, n, true, i), na, nb, true);
+    const Moments b = KIND == 0 ? record(rec + i, n, true)
+                                : merge_records<KIND == 2>(rec, 5, chunks, nb, n, true, false, i);
+    Moments a = b;
+    if (na > 0) {
+      a = record(acc + i, n, true);
+      moments_merge(a, b, na, nb, true);
+    }
     acc[i] = a.mean;
     acc[n + i] = a.m2;
     acc[2 * n + i] = a.c;
@@ -595,12 +618,13 @@ __global__ void record_merge_kernel(float* __restrict__ acc, const float* __rest
 // Merges the `nchunks` consecutive records of one timepoint in frame order and
 // writes the correlations of corr_mask.  full: 5-field records; else one field
 // (the mean) per record.
+template <bool GROUPS>
 __device__ __forceinline__ void finalize_pixel(const float* __restrict__ rec, int F,
                                                int nchunks, int nf, long long n, int corr_mask,
                                                float* __restrict__ out, long long out_stride,
-                                               bool full, long long i) {
+                                               bool full, bool chain, long long i) {
   {
-    const Moments a = merge_records(rec, F, nchunks, nf, n, full, i);
+    const Moments a = merge_records<GROUPS>(rec, F, nchunks, nf, n, full, chain, i);
     const float fn = (float)nf;
     int ci = 0;
     if (corr_mask & NX_CORR_AVG) out[(ci++) * out_stride + i] = a.mean;
@@ -614,6 +638,7 @@ __device__ __forceinline__ void finalize_pixel(const float* __restrict__ rec, in
 
 // every timepoint of one reconstruction in one launch (blockIdx.y): timepoint
 // tp holds nf = min(fpt, T - tp fpt) frames in min(chunks, nf) records
+template <bool GROUPS>
 __global__ void finalize_kernel(const float* __restrict__ rec, int F, int chunks, int T, int fpt,
                                 long long n, int corr_mask, float* __restrict__ out,
                                 long long out_stride, bool full) {
@@ -623,11 +648,13 @@ __global__ void finalize_kernel(const float* __restrict__ rec, int F, int chunks
   float* o = out + (size_t)tp * n;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x)
-    finalize_pixel(r, F, min(chunks, nf), nf, n, corr_mask, o, out_stride, full, i);
+    finalize_pixel<GROUPS>(r, F, min(chunks, nf), nf, n, corr_mask, o, out_stride, full, false,
+                           i);
 }
 
 // a batch's finalisations in one launch: block -> job by binary search on
 // the jobs' first blocks, one pixel per thread
+template <bool GROUPS>
 __global__ void finalize_jobs_kernel(const FinalizeJob* __restrict__ jobs, int njobs) {
   int lo = 0, hi = njobs - 1;
   const int bx = blockIdx.x;
@@ -639,8 +666,8 @@ __global__ void finalize_jobs_kernel(const FinalizeJob* __restrict__ jobs, int n
   const FinalizeJob j = jobs[lo];
   const long long i = (long long)(bx - j.block0) * blockDim.x + threadIdx.x;
   if (i < j.n)
-    finalize_pixel(j.rec, j.F, j.nchunks, j.nf, j.n, j.corr_mask, j.out, j.out_stride,
-                   j.full != 0, i);
+    finalize_pixel<GROUPS>(j.rec, j.F, j.nchunks, j.nf, j.n, j.corr_mask, j.out, j.out_stride,
+                           j.full != 0, j.chain != 0, i);
 }
 
 // sr_temporal_correlations.py:46-75,205-221 on a resident stack, float32 and
@@ -1185,14 +1212,20 @@ cudaError_t launch_record_push_frame(const float* frame, long long n, float* rec
 cudaError_t launch_record_merge(float* acc, const float* rec, long long n, int n_acc, int n_blk,
                                 int chunks, cudaStream_t s) {
   if (n == 0) return cudaSuccess;
-  record_merge_kernel<<<grid_for(n), kBlock, 0, s>>>(acc, rec, n, n_acc, n_blk, chunks);
+  const auto kernel = chunks == 1             ? record_merge_kernel<0>
+                      : chunks <= kMergeGroup ? record_merge_kernel<1>
+                                              : record_merge_kernel<2>;
+  kernel<<<grid_for(n), kBlock, 0, s>>>(acc, rec, n, n_acc, n_blk, chunks);
   return cudaGetLastError();
 }
 
-cudaError_t launch_finalize_jobs(const FinalizeJob* jobs, int njobs, int total_blocks,
+bool merges_in_groups(const FinalizeJob& j) { return !j.chain && j.nchunks > kMergeGroup; }
+
+cudaError_t launch_finalize_jobs(const FinalizeJob* jobs, int njobs, int total_blocks, bool groups,
                                  cudaStream_t s) {
   if (njobs == 0 || total_blocks == 0) return cudaSuccess;
-  finalize_jobs_kernel<<<total_blocks, kBlock, 0, s>>>(jobs, njobs);
+  const auto kernel = groups ? finalize_jobs_kernel<true> : finalize_jobs_kernel<false>;
+  kernel<<<total_blocks, kBlock, 0, s>>>(jobs, njobs);
   return cudaGetLastError();
 }
 
@@ -1200,9 +1233,10 @@ cudaError_t launch_finalize(const float* rec, int F, int chunks, int T, int fpt,
                             long long n, int corr_mask, float* out, long long out_stride,
                             bool full, cudaStream_t s) {
   if (n == 0) return cudaSuccess;
+  const auto kernel = chunks > kMergeGroup ? finalize_kernel<true> : finalize_kernel<false>;
   for (int tp = 0; tp < n_tp; tp += 65535) {  // grid.y limit
     const int cnt = std::min(n_tp - tp, 65535);
-    finalize_kernel<<<dim3(grid_for(n), (unsigned)cnt), kBlock, 0, s>>>(
+    kernel<<<dim3(grid_for(n), (unsigned)cnt), kBlock, 0, s>>>(
         rec + (size_t)tp * chunks * F * n, F, chunks, T - tp * fpt, fpt, n, corr_mask,
         out + (size_t)tp * n, out_stride, full);
     const cudaError_t e = cudaGetLastError();

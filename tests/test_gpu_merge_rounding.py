@@ -40,3 +40,34 @@ def test_chunks_of_pushes(m):
     for a in range(0, 100, 16):
         acc.push(x[a:a + 16])
     assert _error(acc.finalize_device(("AVG",), False)[0], ref) <= 5.5e-8
+
+
+@pytest.mark.parametrize("m", [1, 2])
+def test_sweep_maps_are_one_chain(m):
+    """The maps that sweeps score at m <= 2 are one chain of chunk means whatever the
+    chunks: 174 frames of 103 x 78 in more than 8, against the same chain in float32."""
+    x = torch.from_numpy(np.random.default_rng(3).poisson(100, (174, 103, 78)).astype(np.float32))
+    x = x.cuda()
+    got = nx.esrrf_parameter_sweep(x, magnification=m, sensitivities=[1], radii=[1.0])[0, 0]
+    maps = nx.eSRRF_ST(verbose=False).run(x, magnification=m, radius=1.0, sensitivity=1)
+
+    def chain(chunks):
+        mean, have = None, 0
+        for c in range(chunks):
+            a, b = c * 174 // chunks, (c + 1) * 174 // chunks
+            part = maps[a]
+            for k in range(1, b - a):  # one rounding per frame, as a fused multiply-add
+                inv = np.float32(1) / np.float32(k + 1)
+                part = ((maps[a + k] - part).double() * float(inv) + part.double()).float()
+            if mean is None:
+                mean = part
+            else:
+                q = np.float32(b - a) / (np.float32(have) + np.float32(b - a))
+                mean = ((part - mean).double() * float(q) + mean.double()).float()
+            have = b
+        return mean
+
+    # the kernel's reciprocal is good to an ulp, so a frame's step may round the other way:
+    # most pixels agree with the chain of the right number of chunks and no other way
+    same = max(float((chain(c) == got).float().mean()) for c in range(2, 44))
+    assert same >= 0.9
