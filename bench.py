@@ -40,7 +40,7 @@ CFG = dict(T=500, H=512, W=512, emitters=400, m=5, radius=1.5, sensitivity=2.0,
 SMALL = dict(T=160, fpt=80)
 # DRAM bytes of one fused launch, dram__bytes_read.sum + dram__bytes_write.sum from a
 # 1-pass ncu capture of that launch (large: the full 500-frame launch; small: 160 frames)
-TRAFFIC_BYTES = {"large": 529973248 + 612297216, "small": 171895808 + 217139456}
+TRAFFIC_BYTES = {"large": 530092032 + 607835648, "small": 171895808 + 217139456}
 METRIC = "eSRRF input Mpx*frames/s"
 # frames per reference step: eSRRF_ST and the temporal step scale with the frame
 # count; the per-timepoint macro-pixel correction (2 x ~30 ms on 2560^2) is <1 %
